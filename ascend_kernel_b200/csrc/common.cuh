@@ -164,35 +164,73 @@ __device__ __forceinline__ void s8x4_to_bf16_even_odd(uint32_t w, uint32_t& o02,
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(o13) : "r"(lo), "r"(sg));
 }
 
+// Sum over the lanes below this one and, in `total`, over the whole warp.
+__device__ __forceinline__ int warp_exclusive_sum(int v, int& total) {
+    const int lane = threadIdx.x & 31;
+    int s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += n;
+    }
+    total = __shfl_sync(0xffffffffu, s, 31);
+    return s - v;
+}
+
+// The consecutive experts a lane of the scheduling warp owns: [lo, hi) of G.
+__device__ __forceinline__ void lane_experts(int G, int& lo, int& hi) {
+    const int per = (G + 31) >> 5;
+    lo = min((int)(threadIdx.x & 31) * per, G);
+    hi = min(lo + per, G);
+}
+
 // Row boundaries of every expert from the device-side group_list, clamped into [0, M] and made
 // monotone so no later index can leave the tensors; a violation is reported in the status words.
 // Executed by a whole CTA; row_start has G+1 entries in shared memory.  G <= kMaxExperts.
+// Every thread fetches entries, then the first warp scans them, each lane a stretch of consecutive
+// experts: with one thread walking the 256 entries, the GEMV of one token (8 rows, 7168 x 4096, fp8) took
+// 152 us instead of 110 and that of 37 tokens (2048 x 7168, fp4) 475 instead of 429.
 __device__ __forceinline__ void load_row_starts(const int64_t* __restrict__ gl, int G, int M, int gl_type,
                                                 int* row_start, int* status) {
-    // every thread fetches one entry (clamped into int range), then one thread makes the list
-    // monotone: G is a few hundred and this runs once per CTA
     for (int g = threadIdx.x; g < G; g += blockDim.x) {
-        long long v = gl[g];
+        const long long v = gl[g];
         row_start[g + 1] = (int)(v < -1 ? -1 : (v > (long long)M + 1 ? (long long)M + 1 : v));
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int prev = 0;
-        row_start[0] = 0;
-        bool bad = false;
-        int bad_at = 0;
-        for (int g = 0; g < G; ++g) {
-            const int v = row_start[g + 1];
-            int end = (gl_type == B200MOE_GROUP_LIST_COUNTS) ? prev + v : v;
-            if (v < 0 || end < prev || end > M) {
-                if (!bad) bad_at = g;
-                bad = true;
-                end = (v < 0 || end < prev) ? prev : M;
-            }
-            row_start[g + 1] = end;
-            prev = end;
+    if (threadIdx.x < 32) {
+        const bool counts = gl_type == B200MOE_GROUP_LIST_COUNTS;
+        const int lane = threadIdx.x;
+        int lo, hi;
+        lane_experts(G, lo, hi);
+        // what the lane's stretch adds up to: a sum of counts, or the largest boundary (both without the
+        // invalid negative entries), saturated at M + 1: beyond M nothing changes any more (M < 2^31, so
+        // the sum of two saturated values fits 32 unsigned bits)
+        const uint32_t m = (uint32_t)M, cap = m + 1u;
+        uint32_t mine = 0;
+        for (int g = lo; g < hi; ++g) {
+            const uint32_t v = (uint32_t)max(row_start[g + 1], 0);
+            mine = counts ? min(mine + v, cap) : max(mine, v);
         }
-        if (bad) report_status(status, kDevBadGroupList, bad_at);
+        uint32_t pre = mine;  // inclusive scan, then shifted by one lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre = counts ? min(pre + n, cap) : max(pre, n);
+        }
+        pre = __shfl_up_sync(0xffffffffu, pre, 1);
+        if (lane == 0) pre = 0;
+        int bad_at = G;
+        for (int g = lo; g < hi; ++g) {
+            const int v = row_start[g + 1];
+            const uint32_t end = counts ? pre + (uint32_t)max(v, 0) : (uint32_t)max(v, 0);
+            // (after an end beyond M the list stays at M, so a later boundary below M is a step back)
+            if (v < 0 || end < min(pre, m) || end > m) bad_at = min(bad_at, g);
+            pre = counts ? min(end, cap) : max(pre, end);
+            row_start[g + 1] = (int)min(pre, m);
+        }
+        if (lane == 0) row_start[0] = 0;
+        bad_at = __reduce_min_sync(0xffffffffu, bad_at);
+        if (lane == 0 && bad_at < G) report_status(status, kDevBadGroupList, bad_at);
     }
     __syncthreads();
 }

@@ -494,20 +494,31 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     const int n_kt = a.K / kBK;  // stages per tile
 
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
-    if (threadIdx.x == 0) {
-        int acc = 0, acc1 = 0;
+    if (warp == 0) {
+        // tile-count prefixes, each lane over a stretch of consecutive experts
         int* pref1 = tile_prefix + (a.G + 1);
-        tile_prefix[0] = 0;
-        pref1[0] = 0;
-        for (int g = 0; g < a.G; ++g) {
+        int lo, hi, c2 = 0, c1 = 0, t2, t1;
+        lane_experts(a.G, lo, hi);
+        for (int g = lo; g < hi; ++g) {
             const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
-            acc += (rows / kTileM + (tail > kBM ? 1 : 0)) * n_nt;    // tiles with two row halves
-            acc1 += ((tail >= 1 && tail <= kBM) ? 1 : 0) * n_nt;      // the short last m-tile, if any
-            tile_prefix[g + 1] = acc;
-            pref1[g + 1] = acc1;
+            c2 += rows / kTileM + (tail > kBM ? 1 : 0);   // m-tiles with two row halves
+            c1 += (tail >= 1 && tail <= kBM) ? 1 : 0;      // the short last m-tile, if any
         }
-        acc += acc1;
-        sb->n_tiles = acc;
+        int p2 = warp_exclusive_sum(c2, t2), p1 = warp_exclusive_sum(c1, t1);
+        for (int g = lo; g < hi; ++g) {
+            const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
+            tile_prefix[g] = p2 * n_nt;
+            pref1[g] = p1 * n_nt;
+            p2 += rows / kTileM + (tail > kBM ? 1 : 0);
+            p1 += (tail >= 1 && tail <= kBM) ? 1 : 0;
+        }
+        if (lane == 0) {
+            tile_prefix[a.G] = t2 * n_nt;
+            pref1[a.G] = t1 * n_nt;
+            sb->n_tiles = (t2 + t1) * n_nt;
+        }
+    }
+    if (threadIdx.x == 32) {
         sb->abort = 0;
         for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = 0ull;
         for (int i = 0; i < NS; ++i) {

@@ -243,15 +243,22 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     const int n_kt = a.K / kBK;
 
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        tile_prefix[0] = 0;
-        for (int g = 0; g < a.G; ++g) {
-            const int rows = row_start[g + 1] - row_start[g];
-            acc += ((rows + kMaxR - 1) / kMaxR) * n_nt;
-            tile_prefix[g + 1] = acc;
+    if (warp == 0) {
+        // tile-count prefix, each lane over a stretch of consecutive experts
+        int lo, hi, mine = 0, total;
+        lane_experts(a.G, lo, hi);
+        for (int g = lo; g < hi; ++g) mine += (row_start[g + 1] - row_start[g] + kMaxR - 1) / kMaxR;
+        int at = warp_exclusive_sum(mine, total);
+        for (int g = lo; g < hi; ++g) {
+            tile_prefix[g] = at * n_nt;
+            at += (row_start[g + 1] - row_start[g] + kMaxR - 1) / kMaxR;
         }
-        sb->n_tiles = acc;
+        if (lane == 0) {
+            tile_prefix[a.G] = total * n_nt;
+            sb->n_tiles = total * n_nt;
+        }
+    }
+    if (threadIdx.x == 32) {
         sb->abort = 0;
         for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = make_uint4(0u, 0u, 0u, 0u);
         for (int i = 0; i < kXStages; ++i) {

@@ -828,16 +828,21 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(red + kGvWarps * kGvRows * kGvSlabN);  // [4][K]
 
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         // non-empty experts, those with the most rows first (counting sort on min(rows, 5)): with
         // the ticket counter below the long items start early and the short ones fill the tail
-        int n = 0;
-        for (int b = 5; b >= 1; --b)
-            for (int g = 0; g < a.G; ++g) {
-                const int rows = row_start[g + 1] - row_start[g];
-                if ((rows >= 5 ? 5 : rows) == b) active[n++] = g;
-            }
-        *n_active_p = n;
+        int lo, hi, n = 0;
+        lane_experts(a.G, lo, hi);
+        for (int b = 5; b >= 1; --b) {
+            int mine = 0, total;
+            for (int g = lo; g < hi; ++g) mine += min(row_start[g + 1] - row_start[g], 5) == b;
+            int at = n + warp_exclusive_sum(mine, total);
+            if (total > 0)
+                for (int g = lo; g < hi; ++g)
+                    if (min(row_start[g + 1] - row_start[g], 5) == b) active[at++] = g;
+            n += total;
+        }
+        if (threadIdx.x == 0) *n_active_p = n;
     }
     __syncthreads();
 

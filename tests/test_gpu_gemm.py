@@ -165,3 +165,31 @@ def test_int4_per_group_scales_match_oracle(counts, K, N, with_offset):
     out, st = run_gemm(x, w, scale, offset, cnt, "int4", gl_type=1)
     assert st == (0, 0)
     assert_close_to_golden(out, gold)
+
+
+@pytest.mark.parametrize("gl_type,gl,M,first_bad", [
+    (1, [3] * 33, 99, None),                           # one expert more than the scanning lanes
+    (1, [0] * 31 + [5, 0, 7] + [0] * 30, 12, None),
+    (1, [2] * 40 + [-4] + [1] * 24, 100, 40),          # a negative count counts as none
+    (1, [5] * 70, 123, 24),                            # the 25th expert is cut at the end of x, the rest are empty
+    (1, [1 << 40] + [1] * 64, 10, 0),
+    (0, list(range(2, 202, 2)), 200, None),
+    (0, [4, 9, 7, 20, 500, 30] + [600] * 40, 40, 2),   # a step back is an empty expert, past the end is cut
+])
+def test_group_list_scan(gl_type, gl, M, first_bad):
+    # what one expert after the other would give: rows of expert g are [prev, end)
+    prev, bounds = 0, []
+    for v in gl:
+        end = prev + max(v, 0) if gl_type == 1 else max(v, 0)
+        prev = min(max(end, prev), M)
+        bounds.append(prev)
+    G, K, N = len(gl), 64, 256
+    gen = torch.Generator().manual_seed(G)
+    x = torch.randn(M, K, generator=gen).to(torch.bfloat16)
+    w = torch.randint(-128, 128, (G, K, N), generator=gen, dtype=torch.int8)
+    scale = torch.full((G, N), 0.01, dtype=torch.bfloat16)
+    want = O.golden_f32(x, w, scale, None, torch.tensor(bounds), "int8", O.GROUP_LIST_CUMSUM)
+    out, st = run_gemm(x, w, scale, None, torch.tensor(gl), "int8", gl_type=gl_type)
+    assert st == ((0, 0) if first_bad is None else (1, first_bad))
+    assert_close_to_golden(out, want)
+    assert (out[bounds[-1]:].float() == SENTINEL).all()
