@@ -26,7 +26,7 @@ EXPORTS = [
     "b200moe_moe_route", "b200moe_moe_regroup_index", "b200moe_grouped_gemm_int8_noalloc", "b200moe_grouped_gemm_int8_noalloc_max_rows", "b200moe_noalloc_read_status",
     "b200moe_ep_post_counts", "b200moe_ep_dispatch", "b200moe_ep_wait", "b200moe_ep_post", "b200moe_ep_combine",
     "b200moe_fp4_dequant_bf16_scale", "b200moe_fp8_dequant", "b200moe_fp4_scale_fold",
-    "b200moe_silu_mul_dyn", "b200moe_grouped_gemm_int8_silu", "b200moe_pack_weight_int8", "b200moe_grouped_gemm_int8_packed", "b200moe_grouped_gemm_int8_packed_scatter",
+    "b200moe_silu_mul_dyn", "b200moe_grouped_gemm_int8_silu", "b200moe_grouped_gemm_fp4_e8m0", "b200moe_pack_weight_int8", "b200moe_grouped_gemm_int8_packed", "b200moe_grouped_gemm_int8_packed_scatter",
     "b200moe_set_gemm_reserved_sms", "b200moe_ipc_alloc", "b200moe_ipc_open", "b200moe_ipc_close", "b200moe_ipc_free",
 ]
 
@@ -69,6 +69,8 @@ def _load() -> ctypes.CDLL:
         f.restype = sz
     lib.b200moe_grouped_gemm_int8_silu.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, vp, sz, vp]
     lib.b200moe_grouped_gemm_int8_silu.restype = i32
+    lib.b200moe_grouped_gemm_fp4_e8m0.argtypes = [vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, i32, vp, sz, vp]
+    lib.b200moe_grouped_gemm_fp4_e8m0.restype = i32
     lib.b200moe_pack_weight_int8.argtypes = [vp, vp, i64, i64, i64, i32, vp]
     lib.b200moe_pack_weight_int8.restype = i32
     lib.b200moe_grouped_gemm_int8_packed.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, i32, vp, sz, vp]

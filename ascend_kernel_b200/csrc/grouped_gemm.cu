@@ -70,10 +70,17 @@ constexpr uint32_t kTmemCols = 512;
 // and only the thread -> data assignment of the dequant warps changes: a thread takes 8 rows x 8
 // columns (two 16-byte loads) instead of 4 rows x 16 columns.
 constexpr int kCtFp4Ascend = 16;
+// Internal kernel mode: canonical fp4 codes with one e8m0 scale byte per 32 columns of a k row (the format of
+// b200moe_fp4_dequant), dequantised by the dequant warps to the bits that operator would write.  With SILU the
+// gate columns come first in the matrix and the kernel pairs them with the up columns itself.  Against writing the
+// bf16 weights to memory and reading them back (4 of 4.5 bytes per weight of such a pass, and the bound of it), a
+// layer of 256 experts, 4096 tokens x 8, 7168 x 2048 takes 5.08 instead of 8.80 ms, and one of few tokens an eighth.
+constexpr int kCtFp4E8m0 = 17;
 
 template <int MODE>
 struct GmTraits {
-    static constexpr bool kNibbles = (MODE == B200MOE_CT_FP4 || MODE == B200MOE_CT_INT4 || MODE == kCtFp4Ascend);
+    static constexpr bool kNibbles = (MODE == B200MOE_CT_FP4 || MODE == B200MOE_CT_INT4 || MODE == kCtFp4Ascend ||
+                                      MODE == kCtFp4E8m0);
     // int4 with per-128-k scale/offset: (w + o) * s does not fit bf16, so every k block is fed to
     // the tensor core twice -- a stage carries two weight tiles, hi = bf16(v) and lo = bf16(v - hi),
     // multiplied with the same x block; the fp32 accumulator then holds x @ v to about 2^-16 relative.
@@ -248,6 +255,7 @@ template <int MODE>
 struct PackedRegs {
     uint4 q[kDqRows];  // fp4 / int4 use only .x/.y of each
     uint4 s[2];        // fp4 only: the bf16 scales of the thread's 16 columns (one 16-row group)
+    uint32_t e[kDqRows];  // fp4 with e8m0 scales only: the scale byte of each of the thread's rows
     float sf;          // fp8 only: the fp32 scale of the thread's 128 x 128 block
 };
 
@@ -259,7 +267,13 @@ struct DqIter {
     bool valid;
     const uint8_t* wp;
 };
-template <int MODE>
+// First weight column of 16-column chunk c16 of the tile at n0.  SPLIT: the tile's lower half is the gate
+// columns n0 / 2 .. + 127 and its upper half the up columns N / 2 + the same indices.
+template <bool SPLIT>
+__device__ __forceinline__ int chunk_col(int n0, int c16, int N) {
+    return SPLIT ? (n0 >> 1) + (c16 & 7) * 16 + (c16 >> 3) * (N >> 1) : n0 + c16 * 16;
+}
+template <int MODE, bool SPLIT>
 __device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict__ w, const GemmArgs& a, const DqLane& d,
                                           int n_tiles, const int* tile_prefix, const int* row_start, int n_nt) {
     using T = GmTraits<MODE>;
@@ -271,10 +285,10 @@ __device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict_
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
     it.wp = w + ((size_t)ti.g * a.K + (size_t)it.kt * kBK + d.row) * row_bytes +
             (MODE == kCtFp4Ascend ? (ti.n0 >> 1) + d.src_byte
-             : T::kNibbles        ? (ti.n0 >> 1) + d.c16 * 8
+             : T::kNibbles        ? chunk_col<SPLIT>(ti.n0, d.c16, a.N) >> 1
                                   : ti.n0 + d.c16 * 16);
 }
-template <int MODE>
+template <int MODE, bool SPLIT>
 __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* __restrict__ w, const GemmArgs& a,
                                            const DqLane& d, int n_kt, int n_tiles, const int* tile_prefix,
                                            const int* row_start, int n_nt, GmBarriers* sb) {
@@ -288,10 +302,12 @@ __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* 
         it.kt -= n_kt;
         it.t = next_tile(sb, it.seq, n_tiles, a.status);
     } while (it.kt >= n_kt && it.t < n_tiles);
-    dq_locate<MODE>(it, w, a, d, n_tiles, tile_prefix, row_start, n_nt);
+    dq_locate<MODE, SPLIT>(it, w, a, d, n_tiles, tile_prefix, row_start, n_nt);
 }
 
-template <int MODE>
+constexpr int kScaleAhead = 6;  // stages by which the e8m0 scale lines are requested into L2
+
+template <int MODE, bool SPLIT>
 __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& it, const GemmArgs& a, const DqLane& d) {
     using T = GmTraits<MODE>;
     if constexpr (MODE == kCtFp4Ascend) {
@@ -322,6 +338,19 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
                    ? __ldg(static_cast<const float*>(a.scale) + ((size_t)it.g * (a.K >> 7) + ((it.kt * kBK) >> 7)) * (a.N >> 7) +
                            ((it.n0 + d.c16 * 16) >> 7))
                    : 0.f;
+    }
+    if constexpr (MODE == kCtFp4E8m0) {
+        const uint8_t* sc = static_cast<const uint8_t*>(a.scale);
+        const size_t ld = (size_t)a.N >> 5, row0 = (size_t)it.g * a.K + (size_t)it.kt * kBK;
+        const uint8_t* sp = sc + (row0 + d.row) * ld + (chunk_col<SPLIT>(it.n0, d.c16, a.N) >> 5);
+#pragma unroll
+        for (int j = 0; j < kDqRows; ++j) r.e[j] = __ldg(sp + (size_t)(kDqRowStep * j) * ld);
+        // a tile's scales are 8 bytes of a k row's line: the lines of the warp's eight rows of a later stage are
+        // requested into L2 here (SPLIT: lanes 8 .. 15 those of the up columns)
+        const int l = threadIdx.x & 31, w0 = d.row & ~(kDqWarpRows - 1);
+        if (l < (SPLIT ? 16 : 8) && (it.kt + kScaleAhead + 1) * kBK <= a.K)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(sc + (row0 + (size_t)kScaleAhead * kBK + w0 + (l & 7)) * ld +
+                                                          (chunk_col<SPLIT>(it.n0, l & 8, a.N) >> 5)));
     }
     if constexpr (MODE == B200MOE_CT_FP4) {
         const uint4* sp = reinterpret_cast<const uint4*>(
@@ -386,6 +415,17 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
                     o[2 * i + hp] = pack_bf16x2(f32x2_lo(f), f32x2_hi(f));
                 }
             }
+        } else if constexpr (MODE == kCtFp4E8m0) {
+            // 2^(s-127) as bf16: exponent field s; s = 0 is the subnormal 2^-127, 255 is NaN
+            const uint32_t e = r.e[j];
+            const uint32_t sb = (e == 0 ? 0x0040u : (e == 255 ? 0x7FC0u : (e << 7))) * 0x10001u;
+            uint32_t v[4];
+            e2m1x8_to_bf16(q.x, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = mul_bf16x2(v[i], sb);
+            e2m1x8_to_bf16(q.y, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[4 + i] = mul_bf16x2(v[i], sb);
         } else {  // FP4: 8 bytes = 16 codes; the thread's rows share one 16-row scale group
             const uint4 s0 = r.s[0], s1 = r.s[1];
             uint32_t v[4];
@@ -470,8 +510,8 @@ struct StageIter {
     bool valid;
 };
 
-// SILU (int8 only): the weight columns come as blocks of 128 gate columns followed by the 128 up
-// columns of the same indices, and the epilogue writes bf16(silu(gate) * up), [M, N/2], instead of
+// SILU (int8, fp4 with e8m0 scales): int8 weight columns come as blocks of 128 gate columns followed by the 128
+// up columns of the same indices (fp4: gate columns first, paired here), and the epilogue writes bf16(silu(gate) * up), [M, N/2], instead of
 // the [M, N] product (gate and up are rounded to bf16 first, as the unfused operators would).
 template <int MODE, bool SILU>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -482,6 +522,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* a_ring = base;
     constexpr int NS = T::kStages, P = T::kParts;
+    constexpr bool SPLIT = SILU && MODE == kCtFp4E8m0;
     uint8_t* b_ring = a_ring + NS * kATileBytes;
     GmBarriers* sb = reinterpret_cast<GmBarriers*>(b_ring + NS * P * kBTileBytes);
     static_assert(sizeof(GmBarriers) <= kBarrierBytes, "barrier block");
@@ -572,7 +613,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             far.valid = far.t < n_tiles;
             if (far.valid) far.ti = locate_tile(far.t, tile_prefix, row_start, a.G, n_nt);
             auto far_step = [&]() {
-                if constexpr (!T::kDirect)
+                if constexpr (SPLIT) {
+                    ptx::tma_prefetch_l2_2d(&tmap_w, far.ti.n0 / 4, far.ti.g * a.K + far.kt * kBK);
+                    ptx::tma_prefetch_l2_2d(&tmap_w, (a.N + far.ti.n0) / 4, far.ti.g * a.K + far.kt * kBK);
+                } else if constexpr (!T::kDirect)
                     ptx::tma_prefetch_l2_2d(&tmap_w, T::kNibbles ? far.ti.n0 / 2 : far.ti.n0, far.ti.g * a.K + far.kt * kBK);
                 if (++far.kt < n_kt) return;
                 far.kt = 0;
@@ -686,7 +730,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         // ------------------------------ epilogue ------------------------------
         const int quarter = warp & 3;                 // TMEM lanes 32*quarter .. +31 are the ones this warp may read
         const int grp = (warp - kWarpEpi0) >> 2;      // which accumulator this warp drains
-        const bool per_channel = (MODE == B200MOE_CT_INT8);
+        constexpr bool per_channel = (MODE == B200MOE_CT_INT8);
         const bool has_offset = per_channel && a.offset != nullptr;
         uint32_t use = 0, next1 = 0, seq = 0;
         for (;;) {
@@ -735,19 +779,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                         uint32_t o[8];
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            const float4 sg = *reinterpret_cast<const float4*>(es + c * 16 + 4 * q);
-                            const float4 og = *reinterpret_cast<const float4*>(es + kBN + c * 16 + 4 * q);
-                            const float4 su = *reinterpret_cast<const float4*>(es + kBN / 2 + c * 16 + 4 * q);
-                            const float4 ou = *reinterpret_cast<const float4*>(es + kBN + kBN / 2 + c * 16 + 4 * q);
-                            // accumulator positions (0,2,1,3) of a group of four hold columns 0..3
-                            const uint32_t g01 = pack_bf16x2(fmaf(og.x, rs, sg.x * __uint_as_float(rg[4 * q])),
-                                                             fmaf(og.y, rs, sg.y * __uint_as_float(rg[4 * q + 2])));
-                            const uint32_t g23 = pack_bf16x2(fmaf(og.z, rs, sg.z * __uint_as_float(rg[4 * q + 1])),
-                                                             fmaf(og.w, rs, sg.w * __uint_as_float(rg[4 * q + 3])));
-                            const uint32_t u01 = pack_bf16x2(fmaf(ou.x, rs, su.x * __uint_as_float(ru[4 * q])),
-                                                             fmaf(ou.y, rs, su.y * __uint_as_float(ru[4 * q + 2])));
-                            const uint32_t u23 = pack_bf16x2(fmaf(ou.z, rs, su.z * __uint_as_float(ru[4 * q + 1])),
-                                                             fmaf(ou.w, rs, su.w * __uint_as_float(ru[4 * q + 3])));
+                            uint32_t g01, g23, u01, u23;
+                            if constexpr (per_channel) {
+                                const float4 sg = *reinterpret_cast<const float4*>(es + c * 16 + 4 * q);
+                                const float4 og = *reinterpret_cast<const float4*>(es + kBN + c * 16 + 4 * q);
+                                const float4 su = *reinterpret_cast<const float4*>(es + kBN / 2 + c * 16 + 4 * q);
+                                const float4 ou = *reinterpret_cast<const float4*>(es + kBN + kBN / 2 + c * 16 + 4 * q);
+                                // accumulator positions (0,2,1,3) of a group of four hold columns 0..3
+                                g01 = pack_bf16x2(fmaf(og.x, rs, sg.x * __uint_as_float(rg[4 * q])),
+                                                  fmaf(og.y, rs, sg.y * __uint_as_float(rg[4 * q + 2])));
+                                g23 = pack_bf16x2(fmaf(og.z, rs, sg.z * __uint_as_float(rg[4 * q + 1])),
+                                                  fmaf(og.w, rs, sg.w * __uint_as_float(rg[4 * q + 3])));
+                                u01 = pack_bf16x2(fmaf(ou.x, rs, su.x * __uint_as_float(ru[4 * q])),
+                                                  fmaf(ou.y, rs, su.y * __uint_as_float(ru[4 * q + 2])));
+                                u23 = pack_bf16x2(fmaf(ou.z, rs, su.z * __uint_as_float(ru[4 * q + 1])),
+                                                  fmaf(ou.w, rs, su.w * __uint_as_float(ru[4 * q + 3])));
+                            } else {
+                                g01 = pack_bf16x2(__uint_as_float(rg[4 * q]), __uint_as_float(rg[4 * q + 1]));
+                                g23 = pack_bf16x2(__uint_as_float(rg[4 * q + 2]), __uint_as_float(rg[4 * q + 3]));
+                                u01 = pack_bf16x2(__uint_as_float(ru[4 * q]), __uint_as_float(ru[4 * q + 1]));
+                                u23 = pack_bf16x2(__uint_as_float(ru[4 * q + 2]), __uint_as_float(ru[4 * q + 3]));
+                            }
                             const uint32_t gw[2] = {g01, g23}, uw[2] = {u01, u23};
 #pragma unroll
                             for (int i = 0; i < 2; ++i) {
@@ -817,8 +869,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         pf.seq = 0;
         pf.t = next_tile(sb, pf.seq, n_tiles, a.status);
         pf.kt = 0;
-        dq_locate<MODE>(pf, weight, a, d, n_tiles, tile_prefix, row_start, n_nt);
-        if (grp > 0 && pf.valid) dq_advance<MODE>(pf, grp, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+        dq_locate<MODE, SPLIT>(pf, weight, a, d, n_tiles, tile_prefix, row_start, n_nt);
+        if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT>(pf, grp, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
         DqIter cur = pf;  // int4 only: the stage being converted (its scales are loaded late)
         PackedRegs<MODE> regs[kPrefetch];
         bool loaded[kPrefetch];
@@ -826,8 +878,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         for (int u = 0; u < kPrefetch; ++u) {
             loaded[u] = pf.valid;
             if (pf.valid) {
-                load_packed<MODE>(regs[u], pf, a, d);
-                dq_advance<MODE>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+                load_packed<MODE, SPLIT>(regs[u], pf, a, d);
+                dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
             }
         }
         const uint32_t sa0 = ptx::smem_u32(b_ring) + (MODE == kCtFp4Ascend ? btile_offset(d.k0, d.chunk)
@@ -856,11 +908,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->full[slot]));
                 loaded[u] = pf.valid;
                 if (pf.valid) {
-                    load_packed<MODE>(regs[u], pf, a, d);
-                    dq_advance<MODE>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+                    load_packed<MODE, SPLIT>(regs[u], pf, a, d);
+                    dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
                 }
                 if constexpr (MODE == B200MOE_CT_INT4)
-                    dq_advance<MODE>(cur, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+                    dq_advance<MODE, SPLIT>(cur, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
                 ib += kDqGroups;
             }
         }
@@ -946,7 +998,8 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
         rc = make_tensor_map_2d(&tw, w, 2, (uint64_t)a.G * a.K, a.N, kBK, 64, true);
     else
         rc = make_tensor_map_2d(&tw, w, 1, (uint64_t)a.G * a.K, T::kNibbles ? a.N / 2 : a.N, kBK,
-                                a.N < kBN ? (uint32_t)(T::kNibbles ? a.N / 2 : a.N) : (uint32_t)T::kPRowBytes, false);
+                                SILU && MODE == kCtFp4E8m0 ? kBN / 4  // gate and up halves of a tile: two boxes
+                                : a.N < kBN ? (uint32_t)(T::kNibbles ? a.N / 2 : a.N) : (uint32_t)T::kPRowBytes, false);
     if (rc != B200MOE_OK) return rc;
     const size_t smem = gm_smem_bytes(a.G);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1069,6 +1122,35 @@ extern "C" int b200moe_grouped_gemm_int8_silu(const void* x, const void* weight,
         a.rowsum = rowsum;
     }
     return gm_launch<B200MOE_CT_INT8, true>(x, weight, a, s);
+}
+
+extern "C" int b200moe_grouped_gemm_fp4_e8m0(const void* x, const void* codes, const void* scale_e8m0,
+                                             const int64_t* group_list, void* out, int64_t M, int64_t K, int64_t N, int64_t G,
+                                             int group_list_type, int gate_up_silu, void* workspace, size_t workspace_bytes,
+                                             void* stream) {
+    if (group_list_type != B200MOE_GROUP_LIST_CUMSUM && group_list_type != B200MOE_GROUP_LIST_COUNTS)
+        return B200MOE_ERR_ARGUMENT;
+    if (M < 0 || K <= 0 || N <= 0 || G <= 0 || G > kMaxExperts || M > 0x7FFFFFF0LL || K > 0x7FFFFFF0LL ||
+        N > 0x7FFFFFF0LL || G * K > 0x7FFFFFF0LL)
+        return B200MOE_ERR_SHAPE;
+    if ((K % kBK) != 0 || (N % kBN) != 0) return B200MOE_ERR_SHAPE;
+    if (M == 0) return B200MOE_OK;
+    if (!x || !codes || !scale_e8m0 || !group_list || !out) return B200MOE_ERR_NULL_POINTER;
+    if (!aligned16(x) || !aligned16(codes) || !aligned16(out)) return B200MOE_ERR_ALIGNMENT;
+    const size_t need = b200moe_grouped_gemm_workspace_bytes(M, K, N, G, B200MOE_CT_FP4, B200MOE_LAYOUT_CANONICAL);
+    if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200MOE_ERR_WORKSPACE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
+    GemmArgs a;
+    a.scale = scale_e8m0;
+    a.offset = nullptr;
+    a.rowsum = nullptr;
+    a.group_list = group_list;
+    a.y = static_cast<__nv_bfloat16*>(out);
+    a.M = (int)M; a.K = (int)K; a.N = (int)N; a.G = (int)G;
+    a.gl_type = group_list_type;
+    a.status = static_cast<int*>(workspace);
+    return gate_up_silu ? gm_launch<kCtFp4E8m0, true>(x, codes, a, s) : gm_launch<kCtFp4E8m0>(x, codes, a, s);
 }
 
 // ---------------------------------------------------------------------------------------------

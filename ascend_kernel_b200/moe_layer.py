@@ -67,10 +67,10 @@ class MoELayer:
         ``weight_format="fp4"``: the experts are STORED as FP4 e2m1 -- w13 uint8 [E_local, H, 2I/2] and w2
         uint8 [E_local, I, H/2], two codes per byte along the last dimension, with s13 / s2 one e8m0 byte
         per 32 elements of the last dimension ([E_local, H, 2I/32] / [E_local, I, H/32]); o13 / o2 must be
-        None.  Every pass dequantises them to bf16 buffers owned by the layer (FP4 -> BF16 kernel) and
-        runs the bf16 grouped GEMM on those: the two-phase structure of the reference's own kernel
-        (dequantise to a bf16 workspace, then multiply: grouped_matmul_antiquant.h:632-654,
-        grouped_matmul.h:409-463) with the benchmark's storage format.
+        None.  Every pass reads them in place: the grouped GEMM dequantises them to bf16 inside the kernel, with the
+        bits and the product of the two phases of the reference's own kernel (dequantise to a bf16
+        workspace, then multiply: grouped_matmul_antiquant.h:632-654, grouped_matmul.h:409-463), and
+        SiLU(gate) * up runs in the first GEMM's epilogue.  ``bf13`` / ``bf2`` dequantise them on request.
         ``exchange_buffers=2`` (p2p exchange only) doubles the exchange buffers, which ``OverlappedSteps``
         needs to run one step's token exchange beside the expert GEMMs of the step before."""
         self.ops = row_ops
@@ -90,16 +90,12 @@ class MoELayer:
         if weight_format not in ("int8", "fp4"):
             raise ValueError("weight_format must be 'int8' or 'fp4'")
         self.weight_format = weight_format
-        self.bf13 = self.bf2 = None
         if weight_format == "fp4":
             if o13 is not None or o2 is not None or row_ops is not CudaRowOps:
                 raise ValueError("FP4-stored experts take no offsets and run on the CUDA row operations only")
             if w13.shape[2] != self.inter or w2.shape[2] * 2 != self.hidden:
                 raise ValueError("expected w13 [E, H, 2I/2] and w2 [E, I, H/2] packed codes")
             fuse_silu, gemm = False, "generic"
-            # the bf16 weights of one pass: overwritten by every pass, never read across passes
-            self.bf13 = torch.empty(self.e_local, self.hidden, 2 * self.inter, dtype=torch.bfloat16, device=self.device)
-            self.bf2 = torch.empty(self.e_local, self.inter, self.hidden, dtype=torch.bfloat16, device=self.device)
         self.fuse_silu = (row_ops is CudaRowOps) if fuse_silu is None else bool(fuse_silu)
         if gemm is None:
             gemm = "packed" if (row_ops is CudaRowOps and self.fuse_silu) else "generic"
@@ -129,6 +125,23 @@ class MoELayer:
         # called on the host when the rows of the step have been enqueued to reach their experts and the
         # expert GEMMs come next (HostPipeline starts the neighbouring steps' host copies there)
         self.mid_hook = None
+
+    def _dequantised(self, codes, scale, cols):
+        if self.weight_format != "fp4":
+            return None
+        w = torch.empty(codes.shape[0], codes.shape[1], cols, dtype=torch.bfloat16, device=self.device)
+        ops.fp4_dequant(codes, scale, w)
+        return w
+
+    @property
+    def bf13(self):
+        """FP4-stored experts only: the gate/up weights as the bf16 values a pass multiplies with."""
+        return self._dequantised(self.w13, self.s13, 2 * self.inter)
+
+    @property
+    def bf2(self):
+        """FP4-stored experts only: the down projection's weights as the bf16 values a pass multiplies with."""
+        return self._dequantised(self.w2, self.s2, self.hidden)
 
     def read_status(self, clear: bool = True):
         """Device-side findings of the passes run so far, read at a synchronisation point of the caller's
@@ -164,16 +177,12 @@ class MoELayer:
         if ev:
             ev[0].record()
         if self.weight_format == "fp4":
-            ops.fp4_dequant(self.w13, self.s13, self.bf13)
-            h = torch.empty(R, 2 * self.inter, dtype=torch.bfloat16, device=self.device)
-            ops.grouped_gemm(rows, self.bf13, None, None, counts, "bf16", h, group_list_type=1)
+            act = torch.empty(R, self.inter, dtype=torch.bfloat16, device=self.device)
+            ops.grouped_gemm_fp4_e8m0(rows, self.w13, self.s13, counts, act, group_list_type=1, gate_up_silu=True)
             if ev:
                 ev[1].record()
-            act = ops.silu_mul(h) if n_rows is None else ops.silu_mul_dyn(h, n_rows)
-            if ev:
                 ev[2].record()
-            ops.fp4_dequant(self.w2, self.s2, self.bf2)
-            ops.grouped_gemm(act, self.bf2, None, None, counts, "bf16", y, group_list_type=1)
+            ops.grouped_gemm_fp4_e8m0(act, self.w2, self.s2, counts, y, group_list_type=1)
             if ev:
                 ev[3].record()
                 self.timing = ev

@@ -202,6 +202,34 @@ def grouped_gemm_silu(x, weight, scale, offset, group_list, output, group_list_t
     return ws if return_workspace else None
 
 
+def grouped_gemm_fp4_e8m0(x, codes, scale, group_list, output, group_list_type: int = 0, gate_up_silu: bool = False,
+                          return_workspace: bool = False):
+    """Grouped GEMM on experts stored as fp4 codes [G, K, N/2] with one e8m0 byte per 32 columns [G, K, N/32]:
+    the result of :func:`fp4_dequant` followed by the ``"bf16"`` grouped GEMM, without the bf16 weights' way
+    through memory.  ``gate_up_silu``: N = 2I with the gate columns first, output [M, I] = bf16(silu(gate) * up)."""
+    _need_cuda(x=x, codes=codes, scale=scale, group_list=group_list, output=output)
+    if x.dtype != torch.bfloat16 or output.dtype != torch.bfloat16 or group_list.dtype != torch.int64:
+        raise RuntimeError("x and output must be bfloat16, group_list int64")
+    if codes.dim() != 3 or codes.element_size() != 1:
+        raise RuntimeError("codes must be a 1-byte container [G, K, N/2]")
+    G, K, N = codes.shape[0], codes.shape[1], codes.shape[2] * 2
+    M = x.shape[0]
+    n_out = N // 2 if gate_up_silu else N
+    if x.shape[1] != K or tuple(output.shape) != (M, n_out) or group_list.numel() != G:
+        raise RuntimeError(f"shape mismatch: x {tuple(x.shape)}, codes {tuple(codes.shape)}, output {tuple(output.shape)}")
+    if scale.element_size() != 1 or scale.numel() * 32 != G * K * N:
+        raise RuntimeError("scale must hold one e8m0 byte per 32 elements")
+    need = _lib.b200moe_grouped_gemm_workspace_bytes(M, K, N, G, CT["fp4"], LAYOUT["canonical"])
+    ws = _workspace(need, x.device)
+    with torch.cuda.device(x.device):
+        rc = _lib.b200moe_grouped_gemm_fp4_e8m0(_ptr(x), _ptr(codes), _ptr(scale), _ptr(group_list), _ptr(output), M, K, N, G,
+                                                group_list_type, int(bool(gate_up_silu)), _ptr(ws), need, _stream())
+    _abi.check(rc, "grouped_gemm_fp4_e8m0")
+    if M > 0:
+        _count(1)
+    return ws if return_workspace else None
+
+
 def pack_weight_int8(weight, gate_up: bool = False):
     """int8 [G, K, N] -> the tile-packed order grouped_gemm_packed reads (same shape, opaque contents).
     ``gate_up``: N = 2I with the gate columns first; tiles then pair gate and up columns."""

@@ -108,6 +108,18 @@ int b200moe_grouped_gemm_int8_silu(const void* x, const void* weight, const void
                                    const int64_t* group_list, void* out, int64_t M, int64_t K, int64_t N, int64_t G,
                                    int group_list_type, void* workspace, size_t workspace_bytes, void* stream);
 
+/* Grouped GEMM on fp4 weights in the format of b200moe_fp4_dequant (no reference counterpart): codes
+ * [G, K, N / 2], low nibble = even column, scale_e8m0 one byte per 32 columns of a k row, [G, K, N / 32].  The
+ * weights are dequantised inside the kernel to the bits b200moe_fp4_dequant would write, so the result
+ * equals that operator followed by b200moe_grouped_gemm with compute_type bf16 -- without the bf16 weights'
+ * way through memory.  gate_up_silu != 0: N = 2 * I with the gate columns first, out bf16 [M, I] =
+ * bf16(silu(gate) * up) as b200moe_silu_mul would compute it; otherwise out bf16 [M, N].  K % 64 == 0,
+ * N % 256 == 0; x, codes and out aligned to 16 bytes.  Workspace as for b200moe_grouped_gemm with
+ * compute_type fp4. */
+int b200moe_grouped_gemm_fp4_e8m0(const void* x, const void* codes, const void* scale_e8m0, const int64_t* group_list,
+                                  void* out, int64_t M, int64_t K, int64_t N, int64_t G, int group_list_type,
+                                  int gate_up_silu, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Int8 grouped GEMM on weights repacked once into a tile order (no reference counterpart: the
  * reference reads [G, K, N] on every call; a caller that keeps expert weights resident, like the MoE
  * layer, repacks them at load time).  In the packed order every dequantised weight tile is written by

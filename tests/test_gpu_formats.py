@@ -150,3 +150,39 @@ def test_device_findings_reach_the_caller_without_a_workspace():
     assert tuple(cinfer_ascendc.last_status()) == (1, 1)
     with pytest.raises(RuntimeError, match="group_list"):
         cinfer_ascendc.check_status()
+
+
+@pytest.mark.parametrize("counts,K,N", [
+    ([1], 64, 256),                            # smallest legal problem, one tile, one k-stage
+    ([127, 0, 129, 33, 300, 256, 257], 192, 512),  # one- and two-half tiles, small last boxes, an empty expert
+    ([2100, 5], 448, 256),                     # more than one L2 super-tile; fewer k-stages than the scale prefetch leads
+    ([20] * 40, 1024, 768),                    # many small experts, odd number of tile columns
+])
+@pytest.mark.parametrize("all_scales", [False, True])
+def test_fp4_e8m0_gemm_equals_dequant_then_bf16_gemm(counts, K, N, all_scales):
+    """The fused path against its two phases on the same tensors: the same weight bits, the same products in the
+    same order, hence the same output bits; with every scale byte there are infinities and NaNs among them."""
+    import ascend_kernel_b200 as ak
+    from ascend_kernel_b200 import ops
+
+    gen = torch.Generator().manual_seed(K + N)
+    G, M = len(counts), sum(counts) + 3
+    codes = torch.randint(0, 256, (G, K, N // 2), generator=gen, dtype=torch.uint8).cuda()
+    lo, hi = (0, 256) if all_scales else (119, 128)
+    scale = torch.randint(lo, hi, (G, K, N // 32), generator=gen, dtype=torch.uint8).cuda()
+    x = torch.randn(M, K, generator=gen).to(torch.bfloat16).cuda()
+    cnt = torch.tensor(counts, dtype=torch.int64).cuda()
+    w = torch.empty(G, K, N, dtype=torch.bfloat16, device="cuda")
+    ak.fp4_dequant(codes, scale, w)
+    want = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    got = want.clone()
+    ak.grouped_gemm(x, w, None, None, cnt, "bf16", want, group_list_type=1)
+    ws = ops.grouped_gemm_fp4_e8m0(x, codes, scale, cnt, got, group_list_type=1, return_workspace=True)
+    torch.cuda.synchronize()
+    assert ak.read_status(ws) == (0, 0)
+    assert same_bits(got, want)
+    assert (got[sum(counts):] == 7.0).all()          # rows of no expert are never written
+    act = torch.full((M, N // 2), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.grouped_gemm_fp4_e8m0(x, codes, scale, cnt.cumsum(0), act, gate_up_silu=True)
+    assert same_bits(act[:sum(counts)], ak.silu_mul(want)[:sum(counts)])
+    assert (act[sum(counts):] == 7.0).all()
