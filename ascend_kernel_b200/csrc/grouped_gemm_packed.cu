@@ -5,7 +5,7 @@
 //   y^T[weight columns, rows of expert g] = W[g]^T @ x[rows of expert g]^T
 //
 // The operands are swapped against the generic kernel (grouped_gemm.cu): the 128 lanes of an MMA
-// are weight columns and its N extent is the tile's token rows rounded up to 16 (16 .. 160), so an
+// are weight columns and its N extent is the tile's token rows rounded up to 16 (16 .. 160; in decode steps up to 32), so an
 // expert with 137 rows costs 144 columns of tensor-core time instead of two 128-row halves, and the
 // A operand (bf16 weights) is written by the dequant warps straight into tensor memory
 // (tcgen05.st) and read from there by the MMA.  Shared memory carries only the x tile (TMA, K-major,
@@ -25,7 +25,7 @@
 // warp 2 TMEM allocation and MMA issue; warps 4-11 epilogue (lane = weight column: per-channel
 // scale and offset are per-thread scalars, a warp stores 64 contiguous bytes of one output row
 // per instruction); warps 12-27 dequant in two groups on alternate stages.  TMEM: accumulators of
-// the two halves at columns 0 and 160, the A ring (3 stages x 2 halves x 32 columns) from column
+// the two halves at columns 0 and 160, the A ring (3 stages x 2 halves x 32 columns; Shape has the decode step's sizes) from column
 // 320.  The x ring has its own barriers and twice the depth: an x box takes 700 to 800 cycles from
 // issue to arrival, more than a stage lasts, and shared memory has the room that tensor memory lacks.
 // The MMA warp's loop is serial and every step of it costs tens of cycles, so it sees ONE barrier
@@ -52,9 +52,6 @@ static unsigned grid_ctas() {
 
 constexpr int kBK = 64;        // k per stage
 constexpr int kTileN = 256;    // weight columns per tile: two MMA halves of 128
-constexpr int kMaxR = 160;     // token rows per tile (the MMA's N extent), a multiple of 32
-constexpr int kStages = 3;     // A ring (tensor memory), 64 k per stage
-constexpr int kXStages = 6;    // x ring (shared memory), 64 k per stage (120 KB; 80 KB more hold the epilogue's staging tile)
 constexpr int kThreads = 896;
 constexpr int kWarpProd = 0, kWarpMma = 2, kWarpEpi0 = 4, kEpiWarps = 8, kWarpDq0 = 12;
 constexpr int kDqGroups = 2, kDqGroupWarps = 8;
@@ -62,27 +59,42 @@ constexpr int kPrefetch = 2;    // packed stages a dequant thread holds in regis
 constexpr int kL2Ahead = 4;     // stages by which the L2 prefetch of packed weights leads the x loads
 constexpr int kSuperRows = 8;   // m-tiles per L2 super-tile
 constexpr int kTileRing = 32;
-constexpr int kXSlotBytes = kMaxR * kBK * 2;  // 20 KB, a multiple of 1024
 constexpr int kStageWBytes = kBK * kTileN;    // packed bytes of one stage
 constexpr int kBigBox = 128, kSmallBox = 32;  // rows of the two x boxes
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kACol = 2 * kMaxR;          // first column of the A ring
 constexpr uint32_t kAStageCols = 64;           // 2 halves x 32 columns (64 k as bf16 pairs)
 constexpr int kBarrierBytes = 1024;
-constexpr int kEpiStripBytes = kMaxR * 4;  // per epilogue warp: the row sums of the tile's rows
-constexpr int kStageTileBytes = kMaxR * kTileN * 2;  // the epilogue's bf16 staging tile (80 KB)
-static_assert(kACol + kStages * kAStageCols <= kTmemCols, "tensor memory budget");
+
+// Sizes of the kernel: token rows per tile (the MMA's N extent, a multiple of 32) against the depth of the A ring in tensor
+// memory, 64 k per stage; what the accumulators leave of its 512 columns is the ring.
+template <int MAX_R, int STAGES, int X_STAGES>
+struct Shape {
+    static constexpr int kMaxR = MAX_R;
+    static constexpr int kStages = STAGES;     // A ring (tensor memory)
+    static constexpr int kXStages = X_STAGES;  // x ring (shared memory); the epilogue's staging tile takes the rest
+    static constexpr int kXSlotBytes = MAX_R * kBK * 2;   // a multiple of 1024
+    static constexpr uint32_t kACol = 2 * MAX_R;          // first column of the A ring
+    static constexpr int kEpiStripBytes = MAX_R * 4;      // per epilogue warp: the row sums of the tile's rows
+    static constexpr int kStageTileBytes = MAX_R * kTileN * 2;  // the epilogue's bf16 staging tile
+    static_assert(2 * MAX_R + STAGES * kAStageCols <= kTmemCols, "tensor memory budget");
+    static_assert(kXSlotBytes % 1024 == 0 && MAX_R % 32 == 0, "x slots");
+};
+using Prefill = Shape<160, 3, 6>;
+// Decode steps have few rows an expert and are bound by the weights' way from HBM (about 700 cycles a stage); the round
+// trip of a three-stage ring takes longer than that.  Layer of 256 experts, 32 tokens x 8, 7168 x 2048: 1.65 ms with
+// three stages, 1.53 with seven (4.4 and 4.7 TB/s).
+using Decode = Shape<32, 7, 12>;
 
 struct TileInfo {
-    int g, row0, rows;  // expert, first row, rows of the expert inside the tile (1 .. kMaxR)
+    int g, row0, rows;  // expert, first row, rows of the expert inside the tile (1 .. the shape's kMaxR)
     int j;              // tile column index (256 weight columns each)
 };
 
 struct Barriers {
-    uint64_t x_full[kXStages];   // x ring: TMA bytes; waited for by the relay lane of the stage's dequant group
-    uint64_t x_empty[kXStages];  // x ring: one arrive by the relay lane once the stage's MMAs have completed
-    uint64_t full[kStages];   // the 8 dequant warps of the stage's group: A slot written AND x tile landed
-    uint64_t empty[kStages];  // one tcgen05.commit per stage
+    uint64_t x_full[Decode::kXStages];   // x ring: TMA bytes; waited for by the relay lane of the stage's dequant group
+    uint64_t x_empty[Decode::kXStages];  // x ring: one arrive by the relay lane once the stage's MMAs have completed
+    uint64_t full[Decode::kStages];   // the 8 dequant warps of the stage's group: A slot written AND x tile landed
+    uint64_t empty[Decode::kStages];  // one tcgen05.commit per stage
     uint64_t t_full, t_empty; // accumulator hand-off with the epilogue
     uint64_t stage_full, stage_free;  // the epilogue warps among themselves: staging tile written / stored
     uint64_t drain;
@@ -161,6 +173,7 @@ __device__ __forceinline__ bool next_tile(Barriers* sb, uint32_t& seq, TileInfo&
 // Rows of an m-tile of an expert with `rows` rows: the expert is cut into the fewest tiles of at
 // most kMaxR rows, of equal size rounded up to 16 (a short last tile would still pay a full
 // dequantisation of the weight tile).
+template <int kMaxR>
 __device__ __forceinline__ int tile_rows_of(int rows) {
     const int n_mt = (rows + kMaxR - 1) / kMaxR;
     return n_mt == 0 ? kMaxR : ((((rows + n_mt - 1) / n_mt) + 15) & ~15);
@@ -169,6 +182,7 @@ __device__ __forceinline__ int tile_rows_of(int rows) {
 // tile index -> expert, rows, tile column.  tile_prefix has G + 1 entries.  Inside an expert the
 // tiles run in super-tiles of up to kSuperRows m-tiles x all tile columns, m fastest, so that
 // concurrently running CTAs share a weight tile and the expert's x rows in L2.
+template <int kMaxR>
 __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, const int* row_start, int G, int n_nt) {
     int lo = 0, hi = G;  // largest g with tile_prefix[g] <= t
     while (hi - lo > 1) {
@@ -179,7 +193,7 @@ __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, c
     const int g = lo, j = t - tile_prefix[g];
     const int r0 = row_start[g], rows = row_start[g + 1] - r0;
     const int mt = (tile_prefix[g + 1] - tile_prefix[g]) / n_nt;
-    const int tr = tile_rows_of(rows);
+    const int tr = tile_rows_of<kMaxR>(rows);
     const int per_super = kSuperRows * n_nt;
     const int st = j / per_super, base = st * kSuperRows;
     const int h = min(kSuperRows, mt - base);
@@ -223,10 +237,13 @@ __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* 
 // GATE_UP: a tile's half 0 holds 128 gate columns and half 1 the up columns of the same indices; the
 // epilogue writes bf16(silu(gate) * up), [M, N / 2] (gate and up are rounded to bf16 first, as the
 // unfused operators would).
-template <bool GATE_UP>
+template <bool GATE_UP, class SHAPE>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xs,
                            const uint8_t* __restrict__ weight, const GemmArgs a) {
+    constexpr int kMaxR = SHAPE::kMaxR, kStages = SHAPE::kStages, kXStages = SHAPE::kXStages, kXSlotBytes = SHAPE::kXSlotBytes;
+    constexpr int kStageTileBytes = SHAPE::kStageTileBytes, kEpiStripBytes = SHAPE::kEpiStripBytes;
+    constexpr uint32_t kACol = SHAPE::kACol;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_ring = base;
@@ -301,7 +318,7 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
                 const bool live = held < n_tiles;
                 uint4 entry = make_uint4(published + 1, 0u, 0u, 0u);  // rows 0: the schedule has ended
                 if (live) {
-                    far_ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
+                    far_ti = locate_tile<kMaxR>(held, tile_prefix, row_start, a.G, n_nt);
                     entry.y = (uint32_t)far_ti.row0;
                     entry.z = (uint32_t)far_ti.g | ((uint32_t)far_ti.rows << 16);
                     entry.w = (uint32_t)far_ti.j;
@@ -345,7 +362,7 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
                     const uint32_t dst = ptx::smem_u32(x_ring + s * kXSlotBytes);
                     const int kx = kt * kBK;
                     ptx::mbar_arrive_expect_tx(bar, stage_bytes);
-                    if (n_big) ptx::tma_load_2d(dst, &tmap_x, bar, kx, ti.row0);
+                    if (kMaxR >= kBigBox && n_big) ptx::tma_load_2d(dst, &tmap_x, bar, kx, ti.row0);
                     for (int b = 0; b < n_small; ++b)
                         ptx::tma_load_2d(dst + (uint32_t)((n_big * kBigBox + b * kSmallBox) * kBK * 2), &tmap_xs, bar, kx,
                                          ti.row0 + n_big * kBigBox + b * kSmallBox);
@@ -612,6 +629,17 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     }
 }
 
+template <bool GATE_UP, class SHAPE>
+static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, cudaStream_t s) {
+    const size_t smem = 1024 + (size_t)SHAPE::kXStages * SHAPE::kXSlotBytes + SHAPE::kStageTileBytes + kBarrierBytes +
+                        (size_t)kEpiWarps * SHAPE::kEpiStripBytes + sizeof(int) * 2 * (size_t)(a.G + 1);
+    B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_packed_kernel<GATE_UP, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+    grouped_gemm_packed_kernel<GATE_UP, SHAPE><<<grid_ctas(), kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
+    B200MOE_CUDA_TRY(cudaGetLastError());
+    return B200MOE_OK;
+}
+
 // [G, K, N] int8 -> the packed order.  One thread writes one lane's 16 bytes of a k-chunk.
 __global__ void pack_weight_int8_kernel(const int8_t* __restrict__ w, uint4* __restrict__ out, int K, int N, int gate_up,
                                         long long n_units) {
@@ -716,19 +744,11 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
     if (rc != B200MOE_OK) return rc;
     rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)M, (uint64_t)K, pk::kSmallBox, pk::kBK, true);
     if (rc != B200MOE_OK) return rc;
-    const size_t smem = 1024 + (size_t)pk::kXStages * pk::kXSlotBytes + pk::kStageTileBytes + pk::kBarrierBytes +
-                        (size_t)pk::kEpiWarps * pk::kEpiStripBytes + sizeof(int) * 2 * (size_t)(G + 1);
-    if (gate_up_silu) {
-        B200MOE_CUDA_TRY(cudaFuncSetAttribute(pk::grouped_gemm_packed_kernel<true>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        pk::grouped_gemm_packed_kernel<true><<<pk::grid_ctas(), pk::kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
-    } else {
-        B200MOE_CUDA_TRY(cudaFuncSetAttribute(pk::grouped_gemm_packed_kernel<false>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        pk::grouped_gemm_packed_kernel<false><<<pk::grid_ctas(), pk::kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
-    }
-    B200MOE_CUDA_TRY(cudaGetLastError());
-    return B200MOE_OK;
+    // The 32-row shape where the experts have at most eight rows on average (a decode step): a larger expert is then cut
+    // into tiles of 32 rows that each dequantise its weights, at most M / 32 of them in all.
+    const bool decode = M <= 8 * G;
+    if (gate_up_silu) return decode ? pk::launch<true, pk::Decode>(tx, txs, packed, a, s) : pk::launch<true, pk::Prefill>(tx, txs, packed, a, s);
+    return decode ? pk::launch<false, pk::Decode>(tx, txs, packed, a, s) : pk::launch<false, pk::Prefill>(tx, txs, packed, a, s);
 }
 
 extern "C" int b200moe_grouped_gemm_int8_packed(const void* x, const void* packed, const void* scale, const void* offset,

@@ -138,3 +138,26 @@ def test_row_sums_from_the_gather_give_the_same_bits(K, N):
     assert torch.equal(a.view(torch.int16), b.view(torch.int16))
     gold = O.golden_f32(rows.cpu(), w, scale, offset, cnt, "int8", O.GROUP_LIST_COUNTS)
     assert_close_to_golden(b, gold)
+
+
+@pytest.mark.parametrize("counts,K,N", [
+    ([8], 64, 256),                                    # one stage, exactly eight rows an expert
+    ([1] * 9 + [0, 2, 31, 33, 16, 17], 512, 512),      # eight stages (the ring is seven deep), tile edges at 16 and 32 rows
+    ([0] * 20 + [161], 832, 256),                      # every row on one expert: six 32-row tiles of the same weights
+    ([3] * 150, 1024, 256),                            # more tiles than multiprocessors, 16 stages each
+])
+def test_packed_decode_shape_matches_oracle_and_generic_kernel(counts, K, N):
+    """At most eight rows an expert on average: the kernel's 32-row shape."""
+    x, w, scale, offset, cnt = _int8_case(counts, K, N, 17, True, extra_rows=0)
+    assert x.shape[0] <= 8 * len(counts)
+    gold = O.golden_f32(x, w, scale, offset, cnt, "int8", O.GROUP_LIST_COUNTS)
+    out, st = run_packed(x, w, scale, offset, cnt)
+    assert st == (0, 0)
+    assert_close_to_golden(out, gold)
+    ref, _ = run_gemm(x, w, scale, offset, cnt, "int8", gl_type=1)
+    assert float((out.float() - ref.float()).abs().max()) <= 0.02 * float(ref.float().abs().max())
+    act, st = run_packed(x, w, scale, offset, cnt, gate_up=True)
+    assert st == (0, 0)
+    h = gold.to(torch.bfloat16).float()
+    want = (torch.nn.functional.silu(h[:, :N // 2]) * h[:, N // 2:]).to(torch.bfloat16).float()
+    assert O.rel_l2(act.float().cpu(), want) < 4e-3
