@@ -93,6 +93,10 @@ struct GmTraits {
     // into the B ring (a 64 k x 128-byte box with the 128-byte swizzle is exactly one block of the
     // MN-major operand layout) and the dequant warps have nothing to do
     static constexpr bool kDirect = (MODE == B200MOE_CT_BF16);
+    // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
+    // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
+    // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
+    static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
 };
 
 struct GmBarriers {
@@ -210,6 +214,38 @@ __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, c
     return ti;
 }
 
+// Row boundaries and the tile-count prefixes of locate_tile, by the whole CTA (a barrier must follow).  Not inlined:
+// the main loops then keep their registers (inlined, every mode spilled more; int8, 8192 tokens x 8 over 256
+// experts, 7168 x 4096: 5.22 -> 5.03 ms).
+__device__ __noinline__ void gm_schedule(const int64_t* __restrict__ gl, int G, int M, int gl_type, int n_nt,
+                                         int* row_start, int* tile_prefix, int* n_tiles, int* status) {
+    load_row_starts(gl, G, M, gl_type, row_start, status);
+    if (threadIdx.x < 32) {
+        // tile-count prefixes, each lane over a stretch of consecutive experts
+        int* pref1 = tile_prefix + (G + 1);
+        int lo, hi, c2 = 0, c1 = 0, t2, t1;
+        lane_experts(G, lo, hi);
+        for (int g = lo; g < hi; ++g) {
+            const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
+            c2 += rows / kTileM + (tail > kBM ? 1 : 0);   // m-tiles with two row halves
+            c1 += (tail >= 1 && tail <= kBM) ? 1 : 0;      // the short last m-tile, if any
+        }
+        int p2 = warp_exclusive_sum(c2, t2), p1 = warp_exclusive_sum(c1, t1);
+        for (int g = lo; g < hi; ++g) {
+            const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
+            tile_prefix[g] = p2 * n_nt;
+            pref1[g] = p1 * n_nt;
+            p2 += rows / kTileM + (tail > kBM ? 1 : 0);
+            p1 += (tail >= 1 && tail <= kBM) ? 1 : 0;
+        }
+        if (threadIdx.x == 0) {
+            tile_prefix[G] = t2 * n_nt;
+            pref1[G] = t1 * n_nt;
+            *n_tiles = (t2 + t1) * n_nt;
+        }
+    }
+}
+
 // ---- dequant of one packed stage into the bf16 UMMA tile --------------------------------------
 // bf16 tile layout (MN-major, 128-byte swizzle): four blocks of 64 columns; inside a block row k
 // occupies 128 bytes at k*128 and its eight 16-byte chunks are XOR-swizzled with (k & 7).
@@ -226,8 +262,8 @@ __device__ __forceinline__ uint32_t btile_offset(int k, int nchunk16) {  // nchu
 struct DqLane {
     int row;  // the thread converts k = row + kDqRowStep * j, j < kDqRows, of its stages
     int c16;  // 16-column chunk 0..15
-    // stored-order fp4 only: the thread converts canonical rows k0 .. k0 + 7, columns 8 * chunk .. + 7
-    int k0, chunk, src_row, src_byte;  // where its 32 bytes start inside the 64 x 128-byte box
+    // kEightRows only: the thread converts canonical rows k0 .. k0 + 7, columns 8 * chunk .. + 7
+    int k0, chunk, src_row, src_byte;  // where its first bytes are inside the 64 x 128-byte box
 };
 template <int MODE>
 __device__ __forceinline__ DqLane dq_lane(int tid) {
@@ -240,6 +276,11 @@ __device__ __forceinline__ DqLane dq_lane(int tid) {
         d.src_row = (b * 4 + a) * 8 + (l >> 2);
         d.src_byte = (l & 3) * 32;
         d.row = d.src_row;                    // what dq_locate adds to the stage's first row
+        d.c16 = 0;
+    } else if constexpr (GmTraits<MODE>::kEightRows) {
+        d.k0 = d.row = d.src_row = 8 * w;
+        d.chunk = l;
+        d.src_byte = 4 * l;
         d.c16 = 0;
     } else {
         const int p = l >> 3, q = l & 7, odd = q >> 2;
@@ -255,7 +296,7 @@ template <int MODE>
 struct PackedRegs {
     uint4 q[kDqRows];  // fp4 / int4 use only .x/.y of each
     uint4 s[2];        // fp4 only: the bf16 scales of the thread's 16 columns (one 16-row group)
-    uint32_t e[kDqRows];  // fp4 with e8m0 scales only: the scale byte of each of the thread's rows
+    uint32_t e[kDqRows];  // fp4 with e8m0 scales: the scale byte of each of the thread's rows; int4: e[0] locates its scales
     float sf;          // fp8 only: the fp32 scale of the thread's 128 x 128 block
 };
 
@@ -284,7 +325,7 @@ __device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict_
     it.n0 = ti.n0;
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
     it.wp = w + ((size_t)ti.g * a.K + (size_t)it.kt * kBK + d.row) * row_bytes +
-            (MODE == kCtFp4Ascend ? (ti.n0 >> 1) + d.src_byte
+            (T::kEightRows        ? (ti.n0 >> 1) + d.src_byte
              : T::kNibbles        ? chunk_col<SPLIT>(ti.n0, d.c16, a.N) >> 1
                                   : ti.n0 + d.c16 * 16);
 }
@@ -321,6 +362,16 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
         return;
     }
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
+    if constexpr (MODE == B200MOE_CT_INT4) {
+        uint32_t v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(it.wp + (size_t)i * row_bytes));
+        r.q[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        r.q[1] = make_uint4(v[4], v[5], v[6], v[7]);
+        // in units of the 8 scales a thread loads (fits 32 bits: the weights would be 17 TB otherwise)
+        r.e[0] = (uint32_t)((((size_t)it.g * (a.K >> 7) + ((it.kt * kBK) >> 7)) * a.N + it.n0) >> 3) + d.chunk;
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < kDqRows; ++j) {
         const uint8_t* p = it.wp + (size_t)(kDqRowStep * j) * row_bytes;
@@ -444,62 +495,49 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
 
 // int4 with per-128-k scale / offset: one pass over a k block produces both stages it feeds to the
 // tensor core, hi = bf16(v) and lo = bf16(v - hi) with v = w * s + o * s in fp32.  The thread's
-// rows lie in the same 128-k group, so its 16 scales and offsets are loaded once per k block
+// rows lie in the same 128-k group, so its 8 scales and offsets are loaded once per k block
 // (before the wait for the stage, so that their latency is hidden by it).
 struct Int4Scales {
-    uint4 s[2], o[2];
+    uint4 s, o;
 };
-__device__ __forceinline__ Int4Scales load_int4_scales(const GemmArgs& a, int g, int n0, int kb, const DqLane& d) {
-    const size_t so = ((size_t)g * (a.K >> 7) + ((kb * kBK) >> 7)) * a.N + n0 + d.c16 * 16;
-    const uint4* sp = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.scale) + so);
+__device__ __forceinline__ Int4Scales load_int4_scales(const GemmArgs& a, uint32_t unit) {
     Int4Scales r;
-    r.s[0] = __ldg(sp);
-    r.s[1] = __ldg(sp + 1);
-    if (a.offset != nullptr) {
-        const uint4* op = reinterpret_cast<const uint4*>(a.offset + so);
-        r.o[0] = __ldg(op);
-        r.o[1] = __ldg(op + 1);
-    } else {
-        r.o[0] = r.o[1] = make_uint4(0u, 0u, 0u, 0u);
-    }
+    r.s = __ldg(static_cast<const uint4*>(a.scale) + unit);
+    r.o = a.offset != nullptr ? __ldg(reinterpret_cast<const uint4*>(a.offset) + unit) : make_uint4(0u, 0u, 0u, 0u);
     return r;
 }
 
+// `sa_hi` / `sa_lo`: shared addresses of the thread's chunk in its first row (a multiple of 8, see
+// convert_stage_fp4_ascend).
 __device__ __forceinline__ void convert_block_int4(const PackedRegs<B200MOE_CT_INT4>& r, const Int4Scales& sc,
                                                    uint32_t sa_hi, uint32_t sa_lo) {
     const f32x2 kMagic = pack_f32x2(8388616.0f, 8388616.0f);  // 2^23 + 8
+    const uint32_t sw[4] = {sc.s.x, sc.s.y, sc.s.z, sc.s.w};
+    const uint32_t ow[4] = {sc.o.x, sc.o.y, sc.o.z, sc.o.w};
+    f32x2 s2[4], t2[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // columns 8h .. 8h+7: one 16-byte chunk of the bf16 tile per row
-        const uint32_t sw[4] = {sc.s[h].x, sc.s[h].y, sc.s[h].z, sc.s[h].w};
-        const uint32_t ow[4] = {sc.o[h].x, sc.o[h].y, sc.o[h].z, sc.o[h].w};
-        uint32_t lo_n[kDqRows], hi_n[kDqRows];
+    for (int i = 0; i < 4; ++i) {
+        s2[i] = pack_f32x2(__uint_as_float(sw[i] << 16), __uint_as_float(sw[i] & 0xFFFF0000u));
+        t2[i] = mul_f32x2(pack_f32x2(__uint_as_float(ow[i] << 16), __uint_as_float(ow[i] & 0xFFFF0000u)), s2[i]);
+    }
+    const uint32_t w8[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
 #pragma unroll
-        for (int j = 0; j < kDqRows; ++j) {
-            const uint32_t word = (h == 0 ? r.q[j].x : r.q[j].y) ^ 0x88888888u;  // nibble + 8, unsigned
-            lo_n[j] = word & 0x0F0F0F0Fu;         // even columns, one per byte
-            hi_n[j] = (word >> 4) & 0x0F0F0F0Fu;  // odd columns
+    for (int j = 0; j < 8; ++j) {
+        const uint32_t word = w8[j] ^ 0x88888888u;                                      // nibble + 8, unsigned
+        const uint32_t lo_n = word & 0x0F0F0F0Fu, hi_n = (word >> 4) & 0x0F0F0F0Fu;  // even / odd columns, one per byte
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // column pair 2i, 2i + 1 = byte i of the word
+            // byte i under the fp32 pattern of 2^23: the float 2^23 + nibble + 8
+            const f32x2 wm = pack_u32x2(prmt(lo_n, 0x4B000000u, 0x7440u + i), prmt(hi_n, 0x4B000000u, 0x7440u + i));
+            const f32x2 v = fma_f32x2(sub_f32x2(wm, kMagic), s2[i], t2[i]);
+            hi[i] = pack_bf16x2(f32x2_lo(v), f32x2_hi(v));
+            const f32x2 l = sub_f32x2(v, pack_u32x2(hi[i] << 16, hi[i] & 0xFFFF0000u));
+            lo[i] = pack_bf16x2(f32x2_lo(l), f32x2_hi(l));
         }
-        uint32_t hi[kDqRows][4], lo[kDqRows][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {  // column pair 8h + 2i, 8h + 2i + 1 = byte i of the word
-            const f32x2 s2 = pack_f32x2(__uint_as_float(sw[i] << 16), __uint_as_float(sw[i] & 0xFFFF0000u));
-            const f32x2 t2 = mul_f32x2(pack_f32x2(__uint_as_float(ow[i] << 16), __uint_as_float(ow[i] & 0xFFFF0000u)), s2);
-#pragma unroll
-            for (int j = 0; j < kDqRows; ++j) {
-                // byte i under the fp32 pattern of 2^23: the float 2^23 + nibble + 8
-                const f32x2 wm = pack_u32x2(prmt(lo_n[j], 0x4B000000u, 0x7440u + i), prmt(hi_n[j], 0x4B000000u, 0x7440u + i));
-                const f32x2 v = fma_f32x2(sub_f32x2(wm, kMagic), s2, t2);
-                const uint32_t hh = pack_bf16x2(f32x2_lo(v), f32x2_hi(v));
-                hi[j][i] = hh;
-                const f32x2 l = sub_f32x2(v, pack_u32x2(hh << 16, hh & 0xFFFF0000u));
-                lo[j][i] = pack_bf16x2(f32x2_lo(l), f32x2_hi(l));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kDqRows; ++j) {
-            sts128(dq_row_addr(sa_hi, j) ^ (uint32_t)(h << 4), hi[j][0], hi[j][1], hi[j][2], hi[j][3]);
-            sts128(dq_row_addr(sa_lo, j) ^ (uint32_t)(h << 4), lo[j][0], lo[j][1], lo[j][2], lo[j][3]);
-        }
+        const uint32_t at = (uint32_t)(j << 4), row = (uint32_t)(j * 128);
+        sts128((sa_hi ^ at) + row, hi[0], hi[1], hi[2], hi[3]);
+        sts128((sa_lo ^ at) + row, lo[0], lo[1], lo[2], lo[3]);
     }
 }
 
@@ -534,31 +572,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     const int n_nt = (a.N + kBN - 1) / kBN;  // (fp8 only: the last tile may hold 128 columns)
     const int n_kt = a.K / kBK;  // stages per tile
 
-    load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
-    if (warp == 0) {
-        // tile-count prefixes, each lane over a stretch of consecutive experts
-        int* pref1 = tile_prefix + (a.G + 1);
-        int lo, hi, c2 = 0, c1 = 0, t2, t1;
-        lane_experts(a.G, lo, hi);
-        for (int g = lo; g < hi; ++g) {
-            const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
-            c2 += rows / kTileM + (tail > kBM ? 1 : 0);   // m-tiles with two row halves
-            c1 += (tail >= 1 && tail <= kBM) ? 1 : 0;      // the short last m-tile, if any
-        }
-        int p2 = warp_exclusive_sum(c2, t2), p1 = warp_exclusive_sum(c1, t1);
-        for (int g = lo; g < hi; ++g) {
-            const int rows = row_start[g + 1] - row_start[g], tail = rows % kTileM;
-            tile_prefix[g] = p2 * n_nt;
-            pref1[g] = p1 * n_nt;
-            p2 += rows / kTileM + (tail > kBM ? 1 : 0);
-            p1 += (tail >= 1 && tail <= kBM) ? 1 : 0;
-        }
-        if (lane == 0) {
-            tile_prefix[a.G] = t2 * n_nt;
-            pref1[a.G] = t1 * n_nt;
-            sb->n_tiles = (t2 + t1) * n_nt;
-        }
-    }
+    gm_schedule(a.group_list, a.G, a.M, a.gl_type, n_nt, row_start, tile_prefix, &sb->n_tiles, a.status);
     if (threadIdx.x == 32) {
         sb->abort = 0;
         for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = 0ull;
@@ -871,7 +885,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         pf.kt = 0;
         dq_locate<MODE, SPLIT>(pf, weight, a, d, n_tiles, tile_prefix, row_start, n_nt);
         if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT>(pf, grp, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
-        DqIter cur = pf;  // int4 only: the stage being converted (its scales are loaded late)
         PackedRegs<MODE> regs[kPrefetch];
         bool loaded[kPrefetch];
 #pragma unroll
@@ -882,7 +895,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
             }
         }
-        const uint32_t sa0 = ptx::smem_u32(b_ring) + (MODE == kCtFp4Ascend ? btile_offset(d.k0, d.chunk)
+        const uint32_t sa0 = ptx::smem_u32(b_ring) + (T::kEightRows ? btile_offset(d.k0, d.chunk)
                                                                             : btile_offset(d.row, 2 * d.c16));
         uint32_t ib = grp;
         bool ok = true;
@@ -892,7 +905,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if (!loaded[u]) { ok = false; break; }  // the schedule has ended
                 const uint32_t slot = ib % NS;
                 Int4Scales sc4;
-                if constexpr (MODE == B200MOE_CT_INT4) sc4 = load_int4_scales(a, cur.g, cur.n0, cur.kt, d);
+                if constexpr (MODE == B200MOE_CT_INT4) sc4 = load_int4_scales(a, regs[u].e[0]);  // (late: registers)
                 bool got = true;
                 if (ib >= NS) got = gm_wait(&sb->empty[slot], ((ib / NS) & 1) ^ 1, sb, a.status, 80 + (int)slot);
                 if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
@@ -911,8 +924,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     load_packed<MODE, SPLIT>(regs[u], pf, a, d);
                     dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
                 }
-                if constexpr (MODE == B200MOE_CT_INT4)
-                    dq_advance<MODE, SPLIT>(cur, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
                 ib += kDqGroups;
             }
         }
