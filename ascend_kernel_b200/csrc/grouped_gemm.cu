@@ -680,36 +680,43 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         }
     } else if (warp == kWarpMma) {
         // ------------------------------ MMA issuer ------------------------------
-        // One thread feeds the tensor core; its per-stage instruction count bounds the MMA rate, so
-        // ring positions and parities are carried incrementally and the shared-memory descriptors
-        // are a 64-bit base plus a small stage / k offset.
-        if (lane == 0) {
-            const uint32_t idesc = ptx::umma_idesc_bf16(kBM, kBN, true);
-            // A: K-major, 8-row groups 1024 B apart, 32 B per 16 k inside the swizzle atom
-            const uint64_t da0 = ptx::umma_desc_sw128(ptx::smem_u32(a_ring), 0, 1024);
-            // B: MN-major, 64-column blocks kBK*128 B apart (LBO), 8-k groups 1024 B apart (SBO)
-            const uint64_t db0 = ptx::umma_desc_sw128(ptx::smem_u32(b_ring), kBK * 128, 1024);
-            uint32_t sa = 0, pha = 0;
-            uint32_t uses[2] = {0, 0}, next1 = 0;
-            bool ok = true;
-            uint32_t seq = 0;
-            for (;;) {
-                const int t = next_tile(sb, seq, n_tiles, a.status);
-                if (t >= n_tiles || !ok) break;
-                const TileInfo ti = locate_tile(t, tile_prefix, row_start, a.G, n_nt);
-                // accumulators of this tile: both for two halves, else the one used less recently;
-                // the epilogue of their previous tile must have drained them
-                const uint32_t b0 = ti.halves == 2 ? 0u : next1, b1 = ti.halves == 2 ? 2u : next1 + 1u;
-                if (ti.halves == 1) next1 ^= 1u;
-                for (uint32_t b = b0; b < b1 && ok; ++b)
-                    if (uses[b] >= 1 && !gm_wait(&sb->t_empty[b], (uses[b] - 1) & 1, sb, a.status, 30 + (int)b)) ok = false;
+        // The whole warp walks the loop, so that waits, tile look-up and descriptor arithmetic are warp-uniform, and
+        // one elected lane issues the tcgen05 instructions: with everything in a branch of one lane, the issue of a
+        // stage's MMAs took 750 cycles, as long as they run, and stood in the ring's round trip (8192 tokens x 8 over 256
+        // experts, 7168 x 4096, int8: 5.03 -> 4.90 ms; the fp4-stored layer's GEMMs 5.24 -> 5.05).  Ring positions
+        // and parities are carried incrementally and the shared-memory descriptors are a 64-bit base plus a
+        // small stage / k offset.  The next stage's barrier is polled (non-blocking) right after a stage's MMAs are
+        // issued, so that the poll's latency runs beside the commit's.
+        const bool leader = ptx::elect_one();
+        const uint32_t idesc = ptx::umma_idesc_bf16(kBM, kBN, true);
+        // A: K-major, 8-row groups 1024 B apart, 32 B per 16 k inside the swizzle atom
+        const uint64_t da0 = ptx::umma_desc_sw128(ptx::smem_u32(a_ring), 0, 1024);
+        // B: MN-major, 64-column blocks kBK*128 B apart (LBO), 8-k groups 1024 B apart (SBO)
+        const uint64_t db0 = ptx::umma_desc_sw128(ptx::smem_u32(b_ring), kBK * 128, 1024);
+        uint32_t sa = 0, pha = 0;
+        uint32_t uses0 = 0, uses1 = 0, next1 = 0;
+        bool ok = true, ready = false;  // ready: the next stage's barrier has been seen complete already
+        uint32_t seq = 0;
+        for (;;) {
+            const int t = __shfl_sync(0xffffffffu, next_tile(sb, seq, n_tiles, a.status), 0);
+            if (t >= n_tiles) break;
+            const TileInfo ti = locate_tile(t, tile_prefix, row_start, a.G, n_nt);
+            // accumulators of this tile: both for two halves, else the one used less recently;
+            // the epilogue of their previous tile must have drained them
+            const bool use0 = ti.halves == 2 || next1 == 0, use1 = ti.halves == 2 || next1 == 1;
+            if (ti.halves == 1) next1 ^= 1u;
+            if (use0 && uses0 >= 1) ok = gm_wait(&sb->t_empty[0], (uses0 - 1) & 1, sb, a.status, 30);
+            if (ok && use1 && uses1 >= 1) ok = gm_wait(&sb->t_empty[1], (uses1 - 1) & 1, sb, a.status, 31);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const uint32_t acc0 = tmem_base + (use0 ? 0u : (uint32_t)kBN);
+            ptx::tc_fence_after();
+            uint32_t accumulate = 0;
+            for (int kt = 0; kt < n_kt; ++kt) {
+                if (!ready) ok = __all_sync(0xffffffffu, gm_wait(&sb->full[sa], pha, sb, a.status, 40 + (int)sa));
                 if (!ok) break;
-                const uint32_t acc0 = tmem_base + b0 * kBN;
                 ptx::tc_fence_after();
-                uint32_t accumulate = 0;
-                for (int kt = 0; kt < n_kt; ++kt) {
-                    if (!gm_wait(&sb->full[sa], pha, sb, a.status, 40 + (int)sa)) { ok = false; break; }
-                    ptx::tc_fence_after();
+                const uint32_t sn = sa + 1 == NS ? 0u : sa + 1, phn = sa + 1 == NS ? pha ^ 1u : pha;
+                if (leader) {
                     const uint64_t da = da0 + (uint64_t)(sa * (kATileBytes >> 4));
 #pragma unroll
                     for (int p = 0; p < P; ++p) {  // int4: the hi tile, then the lo tile, against the same x stage
@@ -725,17 +732,24 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                                                db + (uint64_t)(k16 * 128), idesc, accumulate | (uint32_t)(k16 + p));
                         }
                     }
-                    accumulate = 1;
-                    ptx::umma_commit(ptx::smem_u32(&sb->empty[sa]));
-                    if (++sa == NS) { sa = 0; pha ^= 1; }
                 }
-                if (ok)
-                    for (uint32_t b = b0; b < b1; ++b) {
-                        ptx::umma_commit(ptx::smem_u32(&sb->t_full[b]));
-                        ++uses[b];
-                    }
+                ready = ptx::mbar_test_wait(ptx::smem_u32(&sb->full[sn]), phn);
+                if (leader) ptx::umma_commit(ptx::smem_u32(&sb->empty[sa]));
+                ready = __all_sync(0xffffffffu, ready);
+                accumulate = 1;
+                sa = sn;
+                pha = phn;
             }
-            // drain: every issued MMA must have completed before TMEM is released
+            if (!ok) break;
+            if (leader) {
+                if (use0) ptx::umma_commit(ptx::smem_u32(&sb->t_full[0]));
+                if (use1) ptx::umma_commit(ptx::smem_u32(&sb->t_full[1]));
+            }
+            uses0 += use0;
+            uses1 += use1;
+        }
+        // drain: every issued MMA must have completed before TMEM is released
+        if (leader) {
             ptx::umma_commit(ptx::smem_u32(&sb->drain));
             (void)ptx::mbar_wait(ptx::smem_u32(&sb->drain), 0);
         }
