@@ -43,6 +43,28 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
         }                                           \
     } while (0)
 
+// A kernel launched with launch_dependent may start while the kernel before it in the stream is still running, once all of
+// that kernel's blocks have called grid_dep_launch() or ended; grid_dep_wait() returns when it has completed and its
+// writes are visible (at once in a kernel launched the usual way).
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                                    const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // Multiprocessor count of the current device (cached per device).
 int sm_count();
 
@@ -230,7 +252,10 @@ __device__ __forceinline__ void load_row_starts(const int64_t* __restrict__ gl, 
         }
         if (lane == 0) row_start[0] = 0;
         bad_at = __reduce_min_sync(0xffffffffu, bad_at);
-        if (lane == 0 && bad_at < G) report_status(status, kDevBadGroupList, bad_at);
+        if (lane == 0 && bad_at < G) {
+            grid_dep_wait();  // the kernel before this one may still have to zero the status words
+            report_status(status, kDevBadGroupList, bad_at);
+        }
     }
     __syncthreads();
 }

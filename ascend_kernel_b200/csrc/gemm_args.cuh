@@ -21,8 +21,8 @@ struct GemmArgs {
     long long dst_rows = 0;
 };
 
-// out[m] = sum_k x[m, k] in fp32 for the rows the group list uses (grouped_gemm.cu).
+// out[m] = sum_k x[m, k] in fp32 for the rows the group list uses, and status words 0 .. 3 zeroed (grouped_gemm.cu).
 void launch_rowsum(const void* x, float* out, int64_t M, int64_t K, const int64_t* group_list, int64_t G, int gl_type,
-                   cudaStream_t stream);
+                   int* status, cudaStream_t stream);
 
 }  // namespace b200moe

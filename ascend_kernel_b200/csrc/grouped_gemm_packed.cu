@@ -708,7 +708,8 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
     const size_t need = b200moe_grouped_gemm_workspace_bytes(M, K, N, G, B200MOE_CT_INT8, B200MOE_LAYOUT_CANONICAL);
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200MOE_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
+    // (the row sums' kernel zeroes the status words itself)
+    if (offset == nullptr || x_rowsum != nullptr) B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
     GemmArgs a;
     a.scale = scale;
     a.offset = nullptr;
@@ -734,7 +735,7 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
             a.rowsum = x_rowsum;  // the caller already has the fp32 sums of the rows of x (e.g. from the row gather)
         } else {
             float* rowsum = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES);
-            launch_rowsum(x, rowsum, M, K, group_list, G, group_list_type, s);
+            launch_rowsum(x, rowsum, M, K, group_list, G, group_list_type, a.status, s);
             B200MOE_CUDA_TRY(cudaGetLastError());
             a.rowsum = rowsum;
         }
