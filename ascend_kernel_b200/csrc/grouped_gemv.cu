@@ -1,15 +1,17 @@
 // Grouped GEMV for decode-sized expert batches (HBM-bandwidth kernel).
 //
-// Work item = (non-empty expert, slab of 256 output columns); persistent CTAs (two per SM) draw
-// items from a ticket counter, experts with the most rows first, the slabs of an expert next to one another.  The expert's x rows (up to 4 per pass) are copied to shared memory
-// once per item.  Every warp streams its share of the k rows straight from global memory with
+// Work unit = (up to 4 rows of a non-empty expert, slab of 256 output columns, part of the k range);
+// persistent CTAs (two per SM) draw units from a ticket counter, experts with the most rows first, the
+// passes of a slab next to one another (their weights are then read from L2), then the slabs.  K is cut
+// into parts only when whole columns would leave the chip idle (gv_choose_parts); the parts' fp32 sums meet
+// in the workspace and the CTA that finishes a slab last adds them up in a fixed order.  The unit's x
+// rows are copied to shared memory first.  Every warp streams its share of the k rows straight from global memory with
 // 128-bit coalesced loads, eight row pairs (8 x 512 B per warp) in flight before the first is
 // consumed, decodes the packed weights in registers (byte / nibble unpack, no shared-memory
 // staging of weights) and accumulates in fp32 with packed two-wide FMAs.  The 16 half-warp
 // partial sums per column are combined with one shuffle and one pass through shared memory;
 // scale and offset are applied in the fp32 epilogue and the result is rounded to bf16 once.
-// Experts with more than 4 rows are processed 4 rows at a time (the weight slab is then re-read
-// from L2).  int8 items with 2..4 rows, fp8 items and fp4 items use the tensor core for the multiply-adds
+// int8 items with 2..4 rows, fp8 items and fp4 items use the tensor core for the multiply-adds
 // (gv_compute_mma, gv_compute_fp4_mma); fp4 falls back to fp32 FMAs for x rows that are not exact in f16.
 #include <cuda_fp16.h>
 
@@ -42,6 +44,23 @@ struct GemvArgs {
     int fp4_stored;  // fp4 weights in the reference's pre-shuffled order, read in place
     const __half* x16;  // fp4: x as scaled f16 and the rows' exponents (gv_fp4_prepare_x_kernel), or null: fp32 path only
     const int* xexp;
+    unsigned* part_count;  // [kGvMaxParts] finished parts of a slab, zero at the launch
+    float* part_sums;      // [kGvMaxParts][kGvSlotFloats]
+    int* ticket;           // status word 2 (the fp32 kernel of fp4: 3, from 1 on)
+    int by_rows;           // experts in the order of their row counts: shared memory has room for the order
+};
+
+// Split of the k range: parts are multiples of kGvPartRows rows, at most kGvMaxParts of them per launch (four waves of
+// two CTAs on 148 SMs; 4.9 MB of partial sums), each with the sums of 4 rows x 256 columns and of the x rows.
+constexpr int kGvPartRows = 128;
+constexpr int kGvMaxParts = 1184;
+constexpr int kGvSlotFloats = kGvRows * kGvSlabN + 16;
+
+struct GvUnit {
+    int g, r0, rows, n0;  // expert, first row, rows (1 .. kGvRows), first column
+    int k0, k1;           // its part of the k range
+    int split, n_split;
+    int slot;             // first slot of the slab's parts; also its counter
 };
 
 typedef unsigned long long f32x2;  // two packed fp32 (sm_100 two-wide FP32 instructions)
@@ -147,10 +166,71 @@ __device__ __forceinline__ void gv_decode(const uint4& q, f32x2 (&w)[8], const f
     }
 }
 
+// Takes the CTA's next ticket when the weights of a unit are through: its latency then runs beside the sums.  (Drawn
+// earlier, a CTA would sit on a unit while others are idle at the end of the launch.)
+__device__ __forceinline__ void gv_draw(const GemvArgs& a, int& next) {
+    if (threadIdx.x == 0) next = atomicAdd(a.ticket, 1);
+}
+
+// End of a unit: v[m] is the thread's column (threadIdx.x of the slab) of row m summed over the unit's part of k.
+// A slab in one part is stored at once.  Otherwise the sums go to the part's slot and the CTA that arrives last adds
+// the parts in their order, so the result does not depend on which one that is.
+template <int MODE>
+__device__ __forceinline__ void gv_finish(const GemvArgs& a, GvUnit& u, const float* xsum, const int* xexp,
+                                          float (&v)[kGvRows]) {
+    const int t = threadIdx.x, n = u.n0 + t;
+    float xs[kGvRows];
+#pragma unroll
+    for (int m = 0; m < kGvRows; ++m) xs[m] = (MODE == B200MOE_CT_INT8) ? xsum[m] : 0.f;
+    if (u.n_split > 1) {
+        float* slot = a.part_sums + (size_t)(u.slot + u.split) * kGvSlotFloats;
+#pragma unroll
+        for (int m = 0; m < kGvRows; ++m)
+            if (m < u.rows) {
+                __stcg(slot + m * kGvSlabN + t, v[m]);
+                if (MODE == B200MOE_CT_INT8 && t == 0) __stcg(slot + kGvRows * kGvSlabN + m, xs[m]);
+            }
+        __threadfence();
+        __syncthreads();
+        if (t == 0) u.split = atomicAdd(a.part_count + u.slot, 1u) == (unsigned)(u.n_split - 1) ? -1 : 0;  // (no longer needed)
+        __syncthreads();
+        if (u.split != -1) return;
+        __threadfence();
+        const float* first = a.part_sums + (size_t)u.slot * kGvSlotFloats;
+#pragma unroll
+        for (int m = 0; m < kGvRows; ++m) {
+            if (m < u.rows) {
+                v[m] = 0.f;
+                xs[m] = 0.f;
+                for (int p = 0; p < u.n_split; ++p) {
+                    v[m] += __ldcg(first + (size_t)p * kGvSlotFloats + m * kGvSlabN + t);
+                    if (MODE == B200MOE_CT_INT8) xs[m] += __ldcg(first + (size_t)p * kGvSlotFloats + kGvRows * kGvSlabN + m);
+                }
+            }
+        }
+    }
+    if (n >= a.N) return;  // (fp8 only: the upper half of a 128-column last slab)
+    float s_n = 1.f, so_n = 0.f;
+    if constexpr (MODE == B200MOE_CT_INT8) {
+        s_n = __bfloat162float(static_cast<const __nv_bfloat16*>(a.scale)[(size_t)u.g * a.N + n]);
+        if (a.offset != nullptr) so_n = s_n * __bfloat162float(a.offset[(size_t)u.g * a.N + n]);
+    }
+#pragma unroll
+    for (int m = 0; m < kGvRows; ++m) {
+        if (m < u.rows) {
+            float o = v[m];
+            if constexpr (MODE == B200MOE_CT_INT8) o = fmaf(so_n, xs[m], s_n * o);
+            if (xexp != nullptr) o = scalbnf(o, xexp[m]);
+            a.y[(size_t)(u.r0 + m) * a.N + n] = __float2bfloat16_rn(o);
+        }
+    }
+}
+
 template <int MODE, int MB>
-__device__ __forceinline__ void gv_compute(const GemvArgs& a, const __nv_bfloat16* xs, const float* xsum, float* red,
-                                           int g, int r0, int rows_valid, int n0) {
+__device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs, const float* xsum,
+                                           float* red, int& next) {
     using T = GvTraits<MODE>;
+    const int g = un.g, n0 = un.n0, k_begin = un.k0, k_end = un.k1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, l16 = lane & 15;
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
@@ -173,12 +253,12 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, const __nv_bfloat1
     const uint8_t* pf_base = a.weight + (size_t)g * a.K * row_bytes + n0 + 128 * (lane & 1);
     auto prefetch_step = [&](int k) {
         if constexpr (!T::kNibbles) {
-            if (k + (lane >> 1) < a.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t)(k + (lane >> 1)) * row_bytes));
+            if (k + (lane >> 1) < k_end) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t)(k + (lane >> 1)) * row_bytes));
         }
     };
 #pragma unroll
-    for (int i = 0; i < kGvL2Steps; ++i) prefetch_step(warp * kGvWarpRows + i * kGvIterRows);
-    for (int k0 = warp * kGvWarpRows; k0 < a.K; k0 += kGvIterRows) {
+    for (int i = 0; i < kGvL2Steps; ++i) prefetch_step(k_begin + warp * kGvWarpRows + i * kGvIterRows);
+    for (int k0 = k_begin + warp * kGvWarpRows; k0 < k_end; k0 += kGvIterRows) {
         prefetch_step(k0 + kGvL2Steps * kGvIterRows);
         // ---- issue all loads of this step first ----
         uint4 q[kGvUnroll];
@@ -281,27 +361,18 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, const __nv_bfloat1
             for (int c = 0; c < 4; ++c) dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
         }
     }
+    gv_draw(a, next);
     __syncthreads();
-    {
-        const int t = threadIdx.x;  // column inside the slab
-        const int n = n0 + t;
-        float s_n = 1.f, so_n = 0.f;
-        if constexpr (MODE == B200MOE_CT_INT8) {
-            s_n = __bfloat162float(static_cast<const __nv_bfloat16*>(a.scale)[(size_t)g * a.N + n]);
-            if (a.offset != nullptr) so_n = s_n * __bfloat162float(a.offset[(size_t)g * a.N + n]);
-        }
+    float v[kGvRows];
 #pragma unroll
-        for (int m = 0; m < MB; ++m) {
-            if (m < rows_valid) {
-                float v = 0.f;
+    for (int m = 0; m < kGvRows; ++m) {
+        v[m] = 0.f;
+        if (m < un.rows) {
 #pragma unroll
-                for (int w = 0; w < kGvWarps; ++w) v += red[(w * kGvRows + m) * kGvSlabN + t];
-                if constexpr (MODE == B200MOE_CT_INT8) v = fmaf(so_n, xsum[m], s_n * v);
-                a.y[(size_t)(r0 + m) * a.N + n] = __float2bfloat16_rn(v);
-            }
+            for (int w = 0; w < kGvWarps; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    __syncthreads();
+    gv_finish<MODE>(a, un, xsum, nullptr, v);
 }
 
 // ---- 2..4 rows per expert, int8: the multiply-adds go to the tensor core ---------------------
@@ -334,8 +405,9 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 // high bytes of the two 16-bit lanes and decoded by bit placement (exact in bf16); the fp32 scale of
 // the 128 x 128 block, uniform for a warp over a 128-row stretch, multiplies the stretch's partial sums.
 template <int MODE>
-__device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, const __nv_bfloat16* xs, const float* xsum, float* red,
-                                               int g_expert, int r0, int rows_valid, int n0) {
+__device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs,
+                                               const float* xsum, float* red, int& next) {
+    const int g_expert = un.g, rows_valid = un.rows, n0 = un.n0, k_begin = un.k0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int hc = warp & 1, kg = warp >> 1;  // column half of the slab, k group
@@ -357,7 +429,7 @@ __device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, const __nv_bfl
 
     constexpr int kStepRows = 16 * kGvMmaParts;  // k rows the CTA consumes per step
     // (fp8 accepts N % 256 == 128: in the last slab the warps of the second column half have no columns)
-    const int k_end = (n0 + 128 * hc < a.N) ? a.K : 0;
+    const int k1 = un.k1, k_end = (n0 + 128 * hc < a.N) ? k1 : 0;
     // two steps (2 x 16 rows of the warp's 128-byte row segment) per iteration: one line per lane into L2,
     // kGvL2Steps / 2 iterations ahead
     const uint8_t* pf_base = a.weight + (size_t)g_expert * a.K * row_bytes + n0 + 128 * hc;
@@ -366,10 +438,10 @@ __device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, const __nv_bfl
         if (kk < k_end) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t)kk * row_bytes));
     };
 #pragma unroll
-    for (int i = 0; i < kGvL2Steps / 2; ++i) prefetch_iter(kg * 16 + i * 2 * kStepRows);
-    for (int k0 = kg * 16; k0 < k_end; k0 += 2 * kStepRows) {
+    for (int i = 0; i < kGvL2Steps / 2; ++i) prefetch_iter(k_begin + kg * 16 + i * 2 * kStepRows);
+    for (int k0 = k_begin + kg * 16; k0 < k_end; k0 += 2 * kStepRows) {
         prefetch_iter(k0 + (kGvL2Steps / 2) * 2 * kStepRows);
-        const bool second = k0 + kStepRows < a.K;
+        const bool second = k0 + kStepRows < k1;
         float sf = 1.f;
         if constexpr (kBlockScale)  // k0 and k0 + 64 lie in the same 128-row block (K % 128 == 0)
             sf = __ldg(static_cast<const float*>(a.scale) + ((size_t)g_expert * (a.K >> 7) + (k0 >> 7)) * (a.N >> 7) +
@@ -442,27 +514,18 @@ __device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, const __nv_bfl
             }
         }
     }
+    gv_draw(a, next);
     __syncthreads();
-    {
-        const int tc = threadIdx.x;  // column inside the slab
-        const int n = n0 + tc;
-        float s_n = 1.f, so_n = 0.f;
-        if constexpr (MODE == B200MOE_CT_INT8) {
-            s_n = __bfloat162float(static_cast<const __nv_bfloat16*>(a.scale)[(size_t)g_expert * a.N + n]);
-            if (a.offset != nullptr) so_n = s_n * __bfloat162float(a.offset[(size_t)g_expert * a.N + n]);
-        }
+    float v[kGvRows];
 #pragma unroll
-        for (int m = 0; m < kGvRows; ++m) {
-            if (m < rows_valid && n < a.N) {
-                float v = 0.f;
+    for (int m = 0; m < kGvRows; ++m) {
+        v[m] = 0.f;
+        if (m < un.rows) {
 #pragma unroll
-                for (int w = 0; w < kGvMmaParts; ++w) v += red[(w * kGvRows + m) * kGvSlabN + tc];
-                if constexpr (MODE == B200MOE_CT_INT8) v = fmaf(so_n, xsum[m], s_n * v);
-                a.y[(size_t)(r0 + m) * a.N + n] = __float2bfloat16_rn(v);
-            }
+            for (int w = 0; w < kGvMmaParts; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    __syncthreads();
+    gv_finish<MODE>(a, un, xsum, nullptr, v);
 }
 
 // ---- fp4 weights in the reference's stored (pre-shuffled) order, read in place -----------------
@@ -474,8 +537,9 @@ __device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, const __nv_bfl
 // multiplies the fp32 sum of its 16 products (x * e2m1 is exact in fp32) instead of every weight.
 // No conversion pass over the weights.
 template <int MB>
-__device__ __forceinline__ void gv_compute_fp4_stored(const GemvArgs& a, const __nv_bfloat16* xs, float* red, int g,
-                                                      int r0, int rows_valid, int n0) {
+__device__ __forceinline__ void gv_compute_fp4_stored(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs,
+                                                      float* red, int& next) {
+    const int g = un.g, n0 = un.n0, k_begin = un.k0, k_end = un.k1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int J = a.N >> 8, j = n0 >> 8, p = lane >> 2, q = lane & 3;
     const uint8_t* wbase = a.weight + (size_t)g * a.K * ((size_t)a.N >> 1) + (size_t)j * 128 + q * 32;
@@ -488,7 +552,7 @@ __device__ __forceinline__ void gv_compute_fp4_stored(const GemvArgs& a, const _
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[m][c] = 0ull;
 
-    for (int k0 = warp * 16; k0 < a.K; k0 += kGvWarps * 16) {
+    for (int k0 = k_begin + warp * 16; k0 < k_end; k0 += kGvWarps * 16) {
         const int R = k0 >> 6, aa = (k0 >> 4) & 3;
         uint4 wq[4];  // [2b + h]: rows k0 + 8b + 4h .. + 3
 #pragma unroll
@@ -553,20 +617,18 @@ __device__ __forceinline__ void gv_compute_fp4_stored(const GemvArgs& a, const _
         dst[0] = make_float4(v[0], v[1], v[2], v[3]);
         dst[1] = make_float4(v[4], v[5], v[6], v[7]);
     }
+    gv_draw(a, next);
     __syncthreads();
-    {
-        const int t = threadIdx.x;
+    float v[kGvRows];
 #pragma unroll
-        for (int m = 0; m < MB; ++m) {
-            if (m < rows_valid) {
-                float v = 0.f;
+    for (int m = 0; m < kGvRows; ++m) {
+        v[m] = 0.f;
+        if (m < un.rows) {
 #pragma unroll
-                for (int w = 0; w < kGvWarps; ++w) v += red[(w * kGvRows + m) * kGvSlabN + t];
-                a.y[(size_t)(r0 + m) * a.N + n0 + t] = __float2bfloat16_rn(v);
-            }
+            for (int w = 0; w < kGvWarps; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    __syncthreads();
+    gv_finish<B200MOE_CT_FP4>(a, un, nullptr, nullptr, v);
 }
 
 
@@ -608,8 +670,9 @@ constexpr int kGvFp4Ahead = 4;  // steps whose loads are in flight per warp (6: 
 constexpr int kGvFp4L2Ahead = 1;  // batches of kGvFp4Ahead steps requested into L2 before their loads are issued
 
 template <bool kStored>
-__device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __half* xs, const int* xexp, float* red,
-                                                   int g_expert, int r0, int rows_valid, int n0) {
+__device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, GvUnit& un, const __half* xs, const int* xexp,
+                                                   float* red, int& next) {
+    const int g_expert = un.g, rows_valid = un.rows, n0 = un.n0, k_begin = un.k0, k_end = un.k1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int hc = warp & 1, kg = warp >> 1;  // column half of the slab, k group
@@ -660,7 +723,7 @@ __device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __ha
     // lines.  The register loads, issued up to kGvFp4L2Ahead batches later, then wait for L2, not for DRAM.
     auto prefetch_group = [&](int k0) {
         const int h = lane >> 3, k = k0 + h * kStepRows;
-        if (k >= a.K) return;
+        if (k >= k_end) return;
         const uint8_t* w;
         if constexpr (kStored) {
             const int R = k >> 6, aa = (k >> 4) & 3, i = (lane >> 2) & 1, b = (lane >> 1) & 1, gq = lane & 1;
@@ -714,9 +777,9 @@ __device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __ha
         }
     };
     constexpr int kBatchRows = kGvFp4Ahead * kStepRows;
-    int k0 = kg * 16;
+    int k0 = k_begin + kg * 16;
     int k_pf = k0;  // first step not yet requested into L2 (requests go out four steps at a time)
-    for (; k0 + (kGvFp4Ahead - 1) * kStepRows < a.K; k0 += kBatchRows) {
+    for (; k0 + (kGvFp4Ahead - 1) * kStepRows < k_end; k0 += kBatchRows) {
         uint2 q[kGvFp4Ahead][4];
         for (; k_pf < k0 + kGvFp4L2Ahead * kBatchRows; k_pf += 4 * kStepRows) prefetch_group(k_pf);
 #pragma unroll
@@ -724,7 +787,7 @@ __device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __ha
 #pragma unroll
         for (int h = 0; h < kGvFp4Ahead; ++h) compute(k0 + h * kStepRows, q[h]);
     }
-    for (; k0 < a.K; k0 += kStepRows) {
+    for (; k0 < k_end; k0 += kStepRows) {
         uint2 q1[4];
         load(k0, q1);
         compute(k0, q1);
@@ -742,20 +805,18 @@ __device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __ha
             }
         }
     }
+    gv_draw(a, next);
     __syncthreads();
-    {
-        const int tc = threadIdx.x;  // column inside the slab
+    float v[kGvRows];
 #pragma unroll
-        for (int m = 0; m < kGvRows; ++m) {
-            if (m < rows_valid) {
-                float v = 0.f;
+    for (int m = 0; m < kGvRows; ++m) {
+        v[m] = 0.f;
+        if (m < un.rows) {
 #pragma unroll
-                for (int w = 0; w < kGvMmaParts; ++w) v += red[(w * kGvRows + m) * kGvSlabN + tc];
-                a.y[(size_t)(r0 + m) * a.N + n0 + tc] = __float2bfloat16_rn(scalbnf(v, xexp[m]));
-            }
+            for (int w = 0; w < kGvMmaParts; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    __syncthreads();
+    gv_finish<B200MOE_CT_FP4>(a, un, nullptr, xexp, v);
 }
 
 // fp4 prepass, one CTA per x row: the row as f16, times 2^-e with e chosen so that its largest element lies in
@@ -763,8 +824,10 @@ __device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, const __ha
 // than about 2^-32 below the row's largest, a bf16 subnormal, an infinity or a NaN): such rows take the fp32 path.
 constexpr int kGvNotF16 = -(1 << 30);
 
+// A row of the second kind also raises status word 3, the ticket of the fp32 kernel, from 0 (nothing to do) to 1.
 __global__ void __launch_bounds__(256) gv_fp4_prepare_x_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ x16,
-                                                               int* __restrict__ xexp, int K) {
+                                                               int* __restrict__ xexp, int K, int* __restrict__ status) {
+    grid_dep_launch();
     __shared__ int s_max, s_bad;
     const size_t row = blockIdx.x;
     const uint32_t* src = reinterpret_cast<const uint32_t*>(x + row * K);
@@ -809,70 +872,143 @@ __global__ void __launch_bounds__(256) gv_fp4_prepare_x_kernel(const __nv_bfloat
     }
     if (bad) atomicOr(&s_bad, 1);
     __syncthreads();
-    if (threadIdx.x == 0) xexp[row] = s_bad ? kGvNotF16 : sh;
+    if (threadIdx.x == 0) {
+        xexp[row] = s_bad ? kGvNotF16 : sh;
+        if (s_bad) atomicMax(status + 3, 1);
+    }
+}
+
+// Clears what a call starts from: status words 0 .. 3 and the counters of the k parts (words 4, 5 are the caller's).
+__global__ void __launch_bounds__(256) gv_begin_kernel(int* __restrict__ status, unsigned* __restrict__ part_count) {
+    grid_dep_launch();
+    if (threadIdx.x < 4) status[threadIdx.x] = 0;
+    for (int i = threadIdx.x; i < kGvMaxParts; i += blockDim.x) part_count[i] = 0u;
+}
+
+// Parts a slab's k range is cut into, for `slabs` (rows x slab) units on `ctas` CTAs; called by a whole warp, lane i
+// weighs i + 1 parts: waves of CTAs times the blocks of kGvPartRows rows of a part plus kGvPartCost, what a unit costs
+// beyond its weights (x staging, first loads, the sums' way through L2) in blocks.  A launch of many waves has nothing
+// to gain and stays whole.  One token on 8 of 256 experts, 7168 x 4096 fp8 (128 slabs, two parts): 117 -> 72 us = 3.3
+// TB/s; 3 tokens x 4 over 160 experts, 4224 x 3328 int8: 54.6 -> 53.3 us.
+constexpr int kGvPartCost = 2;
+__device__ __forceinline__ int gv_choose_parts(int slabs, int ctas, int K) {
+    const int blocks = (K + kGvPartRows - 1) / kGvPartRows;
+    const int s = (threadIdx.x & 31) + 1, per = (blocks + s - 1) / s;
+    unsigned cost = 0xFFFFFFFFu;
+    if (s == 1 || ((long long)slabs * s <= kGvMaxParts && per > 1 && (blocks + per - 1) / per == s))
+        cost = min((unsigned)((slabs * (long long)s + ctas - 1) / ctas) * (unsigned)(per + kGvPartCost), 0x03FFFFFFu) * 32u + (unsigned)(s - 1);
+    return (int)(__reduce_min_sync(0xffffffffu, cost) & 31u) + 1;
 }
 
 // fp4 is launched as two kernels over the same work items: PATH 1 takes the passes whose x rows are all exact as
 // scaled f16 (tensor-core path), PATH 2 the others (fp32 multiply-adds; normally none, and the kernel leaves after
 // walking the item list); PATH 0: every other mode, and fp4 without the prepass.  Separate kernels keep the
-// registers of one path from weighing on the other.
+// registers of one path from weighing on the other.  PATH 2 leaves at once when the prepass found no such row.
 template <int MODE, int PATH = 0>
 __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     int* row_start = reinterpret_cast<int*>(smem_raw);
-    int* active = row_start + (a.G + 1);
-    int* n_active_p = active + a.G;
-    uintptr_t p = (reinterpret_cast<uintptr_t>(n_active_p + 1) + 15) & ~uintptr_t(15);
-    float* xsum = reinterpret_cast<float*>(p);                                   // [4]
-    float* red = xsum + 4;                                                        // [8][4][256]
+    int* pass_start = row_start + (a.G + 1);  // [G + 1] passes (of up to 4 rows) before the i-th expert in order
+    int* order = pass_start + (a.G + 1);      // [G], with by_rows
+    uintptr_t p = (reinterpret_cast<uintptr_t>(order + (a.by_rows ? a.G : 0)) + 15) & ~uintptr_t(15);
+    float* red = reinterpret_cast<float*>(p);                                     // [8][4][256]
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(red + kGvWarps * kGvRows * kGvSlabN);  // [4][K]
+    float* xsum = reinterpret_cast<float*>(xs + a.K);  // [4], in the pad behind the first row
+    int* xexp = reinterpret_cast<int*>(xsum + kGvRows);  // [4], the other half of it
+    static_assert(kGvXPad * sizeof(__nv_bfloat16) == 2 * kGvRows * sizeof(float), "pad of a staged row");
 
+    if (PATH == 2) {
+        grid_dep_wait();
+        if (*reinterpret_cast<volatile int*>(a.status + 3) == 0) return;
+    }
+    __shared__ GvUnit un;
+    __shared__ int s_ticket;
+    const int n_slabs = (a.N + kGvSlabN - 1) / kGvSlabN;
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
     if (threadIdx.x < 32) {
-        // non-empty experts, those with the most rows first (counting sort on min(rows, 5)): with
-        // the ticket counter below the long items start early and the short ones fill the tail
-        int lo, hi, n = 0;
+        int lo, hi, mine = 0, total;
         lane_experts(a.G, lo, hi);
-        for (int b = 5; b >= 1; --b) {
-            int mine = 0, total;
-            for (int g = lo; g < hi; ++g) mine += min(row_start[g + 1] - row_start[g], 5) == b;
-            int at = n + warp_exclusive_sum(mine, total);
-            if (total > 0)
-                for (int g = lo; g < hi; ++g)
-                    if (min(row_start[g + 1] - row_start[g], 5) == b) active[at++] = g;
-            n += total;
+        if (a.by_rows) {
+            // counting sort on min(rows, 5), the most rows first: units of the same number of rows run together (the
+            // row count picks the code path) and the long ones start early.  32 tokens x 8 over 256 experts,
+            // 7168 x 4096 int8: 3 % slower in the experts' own order.
+            int n = 0;
+            for (int b = 5; b >= 0; --b) {
+                int same = 0, all;
+                for (int g = lo; g < hi; ++g) same += min(row_start[g + 1] - row_start[g], 5) == b;
+                int to = n + warp_exclusive_sum(same, all);
+                if (all > 0)
+                    for (int g = lo; g < hi; ++g)
+                        if (min(row_start[g + 1] - row_start[g], 5) == b) order[to++] = g;
+                n += all;
+            }
+            __syncwarp();
         }
-        if (threadIdx.x == 0) *n_active_p = n;
+        auto passes_of = [&](int i) {
+            const int g = a.by_rows ? order[i] : i;
+            return (row_start[g + 1] - row_start[g] + kGvRows - 1) / kGvRows;
+        };
+        for (int i = lo; i < hi; ++i) mine += passes_of(i);
+        int at = warp_exclusive_sum(mine, total);
+        for (int i = lo; i < hi; ++i) {
+            pass_start[i] = at;
+            at += passes_of(i);
+        }
+        if (threadIdx.x == 0) pass_start[a.G] = total;
+        const int parts = gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K);
+        if (threadIdx.x == 0) un.n_split = parts;
     }
     __syncthreads();
 
-    const int n_slabs = (a.N + kGvSlabN - 1) / kGvSlabN;
-    const int n_act = *n_active_p;
-    const int n_items = n_act * n_slabs;
-    const int kvec = a.K / 8;  // 16-byte vectors per x row
-    int* ticket = a.status + (PATH == 2 ? 3 : 2);  // zeroed by the host before the launch
-    __shared__ int s_item;
-    __shared__ int xexp[kGvRows];
+    grid_dep_wait();  // (the prologue above ran beside the kernel that zeroes the tickets and counters)
+    const int n_parts = un.n_split;
+    const unsigned per_pass = (unsigned)(n_slabs * n_parts);  // units of one pass
+    // (32 bits hold every unit number: y alone would take 2 TB with 2^30 units)
+    const unsigned n_units = (unsigned)pass_start[a.G] * per_pass;
+    const int part_rows = ((a.K + kGvPartRows - 1) / kGvPartRows + n_parts - 1) / n_parts * kGvPartRows;
+    int next = 0;  // thread 0: the ticket drawn last
+    gv_draw(a, next);
     for (;;) {
+        if (threadIdx.x == 0) s_ticket = next;
         __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1);
+        const unsigned unit = (unsigned)(s_ticket - (PATH == 2 ? 1 : 0));
+        if (unit >= n_units) break;
+        // every thread looks at its experts, the one that finds the unit describes it to the others: a binary search
+        // with its divisions by one thread was a tenth of a short unit (2048 rows of fp4)
+        for (int i = threadIdx.x; i < a.G; i += kGvThreads) {
+            const unsigned first = (unsigned)pass_start[i] * per_pass, passes = (unsigned)(pass_start[i + 1] - pass_start[i]);
+            if (unit < first || unit - first >= passes * per_pass) continue;
+            const int g = a.by_rows ? order[i] : i;
+            // expert-major order: the CTAs that run at the same time hold neighbouring slabs of the same experts
+            // and walk the same k rows together, so whole rows of the weight matrix are fetched close in time
+            // (DRAM pages stay open: measured +1..6 % over slab-major order); the passes of a slab are
+            // adjacent, so all but the first find its weights in L2
+            const unsigned j = (unit - first) / passes, pass = (unit - first) - j * passes;
+            const int split = (int)(j / (unsigned)n_slabs), slab = (int)j - split * n_slabs;
+            un.g = g;
+            un.n0 = slab * kGvSlabN;
+            un.r0 = row_start[g] + (int)pass * kGvRows;
+            un.rows = min(kGvRows, row_start[g + 1] - un.r0);
+            un.split = split;
+            un.n_split = n_parts;
+            un.slot = n_parts > 1 ? ((pass_start[i] + (int)pass) * n_slabs + slab) * n_parts : 0;
+            un.k0 = split * part_rows;
+            un.k1 = min(un.k0 + part_rows, a.K);
+        }
         __syncthreads();
-        const int item = s_item;
-        if (item >= n_items) break;
-        // expert-major order: the CTAs that run at the same time hold neighbouring slabs of the same experts and
-        // walk the same k rows together, so whole rows of the weight matrix are fetched close in time (DRAM
-        // pages stay open: measured +1..6 % over slab-major order); the experts with the most rows still come first
-        const int g = active[item / n_slabs];
-        const int n0 = (item % n_slabs) * kGvSlabN;
-        const int r0 = row_start[g], r1 = row_start[g + 1];
-        for (int r = r0; r < r1; r += kGvRows) {
-            const int rows = min(kGvRows, r1 - r);
+        {
+            // (copies: the stores of the staging loop could alias the descriptor)
+            const int r = un.r0, rows = un.rows, v0 = un.k0 / 8, v1 = un.k1 / 8;
             // fp4: the tensor-core path when every row of the pass is exact as scaled f16 (prepared by the prepass)
             bool fp4_mma = false;
             if constexpr (PATH != 0) {
                 fp4_mma = true;
                 for (int m = 0; m < rows; ++m) fp4_mma = fp4_mma && a.xexp[r + m] != kGvNotF16;
-                if (fp4_mma != (PATH == 1)) continue;  // the other kernel's pass
+                if (fp4_mma != (PATH == 1)) {  // the other kernel's pass
+                    gv_draw(a, next);
+                    __syncthreads();
+                    continue;
+                }
                 if (fp4_mma && threadIdx.x < rows) xexp[threadIdx.x] = a.xexp[r + threadIdx.x];
             }
             // ---- stage the x rows (and their sums, for the offset term) ----
@@ -883,7 +1019,8 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
                                            : reinterpret_cast<const uint4*>(a.x + (size_t)(r + m) * a.K);
                 uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)m * (a.K + kGvXPad));
                 float s = 0.f;
-                for (int i = threadIdx.x; i < kvec; i += kGvThreads) {
+#pragma unroll 4
+                for (int i = v0 + threadIdx.x; i < v1; i += kGvThreads) {
                     const uint4 v = __ldg(src + i);
                     dst[i] = v;
                     if (MODE == B200MOE_CT_INT8 && a.offset != nullptr) {
@@ -902,37 +1039,47 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             // fp8: the tensor-core path also wins with one row (its decode is two-wide); int8 with one
             // row is faster on the scalar path; fp4 takes the tensor-core path whenever x is exact in f16
             if constexpr (PATH == 1) {
-                if (a.fp4_stored) gv_compute_fp4_mma<true>(a, reinterpret_cast<const __half*>(xs), xexp, red, g, r, rows, n0);
-                else gv_compute_fp4_mma<false>(a, reinterpret_cast<const __half*>(xs), xexp, red, g, r, rows, n0);
+                if (a.fp4_stored) gv_compute_fp4_mma<true>(a, un, reinterpret_cast<const __half*>(xs), xexp, red, next);
+                else gv_compute_fp4_mma<false>(a, un, reinterpret_cast<const __half*>(xs), xexp, red, next);
             } else if (MODE == B200MOE_CT_FP4 && a.fp4_stored) {
-                if (rows == 1) gv_compute_fp4_stored<1>(a, xs, red, g, r, rows, n0);
-                else if (rows == 2) gv_compute_fp4_stored<2>(a, xs, red, g, r, rows, n0);
-                else gv_compute_fp4_stored<4>(a, xs, red, g, r, rows, n0);
-            } else if constexpr (MODE == B200MOE_CT_FP8) gv_compute_mma<MODE>(a, xs, xsum, red, g, r, rows, n0);
-            else if (rows == 1) gv_compute<MODE, 1>(a, xs, xsum, red, g, r, rows, n0);
-            else if constexpr (MODE == B200MOE_CT_INT8) gv_compute_mma<MODE>(a, xs, xsum, red, g, r, rows, n0);
-            else if (rows == 2) gv_compute<MODE, 2>(a, xs, xsum, red, g, r, rows, n0);
-            else gv_compute<MODE, 4>(a, xs, xsum, red, g, r, rows, n0);
+                if (rows == 1) gv_compute_fp4_stored<1>(a, un, xs, red, next);
+                else if (rows == 2) gv_compute_fp4_stored<2>(a, un, xs, red, next);
+                else gv_compute_fp4_stored<4>(a, un, xs, red, next);
+            } else if constexpr (MODE == B200MOE_CT_FP8) gv_compute_mma<MODE>(a, un, xs, xsum, red, next);
+            else if (rows == 1) gv_compute<MODE, 1>(a, un, xs, xsum, red, next);
+            else if constexpr (MODE == B200MOE_CT_INT8) gv_compute_mma<MODE>(a, un, xs, xsum, red, next);
+            else if (rows == 2) gv_compute<MODE, 2>(a, un, xs, xsum, red, next);
+            else gv_compute<MODE, 4>(a, un, xs, xsum, red, next);
         }
     }
 }
 
-static size_t gv_smem_bytes(int G, int K) {
-    size_t b = sizeof(int) * (size_t)(2 * G + 2) + 16;
-    b += sizeof(float) * (4 + kGvWarps * kGvRows * kGvSlabN);
-    b += (size_t)kGvRows * (K + kGvXPad) * 2;
+static size_t gv_smem_bytes(int G, int K, bool by_rows) {
+    size_t b = (sizeof(int) * (size_t)((by_rows ? 3 : 2) * G + 2) + 15) & ~size_t(15);
+    b += sizeof(float) * kGvWarps * kGvRows * kGvSlabN;
+    b += ((size_t)kGvRows * K + (kGvRows - 1) * kGvXPad) * 2;
     return b;
 }
 
 template <int MODE, int PATH = 0>
-static int gv_launch(const GemvArgs& a, cudaStream_t stream) {
-    const size_t smem = gv_smem_bytes(a.G, a.K);
+static int gv_launch(const GemvArgs& a0, cudaStream_t stream) {
+    GemvArgs a = a0;
+    a.ticket = a.status + (PATH == 2 ? 3 : 2);
+    size_t smem = gv_smem_bytes(a.G, a.K, true);
+    // (the order must not cost the second CTA of a multiprocessor, nor a shape that fits without it)
+    a.by_rows = smem <= 110 * 1024 || (smem <= 226 * 1024 && gv_smem_bytes(a.G, a.K, false) > 110 * 1024);
+    if (!a.by_rows) smem = gv_smem_bytes(a.G, a.K, false);
     if (smem > 227 * 1024) return B200MOE_ERR_SHAPE;
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemv_kernel<MODE, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
     const int per_sm = smem <= 110 * 1024 ? 2 : 1;
-    grouped_gemv_kernel<MODE, PATH><<<per_sm * sm_count(), kGvThreads, smem, stream>>>(a);
-    B200MOE_CUDA_TRY(cudaGetLastError());
+    // (behind gv_begin_kernel or the fp4 prepass; the fp32 kernel of fp4 stays behind the tensor-core one)
+    if (PATH != 2) {
+        B200MOE_CUDA_TRY(launch_dependent(grouped_gemv_kernel<MODE, PATH>, (unsigned)(per_sm * sm_count()), kGvThreads, smem, stream, a));
+    } else {
+        grouped_gemv_kernel<MODE, PATH><<<per_sm * sm_count(), kGvThreads, smem, stream>>>(a);
+        B200MOE_CUDA_TRY(cudaGetLastError());
+    }
     return B200MOE_OK;
 }
 
@@ -940,13 +1087,17 @@ static int gv_launch(const GemvArgs& a, cudaStream_t stream) {
 
 using namespace b200moe;
 
+constexpr size_t kGvCountBytes = (kGvMaxParts * sizeof(unsigned) + 255) / 256 * 256;
+constexpr size_t kGvPartBytes = kGvCountBytes + kGvMaxParts * sizeof(float) * kGvSlotFloats;
+static_assert(kGvPartBytes % 256 == 0, "what follows stays aligned");
 static size_t gv_fp4_exp_bytes(int64_t M) { return ((size_t)M * sizeof(int) + 255) / 256 * 256; }
 
 extern "C" size_t b200moe_grouped_gemv_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
                                                        int weight_layout) {
     (void)N; (void)G; (void)weight_layout;
-    // status words and the work-item ticket; fp4 adds the rows' exponents and x as scaled f16
-    size_t b = B200MOE_STATUS_BYTES;
+    // status words and the work-unit ticket, counters and sums of the k parts; fp4 adds the rows' exponents and x as
+    // scaled f16
+    size_t b = B200MOE_STATUS_BYTES + kGvPartBytes;
     if (compute_type == B200MOE_CT_FP4 && M > 0 && K > 0) b += gv_fp4_exp_bytes(M) + (size_t)M * (size_t)K * 2;
     return b;
 }
@@ -977,7 +1128,6 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200MOE_ERR_WORKSPACE;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
     GemvArgs a;
     a.x = static_cast<const __nv_bfloat16*>(x);
     a.weight = static_cast<const uint8_t*>(weight);
@@ -988,6 +1138,12 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     a.M = (int)M; a.K = (int)K; a.N = (int)N; a.G = (int)G;
     a.gl_type = group_list_type;
     a.status = static_cast<int*>(workspace);
+    uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
+    a.part_count = reinterpret_cast<unsigned*>(ws);
+    a.part_sums = reinterpret_cast<float*>(ws + kGvCountBytes);
+    ws += kGvPartBytes;
+    gv_begin_kernel<<<1, 256, 0, s>>>(a.status, a.part_count);
+    B200MOE_CUDA_TRY(cudaGetLastError());
 
     // fp4 in the stored (pre-shuffled) order is read in place
     a.fp4_stored = (compute_type == B200MOE_CT_FP4 && weight_layout == B200MOE_LAYOUT_ASCEND) ? 1 : 0;
@@ -996,10 +1152,10 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     // (B200MOE_GEMV_FP4_SCALAR=1 keeps fp4 on the fp32 multiply-adds: comparison runs)
     static const bool fp4_scalar = [] { const char* e = getenv("B200MOE_GEMV_FP4_SCALAR"); return e && e[0] == '1'; }();
     if (compute_type == B200MOE_CT_FP4 && !fp4_scalar) {
-        uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
         a.xexp = reinterpret_cast<const int*>(ws);
         a.x16 = reinterpret_cast<const __half*>(ws + gv_fp4_exp_bytes(M));
-        gv_fp4_prepare_x_kernel<<<(unsigned)M, 256, 0, s>>>(a.x, const_cast<__half*>(a.x16), const_cast<int*>(a.xexp), a.K);
+        gv_fp4_prepare_x_kernel<<<(unsigned)M, 256, 0, s>>>(a.x, const_cast<__half*>(a.x16), const_cast<int*>(a.xexp), a.K,
+                                                                a.status);
         B200MOE_CUDA_TRY(cudaGetLastError());
     }
     switch (compute_type) {

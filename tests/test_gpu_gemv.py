@@ -184,3 +184,46 @@ def test_int4_per_group_scales_match_oracle(counts, K, N, with_offset):
     out, st = run_gemv(x, w, scale, cnt, "int4", offset, gl_type=1)
     assert st == (0, 0)
     assert_close_to_golden(out, gold)
+
+
+@pytest.mark.parametrize("ct,counts,K,N", [
+    ("int8", [1, 0, 6, 3], 1088, 512),    # a last part of 64 + 256 rows, one- and two-pass experts, offsets
+    ("int8", [1], 7168, 256),             # a single slab: as many parts as there can be
+    ("int8", [2] * 33, 512, 1024),        # 132 slabs: two parts, near a full wave
+    ("fp8", [1, 4, 0, 5], 1152, 384),     # 9 blocks of 128 rows, a last slab of 128 columns
+    ("int4", [3, 1], 896, 256),
+    ("fp4", [1, 4, 0, 5, 2], 1088, 512),
+    ("fp4_inexact", [1, 4, 0, 5, 2], 1088, 512),  # parts of the tensor-core and of the fp32 kernel in one call
+])
+def test_k_range_in_parts_matches_oracle(ct, counts, K, N):
+    """Few units of work: the k range is cut into parts whose fp32 sums meet in the workspace, with the same
+    bits whichever part arrives last."""
+    import ascend_kernel_b200 as ak
+
+    gen = torch.Generator().manual_seed(57)
+    G, cnt = len(counts), torch.tensor(counts, dtype=torch.int64)
+    offset, layout, ulps = None, "canonical", 2.0
+    if ct == "int8":
+        x, w, scale, offset, cnt = _int8_case(counts, K, N, 57, True)
+        ulps = 1.0
+    elif ct == "fp8":
+        x = torch.randn(int(cnt.sum()), K, generator=gen).to(torch.bfloat16)
+        w = torch.randint(0, 256, (G, K, N), generator=gen, dtype=torch.uint8)
+        scale = torch.randn(G, K // 128, N // 128, generator=gen)
+    elif ct == "int4":
+        x = torch.randn(int(cnt.sum()), K, generator=gen).to(torch.bfloat16)
+        w = torch.randint(0, 256, (G, K, N // 2), generator=gen, dtype=torch.uint8).view(torch.int8)
+        scale = (torch.rand(G, K // 128, N, generator=gen) * 0.045 + 0.005).to(torch.bfloat16)
+    else:
+        x, w, scale, cnt = _fp4_case(counts, K, N, 57)
+        if ct == "fp4_inexact":
+            x[1, 5], x[7, K - 1] = 2.0 ** -100, 2.0 ** -90
+        ct = "fp4"
+    gold = O.golden_f32(x, w, scale, offset, cnt, ct, O.GROUP_LIST_COUNTS, weight_layout=layout, gemv=True)
+    for lay in ("canonical", "ascend") if ct == "fp4" else (layout,):
+        wd = ak.fp4_layout(w.cuda(), to_ascend=True).cpu() if lay == "ascend" else w
+        out, st = run_gemv(x, wd, scale, cnt, ct, offset, gl_type=1, layout=lay)
+        assert st == (0, 0)
+        assert_close_to_golden(out, gold, ulps=ulps)
+        again, _ = run_gemv(x, wd, scale, cnt, ct, offset, gl_type=1, layout=lay)
+        assert torch.equal(out.view(torch.int16), again.view(torch.int16))
