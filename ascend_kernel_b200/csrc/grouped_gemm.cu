@@ -438,7 +438,12 @@ __device__ __forceinline__ void convert_stage_fp4_ascend(const PackedRegs<kCtFp4
 
 template <int MODE>
 __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_t sa) {
-    const float sf = (MODE == B200MOE_CT_FP8) ? r.sf : 1.f;
+    float sf = (MODE == B200MOE_CT_FP8) ? r.sf : 1.f;
+    bool in_scale = false;
+    if constexpr (MODE == B200MOE_CT_FP8) {
+        in_scale = __all_sync(0xffffffffu, fabsf(sf) < 128.f);
+        if (in_scale) sf *= 1.329227995784916e36f;  // 2^120
+    }
     const f32x2 sf2 = pack_f32x2(sf, sf);
 #pragma unroll
     for (int j = 0; j < kDqRows; ++j) {
@@ -451,20 +456,23 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
             s8x4_to_bf16_even_odd(q.z, o[4], o[5]);
             s8x4_to_bf16_even_odd(q.w, o[6], o[7]);
         } else if constexpr (MODE == B200MOE_CT_FP8) {
-            // e4m3 byte -> bf16 with the 4 exponent and 3 mantissa bits placed under the bf16 exponent
-            // (exact after * 2^120, subnormals included), two values per instruction; widened to fp32,
-            // scaled with the block's fp32 scale and rounded once to bf16.
+            // e4m3 byte -> bf16 with the 4 exponent and 3 mantissa bits placed under the bf16 exponent (the value
+            // times 2^-120, subnormals included), bytes 1, 3 and 0, 2 of a word at a time; widened to fp32, scaled
+            // with the block's fp32 scale and rounded once to bf16.  The 2^120 is in the scale where that holds
+            // it (sf2 = scale * 2^120; the product of the two is the same number), else it is a multiply of its own.
             const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-#pragma unroll
-                for (int hp = 0; hp < 2; ++hp) {
-                    const uint32_t t = prmt(w4[i], 0u, hp == 0 ? 0x1404u : 0x3424u);
-                    const uint32_t xb = ((t >> 4) & 0x07F007F0u) | (t & 0x80008000u);
-                    const uint32_t yb = mul_bf16x2(xb, 0x7B807B80u);  // * 2^120
-                    const f32x2 f = mul_f32x2(pack_u32x2(yb << 16, yb & 0xFFFF0000u), sf2);
-                    o[2 * i + hp] = pack_bf16x2(f32x2_lo(f), f32x2_hi(f));
+                uint32_t odd = ((w4[i] >> 4) & 0x07F007F0u) | (w4[i] & 0x80008000u);
+                uint32_t even = ((w4[i] << 4) & 0x07F007F0u) | ((w4[i] << 8) & 0x80008000u);
+                if (!in_scale) {
+                    odd = mul_bf16x2(odd, 0x7B807B80u);  // * 2^120
+                    even = mul_bf16x2(even, 0x7B807B80u);
                 }
+                const f32x2 lo = mul_f32x2(pack_u32x2(even << 16, odd << 16), sf2);
+                const f32x2 hi = mul_f32x2(pack_u32x2(even & 0xFFFF0000u, odd & 0xFFFF0000u), sf2);
+                o[2 * i] = pack_bf16x2(f32x2_lo(lo), f32x2_hi(lo));
+                o[2 * i + 1] = pack_bf16x2(f32x2_lo(hi), f32x2_hi(hi));
             }
         } else if constexpr (MODE == kCtFp4E8m0) {
             // 2^(s-127) as bf16: exponent field s; s = 0 is the subnormal 2^-127, 255 is NaN

@@ -186,3 +186,30 @@ def test_fp4_e8m0_gemm_equals_dequant_then_bf16_gemm(counts, K, N, all_scales):
     ops.grouped_gemm_fp4_e8m0(x, codes, scale, cnt.cumsum(0), act, gate_up_silu=True)
     assert same_bits(act[:sum(counts)], ak.silu_mul(want)[:sum(counts)])
     assert (act[sum(counts):] == 7.0).all()
+
+
+@pytest.mark.parametrize("scales", [(0.5, -127.5), (128.0, 0.25), (-3.0e5, 2.0e-3), (1.0e-40, 1.0e-30)])
+def test_fp8_gemm_equals_dequant_then_bf16_gemm_for_scales_of_any_size(scales):
+    """The decode's power of two rides in the block scale where that can hold it (below 128) and is multiplied on its
+    own elsewhere; blocks of both kinds side by side, subnormal scales, all 256 codes."""
+    import ascend_kernel_b200 as ak
+
+    gen = torch.Generator().manual_seed(61)
+    G, K, N = 2, 256, 384
+    w = torch.randint(0, 256, (G, K, N), generator=gen, dtype=torch.uint8)
+    w[0, 0, :256] = torch.arange(256, dtype=torch.uint8)
+    s = torch.tensor(scales)[torch.randint(0, 2, (G, K // 128, N // 128), generator=gen)] * torch.rand(G, K // 128, N // 128, generator=gen)
+    s[0, 0, 0], s[0, 0, 1], s[1, 0, 0] = scales[0], scales[1], scales[1]
+    x = torch.randn(200, K, generator=gen).to(torch.bfloat16).cuda()
+    cnt = torch.tensor([137, 60]).cuda()
+    wd = torch.empty(G, K, N, dtype=torch.bfloat16, device="cuda")
+    ak.fp8_dequant(w.cuda(), s.cuda(), wd)
+    # (the bf16 GEMM takes whole 256-column tiles)
+    wide = torch.zeros(G, K, 512, dtype=torch.bfloat16, device="cuda")
+    wide[:, :, :N] = wd
+    want = torch.zeros(200, 512, dtype=torch.bfloat16, device="cuda")
+    ak.grouped_gemm(x, wide, None, None, cnt, "bf16", want, group_list_type=1)
+    got = torch.zeros(200, N, dtype=torch.bfloat16, device="cuda")
+    ak.grouped_gemm(x, w.cuda(), s.cuda(), None, cnt, "fp8", got, group_list_type=1)
+    torch.cuda.synchronize()
+    assert same_bits(got, want[:, :N])
