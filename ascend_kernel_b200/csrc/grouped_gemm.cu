@@ -365,7 +365,7 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
     if constexpr (MODE == B200MOE_CT_INT4) {
         uint32_t v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(it.wp + (size_t)i * row_bytes));
+        for (int i = 0; i < 8; ++i) v[i] = ldg_stream4(it.wp + (size_t)i * row_bytes);
         r.q[0] = make_uint4(v[0], v[1], v[2], v[3]);
         r.q[1] = make_uint4(v[4], v[5], v[6], v[7]);
         // in units of the 8 scales a thread loads (fits 32 bits: the weights would be 17 TB otherwise)
@@ -379,7 +379,7 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
             const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
             r.q[j] = make_uint4(v.x, v.y, 0u, 0u);
         } else if (MODE != B200MOE_CT_FP8 || it.n0 + d.c16 * 16 < a.N) {
-            r.q[j] = __ldg(reinterpret_cast<const uint4*>(p));
+            r.q[j] = MODE == B200MOE_CT_FP8 ? ldg_stream(p) : __ldg(reinterpret_cast<const uint4*>(p));
         } else {
             r.q[j] = make_uint4(0u, 0u, 0u, 0u);  // columns past N in the 128-column last tile of an fp8 matrix
         }
