@@ -227,3 +227,47 @@ def test_k_range_in_parts_matches_oracle(ct, counts, K, N):
         assert_close_to_golden(out, gold, ulps=ulps)
         again, _ = run_gemv(x, wd, scale, cnt, ct, offset, gl_type=1, layout=lay)
         assert torch.equal(out.view(torch.int16), again.view(torch.int16))
+
+
+@pytest.mark.parametrize("op,ct", [("gemm", "int8"), ("gemv", "int8"), ("gemv", "fp4")])
+def test_dependent_launches_in_a_captured_graph(op, ct):
+    """The kernels that start beside the one before them (int8 GEMM behind its row sums, GEMV behind the clearing of its
+    counters) in a CUDA graph: three calls in a row, replayed on new inputs, against the same calls made eagerly."""
+    import ascend_kernel_b200 as ak
+
+    if ct == "int8":
+        x, w, scale, offset, cnt = _int8_case([3, 0, 2, 40 if op == "gemm" else 7], 1088, 512, 71, True)
+    else:
+        x, w, scale, cnt = _fp4_case([3, 0, 2, 7], 1088, 512, 71)
+        offset = None
+    xs = [x.cuda(), (x * 0.5).cuda(), (x * -3).cuda()]
+    w, scale, cnt = w.cuda(), scale.cuda(), cnt.cuda()
+    offset = None if offset is None else offset.cuda()
+
+    def call(xi, out):
+        if op == "gemm":
+            ak.grouped_gemm(xi, w, scale, offset, cnt, ct, out, group_list_type=1, weight_layout="canonical")
+        else:
+            ak.grouped_soft_gemv(xi, w, scale, cnt, ct, out, group_list_type=1, weight_layout="canonical", offset=offset)
+
+    outs = [torch.zeros(x.shape[0], 512, dtype=torch.bfloat16, device="cuda") for _ in xs]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for xi, o in zip(xs, outs):  # warm-up on the capture stream: its workspace exists before the capture
+            call(xi, o)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        for xi, o in zip(xs, outs):
+            call(xi, o)
+    for xi in xs:
+        xi.copy_(xi.flip(1))
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for xi, o in zip(xs, outs):
+        want = torch.zeros_like(o)
+        call(xi, want)
+        torch.cuda.synchronize()
+        assert torch.equal(o.view(torch.int16), want.view(torch.int16))
+    assert ak.last_status() == (0, 0)
