@@ -180,7 +180,7 @@ void GroupedSoftGemv(at::Tensor x, at::Tensor weight, at::Tensor scale, at::Tens
     }
     c10::cuda::CUDAGuard guard(x.device());
     auto stream = c10::cuda::getCurrentCUDAStream();
-    const size_t ws_bytes = b200moe_grouped_gemv_workspace_bytes(d.M, d.K, d.N, d.G, ct, layout);
+    const size_t ws_bytes = b200moe_grouped_gemv_split_workspace_bytes(d.M, d.K, d.N, d.G, ct, layout);
     at::Tensor ws = workspace_for(x, ws_bytes, stream.stream());
     raise_on(b200moe_grouped_gemv(x.data_ptr(), weight.data_ptr(), scale.data_ptr(), offset,
                                   groupList.data_ptr<int64_t>(), output.data_ptr(), d.M, d.K, d.N, d.G, ct,

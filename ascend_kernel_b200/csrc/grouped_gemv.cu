@@ -44,7 +44,7 @@ struct GemvArgs {
     int fp4_stored;  // fp4 weights in the reference's pre-shuffled order, read in place
     const __half* x16;  // fp4: x as scaled f16 and the rows' exponents (gv_fp4_prepare_x_kernel), or null: fp32 path only
     const int* xexp;
-    unsigned* part_count;  // [kGvMaxParts] finished parts of a slab, zero at the launch
+    unsigned* part_count;  // [kGvMaxParts] finished parts of a slab, zero at the launch; null: k is not split
     float* part_sums;      // [kGvMaxParts][kGvSlotFloats]
     int* ticket;           // status word 2 (the fp32 kernel of fp4: 3, from 1 on)
     int by_rows;           // experts in the order of their row counts: shared memory has room for the order
@@ -875,7 +875,8 @@ __global__ void __launch_bounds__(256) gv_fp4_prepare_x_kernel(const __nv_bfloat
 __global__ void __launch_bounds__(256) gv_begin_kernel(int* __restrict__ status, unsigned* __restrict__ part_count) {
     grid_dep_launch();
     if (threadIdx.x < 4) status[threadIdx.x] = 0;
-    for (int i = threadIdx.x; i < kGvMaxParts; i += blockDim.x) part_count[i] = 0u;
+    if (part_count != nullptr)
+        for (int i = threadIdx.x; i < kGvMaxParts; i += blockDim.x) part_count[i] = 0u;
 }
 
 // Parts a slab's k range is cut into, for `slabs` (rows x slab) units on `ctas` CTAs; called by a whole warp, lane i
@@ -948,7 +949,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             at += passes_of(i);
         }
         if (threadIdx.x == 0) pass_start[a.G] = total;
-        const int parts = gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K);
+        const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K);
         if (threadIdx.x == 0) un.n_split = parts;
     }
     __syncthreads();
@@ -1088,11 +1089,18 @@ static size_t gv_fp4_exp_bytes(int64_t M) { return ((size_t)M * sizeof(int) + 25
 extern "C" size_t b200moe_grouped_gemv_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
                                                        int weight_layout) {
     (void)N; (void)G; (void)weight_layout;
-    // status words and the work-unit ticket, counters and sums of the k parts; fp4 adds the rows' exponents and x as
-    // scaled f16
-    size_t b = B200MOE_STATUS_BYTES + kGvPartBytes;
+    // status words and the work-unit tickets; fp4 adds the rows' exponents and x as scaled f16
+    size_t b = B200MOE_STATUS_BYTES;
     if (compute_type == B200MOE_CT_FP4 && M > 0 && K > 0) b += gv_fp4_exp_bytes(M) + (size_t)M * (size_t)K * 2;
     return b;
+}
+
+// ... and, behind that, the counters and sums of the k parts.
+static size_t gv_parts_offset(size_t base) { return (base + 255) / 256 * 256; }
+
+extern "C" size_t b200moe_grouped_gemv_split_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
+                                                             int weight_layout) {
+    return gv_parts_offset(b200moe_grouped_gemv_workspace_bytes(M, K, N, G, compute_type, weight_layout)) + kGvPartBytes;
 }
 
 extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const void* scale, const void* offset,
@@ -1132,9 +1140,13 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     a.gl_type = group_list_type;
     a.status = static_cast<int*>(workspace);
     uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
-    a.part_count = reinterpret_cast<unsigned*>(ws);
-    a.part_sums = reinterpret_cast<float*>(ws + kGvCountBytes);
-    ws += kGvPartBytes;
+    a.part_count = nullptr;
+    a.part_sums = nullptr;
+    if (workspace_bytes >= gv_parts_offset(need) + kGvPartBytes) {
+        uint8_t* parts = static_cast<uint8_t*>(workspace) + gv_parts_offset(need);
+        a.part_count = reinterpret_cast<unsigned*>(parts);
+        a.part_sums = reinterpret_cast<float*>(parts + kGvCountBytes);
+    }
     gv_begin_kernel<<<1, 256, 0, s>>>(a.status, a.part_count);
     B200MOE_CUDA_TRY(cudaGetLastError());
 

@@ -329,7 +329,7 @@ def grouped_soft_gemv(x, weight, scale, groupList, computeType, output, group_li
         if ct not in (CT["int8"], CT["int4"]):
             raise RuntimeError("offset is only defined for int8 / int4")
         _check_scale(offset, ct, G, K, N, "offset")
-    ws = _run(_lib.b200moe_grouped_gemv, _lib.b200moe_grouped_gemv_workspace_bytes, "grouped_soft_gemv", x, weight,
+    ws = _run(_lib.b200moe_grouped_gemv, _lib.b200moe_grouped_gemv_split_workspace_bytes, "grouped_soft_gemv", x, weight,
               scale, offset, groupList, output, ct, group_list_type, LAYOUT[weight_layout], M, K, N, G)
     if M > 0:
         _count(1)

@@ -208,6 +208,11 @@ int b200moe_grouped_gemv(const void* x, const void* weight, const void* scale, c
                          int compute_type, int group_list_type, int weight_layout, void* workspace,
                          size_t workspace_bytes, void* stream);
 
+/* The workspace with which calls of few rows also split the k range over the multiprocessors (4.9 MB more, for the
+ * parts' fp32 sums; one token on 8 of 256 experts, 7168 x 4096 fp8: 117 -> 72 us).  b200moe_grouped_gemv takes any
+ * size from b200moe_grouped_gemv_workspace_bytes on and splits from this one on. */
+size_t b200moe_grouped_gemv_split_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
+                                                  int weight_layout);
 size_t b200moe_grouped_gemv_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
                                             int weight_layout);
 

@@ -119,3 +119,14 @@ def test_install_check_lists_the_reference_operators():
             chk.check(verbose=False)
     finally:
         chk.ADDED_OPS.pop()
+
+
+def test_gemv_split_workspace_comes_on_top_of_the_plain_one():
+    """Counters (1184 words, padded to 256 bytes) and sums (4 rows x 256 columns + 16 words each) of the k parts, behind
+    the plain workspace rounded up to 256 bytes."""
+    lib = _lib().lib
+    parts = (1184 * 4 + 255) // 256 * 256 + 1184 * (4 * 256 + 16) * 4
+    for ct in (0, 1, 2, 3):
+        for M, K in ((1, 128), (8, 256), (37, 2048)):
+            plain = lib.b200moe_grouped_gemv_workspace_bytes(M, K, 512, 4, ct, 0)
+            assert lib.b200moe_grouped_gemv_split_workspace_bytes(M, K, 512, 4, ct, 0) == (plain + 255) // 256 * 256 + parts

@@ -271,3 +271,28 @@ def test_dependent_launches_in_a_captured_graph(op, ct):
         torch.cuda.synchronize()
         assert torch.equal(o.view(torch.int16), want.view(torch.int16))
     assert ak.last_status() == (0, 0)
+
+
+@pytest.mark.parametrize("ct,counts", [("int8", [1, 6]), ("fp4", [1, 4, 2])])
+def test_plain_workspace_runs_without_splitting(ct, counts):
+    """A caller with the smaller workspace gets the same results, the k range in one piece."""
+    import ascend_kernel_b200 as ak
+    from ascend_kernel_b200 import _abi
+
+    if ct == "int8":
+        x, w, scale, offset, cnt = _int8_case(counts, 1088, 512, 83, True)
+    else:
+        (x, w, scale, cnt), offset = _fp4_case(counts, 1088, 512, 83), None
+    gold = O.golden_f32(x, w, scale, offset, cnt, ct, O.GROUP_LIST_COUNTS, weight_layout="canonical", gemv=True)
+    d = [t.cuda() if t is not None else None for t in (x, w, scale, offset, cnt)]
+    M, K, N, G = x.shape[0], 1088, 512, len(counts)
+    need = _abi.lib.b200moe_grouped_gemv_workspace_bytes(M, K, N, G, _abi.CT[ct], 0)
+    ws = torch.full((need + 256,), 0x5A, dtype=torch.uint8, device="cuda")   # nothing past `need` may be touched
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+    ptr = [None if t is None else t.data_ptr() for t in d]
+    rc = _abi.lib.b200moe_grouped_gemv(ptr[0], ptr[1], ptr[2], ptr[3], ptr[4], out.data_ptr(), M, K, N, G, _abi.CT[ct], 1, 0,
+                                       ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and ak.read_status(ws) == (0, 0)
+    assert bool((ws[need:] == 0x5A).all())
+    assert_close_to_golden(out, gold, ulps=1.0 if ct == "int8" else 2.0)
