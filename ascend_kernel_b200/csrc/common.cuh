@@ -155,15 +155,19 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
 // mantissa MSB); read as bf16 that is value * 2^-126 including the subnormal code 0.5, so one
 // exact multiply by 2^126 yields the e2m1 value.  Codes i and i+4 sit 16 bits apart and share
 // one bf16x2 lane pair, which makes the sign and magnitude moves two shifts and two logic ops.
-__device__ __forceinline__ void e2m1x8_to_bf16(uint32_t w, uint32_t out[4]) {
+// e2m1x8_to_bf16_pairs leaves them that way: out[i] = elements (i, i + 4).
+__device__ __forceinline__ void e2m1x8_to_bf16_pairs(uint32_t w, uint32_t out[4]) {
     constexpr uint32_t kTwo126 = 0x7E807E80u;
-    uint32_t r[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint32_t m = (i < 2) ? (w << (6 - 4 * i)) : (w >> (4 * i - 6));
         const uint32_t s = w << (12 - 4 * i);
-        r[i] = mul_bf16x2((m & 0x01C001C0u) | (s & 0x80008000u), kTwo126);
+        out[i] = mul_bf16x2((m & 0x01C001C0u) | (s & 0x80008000u), kTwo126);
     }
+}
+__device__ __forceinline__ void e2m1x8_to_bf16(uint32_t w, uint32_t out[4]) {
+    uint32_t r[4];
+    e2m1x8_to_bf16_pairs(w, r);
     out[0] = prmt(r[0], r[1], 0x5410);
     out[1] = prmt(r[2], r[3], 0x5410);
     out[2] = prmt(r[0], r[1], 0x7632);

@@ -54,7 +54,7 @@ constexpr int kSuperRows = 8;  // m-tiles per L2 super-tile
 // stages, those lead the MMAs by the ring depth, the epilogue trails by at most two tiles; with one
 // stage per tile that is kL2Ahead + kNS + 2 tiles.
 constexpr int kTileRing = 32;
-constexpr int kBarrierBytes = 512;  // shared memory reserved for GmBarriers
+constexpr int kBarrierBytes = 1024;  // shared memory reserved for GmBarriers
 constexpr int kEpiScaleFloats = 2 * kBN;  // per epilogue warp: the tile's column scales and scale * offset
 constexpr int kAHalfBytes = kBM * kBK * 2;   // one 128-row box
 constexpr int kATileBytes = 2 * kAHalfBytes;  // an x stage holds both row halves
@@ -96,6 +96,9 @@ struct GmTraits {
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
+    // who resolves a published tile number: the publisher, or (fp8, whose dequant loop spills otherwise and took 6.24
+    // instead of 5.88 ms for 8192 tokens x 8 over 256 experts, 7168 x 4096) each role for itself
+    static constexpr bool kResolved = MODE != B200MOE_CT_FP8;
     static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
 };
 
@@ -111,13 +114,16 @@ struct GmBarriers {
     int n_tiles;
     int pad;
     // Tile schedule of this CTA: tiles are drawn from a global ticket counter (status word 2) by the
-    // thread that runs furthest ahead and published here, entry i % kTileRing = (i + 1) << 32 | tile.
-    // Every role walks the entries in order, so all see the same sequence.
-    unsigned long long tile_ring[kTileRing];
+    // thread that runs furthest ahead, resolved by it and published here, entry i % kTileRing = {i + 1, first row,
+    // expert | rows << 16 (rows 0: the schedule has ended), first column}, written and read as one aligned
+    // 16-byte vector.  Every role walks the entries in order, so all see the same sequence, and none
+    // repeats the search and the divisions at each tile switch (64 experts, 210 rows each, 1280 x 512, int4: 74 -> 48 us).
+    uint4 tile_ring[kTileRing];
 };
 
 struct TileInfo {
-    int g, row0, row_end, n0;
+    int g, row0, n0;
+    int rows;    // of the expert inside the tile, 1 .. kTileM
     int halves;  // 1: at most 128 rows in the tile, 2: more
 };
 
@@ -145,34 +151,34 @@ __device__ __forceinline__ bool gm_wait(uint64_t* bar, uint32_t parity, GmBarrie
     return gm_wait_slow(b, parity, sb, status, id);
 }
 
-// tile index -> expert, first row, row bound, first column.  tile_prefix has G+1 entries.
-// The seq-th tile of this CTA (seq counts from 0 and is advanced), or n_tiles when the schedule has
-// ended, a wait expired or another role aborted.  The publisher is always far ahead, so outside the
-// first microseconds of the kernel the entry is already there.
-__device__ __forceinline__ int next_tile(GmBarriers* sb, uint32_t& seq, int n_tiles, int* status) {
-    const volatile unsigned long long* e = &sb->tile_ring[seq % kTileRing];
-    const uint32_t want = seq + 1;
-    unsigned long long v = *e;
-    if ((uint32_t)(v >> 32) != want) {
-        volatile int* abort = &sb->abort;
-        const uint64_t t0 = ptx::globaltimer_ns();
-        uint32_t spins = 0;
-        while ((uint32_t)((v = *e) >> 32) != want) {
-            if ((++spins & 0xFF) == 0) {
-                if (*abort) return n_tiles;
-                if (ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) {
-                    *abort = 1;
-                    report_status(status, kDevWaitExpired, 90);
-                    return n_tiles;
-                }
+__device__ __forceinline__ uint4 ring_load(const uint4* e) {
+    uint4 v;
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(ptx::smem_u32(e)));
+    return v;
+}
+
+// Waits for entry `e` to carry the sequence number `want`; an entry of no rows when a wait expired or another role aborted.
+__device__ __noinline__ uint4 ring_wait(const uint4* e, uint32_t want, GmBarriers* sb, int* status) {
+    volatile int* abort = &sb->abort;
+    const uint64_t t0 = ptx::globaltimer_ns();
+    uint32_t spins = 0;
+    uint4 v;
+    while ((v = ring_load(e)).x != want) {
+        if ((++spins & 0xFF) == 0) {
+            if (*abort) return make_uint4(want, 0u, 0u, 0u);
+            if (ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) {
+                *abort = 1;
+                report_status(status, kDevWaitExpired, 90);
+                return make_uint4(want, 0u, 0u, 0u);
             }
         }
     }
-    ++seq;
-    const int t = (int)(uint32_t)v;
-    return t < n_tiles ? t : n_tiles;
+    return v;
 }
 
+// tile index -> expert, first row, rows, first column.
 // Tile numbering: first every tile with two row halves (more than 128 rows), expert by expert in
 // super-tiles, then every tile with one row half (the last, short m-tile of an expert).  tile_prefix
 // holds two prefix arrays of G + 1 entries each: two-half tiles before expert g, one-half tiles
@@ -193,7 +199,6 @@ __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, c
     const int r0 = row_start[g], r1 = row_start[g + 1];
     TileInfo ti;
     ti.g = g;
-    ti.row_end = r1;
     if (two) {
         const int mt = (pref[g + 1] - pref[g]) / n_nt;
         // super-tiles of up to kSuperRows m-tiles x all n-tiles keep x rows and the expert's weights
@@ -211,7 +216,31 @@ __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, c
         ti.row0 = r0 + ((r1 - r0) / kTileM) * kTileM;
         ti.halves = 1;
     }
+    ti.rows = min(r1 - ti.row0, kTileM);
     return ti;
+}
+
+// The seq-th tile of this CTA (seq counts from 0 and is advanced) into `ti`; false when the schedule has
+// ended, a wait expired or another role aborted.  The publisher is always far ahead, so outside the
+// first microseconds of the kernel the entry is already there.
+template <bool RESOLVED>
+__device__ __forceinline__ bool next_tile(GmBarriers* sb, uint32_t& seq, TileInfo& ti, const int* tile_prefix, const int* row_start,
+                                          int G, int n_nt, int* status) {
+    const uint4* e = &sb->tile_ring[seq % kTileRing];
+    uint4 v = ring_load(e);
+    if (v.x != seq + 1) v = ring_wait(e, seq + 1, sb, status);
+    ++seq;
+    if constexpr (!RESOLVED) {
+        if (v.z == 0u) return false;
+        ti = locate_tile((int)v.y, tile_prefix, row_start, G, n_nt);
+        return true;
+    }
+    ti.row0 = (int)v.y;
+    ti.g = (int)(v.z & 0xFFFFu);
+    ti.rows = (int)(v.z >> 16);
+    ti.n0 = (int)v.w;
+    ti.halves = ti.rows > kBM ? 2 : 1;
+    return ti.rows != 0;
 }
 
 // Row boundaries and the tile-count prefixes of locate_tile, by the whole CTA (a barrier must follow).  Not inlined:
@@ -303,7 +332,7 @@ struct PackedRegs {
 // Position of a dequant thread in the (tile, k-stage) sequence of its CTA, with the address of the
 // thread's first packed row of that stage carried along (advanced by a constant inside a tile).
 struct DqIter {
-    int t, kt, g, n0;
+    int kt, g, n0;
     uint32_t seq;  // tiles taken from the CTA's schedule so far
     bool valid;
     const uint8_t* wp;
@@ -315,24 +344,18 @@ __device__ __forceinline__ int chunk_col(int n0, int c16, int N) {
     return SPLIT ? (n0 >> 1) + (c16 & 7) * 16 + (c16 >> 3) * (N >> 1) : n0 + c16 * 16;
 }
 template <int MODE, bool SPLIT>
-__device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict__ w, const GemmArgs& a, const DqLane& d,
-                                          int n_tiles, const int* tile_prefix, const int* row_start, int n_nt) {
+__device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict__ w, const GemmArgs& a, const DqLane& d) {
     using T = GmTraits<MODE>;
-    it.valid = it.t < n_tiles;
     if (!it.valid) return;
-    const TileInfo ti = locate_tile(it.t, tile_prefix, row_start, a.G, n_nt);
-    it.g = ti.g;
-    it.n0 = ti.n0;
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
-    it.wp = w + ((size_t)ti.g * a.K + (size_t)it.kt * kBK + d.row) * row_bytes +
-            (T::kEightRows        ? (ti.n0 >> 1) + d.src_byte
-             : T::kNibbles        ? chunk_col<SPLIT>(ti.n0, d.c16, a.N) >> 1
-                                  : ti.n0 + d.c16 * 16);
+    it.wp = w + ((size_t)it.g * a.K + (size_t)it.kt * kBK + d.row) * row_bytes +
+            (T::kEightRows        ? (it.n0 >> 1) + d.src_byte
+             : T::kNibbles        ? chunk_col<SPLIT>(it.n0, d.c16, a.N) >> 1
+                                  : it.n0 + d.c16 * 16);
 }
 template <int MODE, bool SPLIT>
 __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* __restrict__ w, const GemmArgs& a,
-                                           const DqLane& d, int n_kt, int n_tiles, const int* tile_prefix,
-                                           const int* row_start, int n_nt, GmBarriers* sb) {
+                                           const DqLane& d, int n_kt, const int* tile_prefix, const int* row_start, int n_nt, GmBarriers* sb) {
     using T = GmTraits<MODE>;
     it.kt += step;
     if (it.kt < n_kt) {
@@ -341,9 +364,12 @@ __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* 
     }
     do {
         it.kt -= n_kt;
-        it.t = next_tile(sb, it.seq, n_tiles, a.status);
-    } while (it.kt >= n_kt && it.t < n_tiles);
-    dq_locate<MODE, SPLIT>(it, w, a, d, n_tiles, tile_prefix, row_start, n_nt);
+        TileInfo ti;
+        it.valid = next_tile<T::kResolved>(sb, it.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
+        it.g = ti.g;
+        it.n0 = ti.n0;
+    } while (it.kt >= n_kt && it.valid);
+    dq_locate<MODE, SPLIT>(it, w, a, d);
 }
 
 constexpr int kScaleAhead = 6;  // stages by which the e8m0 scale lines are requested into L2
@@ -422,15 +448,25 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, ui
 // the pair is at the returned address ^ 16.
 __device__ __forceinline__ uint32_t dq_row_addr(uint32_t sa, int j) { return (sa ^ (uint32_t)(j << 5)) + (uint32_t)(j * 256); }
 
+// Stored-order fp4 and fp4 with e8m0 scales enter the tile in the column order (0,4,1,5,2,6,3,7) of every eight, the order
+// in which the decode produces them (e2m1x8_to_bf16_pairs); the epilogue undoes it when it picks accumulator
+// registers.  Restoring the order here cost four permutes per eight codes (with resolved tiles, fp4-stored layer of 256
+// experts, 4096 tokens x 8, 7168 x 2048: 4.79 -> 4.61 ms).  The scales of eight columns are
+// brought into the same order, once for all rows of the scale group (the canonical order's 16 columns a thread
+// leave no registers for that).
+__device__ __forceinline__ uint4 pair_scales(const uint4& s) {
+    return make_uint4(prmt(s.x, s.z, 0x5410u), prmt(s.x, s.z, 0x7632u), prmt(s.y, s.w, 0x5410u), prmt(s.y, s.w, 0x7632u));
+}
+
 // Stored-order fp4: eight rows of eight columns; `sa` is the shared address of the thread's chunk in
 // its first row (a multiple of 8, so row i flips the chunk's swizzle bits by i and adds i * 128).
 __device__ __forceinline__ void convert_stage_fp4_ascend(const PackedRegs<kCtFp4Ascend>& r, uint32_t sa) {
-    const uint4 sc = r.s[0];
+    const uint4 sc = pair_scales(r.s[0]);
     const uint32_t w8[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         uint32_t v[4];
-        e2m1x8_to_bf16(w8[i], v);
+        e2m1x8_to_bf16_pairs(w8[i], v);
         sts128((sa ^ (uint32_t)(i << 4)) + (uint32_t)(i * 128), mul_bf16x2(v[0], sc.x), mul_bf16x2(v[1], sc.y),
                mul_bf16x2(v[2], sc.z), mul_bf16x2(v[3], sc.w));
     }
@@ -479,10 +515,10 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
             const uint32_t e = r.e[j];
             const uint32_t sb = (e == 0 ? 0x0040u : (e == 255 ? 0x7FC0u : (e << 7))) * 0x10001u;
             uint32_t v[4];
-            e2m1x8_to_bf16(q.x, v);
+            e2m1x8_to_bf16_pairs(q.x, v);
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[i] = mul_bf16x2(v[i], sb);
-            e2m1x8_to_bf16(q.y, v);
+            e2m1x8_to_bf16_pairs(q.y, v);
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[4 + i] = mul_bf16x2(v[i], sb);
         } else {  // FP4: 8 bytes = 16 codes; the thread's rows share one 16-row scale group
@@ -551,10 +587,19 @@ __device__ __forceinline__ void convert_block_int4(const PackedRegs<B200MOE_CT_I
 
 // Position of the x producer's L2 prefetch in the (tile, k-stage) sequence of its CTA.
 struct StageIter {
-    int t, kt;
+    int kt;
     TileInfo ti;
     bool valid;
 };
+
+// Accumulator position of output column i: the int8 dequant stores columns (0,2,1,3) of every four, the fp4 ones
+// named there (0,4,1,5,2,6,3,7) of every eight.
+template <int MODE>
+__device__ __forceinline__ constexpr int acc_pos(int i) {
+    return MODE == B200MOE_CT_INT8 ? ((i & ~3) | ((i & 1) << 1) | ((i >> 1) & 1))
+           : (MODE == kCtFp4Ascend || MODE == kCtFp4E8m0)   ? ((i & ~7) | ((i & 3) << 1) | ((i >> 2) & 1))
+                                                            : i;
+}
 
 // SILU (int8, fp4 with e8m0 scales): int8 weight columns come as blocks of 128 gate columns followed by the 128
 // up columns of the same indices (fp4: gate columns first, paired here), and the epilogue writes bf16(silu(gate) * up), [M, N/2], instead of
@@ -583,7 +628,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     gm_schedule(a.group_list, a.G, a.M, a.gl_type, n_nt, row_start, tile_prefix, &sb->n_tiles, a.status);
     if (threadIdx.x == 32) {
         sb->abort = 0;
-        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = 0ull;
+        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = make_uint4(0u, 0u, 0u, 0u);
         for (int i = 0; i < NS; ++i) {
             ptx::mbar_init(ptx::smem_u32(&sb->full[i]), T::kDirect ? 1 : 1 + kDqGroupWarps);
             ptx::mbar_init(ptx::smem_u32(&sb->empty[i]), 1);
@@ -624,19 +669,25 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             // tiles.  One ticket is always held in hand, so the atomic's latency is off the path.
             int* ticket = a.status + 2;  // zeroed by the host before the launch
             int held = atomicAdd(ticket, 1);
-            auto publish = [&]() -> int {
-                const int t = held < n_tiles ? held : n_tiles;
-                *reinterpret_cast<volatile unsigned long long*>(&sb->tile_ring[published % kTileRing]) =
-                    ((unsigned long long)(published + 1) << 32) | (uint32_t)t;
-                ++published;
-                if (t < n_tiles) held = atomicAdd(ticket, 1);
-                return t;
-            };
-            StageIter far;
-            far.t = publish();
+            StageIter far;  // the tile published last
             far.kt = 0;
-            far.valid = far.t < n_tiles;
-            if (far.valid) far.ti = locate_tile(far.t, tile_prefix, row_start, a.G, n_nt);
+            auto publish = [&]() {
+                far.valid = held < n_tiles;
+                uint4 entry = make_uint4(published + 1, 0u, 0u, 0u);
+                if (far.valid) {
+                    far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
+                    entry.y = T::kResolved ? (uint32_t)far.ti.row0 : (uint32_t)held;
+                    entry.z = (uint32_t)far.ti.g | ((uint32_t)far.ti.rows << 16);
+                    entry.w = (uint32_t)far.ti.n0;
+                }
+                asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
+                                 ptx::smem_u32(&sb->tile_ring[published % kTileRing])),
+                             "r"(entry.x), "r"(entry.y), "r"(entry.z), "r"(entry.w)
+                             : "memory");
+                ++published;
+                if (far.valid) held = atomicAdd(ticket, 1);
+            };
+            publish();
             auto far_step = [&]() {
                 if constexpr (SPLIT) {
                     ptx::tma_prefetch_l2_2d(&tmap_w, far.ti.n0 / 4, far.ti.g * a.K + far.kt * kBK);
@@ -645,21 +696,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     ptx::tma_prefetch_l2_2d(&tmap_w, T::kNibbles ? far.ti.n0 / 2 : far.ti.n0, far.ti.g * a.K + far.kt * kBK);
                 if (++far.kt < n_kt) return;
                 far.kt = 0;
-                far.t = publish();
-                far.valid = far.t < n_tiles;
-                if (far.valid) far.ti = locate_tile(far.t, tile_prefix, row_start, a.G, n_nt);
+                publish();
             };
             for (int i = 0; i < kL2Ahead && far.valid; ++i) far_step();
             for (;;) {
-                const int t = next_tile(sb, seq, n_tiles, a.status);
-                if (t >= n_tiles || !ok) break;
-                const TileInfo ti = locate_tile(t, tile_prefix, row_start, a.G, n_nt);
+                TileInfo ti;
+                if (!next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status) || !ok) break;
                 // The last row half of a tile often holds only a few rows of the expert (a second half
                 // of a dozen rows when an expert has a little over 128): a box of kSmallRows rows then
                 // replaces the 128-row box.  The MMA still reads 128 rows; what the rows beyond the box
                 // hold is left over from earlier stages and lands in accumulator rows that are never
                 // stored.
-                const int last_rows = ti.row_end - (ti.row0 + (ti.halves - 1) * kBM);
+                const int last_rows = ti.rows - (ti.halves - 1) * kBM;
                 const bool small_last = last_rows <= kSmallRows;
                 const uint32_t stage_bytes = (uint32_t)((ti.halves - 1) * kAHalfBytes + (small_last ? kSmallBytes : kAHalfBytes));
                 const CUtensorMap* last_map = small_last ? &tmap_xs : &tmap_x;
@@ -709,9 +757,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         bool ok = true, ready = false;  // ready: the next stage's barrier has been seen complete already
         uint32_t seq = 0;
         for (;;) {
-            const int t = __shfl_sync(0xffffffffu, next_tile(sb, seq, n_tiles, a.status), 0);
-            if (t >= n_tiles) break;
-            const TileInfo ti = locate_tile(t, tile_prefix, row_start, a.G, n_nt);
+            TileInfo ti;
+            if (!__all_sync(0xffffffffu, next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
             // accumulators of this tile: both for two halves, else the one used less recently;
             // the epilogue of their previous tile must have drained them
             const bool use0 = ti.halves == 2 || next1 == 0, use1 = ti.halves == 2 || next1 == 1;
@@ -773,9 +820,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         const bool has_offset = per_channel && a.offset != nullptr;
         uint32_t use = 0, next1 = 0, seq = 0;
         for (;;) {
-            const int t = next_tile(sb, seq, n_tiles, a.status);
-            if (t >= n_tiles) break;
-            const TileInfo ti = locate_tile(t, tile_prefix, row_start, a.G, n_nt);
+            TileInfo ti;
+            if (!__all_sync(0xffffffffu, next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
             // a two-half tile: this group takes row half `grp`; a one-half tile sits in one accumulator
             bool mine = true;
             int half = grp;
@@ -804,7 +850,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             ptx::tc_fence_after();
             {
                 const int row = ti.row0 + half * kBM + quarter * 32 + lane;
-                const bool row_ok = row < ti.row_end;
+                const bool row_ok = row < ti.row0 + ti.rows;
                 const float rs = (has_offset && row_ok) ? __ldg(a.rowsum + row) : 0.f;
                 if constexpr (SILU) {
                     __nv_bfloat16* arow = a.y + (size_t)row * (a.N >> 1) + (ti.n0 >> 1);
@@ -834,10 +880,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                                 u23 = pack_bf16x2(fmaf(ou.z, rs, su.z * __uint_as_float(ru[4 * q + 1])),
                                                   fmaf(ou.w, rs, su.w * __uint_as_float(ru[4 * q + 3])));
                             } else {
-                                g01 = pack_bf16x2(__uint_as_float(rg[4 * q]), __uint_as_float(rg[4 * q + 1]));
-                                g23 = pack_bf16x2(__uint_as_float(rg[4 * q + 2]), __uint_as_float(rg[4 * q + 3]));
-                                u01 = pack_bf16x2(__uint_as_float(ru[4 * q]), __uint_as_float(ru[4 * q + 1]));
-                                u23 = pack_bf16x2(__uint_as_float(ru[4 * q + 2]), __uint_as_float(ru[4 * q + 3]));
+                                auto two = [&](const uint32_t (&r)[16], int c) {
+                                    return pack_bf16x2(__uint_as_float(r[acc_pos<MODE>(c)]), __uint_as_float(r[acc_pos<MODE>(c + 1)]));
+                                };
+                                g01 = two(rg, 4 * q);
+                                g23 = two(rg, 4 * q + 2);
+                                u01 = two(ru, 4 * q);
+                                u23 = two(ru, 4 * q + 2);
                             }
                             const uint32_t gw[2] = {g01, g23}, uw[2] = {u01, u23};
 #pragma unroll
@@ -869,11 +918,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                             s4 = *reinterpret_cast<const float4*>(es + c * 32 + 4 * q);
                             o4 = *reinterpret_cast<const float4*>(es + kBN + c * 32 + 4 * q);
                         }
-                        // the int8 dequant stores columns (0,2,1,3) of every group of four, so output
-                        // column 4q + i sits at accumulator position 4q + (0,2,1,3)[i]
-                        constexpr bool kPerm = (MODE == B200MOE_CT_INT8);
-                        float v0 = __uint_as_float(r[4 * q]), v1 = __uint_as_float(r[4 * q + (kPerm ? 2 : 1)]);
-                        float v2 = __uint_as_float(r[4 * q + (kPerm ? 1 : 2)]), v3 = __uint_as_float(r[4 * q + 3]);
+                        float v0 = __uint_as_float(r[acc_pos<MODE>(4 * q)]), v1 = __uint_as_float(r[acc_pos<MODE>(4 * q + 1)]);
+                        float v2 = __uint_as_float(r[acc_pos<MODE>(4 * q + 2)]), v3 = __uint_as_float(r[acc_pos<MODE>(4 * q + 3)]);
                         if (per_channel) {
                             v0 = fmaf(o4.x, rs, s4.x * v0);
                             v1 = fmaf(o4.y, rs, s4.y * v1);
@@ -906,10 +952,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         const DqLane d = dq_lane<MODE>(dq_tid % (kDqGroupWarps * 32));
         DqIter pf;
         pf.seq = 0;
-        pf.t = next_tile(sb, pf.seq, n_tiles, a.status);
+        {
+            TileInfo ti;
+            pf.valid = next_tile<T::kResolved>(sb, pf.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
+            pf.g = ti.g;
+            pf.n0 = ti.n0;
+        }
         pf.kt = 0;
-        dq_locate<MODE, SPLIT>(pf, weight, a, d, n_tiles, tile_prefix, row_start, n_nt);
-        if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT>(pf, grp, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+        dq_locate<MODE, SPLIT>(pf, weight, a, d);
+        if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT>(pf, grp, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
         PackedRegs<MODE> regs[kPrefetch];
         bool loaded[kPrefetch];
 #pragma unroll
@@ -917,7 +968,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             loaded[u] = pf.valid;
             if (pf.valid) {
                 load_packed<MODE, SPLIT>(regs[u], pf, a, d);
-                dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+                dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
             }
         }
         const uint32_t sa0 = ptx::smem_u32(b_ring) + (T::kEightRows ? btile_offset(d.k0, d.chunk)
@@ -947,7 +998,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 loaded[u] = pf.valid;
                 if (pf.valid) {
                     load_packed<MODE, SPLIT>(regs[u], pf, a, d);
-                    dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, n_tiles, tile_prefix, row_start, n_nt, sb);
+                    dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
                 }
                 ib += kDqGroups;
             }
