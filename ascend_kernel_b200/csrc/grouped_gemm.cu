@@ -97,7 +97,7 @@ struct GmTraits {
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
     // who resolves a published tile number: the publisher, or (fp8, whose dequant loop spills otherwise and took 6.24
-    // instead of 5.88 ms for 8192 tokens x 8 over 256 experts, 7168 x 4096) each role for itself
+    // instead of 5.78 ms for 8192 tokens x 8 over 256 experts, 7168 x 4096) each role for itself
     static constexpr bool kResolved = MODE != B200MOE_CT_FP8;
     static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
 };
@@ -227,14 +227,35 @@ template <bool RESOLVED>
 __device__ __forceinline__ bool next_tile(GmBarriers* sb, uint32_t& seq, TileInfo& ti, const int* tile_prefix, const int* row_start,
                                           int G, int n_nt, int* status) {
     const uint4* e = &sb->tile_ring[seq % kTileRing];
+    if constexpr (!RESOLVED) {
+        // the first two words: the sequence number and the tile, ~0 past the end
+        const volatile unsigned long long* e2 = reinterpret_cast<const volatile unsigned long long*>(e);
+        const uint32_t want = seq + 1;
+        unsigned long long v = *e2;
+        if ((uint32_t)v != want) {
+            volatile int* abort = &sb->abort;
+            const uint64_t t0 = ptx::globaltimer_ns();
+            uint32_t spins = 0;
+            while ((uint32_t)(v = *e2) != want) {
+                if ((++spins & 0xFF) == 0) {
+                    if (*abort) return false;
+                    if (ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) {
+                        *abort = 1;
+                        report_status(status, kDevWaitExpired, 90);
+                        return false;
+                    }
+                }
+            }
+        }
+        ++seq;
+        const uint32_t t = (uint32_t)(v >> 32);
+        if (t == ~0u) return false;
+        ti = locate_tile((int)t, tile_prefix, row_start, G, n_nt);
+        return true;
+    }
     uint4 v = ring_load(e);
     if (v.x != seq + 1) v = ring_wait(e, seq + 1, sb, status);
     ++seq;
-    if constexpr (!RESOLVED) {
-        if (v.z == 0u) return false;
-        ti = locate_tile((int)v.y, tile_prefix, row_start, G, n_nt);
-        return true;
-    }
     ti.row0 = (int)v.y;
     ti.g = (int)(v.z & 0xFFFFu);
     ti.rows = (int)(v.z >> 16);
@@ -673,7 +694,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             far.kt = 0;
             auto publish = [&]() {
                 far.valid = held < n_tiles;
-                uint4 entry = make_uint4(published + 1, 0u, 0u, 0u);
+                uint4 entry = make_uint4(published + 1, T::kResolved ? 0u : ~0u, 0u, 0u);
                 if (far.valid) {
                     far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
                     entry.y = T::kResolved ? (uint32_t)far.ti.row0 : (uint32_t)held;
