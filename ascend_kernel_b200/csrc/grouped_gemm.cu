@@ -96,10 +96,10 @@ struct GmTraits {
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
+    static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
     // who resolves a published tile number: the publisher, or (fp8, whose dequant loop spills otherwise and took 6.24
     // instead of 5.78 ms for 8192 tokens x 8 over 256 experts, 7168 x 4096) each role for itself
     static constexpr bool kResolved = MODE != B200MOE_CT_FP8;
-    static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
 };
 
 struct GmBarriers {
