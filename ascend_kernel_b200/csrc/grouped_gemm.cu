@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "gemm_args.cuh"
 #include "ptx.cuh"
+#include "tile_ring.h"
 
 namespace b200moe {
 
@@ -53,7 +54,7 @@ constexpr int kSuperRows = 8;  // m-tiles per L2 super-tile
 // Published tiles a role may lag behind the publisher: the publisher leads the x loads by kL2Ahead
 // stages, those lead the MMAs by the ring depth, the epilogue trails by at most two tiles; with one
 // stage per tile that is kL2Ahead + kNS + 2 tiles.
-constexpr int kTileRing = 32;
+static_assert(kL2Ahead + kNS + 2 < kTileRing, "a slot is read before it is written again");
 constexpr int kBarrierBytes = 1024;  // shared memory reserved for GmBarriers
 constexpr int kEpiScaleFloats = 2 * kBN;  // per epilogue warp: the tile's column scales and scale * offset
 constexpr int kAHalfBytes = kBM * kBK * 2;   // one 128-row box
@@ -114,11 +115,11 @@ struct GmBarriers {
     int n_tiles;
     int pad;
     // Tile schedule of this CTA: tiles are drawn from a global ticket counter (status word 2) by the
-    // thread that runs furthest ahead, resolved by it and published here, entry i % kTileRing = {i + 1, first row,
-    // expert | rows << 16 (rows 0: the schedule has ended), first column}, written and read as one aligned
-    // 16-byte vector.  Every role walks the entries in order, so all see the same sequence, and none
+    // thread that runs furthest ahead, resolved by it and published here (tile_ring.h), the i-th tile with number i + 1.
+    // Every role walks the entries in order, so all see the same sequence, and none
     // repeats the search and the divisions at each tile switch (64 experts, 210 rows each, 1280 x 512, int4: 74 -> 48 us).
-    uint4 tile_ring[kTileRing];
+    // Where the roles resolve the tiles themselves, an entry's first word is {i + 1, tile number, ~0 past the end}.
+    alignas(16) TileEntry tile_ring[kTileRing];
 };
 
 struct TileInfo {
@@ -151,27 +152,19 @@ __device__ __forceinline__ bool gm_wait(uint64_t* bar, uint32_t parity, GmBarrie
     return gm_wait_slow(b, parity, sb, status, id);
 }
 
-__device__ __forceinline__ uint4 ring_load(const uint4* e) {
-    uint4 v;
-    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(ptx::smem_u32(e)));
-    return v;
-}
-
-// Waits for entry `e` to carry the sequence number `want`; an entry of no rows when a wait expired or another role aborted.
-__device__ __noinline__ uint4 ring_wait(const uint4* e, uint32_t want, GmBarriers* sb, int* status) {
+// Waits for slot `e` to hold the tile numbered `want`; an entry of no rows when a wait expired or another role aborted.
+__device__ __noinline__ TileEntry ring_wait(const TileEntry* e, uint32_t want, GmBarriers* sb, int* status) {
     volatile int* abort = &sb->abort;
     const uint64_t t0 = ptx::globaltimer_ns();
     uint32_t spins = 0;
-    uint4 v;
-    while ((v = ring_load(e)).x != want) {
+    TileEntry v;
+    while (!tile_entry_is(v = ring_load(e), want)) {
         if ((++spins & 0xFF) == 0) {
-            if (*abort) return make_uint4(want, 0u, 0u, 0u);
+            if (*abort) return tile_entry(want, 0u, 0u, 0u, 0u);
             if (ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) {
                 *abort = 1;
                 report_status(status, kDevWaitExpired, 90);
-                return make_uint4(want, 0u, 0u, 0u);
+                return tile_entry(want, 0u, 0u, 0u, 0u);
             }
         }
     }
@@ -226,12 +219,11 @@ __device__ __forceinline__ TileInfo locate_tile(int t, const int* tile_prefix, c
 template <bool RESOLVED>
 __device__ __forceinline__ bool next_tile(GmBarriers* sb, uint32_t& seq, TileInfo& ti, const int* tile_prefix, const int* row_start,
                                           int G, int n_nt, int* status) {
-    const uint4* e = &sb->tile_ring[seq % kTileRing];
+    const TileEntry* e = &sb->tile_ring[seq % kTileRing];
     if constexpr (!RESOLVED) {
-        // the first two words: the sequence number and the tile, ~0 past the end
-        const volatile unsigned long long* e2 = reinterpret_cast<const volatile unsigned long long*>(e);
+        const volatile uint64_t* e2 = &e->a;
         const uint32_t want = seq + 1;
-        unsigned long long v = *e2;
+        uint64_t v = *e2;
         if ((uint32_t)v != want) {
             volatile int* abort = &sb->abort;
             const uint64_t t0 = ptx::globaltimer_ns();
@@ -253,13 +245,13 @@ __device__ __forceinline__ bool next_tile(GmBarriers* sb, uint32_t& seq, TileInf
         ti = locate_tile((int)t, tile_prefix, row_start, G, n_nt);
         return true;
     }
-    uint4 v = ring_load(e);
-    if (v.x != seq + 1) v = ring_wait(e, seq + 1, sb, status);
+    TileEntry v = ring_load(e);
+    if (!tile_entry_is(v, seq + 1)) v = ring_wait(e, seq + 1, sb, status);
     ++seq;
-    ti.row0 = (int)v.y;
-    ti.g = (int)(v.z & 0xFFFFu);
-    ti.rows = (int)(v.z >> 16);
-    ti.n0 = (int)v.w;
+    ti.row0 = tile_entry_row0(v);
+    ti.g = tile_entry_expert(v);
+    ti.rows = tile_entry_rows(v);
+    ti.n0 = tile_entry_column(v) * kBN;
     ti.halves = ti.rows > kBM ? 2 : 1;
     return ti.rows != 0;
 }
@@ -649,7 +641,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     gm_schedule(a.group_list, a.G, a.M, a.gl_type, n_nt, row_start, tile_prefix, &sb->n_tiles, a.status);
     if (threadIdx.x == 32) {
         sb->abort = 0;
-        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = tile_entry(0u, 0u, 0u, 0u, 0u);
         for (int i = 0; i < NS; ++i) {
             ptx::mbar_init(ptx::smem_u32(&sb->full[i]), T::kDirect ? 1 : 1 + kDqGroupWarps);
             ptx::mbar_init(ptx::smem_u32(&sb->empty[i]), 1);
@@ -694,17 +686,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             far.kt = 0;
             auto publish = [&]() {
                 far.valid = held < n_tiles;
-                uint4 entry = make_uint4(published + 1, T::kResolved ? 0u : ~0u, 0u, 0u);
+                TileEntry entry = tile_entry(published + 1, T::kResolved ? 0u : ~0u, 0u, 0u, 0u);
                 if (far.valid) {
                     far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
-                    entry.y = T::kResolved ? (uint32_t)far.ti.row0 : (uint32_t)held;
-                    entry.z = (uint32_t)far.ti.g | ((uint32_t)far.ti.rows << 16);
-                    entry.w = (uint32_t)far.ti.n0;
+                    entry = tile_entry(published + 1, (uint32_t)(T::kResolved ? far.ti.row0 : held), (uint32_t)far.ti.rows,
+                                       (uint32_t)far.ti.g, (uint32_t)far.ti.n0 / kBN);
                 }
-                asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                 ptx::smem_u32(&sb->tile_ring[published % kTileRing])),
-                             "r"(entry.x), "r"(entry.y), "r"(entry.z), "r"(entry.w)
-                             : "memory");
+                ring_store(&sb->tile_ring[published % kTileRing], entry);
                 ++published;
                 if (far.valid) held = atomicAdd(ticket, 1);
             };

@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "gemm_args.cuh"
 #include "ptx.cuh"
+#include "tile_ring.h"
 
 namespace b200moe {
 namespace pk {
@@ -58,7 +59,6 @@ constexpr int kDqGroups = 2, kDqGroupWarps = 8;
 constexpr int kPrefetch = 2;    // packed stages a dequant thread holds in registers ahead of the conversion
 constexpr int kL2Ahead = 4;     // stages by which the L2 prefetch of packed weights leads the x loads
 constexpr int kSuperRows = 8;   // m-tiles per L2 super-tile
-constexpr int kTileRing = 32;
 constexpr int kStageWBytes = kBK * kTileN;    // packed bytes of one stage
 constexpr int kBigBox = 128, kSmallBox = 32;  // rows of the two x boxes
 constexpr uint32_t kTmemCols = 512;
@@ -102,11 +102,9 @@ struct Barriers {
     int abort;
     int n_tiles;
     int pad;
-    // The published tiles, resolved once by the publisher: entry i % kTileRing = {i + 1, first row,
-    // expert | rows << 16 (rows 0 = end of the schedule), tile column}, written and read as one aligned
-    // 16-byte vector, so a reader sees the sequence number and the tile together.  Every other role reads
+    // The published tiles (tile_ring.h), the i-th with number i + 1, resolved once by the publisher.  Every other role reads
     // the entry instead of repeating the search and the divisions at each tile switch.
-    uint4 tile_ring[kTileRing];
+    alignas(16) TileEntry tile_ring[kTileRing];
 };
 static_assert(sizeof(Barriers) <= kBarrierBytes, "barrier block");
 
@@ -133,25 +131,17 @@ __device__ __forceinline__ bool pk_wait(uint64_t* bar, uint32_t parity, Barriers
     return wait_slow(b, parity, sb, status, id);
 }
 
-__device__ __forceinline__ uint4 ring_load(const uint4* e) {
-    uint4 v;
-    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(ptx::smem_u32(e)));
-    return v;
-}
-
 // The seq-th tile of this CTA (seq is advanced) into `ti`; false when the schedule has ended, a wait
 // expired or another role aborted.
 __device__ __forceinline__ bool next_tile(Barriers* sb, uint32_t& seq, TileInfo& ti, int* status) {
-    const uint4* e = &sb->tile_ring[seq % kTileRing];
+    const TileEntry* e = &sb->tile_ring[seq % kTileRing];
     const uint32_t want = seq + 1;
-    uint4 v = ring_load(e);
-    if (v.x != want) {
+    TileEntry v = ring_load(e);
+    if (!tile_entry_is(v, want)) {
         volatile int* abort = &sb->abort;
         const uint64_t t0 = ptx::globaltimer_ns();
         uint32_t spins = 0;
-        while ((v = ring_load(e)).x != want) {
+        while (!tile_entry_is(v = ring_load(e), want)) {
             if ((++spins & 0xFF) == 0) {
                 if (*abort) return false;
                 if (ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) {
@@ -163,10 +153,10 @@ __device__ __forceinline__ bool next_tile(Barriers* sb, uint32_t& seq, TileInfo&
         }
     }
     ++seq;
-    ti.row0 = (int)v.y;
-    ti.g = (int)(v.z & 0xFFFFu);
-    ti.rows = (int)(v.z >> 16);
-    ti.j = (int)v.w;
+    ti.row0 = tile_entry_row0(v);
+    ti.g = tile_entry_expert(v);
+    ti.rows = tile_entry_rows(v);
+    ti.j = tile_entry_column(v);
     return ti.rows != 0;
 }
 
@@ -277,7 +267,7 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     }
     if (threadIdx.x == 32) {
         sb->abort = 0;
-        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = tile_entry(0u, 0u, 0u, 0u, 0u);
         for (int i = 0; i < kXStages; ++i) {
             ptx::mbar_init(ptx::smem_u32(&sb->x_full[i]), 1);
             ptx::mbar_init(ptx::smem_u32(&sb->x_empty[i]), 1);
@@ -316,17 +306,12 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
             TileInfo far_ti;  // the tile published last, resolved
             auto publish = [&]() -> bool {
                 const bool live = held < n_tiles;
-                uint4 entry = make_uint4(published + 1, 0u, 0u, 0u);  // rows 0: the schedule has ended
+                TileEntry entry = tile_entry(published + 1, 0u, 0u, 0u, 0u);  // rows 0: the schedule has ended
                 if (live) {
                     far_ti = locate_tile<kMaxR>(held, tile_prefix, row_start, a.G, n_nt);
-                    entry.y = (uint32_t)far_ti.row0;
-                    entry.z = (uint32_t)far_ti.g | ((uint32_t)far_ti.rows << 16);
-                    entry.w = (uint32_t)far_ti.j;
+                    entry = tile_entry(published + 1, (uint32_t)far_ti.row0, (uint32_t)far_ti.rows, (uint32_t)far_ti.g, (uint32_t)far_ti.j);
                 }
-                asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                 ptx::smem_u32(&sb->tile_ring[published % kTileRing])),
-                             "r"(entry.x), "r"(entry.y), "r"(entry.z), "r"(entry.w)
-                             : "memory");
+                ring_store(&sb->tile_ring[published % kTileRing], entry);
                 ++published;
                 if (live) held = atomicAdd(ticket, 1);
                 return live;
