@@ -45,7 +45,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 // A kernel launched with launch_dependent may start while the kernel before it in the stream is still running, once all of
 // that kernel's blocks have called grid_dep_launch() or ended; grid_dep_wait() returns when it has completed and its
-// writes are visible (at once in a kernel launched the usual way).
+// writes are visible (at once in a kernel launched the usual way).  What that kernel writes is not read-only for the whole
+// of this one's lifetime, so it is read with ordinary loads (__ldca, __ldcg), never with __ldg: non-coherent
+// loads are defined for data that nothing writes while the kernel is there.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -860,7 +860,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             {
                 const int row = ti.row0 + half * kBM + quarter * 32 + lane;
                 const bool row_ok = row < ti.row0 + ti.rows;
-                const float rs = (has_offset && row_ok) ? __ldg(a.rowsum + row) : 0.f;
+                const float rs = (has_offset && row_ok) ? __ldca(a.rowsum + row) : 0.f;
                 if constexpr (SILU) {
                     __nv_bfloat16* arow = a.y + (size_t)row * (a.N >> 1) + (ti.n0 >> 1);
                     const uint32_t acc = tmem_base + grp * kBN + ((uint32_t)(quarter * 32) << 16);

@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
                 float s = 0.f;
 #pragma unroll 4
                 for (int i = v0 + threadIdx.x; i < v1; i += kGvThreads) {
-                    const uint4 v = __ldg(src + i);
+                    const uint4 v = PATH == 1 ? __ldca(src + i) : __ldg(src + i);
                     dst[i] = v;
                     if (MODE == B200MOE_CT_INT8 && a.offset != nullptr) {
                         const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
