@@ -14,6 +14,7 @@
 #include <stdexcept>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "../../../include/b200moe.h"
 
@@ -58,16 +59,30 @@ struct Dims {
 // a mutex, and it exists for a second reason: words 4 / 5 of a workspace keep the first device-side
 // finding (invalid group list, expired wait) of every call that used it, so last_status() can report
 // at the caller's synchronisation point what no asynchronous call can report by itself.
+// A captured CUDA graph keeps the address of the workspace its calls got.  So a workspace that became too small is
+// kept, not freed, or replays would write into memory that has become somebody else's.  The first one holds what
+// every operator needs whatever its sizes (the split GEMV's 4.9 MB is the largest such part) and a larger one is at
+// least twice its predecessor, so the kept ones of a stream are together no larger than the one in use.  Findings of
+// replays land in the kept ones, so the status calls read those too.
 std::mutex g_ws_mutex;
-std::map<std::pair<int, void*>, at::Tensor> g_workspaces;
+using StreamKey = std::pair<int, void*>;
+std::map<StreamKey, at::Tensor> g_workspaces;
+std::vector<std::pair<StreamKey, at::Tensor>> g_kept_workspaces;
+constexpr size_t kFirstWorkspace = size_t(8) << 20;
 
 at::Tensor workspace_for(const at::Tensor& like, size_t bytes, void* stream) {
     std::lock_guard<std::mutex> lock(g_ws_mutex);
-    const auto key = std::make_pair((int)like.get_device(), stream);
+    const StreamKey key((int)like.get_device(), stream);
     auto it = g_workspaces.find(key);
     if (it == g_workspaces.end() || (size_t)it->second.numel() < bytes) {
-        at::Tensor fresh = at::zeros({(int64_t)std::max<size_t>(bytes, size_t(1) << 20)}, like.options().dtype(at::kByte));
-        if (it != g_workspaces.end()) fresh.slice(0, 16, 24).copy_(it->second.slice(0, 16, 24));
+        const bool first = it == g_workspaces.end();
+        const size_t size = std::max(bytes, first ? kFirstWorkspace : 2 * (size_t)it->second.numel());
+        at::Tensor fresh = at::empty({(int64_t)size}, like.options().dtype(at::kByte));
+        fresh.slice(0, 0, B200MOE_STATUS_BYTES).zero_();  // (the operators clear what else they start from)
+        if (!first) {
+            fresh.slice(0, 16, 24).copy_(it->second.slice(0, 16, 24));
+            g_kept_workspaces.emplace_back(key, it->second);
+        }
         g_workspaces[key] = fresh;
         return fresh;
     }
@@ -79,13 +94,15 @@ std::pair<int, int> LastStatus(bool clear) {
     int dev = 0;
     TORCH_CHECK(cudaGetDevice(&dev) == cudaSuccess, "cudaGetDevice failed");
     std::pair<int, int> found{0, 0};
-    for (auto& kv : g_workspaces) {
-        if (kv.first.first != dev) continue;
+    auto read = [&](const StreamKey& key, const at::Tensor& ws) {
+        if (key.first != dev) return;
         int32_t out[2] = {0, 0};
-        const int rc = b200moe_read_sticky_status(kv.second.data_ptr(), out, clear ? 1 : 0, kv.first.second);
+        const int rc = b200moe_read_sticky_status(ws.data_ptr(), out, clear ? 1 : 0, key.second);
         TORCH_CHECK(rc == B200MOE_OK, "read_sticky_status: ", b200moe_strerror(rc));
         if (found.first == 0 && out[0] != 0) found = {out[0], out[1]};
-    }
+    };
+    for (auto& kv : g_workspaces) read(kv.first, kv.second);
+    for (auto& kv : g_kept_workspaces) read(kv.first, kv.second);
     return found;
 }
 

@@ -83,7 +83,15 @@ def _check_scale(scale, ct, G, K, N, what):
 # list that was clamped, a bounded wait that expired).  `last_status` / `check_status` read them at the
 # caller's synchronisation points, so a failed call cannot pass unnoticed even though no operator
 # synchronises.  Calls on one stream run one after the other, so they can share the buffer.
+#
+# A captured CUDA graph keeps the address of the workspace its calls got.  So a workspace that became too small is
+# kept, not freed, or replays would write into memory that has become somebody else's.  The first one holds what
+# every operator needs whatever its sizes (the split GEMV's 4.9 MB is the largest such part) and a larger one is at
+# least twice its predecessor, so the kept ones of a stream are together no larger than the one in use.  Findings of
+# replays land in the kept ones, so the status calls read those too.
 _WS = {}
+_WS_KEPT = []
+_WS_FIRST = 8 << 20
 
 
 def _workspace(need, device):
@@ -92,9 +100,12 @@ def _workspace(need, device):
     key = (idx, torch.cuda.current_stream(idx).cuda_stream)
     ws = _WS.get(key)
     if ws is None or ws.numel() < need:
-        new = torch.zeros(max(int(need), 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
+        size = max(int(need), _WS_FIRST if ws is None else 2 * ws.numel())
+        new = torch.empty(size, dtype=torch.uint8, device=torch.device("cuda", idx))
+        new[:_abi.STATUS_BYTES].zero_()  # (the operators clear what else they start from)
         if ws is not None:
             new[16:24].copy_(ws[16:24])  # carry the sticky status words over
+            _WS_KEPT.append((key, ws))
         _WS[key] = ws = new
     return ws
 
@@ -108,7 +119,7 @@ def last_status(device=None, clear: bool = False):
 
     idx = torch.cuda.current_device() if device is None else torch.device(device).index
     found = (0, 0)
-    for (d, stream), ws in list(_WS.items()):
+    for (d, stream), ws in list(_WS.items()) + _WS_KEPT:
         if d != idx:
             continue
         out = (ctypes.c_int32 * 2)()
