@@ -98,9 +98,14 @@ struct GmTraits {
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
     static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
-    // who resolves a published tile number: the publisher, or (fp8, whose dequant loop spills otherwise and took 6.24
-    // instead of 5.78 ms for 8192 tokens x 8 over 256 experts, 7168 x 4096) each role for itself
-    static constexpr bool kResolved = MODE != B200MOE_CT_FP8;
+    // Who turns a published tile number into rows and columns: the publisher, once, or each role for itself.  Resolved
+    // entries cost the roles less at a tile switch but leave the dequant loop of the modes with 4 rows x 16 columns a thread
+    // fewer registers.  Each role | publisher, us, libraries called in turn: 8192 tokens x 8 by popularity over 256 experts,
+    // 7168 x 4096: int8 4919 | 4992, its SiLU form 4984 | 5328, fp8 5579 | 7086, canonical fp4 5089 | 6088, bf16 5072 | 5001;
+    // (in runs of their own) int4 9000 | 8616, stored fp4 4838 | 4875, fp4 with e8m0 scales 4602 | 4598, SiLU 5265 | 5039.  32 rows an
+    // expert, 2048 x 7168: int8 1282 | 1299, fp8 1490 | 1921, canonical fp4 1288 | 1619, int4 2326 | 2104, stored fp4 1238 |
+    // 1181, e8m0 1425 | 1159.  64 experts of 210 rows, 1280 x 512: int8 52.3 | 50.3, bf16 35.9 | 34.9, stored fp4 30.8 | 28.9.
+    static constexpr bool kResolved = MODE != B200MOE_CT_INT8 && MODE != B200MOE_CT_FP8 && MODE != B200MOE_CT_FP4;
 };
 
 struct GmBarriers {
