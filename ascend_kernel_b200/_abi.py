@@ -22,7 +22,7 @@ STATUS_BYTES = 256
 EXPORTS = [
     "b200moe_grouped_gemm", "b200moe_grouped_gemm_workspace_bytes", "b200moe_grouped_gemv",
     "b200moe_grouped_gemv_workspace_bytes", "b200moe_grouped_gemv_split_workspace_bytes", "b200moe_fp4_dequant", "b200moe_fp4_layout", "b200moe_silu_mul",
-    "b200moe_ep_finish", "b200moe_gather_rows", "b200moe_gather_rows_sum", "b200moe_grouped_gemm_int8_packed_rowsum", "b200moe_combine", "b200moe_read_status", "b200moe_read_sticky_status", "b200moe_strerror", "b200moe_version",
+    "b200moe_ep_finish", "b200moe_gather_rows", "b200moe_gather_rows_sum", "b200moe_grouped_gemm_int8_packed_rowsum", "b200moe_grouped_gemm_int8_packed_bounded", "b200moe_combine", "b200moe_read_status", "b200moe_read_sticky_status", "b200moe_strerror", "b200moe_version",
     "b200moe_moe_route", "b200moe_moe_regroup_index", "b200moe_grouped_gemm_int8_noalloc", "b200moe_grouped_gemm_int8_noalloc_max_rows", "b200moe_noalloc_read_status",
     "b200moe_ep_post_counts", "b200moe_ep_dispatch", "b200moe_ep_wait", "b200moe_ep_post", "b200moe_ep_combine",
     "b200moe_fp4_dequant_bf16_scale", "b200moe_fp8_dequant", "b200moe_fp4_scale_fold",
@@ -78,6 +78,8 @@ def _load() -> ctypes.CDLL:
     lib.b200moe_grouped_gemm_int8_packed.restype = i32
     lib.b200moe_grouped_gemm_int8_packed_rowsum.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, i32, vp, sz, vp]
     lib.b200moe_grouped_gemm_int8_packed_rowsum.restype = i32
+    lib.b200moe_grouped_gemm_int8_packed_bounded.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, i32, i64, vp, sz, vp]
+    lib.b200moe_grouped_gemm_int8_packed_bounded.restype = i32
     lib.b200moe_grouped_gemm_int8_packed_scatter.argtypes = [vp, vp, vp, vp, vp, vp, ctypes.POINTER(vp), i64, i64, i64, i64, i64,
                                                              i64, i32, vp, sz, vp]
     lib.b200moe_grouped_gemm_int8_packed_scatter.restype = i32

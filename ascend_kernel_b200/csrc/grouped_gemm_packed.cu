@@ -32,7 +32,9 @@
 // pair: a relay lane of the dequant group (which has slack) waits for the stage's x tile before the
 // group reports the stage full, and hands the x slot back to the producer when it observes the
 // completion of the MMAs that read it.  Every wait is bounded.
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_args.cuh"
@@ -78,6 +80,8 @@ struct Shape {
     static constexpr int kStageTileBytes = MAX_R * kTileN * 2;  // the epilogue's bf16 staging tile
     static_assert(2 * MAX_R + STAGES * kAStageCols <= kTmemCols, "tensor memory budget");
     static_assert(kXSlotBytes % 1024 == 0 && MAX_R % 32 == 0, "x slots");
+    // shared memory of the rings, the staging tile, the barriers and the epilogue's strips
+    static constexpr int kBytes = X_STAGES * kXSlotBytes + kStageTileBytes + kBarrierBytes + kEpiWarps * kEpiStripBytes;
 };
 using Prefill = Shape<160, 3, 6>;
 // Decode steps have few rows an expert and are bound by the weights' way from HBM (about 700 cycles a stage); the round
@@ -228,28 +232,20 @@ __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* 
 // epilogue writes bf16(silu(gate) * up), [M, N / 2] (gate and up are rounded to bf16 first, as the
 // unfused operators would).
 template <bool GATE_UP, class SHAPE>
-__global__ void __launch_bounds__(kThreads, 1)
-grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xs,
-                           const uint8_t* __restrict__ weight, const GemmArgs a) {
+__device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUtensorMap& tmap_xs, const uint8_t* __restrict__ weight,
+                                            const GemmArgs& a, uint8_t* base, const int* row_start, int* tile_prefix,
+                                            __nv_bfloat16* const* s_dst_base) {
     constexpr int kMaxR = SHAPE::kMaxR, kStages = SHAPE::kStages, kXStages = SHAPE::kXStages, kXSlotBytes = SHAPE::kXSlotBytes;
-    constexpr int kStageTileBytes = SHAPE::kStageTileBytes, kEpiStripBytes = SHAPE::kEpiStripBytes;
     constexpr uint32_t kACol = SHAPE::kACol;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_ring = base;
     uint8_t* epi_stage = x_ring + kXStages * kXSlotBytes;
-    Barriers* sb = reinterpret_cast<Barriers*>(epi_stage + kStageTileBytes);
-    __shared__ __nv_bfloat16* s_dst_base[8];  // scatter mode: the destination tensors (indexed per row)
-    if (threadIdx.x < 8) s_dst_base[threadIdx.x] = a.dst_base[threadIdx.x];
+    Barriers* sb = reinterpret_cast<Barriers*>(epi_stage + SHAPE::kStageTileBytes);
     float* epi_rowsum = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sb) + kBarrierBytes);
-    int* row_start = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(epi_rowsum) + kEpiWarps * kEpiStripBytes);
-    int* tile_prefix = row_start + (a.G + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_nt = a.N / kTileN;
     const int n_kt = a.K / kBK;
 
-    load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
     if (warp == 0) {
         // tile-count prefix, each lane over a stretch of consecutive experts
         int lo, hi, mine = 0, total;
@@ -614,15 +610,78 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     }
 }
 
-template <bool GATE_UP, class SHAPE>
-static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, cudaStream_t s) {
-    const size_t smem = 1024 + (size_t)SHAPE::kXStages * SHAPE::kXSlotBytes + SHAPE::kStageTileBytes + kBarrierBytes +
-                        (size_t)kEpiWarps * SHAPE::kEpiStripBytes + sizeof(int) * 2 * (size_t)(a.G + 1);
-    B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_packed_kernel<GATE_UP, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+// What a kernel holds: one shape, or both and the choice between them.
+enum class Which { kDecode, kPrefill, kEither };
+template <Which WHICH>
+constexpr int kRingBytes = WHICH == Which::kDecode ? Decode::kBytes : Prefill::kBytes;
+static_assert(Decode::kBytes <= Prefill::kBytes, "kEither has room for both");
+
+// kEither: the decode step's shape where 32-row tiles make (nearly) no more waves of the grid than 160-row ones, and so
+// (nearly) no more dequantisation.  Time of the 160-row shape over that of the 32-row one, 256 experts, 7168 x 4096 / 2048 x 7168: one to
+// eight rows an expert, evenly or 8 of 256 experts a token: 1.03 .. 1.25 / 1.08 .. 1.22, with the same tiles; by popularity
+// (Zipf 1.2), 1, 2, 4 rows on average: 1.03, 1.11, 1.15 / 1.15, 1.14, 1.04 with 1.04 .. 1.11 times the waves; 6 and 8 rows: 0.99,
+// 0.94 / 0.98, 1.00 with 1.08 .. 1.12; all rows on one expert: 0.67 / 0.46 with 2 / 4 times the waves, 0.36 / 0.35 with 3.5 / 4.3.  In one
+// wave (64 experts, 2048 x 1024, any list) 1.09 .. 1.43.
+template <bool GATE_UP, Which WHICH>
+__global__ void __launch_bounds__(kThreads, 1)
+grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xs,
+                           const uint8_t* __restrict__ weight, const GemmArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __nv_bfloat16* s_dst_base[8];  // scatter mode: the destination tensors (indexed per row)
+    if (threadIdx.x < 8) s_dst_base[threadIdx.x] = a.dst_base[threadIdx.x];
+    int* row_start = reinterpret_cast<int*>(base + kRingBytes<WHICH>);
+    int* tile_prefix = row_start + (a.G + 1);
+
+    load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
+    if constexpr (WHICH == Which::kEither) {
+        __shared__ int s_decode;
+        if (threadIdx.x < 32) {
+            int lo, hi, t32 = 0, t160 = 0;
+            lane_experts(a.G, lo, hi);
+            for (int g = lo; g < hi; ++g) {
+                const int rows = row_start[g + 1] - row_start[g];
+                t32 += (rows + Decode::kMaxR - 1) / Decode::kMaxR;
+                t160 += (rows + Prefill::kMaxR - 1) / Prefill::kMaxR;
+            }
+            const int n_nt = a.N / kTileN, ctas = (int)gridDim.x;
+            const int w32 = (__reduce_add_sync(0xffffffffu, t32) * n_nt + ctas - 1) / ctas;
+            const int w160 = (__reduce_add_sync(0xffffffffu, t160) * n_nt + ctas - 1) / ctas;
+            if (threadIdx.x == 0) s_decode = 16LL * w32 <= 17LL * w160;
+        }
+        __syncthreads();
+        if (s_decode) packed_body<GATE_UP, Decode>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+        else packed_body<GATE_UP, Prefill>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+    } else {
+        using Only = std::conditional_t<WHICH == Which::kDecode, Decode, Prefill>;
+        packed_body<GATE_UP, Only>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+    }
+}
+
+template <bool GATE_UP, Which WHICH>
+static int launch_one(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, cudaStream_t s) {
+    const size_t smem = 1024 + (size_t)kRingBytes<WHICH> + sizeof(int) * 2 * (size_t)(a.G + 1);
+    B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_packed_kernel<GATE_UP, WHICH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    grouped_gemm_packed_kernel<GATE_UP, SHAPE><<<grid_ctas(), kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
+    grouped_gemm_packed_kernel<GATE_UP, WHICH><<<grid_ctas(), kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
     B200MOE_CUDA_TRY(cudaGetLastError());
     return B200MOE_OK;
+}
+
+// More than eight rows an expert on average: prefill.  No expert with more than 32 rows (the caller says so, or there are no more),
+// or 32-row tiles in one wave however the rows are spread: decode.  Otherwise only the group list tells, and the kernel that holds
+// both shapes decides; it needs the larger one's shared memory, whose place L1 then lacks.  256 experts, 7168 x 4096 with SiLU /
+// 2048 x 7168, us on the 160-row shape, the 32-row shape, through the choice: 32 tokens x 8: 1124, 999, 1029 / 590, 525, 545; 256 tokens
+// x 8: 1706, 1532, 1570 / 902, 797, 830; 1024 rows by popularity: 1245, 1234, 1281; 2048 rows on one expert: 123, 337, 122.  Two
+// launches of which one leaves at once came to the same for long calls and cost short ones 4 us.
+template <bool GATE_UP>
+static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, int64_t max_rows, cudaStream_t s) {
+    if (a.M > 8LL * a.G) return launch_one<GATE_UP, Which::kPrefill>(tx, txs, packed, a, s);
+    const long long experts = std::min(a.G, a.M);
+    const long long tiles = (experts + (a.M - experts) / Decode::kMaxR) * (a.N / kTileN);  // at most
+    if (std::min<int64_t>(max_rows, a.M) <= Decode::kMaxR || tiles <= grid_ctas())
+        return launch_one<GATE_UP, Which::kDecode>(tx, txs, packed, a, s);
+    return launch_one<GATE_UP, Which::kEither>(tx, txs, packed, a, s);
 }
 
 // [G, K, N] int8 -> the packed order.  One thread writes one lane's 16 bytes of a k-chunk.
@@ -677,7 +736,7 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
                          const float* x_rowsum, const int64_t* group_list, void* y, const int64_t* row_code,
                          void* const* dst_base, int64_t n_base,
                          int64_t dst_rows, int64_t M, int64_t K, int64_t N, int64_t G, int group_list_type, int gate_up_silu,
-                         void* workspace, size_t workspace_bytes, void* stream) {
+                         int64_t max_rows, void* workspace, size_t workspace_bytes, void* stream) {
     if (group_list_type != B200MOE_GROUP_LIST_CUMSUM && group_list_type != B200MOE_GROUP_LIST_COUNTS)
         return B200MOE_ERR_ARGUMENT;
     if (M < 0 || K <= 0 || N <= 0 || G <= 0 || G > kMaxExperts || M > 0x7FFFFFF0LL || K > 0x7FFFFFF0LL ||
@@ -730,11 +789,7 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
     if (rc != B200MOE_OK) return rc;
     rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)M, (uint64_t)K, pk::kSmallBox, pk::kBK, true);
     if (rc != B200MOE_OK) return rc;
-    // The 32-row shape where the experts have at most eight rows on average (a decode step): a larger expert is then cut
-    // into tiles of 32 rows that each dequantise its weights, at most M / 32 of them in all.
-    const bool decode = M <= 8 * G;
-    if (gate_up_silu) return decode ? pk::launch<true, pk::Decode>(tx, txs, packed, a, s) : pk::launch<true, pk::Prefill>(tx, txs, packed, a, s);
-    return decode ? pk::launch<false, pk::Decode>(tx, txs, packed, a, s) : pk::launch<false, pk::Prefill>(tx, txs, packed, a, s);
+    return gate_up_silu ? pk::launch<true>(tx, txs, packed, a, max_rows, s) : pk::launch<false>(tx, txs, packed, a, max_rows, s);
 }
 
 extern "C" int b200moe_grouped_gemm_int8_packed(const void* x, const void* packed, const void* scale, const void* offset,
@@ -742,7 +797,7 @@ extern "C" int b200moe_grouped_gemm_int8_packed(const void* x, const void* packe
                                                 int64_t G, int group_list_type, int gate_up_silu, void* workspace,
                                                 size_t workspace_bytes, void* stream) {
     return packed_launch(x, packed, scale, offset, nullptr, group_list, y, nullptr, nullptr, 0, 0, M, K, N, G, group_list_type,
-                         gate_up_silu, workspace, workspace_bytes, stream);
+                         gate_up_silu, M, workspace, workspace_bytes, stream);
 }
 
 extern "C" int b200moe_grouped_gemm_int8_packed_rowsum(const void* x, const void* packed, const void* scale,
@@ -752,7 +807,17 @@ extern "C" int b200moe_grouped_gemm_int8_packed_rowsum(const void* x, const void
                                                        size_t workspace_bytes, void* stream) {
     if (offset != nullptr && x_rowsum == nullptr) return B200MOE_ERR_NULL_POINTER;
     return packed_launch(x, packed, scale, offset, x_rowsum, group_list, y, nullptr, nullptr, 0, 0, M, K, N, G,
-                         group_list_type, gate_up_silu, workspace, workspace_bytes, stream);
+                         group_list_type, gate_up_silu, M, workspace, workspace_bytes, stream);
+}
+
+extern "C" int b200moe_grouped_gemm_int8_packed_bounded(const void* x, const void* packed, const void* scale,
+                                                        const void* offset, const float* x_rowsum, const int64_t* group_list,
+                                                        void* y, int64_t M, int64_t K, int64_t N, int64_t G,
+                                                        int group_list_type, int gate_up_silu, int64_t max_rows,
+                                                        void* workspace, size_t workspace_bytes, void* stream) {
+    if (max_rows < 0) return B200MOE_ERR_ARGUMENT;
+    return packed_launch(x, packed, scale, offset, x_rowsum, group_list, y, nullptr, nullptr, 0, 0, M, K, N, G,
+                         group_list_type, gate_up_silu, max_rows, workspace, workspace_bytes, stream);
 }
 
 extern "C" int b200moe_grouped_gemm_int8_packed_scatter(const void* x, const void* packed, const void* scale,
@@ -763,5 +828,5 @@ extern "C" int b200moe_grouped_gemm_int8_packed_scatter(const void* x, const voi
                                                         void* stream) {
     if (row_code == nullptr) return B200MOE_ERR_NULL_POINTER;
     return packed_launch(x, packed, scale, offset, nullptr, group_list, nullptr, row_code, dst_base, n_base, dst_rows, M, K, N, G,
-                         group_list_type, 0, workspace, workspace_bytes, stream);
+                         group_list_type, 0, M, workspace, workspace_bytes, stream);
 }

@@ -160,13 +160,14 @@ class MoELayer:
         if self.mid_hook is not None:
             self.mid_hook()
 
-    def _experts(self, rows, counts, record, y=None, n_rows=None, scatter=None, rows_sum=None):
+    def _experts(self, rows, counts, record, y=None, n_rows=None, scatter=None, rows_sum=None, max_rows=None):
         """rows [R, H] expert-major with per-local-expert counts -> [R, H] (into ``y`` when given).
         ``n_rows``: int64 device tensor with the number of rows in use when R is only a capacity.
         ``scatter`` = (row_code, destination pointers, destination rows): the down projection stores
         each result row where its code says (the return buffer of the rank the token came from) instead
         of into ``y``; packed GEMMs only.  ``rows_sum``: fp32 sums of the rows when the caller has them (the
-        packed gate/up GEMM then skips its own pass over the rows)."""
+        packed gate/up GEMM then skips its own pass over the rows).  ``max_rows``: rows an expert has at most,
+        where that is known."""
         R = rows.shape[0]
         if y is None:
             y = torch.empty(R, self.hidden, dtype=torch.bfloat16, device=self.device)
@@ -190,7 +191,7 @@ class MoELayer:
         if self.gemm == "packed":
             act = torch.empty(R, self.inter, dtype=torch.bfloat16, device=self.device)
             ops.grouped_gemm_packed(rows, self.w13, self.s13, self.o13, counts, act, group_list_type=1,
-                                    gate_up_silu=True, x_rowsum=rows_sum)
+                                    gate_up_silu=True, x_rowsum=rows_sum, max_rows=max_rows)
             if ev:
                 ev[1].record()
                 ev[2].record()
@@ -198,7 +199,7 @@ class MoELayer:
                 ops.grouped_gemm_packed_scatter(act, self.w2, self.s2, self.o2, counts, scatter[0], scatter[1], scatter[2],
                                                 group_list_type=1)
             else:
-                ops.grouped_gemm_packed(act, self.w2, self.s2, self.o2, counts, y, group_list_type=1)
+                ops.grouped_gemm_packed(act, self.w2, self.s2, self.o2, counts, y, group_list_type=1, max_rows=max_rows)
             if ev:
                 ev[3].record()
                 self.timing = ev
@@ -285,7 +286,8 @@ class MoELayer:
 
         if self.world == 1:
             self._mid()
-            y = self._experts(send, counts, record, rows_sum=sums)
+            # (a token's experts differ, so none has more rows than there are tokens)
+            y = self._experts(send, counts, record, rows_sum=sums, max_rows=x.shape[0])
             mark("experts")
             out = finish(y, slot, wts)
             mark("combine")

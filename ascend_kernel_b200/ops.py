@@ -257,11 +257,12 @@ def pack_weight_int8(weight, gate_up: bool = False):
 
 
 def grouped_gemm_packed(x, packed, scale, offset, group_list, output, group_list_type: int = 0,
-                        gate_up_silu: bool = False, return_workspace: bool = False, x_rowsum=None):
+                        gate_up_silu: bool = False, return_workspace: bool = False, x_rowsum=None, max_rows=None):
     """int8 grouped GEMM on weights from :func:`pack_weight_int8`; ``scale`` / ``offset`` bf16 [G, N] in
     the original column order.  ``gate_up_silu``: output [M, N/2] = bf16(silu(gate) * up).  ``x_rowsum``: fp32
     [M] sums of the rows of x when the caller has them (``gather_rows(..., with_sums=True)``): the launch then
-    makes no pass of its own over x for the offset term."""
+    makes no pass of its own over x for the offset term.  ``max_rows``: rows an expert has at most where the caller knows it
+    (it helps to choose the kernel, the result does not depend on it)."""
     _need_cuda(x=x, packed=packed, scale=scale, offset=offset, group_list=group_list, output=output, x_rowsum=x_rowsum)
     if x_rowsum is not None and (x_rowsum.dtype != torch.float32 or x_rowsum.numel() < x.shape[0]):
         raise RuntimeError("x_rowsum must be float32 with one element per row of x")
@@ -280,15 +281,10 @@ def grouped_gemm_packed(x, packed, scale, offset, group_list, output, group_list
     need = _lib.b200moe_grouped_gemm_workspace_bytes(M, K, N, G, CT["int8"], LAYOUT["canonical"])
     ws = _workspace(need, x.device)
     with torch.cuda.device(x.device):
-        if x_rowsum is not None and offset is not None:
-            rc = _lib.b200moe_grouped_gemm_int8_packed_rowsum(_ptr(x), _ptr(packed), _ptr(scale), _ptr(offset),
-                                                              _ptr(x_rowsum), _ptr(group_list), _ptr(output), M, K, N, G,
-                                                              group_list_type, int(bool(gate_up_silu)), _ptr(ws), need,
-                                                              _stream())
-        else:
-            rc = _lib.b200moe_grouped_gemm_int8_packed(_ptr(x), _ptr(packed), _ptr(scale), _ptr(offset), _ptr(group_list),
-                                                       _ptr(output), M, K, N, G, group_list_type, int(bool(gate_up_silu)),
-                                                       _ptr(ws), need, _stream())
+        rc = _lib.b200moe_grouped_gemm_int8_packed_bounded(_ptr(x), _ptr(packed), _ptr(scale), _ptr(offset), _ptr(x_rowsum),
+                                                           _ptr(group_list), _ptr(output), M, K, N, G, group_list_type,
+                                                           int(bool(gate_up_silu)), M if max_rows is None else int(max_rows),
+                                                           _ptr(ws), need, _stream())
     _abi.check(rc, "grouped_gemm_packed")
     if M > 0:
         _count(1 + (offset is not None and x_rowsum is None))

@@ -147,6 +147,14 @@ int b200moe_grouped_gemm_int8_packed_rowsum(const void* x, const void* packed, c
                                             const float* x_rowsum, const int64_t* group_list, void* y, int64_t M,
                                             int64_t K, int64_t N, int64_t G, int group_list_type, int gate_up_silu,
                                             void* workspace, size_t workspace_bytes, void* stream);
+/* Both (x_rowsum as above or NULL: the launch makes the sums), for a caller that knows how many rows an expert can have, e.g. a
+ * layer's number of tokens where each picks different experts.  max_rows only helps to choose the kernel's tile
+ * shape on the host; the result does not depend on it, also where an expert has more rows.  (No reference
+ * counterpart.) */
+int b200moe_grouped_gemm_int8_packed_bounded(const void* x, const void* packed, const void* scale, const void* offset,
+                                             const float* x_rowsum, const int64_t* group_list, void* y, int64_t M,
+                                             int64_t K, int64_t N, int64_t G, int group_list_type, int gate_up_silu,
+                                             int64_t max_rows, void* workspace, size_t workspace_bytes, void* stream);
 
 /* b200moe_grouped_gemm_int8_packed (gate_up_silu == 0) whose result rows go where a table says instead of
  * into one [M, N] tensor (no reference counterpart; it is the down projection of an expert-parallel layer

@@ -161,3 +161,29 @@ def test_packed_decode_shape_matches_oracle_and_generic_kernel(counts, K, N):
     h = gold.to(torch.bfloat16).float()
     want = (torch.nn.functional.silu(h[:, :N // 2]) * h[:, N // 2:]).to(torch.bfloat16).float()
     assert O.rel_l2(act.float().cpu(), want) < 4e-3
+
+
+@pytest.mark.parametrize("counts,N", [
+    ([8] * 64, 4096),                        # the same tiles in both shapes: 32 rows
+    ([512] + [0] * 63, 4096),                # two waves of 32-row tiles, one of 160-row tiles: 160 rows
+    ([300] + [0] * 39, 1024),                # more tiles, but one wave of either: 32 rows
+    ([33] * 8 + [0, 1, 2] + [0] * 53, 4096), # one row over a tile on every large expert
+])
+def test_tile_shape_chosen_from_the_group_list(counts, N):
+    """At most eight rows an expert on average, spread in a way that only the group list tells: whatever the kernel chooses,
+    and whatever bound the caller states (a wrong one among them), the result is the same."""
+    import ascend_kernel_b200 as ak
+
+    x, w, scale, offset, cnt = _int8_case(counts, 192, N, 23, True, extra_rows=0)
+    assert 32 < x.shape[0] <= 8 * len(counts)
+    gold = O.golden_f32(x, w, scale, offset, cnt, "int8", O.GROUP_LIST_COUNTS)
+    d = [t.cuda() for t in (x, ak.pack_weight_int8(w.cuda()), scale, offset, cnt)]
+    outs = []
+    for bound in (None, max(counts), 1):
+        out = torch.full((x.shape[0], N), SENTINEL, dtype=torch.bfloat16, device="cuda")
+        ws = ak.grouped_gemm_packed(*d, out, group_list_type=1, return_workspace=True, max_rows=bound)
+        torch.cuda.synchronize()
+        assert ak.read_status(ws) == (0, 0)
+        outs.append(out)
+    assert_close_to_golden(outs[0], gold)
+    assert all(torch.equal(o.view(torch.int16), outs[0].view(torch.int16)) for o in outs[1:])
