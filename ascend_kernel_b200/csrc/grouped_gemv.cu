@@ -13,6 +13,8 @@
 // scale and offset are applied in the fp32 epilogue and the result is rounded to bf16 once.
 // int8 items with 2..4 rows, fp8 items and fp4 items use the tensor core for the multiply-adds
 // (gv_compute_mma, gv_compute_fp4_mma); fp4 falls back to fp32 FMAs for x rows that are not exact in f16.
+#include <algorithm>
+
 #include <cuda_fp16.h>
 
 #include <cstdlib>
@@ -1064,9 +1066,13 @@ static int gv_launch(const GemvArgs& a0, cudaStream_t stream) {
     a.by_rows = smem <= 110 * 1024 || (smem <= 226 * 1024 && gv_smem_bytes(a.G, a.K, false) > 110 * 1024);
     if (!a.by_rows) smem = gv_smem_bytes(a.G, a.K, false);
     if (smem > 227 * 1024) return B200MOE_ERR_SHAPE;
+    // One CTA a multiprocessor: room for exactly one.  A kernel that starts beside the one before it has its CTAs put wherever
+    // there is room, and where two fitted, some SMs got two and others none (stored fp4, 16 tokens x 8 over 64 experts,
+    // 10240 x 1024, 115 KB: 236 us; 188 with one on each).
+    const int per_sm = smem <= 110 * 1024 ? 2 : 1;
+    if (per_sm == 1) smem = std::max<size_t>(smem, 116 * 1024);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemv_kernel<MODE, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    const int per_sm = smem <= 110 * 1024 ? 2 : 1;
     // (behind gv_begin_kernel or the fp4 prepass; the fp32 kernel of fp4 stays behind the tensor-core one)
     if (PATH != 2) {
         B200MOE_CUDA_TRY(launch_dependent(grouped_gemv_kernel<MODE, PATH>, (unsigned)(per_sm * sm_count()), kGvThreads, smem, stream, a));

@@ -296,3 +296,39 @@ def test_plain_workspace_runs_without_splitting(ct, counts):
     assert rc == 0 and ak.read_status(ws) == (0, 0)
     assert bool((ws[need:] == 0x5A).all())
     assert_close_to_golden(out, gold, ulps=1.0 if ct == "int8" else 2.0)
+
+
+@pytest.mark.parametrize("ct,G,K", [
+    ("int8", 4, 10240),    # one CTA a multiprocessor, with room for a second but for the padding
+    ("fp4", 4, 10240),
+    ("int8", 36, 9920),    # the order by rows would cost the second CTA of a multiprocessor: the experts' own order
+    ("fp8", 80, 9856),
+    ("fp4", 36, 9920),
+    ("fp4", 36, 24832),    # the order by rows does not fit at all
+])
+def test_large_k_matches_oracle(ct, G, K):
+    import ascend_kernel_b200 as ak
+
+    gen = torch.Generator().manual_seed(K)
+    N, used = 256, [0, 1, G - 2, G - 1]
+    cnt = torch.zeros(G, dtype=torch.int64)
+    cnt[used] = torch.tensor([2, 5, 1, 4])
+    x = torch.randn(12, K, generator=gen).to(torch.bfloat16)
+    if ct == "fp4":
+        w = torch.randint(0, 256, (4, K, N // 2), generator=gen, dtype=torch.uint8)
+        scale = (torch.rand(4, K // 16, N, generator=gen) * 0.09 + 0.01).to(torch.bfloat16)
+    elif ct == "fp8":
+        w = torch.randint(0, 256, (4, K, N), generator=gen, dtype=torch.uint8)
+        scale = torch.randn(4, K // 128, N // 128, generator=gen)
+    else:
+        w = torch.randint(-128, 128, (4, K, N), generator=gen, dtype=torch.int8)
+        scale = (torch.rand(4, N, generator=gen) * 0.009 + 0.001).to(torch.bfloat16)
+    gold = O.golden_f32(x, w, scale, None, cnt[used], ct, O.GROUP_LIST_COUNTS, weight_layout="canonical", gemv=True)
+    wd = torch.zeros(G, *w.shape[1:], dtype=w.dtype, device="cuda")
+    sd = torch.zeros(G, *scale.shape[1:], dtype=scale.dtype, device="cuda")
+    wd[used], sd[used] = w.cuda(), scale.cuda()
+    for lay in ("canonical", "ascend") if ct == "fp4" else ("canonical",):
+        weights = ak.fp4_layout(wd, to_ascend=True) if lay == "ascend" else wd
+        out, st = run_gemv(x, weights, sd, cnt, ct, gl_type=1, layout=lay)
+        assert st == (0, 0)
+        assert_close_to_golden(out, gold, ulps=1.0 if ct == "int8" else 2.0)
