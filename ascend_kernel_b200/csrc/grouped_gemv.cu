@@ -918,7 +918,8 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
         if (*reinterpret_cast<volatile int*>(a.status + 3) == 0) return;
     }
     __shared__ GvUnit un;
-    __shared__ int s_ticket;
+    __shared__ int s_ticket, s_parts, s_part_rows;
+    __shared__ unsigned s_per_pass, s_units;
     const int n_slabs = (a.N + kGvSlabN - 1) / kGvSlabN;
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
     if (threadIdx.x < 32) {
@@ -952,27 +953,28 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
         }
         if (threadIdx.x == 0) pass_start[a.G] = total;
         const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K);
-        if (threadIdx.x == 0) un.n_split = parts;
+        if (threadIdx.x == 0) {
+            // (kept in shared memory: a unit's loop needs every register)
+            s_parts = parts;
+            s_per_pass = (unsigned)(n_slabs * parts);  // units of one pass
+            s_units = (unsigned)total * s_per_pass;    // (32 bits hold every unit number: y alone would take 2 TB with 2^30 units)
+            s_part_rows = ((a.K + kGvPartRows - 1) / kGvPartRows + parts - 1) / parts * kGvPartRows;
+        }
     }
     __syncthreads();
 
     grid_dep_wait();  // (the prologue above ran beside the kernel that zeroes the tickets and counters)
-    const int n_parts = un.n_split;
-    const unsigned per_pass = (unsigned)(n_slabs * n_parts);  // units of one pass
-    // (32 bits hold every unit number: y alone would take 2 TB with 2^30 units)
-    const unsigned n_units = (unsigned)pass_start[a.G] * per_pass;
-    const int part_rows = ((a.K + kGvPartRows - 1) / kGvPartRows + n_parts - 1) / n_parts * kGvPartRows;
     int next = 0;  // thread 0: the ticket drawn last
     gv_draw(a, next);
     for (;;) {
         if (threadIdx.x == 0) s_ticket = next;
         __syncthreads();
         const unsigned unit = (unsigned)(s_ticket - (PATH == 2 ? 1 : 0));
-        if (unit >= n_units) break;
+        if (unit >= s_units) break;
         // every thread looks at its experts, the one that finds the unit describes it to the others: a binary search
         // with its divisions by one thread was a tenth of a short unit (2048 rows of fp4)
         for (int i = threadIdx.x; i < a.G; i += kGvThreads) {
-            const unsigned first = (unsigned)pass_start[i] * per_pass, passes = (unsigned)(pass_start[i + 1] - pass_start[i]);
+            const unsigned per_pass = s_per_pass, first = (unsigned)pass_start[i] * per_pass, passes = (unsigned)(pass_start[i + 1] - pass_start[i]);
             if (unit < first || unit - first >= passes * per_pass) continue;
             const int g = a.by_rows ? order[i] : i;
             // expert-major order: the CTAs that run at the same time hold neighbouring slabs of the same experts
@@ -980,6 +982,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             // (DRAM pages stay open: measured +1..6 % over slab-major order); the passes of a slab are
             // adjacent, so all but the first find its weights in L2
             const unsigned j = (unit - first) / passes, pass = (unit - first) - j * passes;
+            const int n_slabs = (a.N + kGvSlabN - 1) / kGvSlabN, n_parts = s_parts;
             const int split = (int)(j / (unsigned)n_slabs), slab = (int)j - split * n_slabs;
             un.g = g;
             un.n0 = slab * kGvSlabN;
@@ -988,8 +991,8 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             un.split = split;
             un.n_split = n_parts;
             un.slot = n_parts > 1 ? ((pass_start[i] + (int)pass) * n_slabs + slab) * n_parts : 0;
-            un.k0 = split * part_rows;
-            un.k1 = min(un.k0 + part_rows, a.K);
+            un.k0 = split * s_part_rows;
+            un.k1 = min(un.k0 + s_part_rows, a.K);
         }
         __syncthreads();
         {
