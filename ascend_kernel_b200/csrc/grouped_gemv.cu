@@ -867,6 +867,7 @@ __global__ void __launch_bounds__(256) gv_fp4_prepare_x_kernel(const __nv_bfloat
     }
     if (bad) atomicOr(&s_bad, 1);
     __syncthreads();
+    grid_dep_wait();  // (launched beside gv_begin_kernel, which zeroes the status words; what follows this kernel also follows that)
     if (threadIdx.x == 0) {
         xexp[row] = s_bad ? kGvNotF16 : sh;
         if (s_bad) atomicMax(status + 3, 1);
@@ -1168,9 +1169,10 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     if (compute_type == B200MOE_CT_FP4 && !fp4_scalar) {
         a.xexp = reinterpret_cast<const int*>(ws);
         a.x16 = reinterpret_cast<const __half*>(ws + gv_fp4_exp_bytes(M));
-        gv_fp4_prepare_x_kernel<<<(unsigned)M, 256, 0, s>>>(a.x, const_cast<__half*>(a.x16), const_cast<int*>(a.xexp), a.K,
-                                                                a.status);
-        B200MOE_CUDA_TRY(cudaGetLastError());
+        // (beside gv_begin_kernel: 8 experts, 4 tokens x 2, 512 x 1024, stored order: 22.6 us one after the other, 20.5 so; a memset
+        // in the place of gv_begin_kernel: 21 .. 24)
+        B200MOE_CUDA_TRY(launch_dependent(gv_fp4_prepare_x_kernel, (unsigned)M, 256, 0, s, a.x, const_cast<__half*>(a.x16),
+                                          const_cast<int*>(a.xexp), a.K, a.status));
     }
     switch (compute_type) {
         case B200MOE_CT_INT8: return gv_launch<B200MOE_CT_INT8>(a, s);
