@@ -135,12 +135,14 @@ class MoELayer:
 
     @property
     def bf13(self):
-        """FP4-stored experts only: the gate/up weights as the bf16 values a pass multiplies with."""
+        """FP4-stored experts only: the gate/up weights as the bf16 values a pass multiplies with, in a new tensor at each
+        access (four times the stored size; a pass itself needs none)."""
         return self._dequantised(self.w13, self.s13, 2 * self.inter)
 
     @property
     def bf2(self):
-        """FP4-stored experts only: the down projection's weights as the bf16 values a pass multiplies with."""
+        """FP4-stored experts only: the down projection's weights as the bf16 values a pass multiplies with, in a new tensor
+        at each access."""
         return self._dequantised(self.w2, self.s2, self.hidden)
 
     def read_status(self, clear: bool = True):

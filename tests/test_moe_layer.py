@@ -354,6 +354,39 @@ def test_layer_on_fp4_stored_experts_matches_oracle():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,k", [(1, 1), (300, 2)])
+def test_fp4_layer_multiplies_with_the_dequantised_weights(T, k):
+    """The pass itself against its phases one after the other on the same routed rows -- dequantise, bf16 grouped GEMM, SiLU(gate) *
+    up, dequantise, bf16 grouped GEMM, weighted sum: the same bits."""
+    import ascend_kernel_b200 as ak
+    from ascend_kernel_b200.moe_layer import CudaRowOps, MoELayer
+
+    gen = torch.Generator().manual_seed(19)
+    H, E, I = 256, 8, 384
+    x = torch.randn(T, H, generator=gen).to(torch.bfloat16).cuda()
+    logits = torch.randn(T, E, generator=gen).to(torch.bfloat16).cuda()
+    c13 = torch.randint(0, 256, (E, H, I), generator=gen, dtype=torch.uint8).cuda()
+    s13 = torch.randint(119, 128, (E, H, 2 * I // 32), generator=gen, dtype=torch.uint8).cuda()
+    c2 = torch.randint(0, 256, (E, I, H // 2), generator=gen, dtype=torch.uint8).cuda()
+    s2 = torch.randint(119, 128, (E, I, H // 32), generator=gen, dtype=torch.uint8).cuda()
+    got = MoELayer(c13, s13, None, c2, s2, None, E, k, weight_format="fp4").forward(x, logits)
+
+    _, wts, counts, token_of, slot = CudaRowOps.route(logits, k)
+    rows = CudaRowOps.gather_rows(x, token_of)
+    w13 = torch.empty(E, H, 2 * I, dtype=torch.bfloat16, device="cuda")
+    w2 = torch.empty(E, I, H, dtype=torch.bfloat16, device="cuda")
+    ak.fp4_dequant(c13, s13, w13)
+    ak.fp4_dequant(c2, s2, w2)
+    h = torch.empty(T * k, 2 * I, dtype=torch.bfloat16, device="cuda")
+    y = torch.empty(T * k, H, dtype=torch.bfloat16, device="cuda")
+    ak.grouped_gemm(rows, w13, None, None, counts, "bf16", h, group_list_type=1)
+    ak.grouped_gemm(ak.silu_mul(h), w2, None, None, counts, "bf16", y, group_list_type=1)
+    want = CudaRowOps.combine(y, slot, wts)
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.gpu
 def test_layer_reports_device_findings():
     """MoELayer.read_status raises when a kernel of an earlier pass left a finding (here: a grouped GEMM
     called directly with a group list that is not monotone) and is quiet otherwise."""
