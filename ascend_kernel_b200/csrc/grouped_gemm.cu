@@ -20,7 +20,7 @@
 //               registers (128-bit coalesced loads, prefetched two of the group's stages ahead) ->
 //               bf16 tile in the UMMA MN-major 128-byte-swizzle layout
 // One ring of 3 stages (x boxes 32 KB + bf16 weights 32 KB), one full and one empty barrier per
-// stage: the single MMA-issuing thread pays one wait and one commit per stage.  Shared-memory bandwidth bounds this kernel (the
+// stage: the MMA warp pays one wait and one commit per stage.  Shared-memory bandwidth bounds this kernel (the
 // tensor core alone reads 48 KB per 64-k stage), so packed weights go through registers, not
 // through a shared-memory staging ring, and the bf16 tile is written without bank conflicts.
 // Weights never make a round trip through global memory.  Every wait is bounded; on expiry the
@@ -96,7 +96,7 @@ struct GmTraits {
     static constexpr bool kDirect = (MODE == B200MOE_CT_BF16);
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
-    // columns instead of 16 (222 -> 22 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
+    // columns instead of 16 (222 -> 14 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
     static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
     // Who turns a published tile number into rows and columns: the publisher, once, or each role for itself.  Resolved
     // entries cost the roles less at a tile switch but leave the dequant loop of the modes with 4 rows x 16 columns a thread
@@ -412,7 +412,7 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
         for (int i = 0; i < 8; ++i) v[i] = ldg_stream4(it.wp + (size_t)i * row_bytes);
         r.q[0] = make_uint4(v[0], v[1], v[2], v[3]);
         r.q[1] = make_uint4(v[4], v[5], v[6], v[7]);
-        // in units of the 8 scales a thread loads (fits 32 bits: the weights would be 17 TB otherwise)
+        // in units of the 8 scales a thread loads (fits 32 bits: 2^32 of them are the scales of 2.2 TB of weights)
         r.e[0] = (uint32_t)((((size_t)it.g * (a.K >> 7) + ((it.kt * kBK) >> 7)) * a.N + it.n0) >> 3) + d.chunk;
         return;
     }
@@ -685,7 +685,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             bool ok = true;
             // This thread runs furthest ahead (its L2 prefetch leads everything else), so it draws the
             // tiles.  One ticket is always held in hand, so the atomic's latency is off the path.
-            int* ticket = a.status + 2;  // zeroed by the host before the launch
+            int* ticket = a.status + 2;  // zero at the start: by a memset before the launch, or by the row sums' kernel
             int held = atomicAdd(ticket, 1);
             StageIter far;  // the tile published last
             far.kt = 0;

@@ -297,7 +297,7 @@ __device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUt
         if (lane == 0) {
             uint32_t ia = 0, seq = 0, published = 0;
             bool ok = true;
-            int* ticket = a.status + 2;  // zeroed by the host before the launch
+            int* ticket = a.status + 2;  // zero at the start: by a memset before the launch, or by the row sums' kernel
             int held = atomicAdd(ticket, 1);
             TileInfo far_ti;  // the tile published last, resolved
             auto publish = [&]() -> bool {

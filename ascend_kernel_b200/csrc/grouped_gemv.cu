@@ -898,9 +898,9 @@ __device__ __forceinline__ int gv_choose_parts(int slabs, int ctas, int K) {
 }
 
 // fp4 is launched as two kernels over the same work items: PATH 1 takes the passes whose x rows are all exact as
-// scaled f16 (tensor-core path), PATH 2 the others (fp32 multiply-adds; normally none, and the kernel leaves after
-// walking the item list); PATH 0: every other mode, and fp4 without the prepass.  Separate kernels keep the
-// registers of one path from weighing on the other.  PATH 2 leaves at once when the prepass found no such row.
+// scaled f16 (tensor-core path), PATH 2 the others (fp32 multiply-adds; normally none: the kernel leaves at once when the
+// prepass found no such row); PATH 0: every other mode, and fp4 without the prepass.  Separate kernels keep the
+// registers of one path from weighing on the other.
 template <int MODE, int PATH = 0>
 __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
