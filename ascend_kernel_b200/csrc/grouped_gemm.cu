@@ -105,6 +105,7 @@ struct GmTraits {
     // (in runs of their own) int4 9000 | 8616, stored fp4 4838 | 4875, fp4 with e8m0 scales 4602 | 4598, SiLU 5265 | 5039.  32 rows an
     // expert, 2048 x 7168: int8 1282 | 1299, fp8 1490 | 1921, canonical fp4 1288 | 1619, int4 2326 | 2104, stored fp4 1238 |
     // 1181, e8m0 1425 | 1159.  64 experts of 210 rows, 1280 x 512: int8 52.3 | 50.3, bf16 35.9 | 34.9, stored fp4 30.8 | 28.9.
+    // int8 has both, by the length of its tiles (kInt8RolesK).
     static constexpr bool kResolved = MODE != B200MOE_CT_INT8 && MODE != B200MOE_CT_FP8 && MODE != B200MOE_CT_FP4;
 };
 
@@ -371,7 +372,7 @@ __device__ __forceinline__ void dq_locate(DqIter& it, const uint8_t* __restrict_
              : T::kNibbles        ? chunk_col<SPLIT>(it.n0, d.c16, a.N) >> 1
                                   : it.n0 + d.c16 * 16);
 }
-template <int MODE, bool SPLIT>
+template <int MODE, bool SPLIT, bool RESOLVED>
 __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* __restrict__ w, const GemmArgs& a,
                                            const DqLane& d, int n_kt, const int* tile_prefix, const int* row_start, int n_nt, GmBarriers* sb) {
     using T = GmTraits<MODE>;
@@ -383,7 +384,7 @@ __device__ __forceinline__ void dq_advance(DqIter& it, int step, const uint8_t* 
     do {
         it.kt -= n_kt;
         TileInfo ti;
-        it.valid = next_tile<T::kResolved>(sb, it.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
+        it.valid = next_tile<RESOLVED>(sb, it.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
         it.g = ti.g;
         it.n0 = ti.n0;
     } while (it.kt >= n_kt && it.valid);
@@ -622,7 +623,7 @@ __device__ __forceinline__ constexpr int acc_pos(int i) {
 // SILU (int8, fp4 with e8m0 scales): int8 weight columns come as blocks of 128 gate columns followed by the 128
 // up columns of the same indices (fp4: gate columns first, paired here), and the epilogue writes bf16(silu(gate) * up), [M, N/2], instead of
 // the [M, N] product (gate and up are rounded to bf16 first, as the unfused operators would).
-template <int MODE, bool SILU>
+template <int MODE, bool SILU, bool RESOLVED>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xs,
                     const __grid_constant__ CUtensorMap tmap_w, const uint8_t* __restrict__ weight, const GemmArgs a) {
@@ -691,10 +692,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             far.kt = 0;
             auto publish = [&]() {
                 far.valid = held < n_tiles;
-                TileEntry entry = tile_entry(published + 1, T::kResolved ? 0u : ~0u, 0u, 0u, 0u);
+                TileEntry entry = tile_entry(published + 1, RESOLVED ? 0u : ~0u, 0u, 0u, 0u);
                 if (far.valid) {
                     far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
-                    entry = tile_entry(published + 1, (uint32_t)(T::kResolved ? far.ti.row0 : held), (uint32_t)far.ti.rows,
+                    entry = tile_entry(published + 1, (uint32_t)(RESOLVED ? far.ti.row0 : held), (uint32_t)far.ti.rows,
                                        (uint32_t)far.ti.g, (uint32_t)far.ti.n0 / kBN);
                 }
                 ring_store(&sb->tile_ring[published % kTileRing], entry);
@@ -715,7 +716,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             for (int i = 0; i < kL2Ahead && far.valid; ++i) far_step();
             for (;;) {
                 TileInfo ti;
-                if (!next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status) || !ok) break;
+                if (!next_tile<RESOLVED>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status) || !ok) break;
                 // The last row half of a tile often holds only a few rows of the expert (a second half
                 // of a dozen rows when an expert has a little over 128): a box of kSmallRows rows then
                 // replaces the 128-row box.  The MMA still reads 128 rows; what the rows beyond the box
@@ -772,7 +773,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         uint32_t seq = 0;
         for (;;) {
             TileInfo ti;
-            if (!__all_sync(0xffffffffu, next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
+            if (!__all_sync(0xffffffffu, next_tile<RESOLVED>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
             // accumulators of this tile: both for two halves, else the one used less recently;
             // the epilogue of their previous tile must have drained them
             const bool use0 = ti.halves == 2 || next1 == 0, use1 = ti.halves == 2 || next1 == 1;
@@ -835,7 +836,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         uint32_t use = 0, next1 = 0, seq = 0;
         for (;;) {
             TileInfo ti;
-            if (!__all_sync(0xffffffffu, next_tile<T::kResolved>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
+            if (!__all_sync(0xffffffffu, next_tile<RESOLVED>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status))) break;
             // a two-half tile: this group takes row half `grp`; a one-half tile sits in one accumulator
             bool mine = true;
             int half = grp;
@@ -968,13 +969,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         pf.seq = 0;
         {
             TileInfo ti;
-            pf.valid = next_tile<T::kResolved>(sb, pf.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
+            pf.valid = next_tile<RESOLVED>(sb, pf.seq, ti, tile_prefix, row_start, a.G, n_nt, a.status);
             pf.g = ti.g;
             pf.n0 = ti.n0;
         }
         pf.kt = 0;
         dq_locate<MODE, SPLIT>(pf, weight, a, d);
-        if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT>(pf, grp, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
+        if (grp > 0 && pf.valid) dq_advance<MODE, SPLIT, RESOLVED>(pf, grp, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
         PackedRegs<MODE> regs[kPrefetch];
         bool loaded[kPrefetch];
 #pragma unroll
@@ -982,7 +983,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             loaded[u] = pf.valid;
             if (pf.valid) {
                 load_packed<MODE, SPLIT>(regs[u], pf, a, d);
-                dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
+                dq_advance<MODE, SPLIT, RESOLVED>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
             }
         }
         const uint32_t sa0 = ptx::smem_u32(b_ring) + (T::kEightRows ? btile_offset(d.k0, d.chunk)
@@ -1012,7 +1013,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 loaded[u] = pf.valid;
                 if (pf.valid) {
                     load_packed<MODE, SPLIT>(regs[u], pf, a, d);
-                    dq_advance<MODE, SPLIT>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
+                    dq_advance<MODE, SPLIT, RESOLVED>(pf, kDqGroups, weight, a, d, n_kt, tile_prefix, row_start, n_nt, sb);
                 }
                 ib += kDqGroups;
             }
@@ -1086,14 +1087,21 @@ void launch_rowsum(const void* x, float* out, int64_t M, int64_t K, const int64_
                                                         reinterpret_cast<const long long*>(group_list), (int)G, gl_type, status);
 }
 
+// int8 tiles of fewer than 32 stages are resolved by the publisher.  Each role | publisher, us: 4 experts of 32 rows, 256 x 512: 13.2 |
+// 12.3; 32 of 300, 64 x 2048: 45.0 | 41.0; 128 experts, 32768 rows by popularity, 1024 x 4096: 489 | 474, its SiLU form 526 | 513; 64 of
+// 210, 1536 x 2048: 139.2 | 137.4, SiLU 154.7 | 155.9, 2048 x 2048: 172.6 | 170.8, SiLU 189.9 | 191.2; 128 of 32, 4096 x 2048: 363 |
+// 378, SiLU 376 | 398.
+constexpr int kInt8RolesK = 2048;
+
 static size_t gm_smem_bytes(int G) {
     return 1024 + (size_t)kNS * (kATileBytes + kBTileBytes) + kBarrierBytes + sizeof(float) * kEpiWarps * kEpiScaleFloats +
            sizeof(int) * 3 * (size_t)(G + 1);
 }
 
-template <int MODE, bool SILU = false>
+template <int MODE, bool SILU = false, bool RESOLVED = GmTraits<MODE>::kResolved>
 static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream_t stream) {
     using T = GmTraits<MODE>;
+    if (MODE == B200MOE_CT_INT8 && !RESOLVED && a.K < kInt8RolesK) return gm_launch<MODE, SILU, true>(x, w, a, stream);
     CUtensorMap tx, txs, tw;
     int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)a.M, a.K, kBM, kBK, true);
     if (rc != B200MOE_OK) return rc;
@@ -1107,13 +1115,13 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
                                 : a.N < kBN ? (uint32_t)(T::kNibbles ? a.N / 2 : a.N) : (uint32_t)T::kPRowBytes, false);
     if (rc != B200MOE_OK) return rc;
     const size_t smem = gm_smem_bytes(a.G);
-    B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, SILU, RESOLVED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
     if (a.rowsum != nullptr) {  // launch_rowsum came directly before
-        B200MOE_CUDA_TRY(launch_dependent(grouped_gemm_kernel<MODE, SILU>, (unsigned)sm_count(), kGemmThreads, smem, stream, tx, txs, tw,
+        B200MOE_CUDA_TRY(launch_dependent(grouped_gemm_kernel<MODE, SILU, RESOLVED>, (unsigned)sm_count(), kGemmThreads, smem, stream, tx, txs, tw,
                                           static_cast<const uint8_t*>(w), a));
     } else {
-        grouped_gemm_kernel<MODE, SILU><<<sm_count(), kGemmThreads, smem, stream>>>(tx, txs, tw, static_cast<const uint8_t*>(w), a);
+        grouped_gemm_kernel<MODE, SILU, RESOLVED><<<sm_count(), kGemmThreads, smem, stream>>>(tx, txs, tw, static_cast<const uint8_t*>(w), a);
         B200MOE_CUDA_TRY(cudaGetLastError());
     }
     return B200MOE_OK;

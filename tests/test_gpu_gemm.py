@@ -193,3 +193,22 @@ def test_group_list_scan(gl_type, gl, M, first_bad):
     assert st == ((0, 0) if first_bad is None else (1, first_bad))
     assert_close_to_golden(out, want)
     assert (out[bounds[-1]:].float() == SENTINEL).all()
+
+
+@pytest.mark.parametrize("K", [1984, 2048, 2112])  # 31, 32 and 33 stages a tile: the tiles' numbers are resolved in two places
+def test_int8_tiles_resolved_by_the_publisher_or_by_each_role(K):
+    import ascend_kernel_b200 as ak
+    from ascend_kernel_b200 import ops
+
+    counts, N = [300, 0, 129, 128, 1, 17], 768
+    x, w, scale, offset, cnt = _int8_case(counts, K, N, 33, True)
+    out, st = run_gemm(x, w, scale, offset, cnt, "int8", gl_type=1)
+    assert st == (0, 0)
+    assert_close_to_golden(out, O.golden_f32(x, w, scale, offset, cnt, "int8", O.GROUP_LIST_COUNTS))
+    wi, si, oi = (ops.interleave_gate_up(t.cuda()) for t in (w, scale, offset))
+    act = torch.full((x.shape[0], N // 2), SENTINEL, dtype=torch.bfloat16, device="cuda")
+    ws = ops.grouped_gemm_silu(x.cuda(), wi, si, oi, cnt.cuda(), act, group_list_type=1, return_workspace=True)
+    torch.cuda.synchronize()
+    assert ak.read_status(ws) == (0, 0)
+    n = sum(counts)
+    assert torch.equal(act[:n].view(torch.int16), ak.silu_mul(out)[:n].view(torch.int16))
