@@ -886,14 +886,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                                 const float4 su = *reinterpret_cast<const float4*>(es + kBN / 2 + c * 16 + 4 * q);
                                 const float4 ou = *reinterpret_cast<const float4*>(es + kBN + kBN / 2 + c * 16 + 4 * q);
                                 // accumulator positions (0,2,1,3) of a group of four hold columns 0..3
-                                g01 = pack_bf16x2(fmaf(og.x, rs, sg.x * __uint_as_float(rg[4 * q])),
-                                                  fmaf(og.y, rs, sg.y * __uint_as_float(rg[4 * q + 2])));
-                                g23 = pack_bf16x2(fmaf(og.z, rs, sg.z * __uint_as_float(rg[4 * q + 1])),
-                                                  fmaf(og.w, rs, sg.w * __uint_as_float(rg[4 * q + 3])));
-                                u01 = pack_bf16x2(fmaf(ou.x, rs, su.x * __uint_as_float(ru[4 * q])),
-                                                  fmaf(ou.y, rs, su.y * __uint_as_float(ru[4 * q + 2])));
-                                u23 = pack_bf16x2(fmaf(ou.z, rs, su.z * __uint_as_float(ru[4 * q + 1])),
-                                                  fmaf(ou.w, rs, su.w * __uint_as_float(ru[4 * q + 3])));
+                                g01 = pack_bf16x2(fmaf(og.x, rs, sg.x * s8_sum(rg[4 * q])),
+                                                  fmaf(og.y, rs, sg.y * s8_sum(rg[4 * q + 2])));
+                                g23 = pack_bf16x2(fmaf(og.z, rs, sg.z * s8_sum(rg[4 * q + 1])),
+                                                  fmaf(og.w, rs, sg.w * s8_sum(rg[4 * q + 3])));
+                                u01 = pack_bf16x2(fmaf(ou.x, rs, su.x * s8_sum(ru[4 * q])),
+                                                  fmaf(ou.y, rs, su.y * s8_sum(ru[4 * q + 2])));
+                                u23 = pack_bf16x2(fmaf(ou.z, rs, su.z * s8_sum(ru[4 * q + 1])),
+                                                  fmaf(ou.w, rs, su.w * s8_sum(ru[4 * q + 3])));
                             } else {
                                 auto two = [&](const uint32_t (&r)[16], int c) {
                                     return pack_bf16x2(__uint_as_float(r[acc_pos<MODE>(c)]), __uint_as_float(r[acc_pos<MODE>(c + 1)]));
@@ -936,10 +936,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                         float v0 = __uint_as_float(r[acc_pos<MODE>(4 * q)]), v1 = __uint_as_float(r[acc_pos<MODE>(4 * q + 1)]);
                         float v2 = __uint_as_float(r[acc_pos<MODE>(4 * q + 2)]), v3 = __uint_as_float(r[acc_pos<MODE>(4 * q + 3)]);
                         if (per_channel) {
-                            v0 = fmaf(o4.x, rs, s4.x * v0);
-                            v1 = fmaf(o4.y, rs, s4.y * v1);
-                            v2 = fmaf(o4.z, rs, s4.z * v2);
-                            v3 = fmaf(o4.w, rs, s4.w * v3);
+                            v0 = fmaf(o4.x, rs, s4.x * (kS8Unit * v0));
+                            v1 = fmaf(o4.y, rs, s4.y * (kS8Unit * v1));
+                            v2 = fmaf(o4.z, rs, s4.z * (kS8Unit * v2));
+                            v3 = fmaf(o4.w, rs, s4.w * (kS8Unit * v3));
                         }
                         o[2 * q] = pack_bf16x2(v0, v1);
                         o[2 * q + 1] = pack_bf16x2(v2, v3);

@@ -482,10 +482,10 @@ __device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUt
                 unsigned short ob[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    float o = fmaf(so0, rs[i], s0 * __uint_as_float(v0[i]));
+                    float o = fmaf(so0, rs[i], s0 * s8_sum(v0[i]));
                     if constexpr (GATE_UP) {
                         const float g = __bfloat162float(__float2bfloat16_rn(o));
-                        const float u = __bfloat162float(__float2bfloat16_rn(fmaf(so1, rs[i], s1 * __uint_as_float(v1[i]))));
+                        const float u = __bfloat162float(__float2bfloat16_rn(fmaf(so1, rs[i], s1 * s8_sum(v1[i]))));
                         o = __fdividef(g, 1.f + __expf(-g)) * u;
                     }
                     ob[i] = __bfloat16_as_ushort(__float2bfloat16_rn(o));

@@ -518,6 +518,7 @@ __device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, GvUnit& un, co
         if (m < un.rows) {
 #pragma unroll
             for (int w = 0; w < kGvMmaParts; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
+            if constexpr (MODE == B200MOE_CT_INT8) v[m] *= kS8Unit;
         }
     }
     gv_finish<MODE>(a, un, xsum, nullptr, v);
