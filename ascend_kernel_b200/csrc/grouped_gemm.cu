@@ -477,15 +477,29 @@ __device__ __forceinline__ uint4 pair_scales(const uint4& s) {
     return make_uint4(prmt(s.x, s.z, 0x5410u), prmt(s.x, s.z, 0x7632u), prmt(s.y, s.w, 0x5410u), prmt(s.y, s.w, 0x7632u));
 }
 
+// Whether the 2^126 that e2m1x8_to_bf16_tiny leaves out fits into the whole warp's scales (magnitudes below 4; no infinity or
+// NaN): the product of the scaled scale and the tiny code is then the one rounding of code * scale.
+__device__ __forceinline__ bool scales_take_2p126(const uint4& s) {
+    constexpr uint32_t kMag = 0x7FFF7FFFu, kUp = 0x3F803F80u;  // 0x4080 is the bf16 4.0: + 0x3F80 carries into bit 15
+    const uint32_t big = ((s.x & kMag) + kUp) | ((s.y & kMag) + kUp) | ((s.z & kMag) + kUp) | ((s.w & kMag) + kUp);
+    return __all_sync(0xffffffffu, (big & 0x80008000u) == 0u);
+}
+
 // Stored-order fp4: eight rows of eight columns; `sa` is the shared address of the thread's chunk in
 // its first row (a multiple of 8, so row i flips the chunk's swizzle bits by i and adds i * 128).
 __device__ __forceinline__ void convert_stage_fp4_ascend(const PackedRegs<kCtFp4Ascend>& r, uint32_t sa) {
-    const uint4 sc = pair_scales(r.s[0]);
+    uint4 sc = pair_scales(r.s[0]);
+    const bool tiny = scales_take_2p126(sc);
+    if (tiny) sc = make_uint4(mul_bf16x2(sc.x, kTwo126), mul_bf16x2(sc.y, kTwo126), mul_bf16x2(sc.z, kTwo126), mul_bf16x2(sc.w, kTwo126));
     const uint32_t w8[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         uint32_t v[4];
-        e2m1x8_to_bf16_pairs(w8[i], v);
+        e2m1x8_to_bf16_tiny(w8[i], v);
+        if (!tiny) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = mul_bf16x2(v[j], kTwo126);
+        }
         sts128((sa ^ (uint32_t)(i << 4)) + (uint32_t)(i * 128), mul_bf16x2(v[0], sc.x), mul_bf16x2(v[1], sc.y),
                mul_bf16x2(v[2], sc.z), mul_bf16x2(v[3], sc.w));
     }
@@ -500,6 +514,12 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
         if (in_scale) sf *= 1.329227995784916e36f;  // 2^120
     }
     const f32x2 sf2 = pack_f32x2(sf, sf);
+    bool tiny = false;
+    if constexpr (MODE == kCtFp4E8m0) {
+        // 2^(s - 127) * 2^126 = 2^(s - 1) is a bf16 up to s = 128 (s = 0 included: 2^-127 is a subnormal, 2^-1 is not)
+        tiny = __all_sync(0xffffffffu, max(max(r.e[0], r.e[1]), max(r.e[2], r.e[3])) <= 128u);
+    }
+    static_assert(kDqRows == 4, "scale bytes of a thread");
 #pragma unroll
     for (int j = 0; j < kDqRows; ++j) {
         const uint4 q = r.q[j];
@@ -532,14 +552,15 @@ __device__ __forceinline__ void convert_stage(const PackedRegs<MODE>& r, uint32_
         } else if constexpr (MODE == kCtFp4E8m0) {
             // 2^(s-127) as bf16: exponent field s; s = 0 is the subnormal 2^-127, 255 is NaN
             const uint32_t e = r.e[j];
-            const uint32_t sb = (e == 0 ? 0x0040u : (e == 255 ? 0x7FC0u : (e << 7))) * 0x10001u;
-            uint32_t v[4];
-            e2m1x8_to_bf16_pairs(q.x, v);
+            const uint32_t sb = tiny ? (e + 126u) * 0x800080u : (e == 0 ? 0x0040u : (e == 255 ? 0x7FC0u : (e << 7))) * 0x10001u;
+            e2m1x8_to_bf16_tiny(q.x, o);
+            e2m1x8_to_bf16_tiny(q.y, o + 4);
+            if (!tiny) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = mul_bf16x2(v[i], sb);
-            e2m1x8_to_bf16_pairs(q.y, v);
+                for (int i = 0; i < 8; ++i) o[i] = mul_bf16x2(o[i], kTwo126);
+            }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[4 + i] = mul_bf16x2(v[i], sb);
+            for (int i = 0; i < 8; ++i) o[i] = mul_bf16x2(o[i], sb);
         } else {  // FP4: 8 bytes = 16 codes; the thread's rows share one 16-row scale group
             const uint4 s0 = r.s[0], s1 = r.s[1];
             uint32_t v[4];
