@@ -29,3 +29,21 @@ def test_fp4_weights_for_scales_on_both_sides_of_four(layout):
     s[2] *= -1
     got = _readback(O.ascend_shuffle(w) if layout == "ascend" else w, s, "fp4", layout, G, K, N)
     assert torch.equal(got, O.dequant_fp4(w, s, round_bf16=True))
+
+
+def test_fp8_weights_for_scales_of_every_kind():
+    """Two-term bf16 products where the scale allows it, fp32 products elsewhere (large, tiny and tie-prone scales), every code."""
+    gen = torch.Generator().manual_seed(11)
+    G, K, N = 24, 256, 384
+    w = torch.arange(256, dtype=torch.uint8).repeat(G * K * N // 256).reshape(G, K, N)
+    w = w[:, torch.randperm(K, generator=gen)][:, :, torch.randperm(N, generator=gen)].contiguous()
+    s = torch.randn(G, K // 128, N // 128, generator=gen)
+    flat = s.view(-1)
+    # exact middles of two bf16 numbers for some significand, and one fp32 step to either side of them
+    tie = (257.0 / 256.0) / (1 + torch.arange(8, dtype=torch.float64) / 8)
+    special = torch.cat([torch.tensor([0.0, 127.9, -128.0, 300.0, 2.0 ** -90, 2.0 ** -91, 2.0 ** -100, 1.0, 1.00390625, -0.75]),
+                         tie.float(), torch.nextafter(tie.float(), torch.tensor(2.0)), torch.nextafter(tie.float(), torch.tensor(0.0)),
+                         torch.exp2(torch.rand(40, generator=gen) * 96 - 90)])
+    flat[:special.numel()] = special
+    got = _readback(w, s, "fp8", "canonical", G, K, N)
+    assert torch.equal(got, O.dequant_fp8(w, s, round_bf16=True))
