@@ -1,18 +1,15 @@
-// Grouped GEMV for decode-sized expert batches (HBM-bandwidth kernel).
+// Grouped GEMV for decode-sized expert batches (HBM-bandwidth kernels).
 //
-// Work unit = (up to 4 rows of a non-empty expert, slab of 256 output columns, part of the k range);
-// persistent CTAs (two per SM) draw units from a ticket counter, experts with the most rows first, the
-// passes of a slab next to one another (their weights are then read from L2), then the slabs.  K is cut
-// into parts only when whole columns would leave the chip idle (gv_choose_parts); the parts' fp32 sums meet
-// in the workspace and the CTA that finishes a slab last adds them up in a fixed order.  The unit's x
-// rows are copied to shared memory first.  Every warp streams its share of the k rows straight from global memory with
-// 128-bit coalesced loads, eight row pairs (8 x 512 B per warp) in flight before the first is
-// consumed, decodes the packed weights in registers (byte / nibble unpack, no shared-memory
-// staging of weights) and accumulates in fp32 with packed two-wide FMAs.  The 16 half-warp
-// partial sums per column are combined with one shuffle and one pass through shared memory;
-// scale and offset are applied in the fp32 epilogue and the result is rounded to bf16 once.
-// int8 items with 2..4 rows, fp8 items and fp4 items use the tensor core for the multiply-adds
-// (gv_compute_mma, gv_compute_fp4_mma); fp4 falls back to fp32 FMAs for x rows that are not exact in f16.
+// Work unit = (up to 4 or 8 rows of a non-empty expert, slab of 256 output columns, part of the k range);
+// persistent CTAs draw units from a ticket counter, the passes of a slab next to one another (their weights are then read from L2),
+// then the slabs.  K is cut into parts only when whole columns would leave the chip idle (gv_choose_parts); the parts' fp32 sums meet
+// in the workspace and the CTA that finishes a slab last adds them up in a fixed order.  Scale and offset are applied in
+// the fp32 epilogue and the result is rounded to bf16 once.
+// Two kernels.  int8, fp8 and fp4 run on the tensor core with their operands streamed through shared memory (gemv_ring.cuh).  int4, and
+// the fp4 rows whose x is not exact in f16, run on fp32 multiply-adds (this file, two CTAs per SM): the unit's x rows are copied to
+// shared memory, every warp streams its share of the k rows straight from global memory with coalesced loads, eight row pairs
+// in flight before the first is consumed, decodes the packed weights in registers and accumulates with packed two-wide FMAs; the
+// 16 half-warp partial sums per column are combined with one shuffle and one pass through shared memory.
 #include <algorithm>
 
 #include <cuda_fp16.h>
@@ -31,8 +28,6 @@ constexpr int kGvWarpRows = 2 * kGvUnroll;              // k rows a warp consume
 constexpr int kGvIterRows = kGvWarps * kGvWarpRows;     // k rows a CTA consumes per step
 constexpr int kGvRows = 4;                              // x rows per pass
 constexpr int kGvXPad = 16;                             // bf16 elements between staged x rows (bank spread)
-constexpr int kGvMmaParts = 4;                          // k groups of the tensor-core path
-constexpr int kGvL2Steps = 4;                           // steps a warp requests into L2 ahead of its register loads
 
 struct GemvArgs {
     const __nv_bfloat16* x;
@@ -48,6 +43,7 @@ struct GemvArgs {
     const int* xexp;
     unsigned* part_count;  // [kGvMaxParts] finished parts of a slab, zero at the launch; null: k is not split
     float* part_sums;      // [kGvMaxParts][kGvSlotFloats]
+    int max_parts;         // parts there is room for
     int* ticket;           // status word 2 (the fp32 kernel of fp4: 3, from 1 on)
     int by_rows;           // experts in the order of their row counts: shared memory has room for the order
 };
@@ -97,43 +93,10 @@ __device__ __forceinline__ uint2 ldg_stream8(const uint8_t* p) {
     return v;
 }
 
-template <int MODE>
-struct GvTraits {
-    static constexpr bool kNibbles = (MODE == B200MOE_CT_FP4 || MODE == B200MOE_CT_INT4);
-    static constexpr int kLaneBytes = kNibbles ? 8 : 16;  // 16 columns per lane
-};
-
 // Decode the lane's 16 columns of one weight row into eight fp32 pairs.
 template <int MODE, bool kScaleFp4 = true>
 __device__ __forceinline__ void gv_decode(const uint4& q, f32x2 (&w)[8], const f32x2 (&sc)[8], const f32x2 (&tc)[8]) {
-    if constexpr (MODE == B200MOE_CT_INT8) {
-        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
-        const f32x2 kneg = pack2(-8388736.0f, -8388736.0f);  // -(2^23 + 128)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t u = w4[i] ^ 0x80808080u;  // biased byte: value + 128
-            // 0x4B0000uu is the fp32 2^23 + uu
-            const float f0 = __uint_as_float(prmt(u, 0x4B000000u, 0x7440u)), f1 = __uint_as_float(prmt(u, 0x4B000000u, 0x7441u));
-            const float f2 = __uint_as_float(prmt(u, 0x4B000000u, 0x7442u)), f3 = __uint_as_float(prmt(u, 0x4B000000u, 0x7443u));
-            w[2 * i] = add2(pack2(f0, f1), kneg);
-            w[2 * i + 1] = add2(pack2(f2, f3), kneg);
-        }
-    } else if constexpr (MODE == B200MOE_CT_FP8) {
-        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
-        const f32x2 k120 = pack2(1.329227995784916e36f, 1.329227995784916e36f);  // 2^120
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float f[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                // e4m3 bits moved under the fp32 exponent: value * 2^-120 (subnormals included)
-                const uint32_t p = prmt(w4[i], 0u, 0x0444u | (b << 12));  // byte b -> bits 31..24
-                f[b] = __uint_as_float(((p >> 4) & 0x07F00000u) | (p & 0x80000000u));
-            }
-            w[2 * i] = mul2(pack2(f[0], f[1]), k120);
-            w[2 * i + 1] = mul2(pack2(f[2], f[3]), k120);
-        }
-    } else if constexpr (MODE == B200MOE_CT_INT4) {
+    if constexpr (MODE == B200MOE_CT_INT4) {
         // (w + o) * s = w * s + o * s in fp32: sc holds s, tc holds o * s of the row's 128-k group
         const uint32_t w2[2] = {q.x ^ 0x88888888u, q.y ^ 0x88888888u};  // nibble + 8
         const f32x2 kneg = pack2(-8388616.0f, -8388616.0f);             // -(2^23 + 8)
@@ -170,21 +133,13 @@ __device__ __forceinline__ void gv_draw(const GemvArgs& a, int& next) {
 // End of a unit: v[m] is the thread's column (threadIdx.x of the slab) of row m summed over the unit's part of k.
 // A slab in one part is stored at once.  Otherwise the sums go to the part's slot and the CTA that arrives last adds
 // the parts in their order, so the result does not depend on which one that is.
-template <int MODE>
-__device__ __forceinline__ void gv_finish(const GemvArgs& a, GvUnit& u, const float* xsum, const int* xexp,
-                                          float (&v)[kGvRows]) {
+__device__ __forceinline__ void gv_finish(const GemvArgs& a, GvUnit& u, float (&v)[kGvRows]) {
     const int t = threadIdx.x, n = u.n0 + t;
-    float xs[kGvRows];
-#pragma unroll
-    for (int m = 0; m < kGvRows; ++m) xs[m] = (MODE == B200MOE_CT_INT8) ? xsum[m] : 0.f;
     if (u.n_split > 1) {
         float* slot = a.part_sums + (size_t)(u.slot + u.split) * kGvSlotFloats;
 #pragma unroll
         for (int m = 0; m < kGvRows; ++m)
-            if (m < u.rows) {
-                __stcg(slot + m * kGvSlabN + t, v[m]);
-                if (MODE == B200MOE_CT_INT8 && t == 0) __stcg(slot + kGvRows * kGvSlabN + m, xs[m]);
-            }
+            if (m < u.rows) __stcg(slot + m * kGvSlabN + t, v[m]);
         __threadfence();
         __syncthreads();
         if (t == 0) u.split = atomicAdd(a.part_count + u.slot, 1u) == (unsigned)(u.n_split - 1) ? -1 : 0;  // (no longer needed)
@@ -196,40 +151,22 @@ __device__ __forceinline__ void gv_finish(const GemvArgs& a, GvUnit& u, const fl
         for (int m = 0; m < kGvRows; ++m) {
             if (m < u.rows) {
                 v[m] = 0.f;
-                xs[m] = 0.f;
-                for (int p = 0; p < u.n_split; ++p) {
-                    v[m] += __ldcg(first + (size_t)p * kGvSlotFloats + m * kGvSlabN + t);
-                    if (MODE == B200MOE_CT_INT8) xs[m] += __ldcg(first + (size_t)p * kGvSlotFloats + kGvRows * kGvSlabN + m);
-                }
+                for (int p = 0; p < u.n_split; ++p) v[m] += __ldcg(first + (size_t)p * kGvSlotFloats + m * kGvSlabN + t);
             }
         }
     }
-    if (n >= a.N) return;  // (fp8 only: the upper half of a 128-column last slab)
-    float s_n = 1.f, so_n = 0.f;
-    if constexpr (MODE == B200MOE_CT_INT8) {
-        s_n = __bfloat162float(static_cast<const __nv_bfloat16*>(a.scale)[(size_t)u.g * a.N + n]);
-        if (a.offset != nullptr) so_n = s_n * __bfloat162float(a.offset[(size_t)u.g * a.N + n]);
-    }
 #pragma unroll
-    for (int m = 0; m < kGvRows; ++m) {
-        if (m < u.rows) {
-            float o = v[m];
-            if constexpr (MODE == B200MOE_CT_INT8) o = fmaf(so_n, xs[m], s_n * o);
-            if (xexp != nullptr) o = scalbnf(o, xexp[m]);
-            a.y[(size_t)(u.r0 + m) * a.N + n] = __float2bfloat16_rn(o);
-        }
-    }
+    for (int m = 0; m < kGvRows; ++m)
+        if (m < u.rows) a.y[(size_t)(u.r0 + m) * a.N + n] = __float2bfloat16_rn(v[m]);
 }
 
 template <int MODE, int MB>
-__device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs, const float* xsum,
-                                           float* red, int& next) {
-    using T = GvTraits<MODE>;
+__device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs, float* red, int& next) {
     const int g = un.g, n0 = un.n0, k_begin = un.k0, k_end = un.k1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = lane >> 4, l16 = lane & 15;
-    const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
-    const uint8_t* wbase = a.weight + (size_t)g * a.K * row_bytes + (T::kNibbles ? n0 / 2 : n0) + l16 * T::kLaneBytes;
+    const size_t row_bytes = (size_t)a.N / 2;
+    const uint8_t* wbase = a.weight + (size_t)g * a.K * row_bytes + n0 / 2 + l16 * 8;  // 16 columns per lane
     const int col0 = n0 + l16 * 16;
 
     f32x2 acc[MB][8];
@@ -242,30 +179,14 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const 
 #pragma unroll
     for (int c = 0; c < 8; ++c) sc[c] = tc[c] = 0ull;
 
-    // int8 / fp8: the warp's rows of the steps kGvL2Steps ahead are requested into L2, one line per lane (16 rows
-    // x the slab's 256-byte row segment): the register loads then wait for L2 instead of DRAM.  (The nibble
-    // formats' versions of this function have no registers to spare for it.)
-    const uint8_t* pf_base = a.weight + (size_t)g * a.K * row_bytes + n0 + 128 * (lane & 1);
-    auto prefetch_step = [&](int k) {
-        if constexpr (!T::kNibbles) {
-            if (k + (lane >> 1) < k_end) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t)(k + (lane >> 1)) * row_bytes));
-        }
-    };
-#pragma unroll
-    for (int i = 0; i < kGvL2Steps; ++i) prefetch_step(k_begin + warp * kGvWarpRows + i * kGvIterRows);
     for (int k0 = k_begin + warp * kGvWarpRows; k0 < k_end; k0 += kGvIterRows) {
-        prefetch_step(k0 + kGvL2Steps * kGvIterRows);
         // ---- issue all loads of this step first ----
         uint4 q[kGvUnroll];
         const uint8_t* p = wbase + (size_t)(k0 + half) * row_bytes;
 #pragma unroll
         for (int u = 0; u < kGvUnroll; ++u) {
-            if constexpr (T::kNibbles) {
-                const uint2 v = ldg_stream8(p + (size_t)(2 * u) * row_bytes);
-                q[u] = make_uint4(v.x, v.y, 0u, 0u);
-            } else {
-                q[u] = ldg_stream(p + (size_t)(2 * u) * row_bytes);
-            }
+            const uint2 v = ldg_stream8(p + (size_t)(2 * u) * row_bytes);
+            q[u] = make_uint4(v.x, v.y, 0u, 0u);
         }
         // ---- x values of the 16 rows: lane uses rows k0 + 2u + half ----
         uint32_t xw[MB][kGvUnroll];
@@ -276,10 +197,7 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const 
             xw[m][0] = x0.x; xw[m][1] = x0.y; xw[m][2] = x0.z; xw[m][3] = x0.w;
             xw[m][4] = x1.x; xw[m][5] = x1.y; xw[m][6] = x1.z; xw[m][7] = x1.w;
         }
-        float sf = 1.f;
-        if constexpr (MODE == B200MOE_CT_FP8) {
-            sf = __ldg(static_cast<const float*>(a.scale) + ((size_t)g * (a.K >> 7) + (k0 >> 7)) * (a.N >> 7) + (col0 >> 7));
-        } else if constexpr (MODE == B200MOE_CT_FP4) {
+        if constexpr (MODE == B200MOE_CT_FP4) {
             // one scale row per 16 k rows: exactly the rows of this step
             const uint4* sp = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.scale) +
                                                              ((size_t)g * (a.K >> 4) + (k0 >> 4)) * a.N + col0);
@@ -322,8 +240,7 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const 
             gv_decode<MODE, !kGroupScale>(q[u], w, sc, tc);
 #pragma unroll
             for (int m = 0; m < MB; ++m) {
-                float xv = __uint_as_float(half ? (xw[m][u] & 0xFFFF0000u) : (xw[m][u] << 16));
-                if constexpr (MODE == B200MOE_CT_FP8) xv *= sf;
+                const float xv = __uint_as_float(half ? (xw[m][u] & 0xFFFF0000u) : (xw[m][u] << 16));
                 const f32x2 xx = pack2(xv, xv);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
@@ -367,21 +284,9 @@ __device__ __forceinline__ void gv_compute(const GemvArgs& a, GvUnit& un, const 
             for (int w = 0; w < kGvWarps; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    gv_finish<MODE>(a, un, xsum, nullptr, v);
+    gv_finish(a, un, v);
 }
 
-// ---- 2..4 rows per expert, int8: the multiply-adds go to the tensor core ---------------------
-// With more than one row the scalar path spends most of its issue slots on FMAs.  Here a warp
-// multiplies a 16 (k) x 128 (columns) block of weights with up to four x rows per step using eight
-// mma.sync m16n8k16 instructions, the weights as the 16 x 16 operand:
-//   lane (g, t) = (lane / 4, lane % 4) loads rows k0 + 4t .. 4t+3, columns 16g .. 16g+15 (each load
-//   instruction reads four full 128-byte lines) and feeds instruction j with columns 16g + 2j, +1:
-//   operand row g <-> column 16g + 2j, row g + 8 <-> column 16g + 2j + 1, and the instruction's
-//   k index {2t, 2t+1, 2t+8, 2t+9} <-> weight rows 4t .. 4t+3 (a summation index: any assignment
-//   works as long as the x operand uses the same one).  One byte permute per two rows and two
-//   columns puts (row, row + 1) pairs of a column side by side, then the exact int8 -> bf16
-//   conversion of common.cuh applies; x pairs come from shared memory with one 8-byte load per step.
-// The instruction count per weight byte no longer depends on the number of rows.
 // Two e4m3 codes in the high bytes of the two 16-bit lanes (low bytes ignored) -> bf16x2, exact:
 // exponent and mantissa bits go under the bf16 exponent, times 2^120 (subnormals included).
 __device__ __forceinline__ uint32_t e4m3x2_hi_to_bf16(uint32_t t) {
@@ -394,134 +299,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// fp8 (e4m3) follows the same scheme: the bytes of rows (k, k+1) of a column are permuted into the
-// high bytes of the two 16-bit lanes and decoded by bit placement (exact in bf16); the fp32 scale of
-// the 128 x 128 block, uniform for a warp over a 128-row stretch, multiplies the stretch's partial sums.
-template <int MODE>
-__device__ __forceinline__ void gv_compute_mma(const GemvArgs& a, GvUnit& un, const __nv_bfloat16* xs,
-                                               const float* xsum, float* red, int& next) {
-    const int g_expert = un.g, rows_valid = un.rows, n0 = un.n0, k_begin = un.k0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int hc = warp & 1, kg = warp >> 1;  // column half of the slab, k group
-    const size_t row_bytes = (size_t)a.N;
-    const uint8_t* wbase = a.weight + (size_t)g_expert * a.K * row_bytes + n0 + 128 * hc + 16 * g + (size_t)(4 * t) * row_bytes;
-    // x pairs of token g at the lane's four k rows (tokens beyond the valid rows contribute zeros)
-    const __nv_bfloat16* xrow = xs + (size_t)(g < rows_valid ? g : 0) * (a.K + kGvXPad) + 4 * t;
-    const bool x_on = g < rows_valid;
-
-    float c[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
-    constexpr bool kBlockScale = (MODE == B200MOE_CT_FP8);
-    float ct[kBlockScale ? 8 : 1][4];  // fp8: totals; `c` then holds the current 128-row stretch
-    if constexpr (kBlockScale) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ct[j][0] = ct[j][1] = ct[j][2] = ct[j][3] = 0.f;
-    }
-
-    constexpr int kStepRows = 16 * kGvMmaParts;  // k rows the CTA consumes per step
-    // (fp8 accepts N % 256 == 128: in the last slab the warps of the second column half have no columns)
-    const int k1 = un.k1, k_end = (n0 + 128 * hc < a.N) ? k1 : 0;
-    // two steps (2 x 16 rows of the warp's 128-byte row segment) per iteration: one line per lane into L2,
-    // kGvL2Steps / 2 iterations ahead
-    const uint8_t* pf_base = a.weight + (size_t)g_expert * a.K * row_bytes + n0 + 128 * hc;
-    auto prefetch_iter = [&](int k) {
-        const int kk = k + (lane >> 4) * kStepRows + (lane & 15);
-        if (kk < k_end) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t)kk * row_bytes));
-    };
-#pragma unroll
-    for (int i = 0; i < kGvL2Steps / 2; ++i) prefetch_iter(k_begin + kg * 16 + i * 2 * kStepRows);
-    for (int k0 = k_begin + kg * 16; k0 < k_end; k0 += 2 * kStepRows) {
-        prefetch_iter(k0 + (kGvL2Steps / 2) * 2 * kStepRows);
-        const bool second = k0 + kStepRows < k1;
-        float sf = 1.f;
-        if constexpr (kBlockScale)  // k0 and k0 + 64 lie in the same 128-row block (K % 128 == 0)
-            sf = __ldg(static_cast<const float*>(a.scale) + ((size_t)g_expert * (a.K >> 7) + (k0 >> 7)) * (a.N >> 7) +
-                       ((n0 + 128 * hc) >> 7));
-        uint4 q[2][4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !second) break;
-            const uint8_t* p = wbase + (size_t)(k0 + h * kStepRows) * row_bytes;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) q[h][i] = ldg_stream(p + (size_t)i * row_bytes);
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !second) break;
-            uint2 xb = make_uint2(0u, 0u);
-            if (x_on) xb = *reinterpret_cast<const uint2*>(xrow + k0 + h * kStepRows);
-            const uint32_t r0w[4] = {q[h][0].x, q[h][0].y, q[h][0].z, q[h][0].w};
-            const uint32_t r1w[4] = {q[h][1].x, q[h][1].y, q[h][1].z, q[h][1].w};
-            const uint32_t r2w[4] = {q[h][2].x, q[h][2].y, q[h][2].z, q[h][2].w};
-            const uint32_t r3w[4] = {q[h][3].x, q[h][3].y, q[h][3].z, q[h][3].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-#pragma unroll
-                for (int o = 0; o < 2; ++o) {  // byte pairs (0,1) and (2,3) of word i: instruction j = 2i + o
-                    uint32_t a0, a1, a2, a3;
-                    if constexpr (MODE == B200MOE_CT_INT8) {
-                        const uint32_t sel = o == 0 ? 0x5410u : 0x7632u;
-                        s8x4_to_bf16_even_odd(prmt(r0w[i], r1w[i], sel), a0, a1);  // (row 4t, 4t+1) at the two columns
-                        s8x4_to_bf16_even_odd(prmt(r2w[i], r3w[i], sel), a2, a3);  // (row 4t+2, 4t+3)
-                    } else {
-                        // byte b of both rows into the high bytes of the two lanes (the low bytes are masked off)
-                        const uint32_t s0 = o == 0 ? 0x4000u : 0x6020u, s1 = o == 0 ? 0x5010u : 0x7030u;
-                        a0 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s0));
-                        a1 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s1));
-                        a2 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s0));
-                        a3 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s1));
-                    }
-                    mma_16816(c[2 * i + o], a0, a1, a2, a3, xb.x, xb.y);
-                }
-            }
-        }
-        if constexpr (kBlockScale) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    ct[j][e] = fmaf(sf, c[j][e], ct[j][e]);
-                    c[j][e] = 0.f;
-                }
-        }
-    }
-    if constexpr (kBlockScale) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) c[j][e] = ct[j][e];
-    }
-
-    // ---- partial sums of the four k groups -> shared memory -> per-column epilogue ----------------
-    if (t < 2) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int col = 128 * hc + 16 * g + 2 * j;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {  // tokens 2t, 2t + 1
-                const int tok = 2 * t + e;
-                float* dst = red + (size_t)(kg * kGvRows + tok) * kGvSlabN + col;
-                *reinterpret_cast<float2*>(dst) = make_float2(c[j][e], c[j][2 + e]);
-            }
-        }
-    }
-    gv_draw(a, next);
-    __syncthreads();
-    float v[kGvRows];
-#pragma unroll
-    for (int m = 0; m < kGvRows; ++m) {
-        v[m] = 0.f;
-        if (m < un.rows) {
-#pragma unroll
-            for (int w = 0; w < kGvMmaParts; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
-            if constexpr (MODE == B200MOE_CT_INT8) v[m] *= kS8Unit;
-        }
-    }
-    gv_finish<MODE>(a, un, xsum, nullptr, v);
 }
 
 // ---- fp4 weights in the reference's stored (pre-shuffled) order, read in place -----------------
@@ -624,27 +401,16 @@ __device__ __forceinline__ void gv_compute_fp4_stored(const GemvArgs& a, GvUnit&
             for (int w = 0; w < kGvWarps; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
         }
     }
-    gv_finish<B200MOE_CT_FP4>(a, un, nullptr, nullptr, v);
+    gv_finish(a, un, v);
 }
 
 
-// ---- fp4, 1..4 rows per expert: decode by the e2m1 -> f16 conversion instruction, multiply-adds on the tensor core --
-// The scalar fp4 paths spend their issue slots on the decode and the FMAs (about 6 instructions per weight with
-// four rows; the HBM rate leaves room for fewer than 3).  Here the x rows are held in shared memory as f16 --
-// each row scaled by a power of two so that its largest element lies in [2^14, 2^15); the staging code only
-// takes this path when every element is then exactly representable, so x' * e2m1 products stay exact -- and a
-// warp multiplies a 16 (k) x 128 (columns) block of weights with the x rows using eight mma.sync m16n8k16
-// (f16 operands, fp32 accumulation), the weights as the 16 x 16 operand.  The 16 rows of a step are one scale
-// group: the instruction starts from zero and its fp32 sums are multiplied by the group's bf16 scale per column
-// into the running totals (the scale never touches a weight; gemv_impl.h:147-199 keeps the weights in fp32
-// the same way).  The row's power of two is undone in the epilogue.
-//   lane (g, t) = (lane / 4, lane % 4) owns k rows {2t, 2t+1, 2t+8, 2t+9} of the step -- the instruction's own k
-//   indices -- and 16 columns: rows (2t, 2t+1) of eight columns are two 32-bit words; one shift and two logic
-//   operations put the two rows' codes of a column into one byte, which the conversion instruction turns into
-//   the f16 pair (row 2t, row 2t+1) the operand register wants.
-//   canonical layout: columns 16g .. 16g+15 of the warp's 128 (four 8-byte loads cover four rows x 64 bytes);
-//   stored order: the 8-column groups (p, q) = (4 hc + g / 4 + 2 i, g % 4), i = 0, 1, whose rows (2t, 2t+1) of
-//   an 8-row block are 8 consecutive bytes (each load instruction covers two full 128-byte lines).
+// Operands of the tensor-core kernel (gemv_ring.cuh).  fp4: the scalar paths spend their issue slots on the decode and the FMAs (about 6
+// instructions per weight with four rows; the HBM rate leaves room for fewer than 3).  There the x rows are held as f16 --
+// each row scaled by a power of two so that its largest element lies in [2^14, 2^15); that path is only
+// taken when every element is then exactly representable, so x' * e2m1 products stay exact.  One shift and two logic
+// operations put the two rows' codes of a column into one byte, which the conversion instruction turns into
+// the f16 pair (row 2t, row 2t+1) the operand register wants.  The row's power of two is undone in the epilogue.
 __device__ __forceinline__ void cvt_e2m1x8_f16(uint32_t w, uint32_t (&o)[4]) {
     // byte i of w = two codes -> f16x2 (low nibble in the low half)
     asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4; cvt.rn.f16x2.e2m1x2 %0, b0; "
@@ -659,160 +425,6 @@ __device__ __forceinline__ void mma_16816_f16_zero(float (&d)[4], uint32_t a0, u
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-
-constexpr int kGvFp4Ahead = 4;  // steps whose loads are in flight per warp (6: slower, measured)
-
-constexpr int kGvFp4L2Ahead = 1;  // batches of kGvFp4Ahead steps requested into L2 before their loads are issued
-
-template <bool kStored>
-__device__ __forceinline__ void gv_compute_fp4_mma(const GemvArgs& a, GvUnit& un, const __half* xs, const int* xexp,
-                                                   float* red, int& next) {
-    const int g_expert = un.g, rows_valid = un.rows, n0 = un.n0, k_begin = un.k0, k_end = un.k1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int hc = warp & 1, kg = warp >> 1;  // column half of the slab, k group
-    const size_t row_bytes = (size_t)a.N >> 1;
-    const uint8_t* wexp = a.weight + (size_t)g_expert * a.K * row_bytes;
-    // first of the lane's 16 columns inside the slab (stored order: of its first group; the second is 64 further)
-    const int c_first = kStored ? 128 * hc + 32 * (g >> 2) + 8 * (g & 3) : 128 * hc + 16 * g;
-    const uint8_t* wbase;
-    size_t p_stride = 0;
-    if constexpr (kStored) {
-        const int J = a.N >> 8, j = n0 >> 8;
-        p_stride = (size_t)J * 128;
-        wbase = wexp + (size_t)j * 128 + (g & 3) * 32 + 8 * t;
-    } else {
-        wbase = wexp + (size_t)(n0 >> 1) + 64 * hc + 8 * g + (size_t)(2 * t) * row_bytes;
-    }
-    const __half* xrow = xs + (size_t)(g < rows_valid ? g : 0) * (a.K + kGvXPad) + 2 * t;
-    const bool x_on = g < rows_valid;
-    const __nv_bfloat16* sbase = static_cast<const __nv_bfloat16*>(a.scale) + (size_t)g_expert * (a.K >> 4) * a.N + n0 + c_first;
-
-    float acc[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-
-    constexpr int kStepRows = 16 * kGvMmaParts;  // k rows the CTA consumes per step
-    // q[0], q[1]: rows (2t, 2t+1) and (2t+8, 2t+9) of the lane's columns 0..7; q[2], q[3]: of its columns 8..15
-    auto load = [&](int k, uint2 (&q)[4]) {
-        if constexpr (kStored) {
-            const int R = k >> 6, aa = (k >> 4) & 3;
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    q[2 * i + b] = ldg_stream8(wbase + ((size_t)((2 * R + b) * 4 + aa) * 8 + 4 * hc + (g >> 2) + 2 * i) * p_stride);
-        } else {
-            const uint8_t* p = wbase + (size_t)k * row_bytes;
-            // rows 2t, 2t+1, 2t+8, 2t+9: 16 columns = 8 bytes each
-            const uint2 r0w = ldg_stream8(p), r1w = ldg_stream8(p + row_bytes);
-            const uint2 r8w = ldg_stream8(p + 8 * row_bytes), r9w = ldg_stream8(p + 9 * row_bytes);
-            q[0] = make_uint2(r0w.x, r1w.x);
-            q[1] = make_uint2(r8w.x, r9w.x);
-            q[2] = make_uint2(r0w.y, r1w.y);
-            q[3] = make_uint2(r8w.y, r9w.y);
-        }
-    };
-    // Four steps of the warp's weights and scales into L2, one line per lane: the weights of a step are 8 lines
-    // (stored order: 2 row blocks x 4 line rows; canonical: 16 rows x 64 bytes, half a line each), its scales 2
-    // lines.  The register loads, issued up to kGvFp4L2Ahead batches later, then wait for L2, not for DRAM.
-    auto prefetch_group = [&](int k0) {
-        const int h = lane >> 3, k = k0 + h * kStepRows;
-        if (k >= k_end) return;
-        const uint8_t* w;
-        if constexpr (kStored) {
-            const int R = k >> 6, aa = (k >> 4) & 3, i = (lane >> 2) & 1, b = (lane >> 1) & 1, gq = lane & 1;
-            w = wexp + (size_t)(n0 >> 8) * 128 + ((size_t)((2 * R + b) * 4 + aa) * 8 + 4 * hc + gq + 2 * i) * p_stride;
-        } else {
-            w = wexp + (size_t)(n0 >> 1) + 64 * hc + (size_t)(k + 2 * (lane & 7)) * row_bytes;  // rows 2l and (same line pair) 2l+1
-        }
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(w));
-        if constexpr (!kStored) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + row_bytes));
-        if ((lane & 7) < 2) {
-            const __nv_bfloat16* sp = static_cast<const __nv_bfloat16*>(a.scale) + ((size_t)g_expert * (a.K >> 4) + (k >> 4)) * a.N +
-                                      n0 + 128 * hc + 64 * (lane & 7);
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(sp));
-        }
-    };
-    auto compute = [&](int k, const uint2 (&q)[4]) {
-        uint32_t b0 = 0u, b1 = 0u;
-        if (x_on) {
-            b0 = *reinterpret_cast<const uint32_t*>(xrow + k);
-            b1 = *reinterpret_cast<const uint32_t*>(xrow + k + 8);
-        }
-        // the group's scales of the lane's 16 columns
-        const __nv_bfloat16* sp = sbase + (size_t)(k >> 4) * a.N;
-        const uint4 s0 = __ldg(reinterpret_cast<const uint4*>(sp));
-        const uint4 s1 = __ldg(reinterpret_cast<const uint4*>(sp + (kStored ? 64 : 8)));
-        const uint32_t sw[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {  // columns 8i .. 8i+7 of the lane's 16
-            const uint2 lo = q[2 * i], hi = q[2 * i + 1];
-            // byte b: the codes of rows (r, r + 1) at column 2b (e_*) / 2b + 1 (o_*)
-            const uint32_t e_lo = (lo.x & 0x0F0F0F0Fu) | ((lo.y << 4) & 0xF0F0F0F0u);
-            const uint32_t o_lo = ((lo.x >> 4) & 0x0F0F0F0Fu) | (lo.y & 0xF0F0F0F0u);
-            const uint32_t e_hi = (hi.x & 0x0F0F0F0Fu) | ((hi.y << 4) & 0xF0F0F0F0u);
-            const uint32_t o_hi = ((hi.x >> 4) & 0x0F0F0F0Fu) | (hi.y & 0xF0F0F0F0u);
-            uint32_t a0[4], a1[4], a2[4], a3[4];
-            cvt_e2m1x8_f16(e_lo, a0);
-            cvt_e2m1x8_f16(o_lo, a1);
-            cvt_e2m1x8_f16(e_hi, a2);
-            cvt_e2m1x8_f16(o_hi, a3);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                float d[4];
-                mma_16816_f16_zero(d, a0[b], a1[b], a2[b], a3[b], b0, b1);
-                const float sc_e = __uint_as_float(sw[4 * i + b] << 16), sc_o = __uint_as_float(sw[4 * i + b] & 0xFFFF0000u);
-                float* c = acc[4 * i + b];
-                c[0] = fmaf(d[0], sc_e, c[0]);
-                c[1] = fmaf(d[1], sc_e, c[1]);
-                c[2] = fmaf(d[2], sc_o, c[2]);
-                c[3] = fmaf(d[3], sc_o, c[3]);
-            }
-        }
-    };
-    constexpr int kBatchRows = kGvFp4Ahead * kStepRows;
-    int k0 = k_begin + kg * 16;
-    int k_pf = k0;  // first step not yet requested into L2 (requests go out four steps at a time)
-    for (; k0 + (kGvFp4Ahead - 1) * kStepRows < k_end; k0 += kBatchRows) {
-        uint2 q[kGvFp4Ahead][4];
-        for (; k_pf < k0 + kGvFp4L2Ahead * kBatchRows; k_pf += 4 * kStepRows) prefetch_group(k_pf);
-#pragma unroll
-        for (int h = 0; h < kGvFp4Ahead; ++h) load(k0 + h * kStepRows, q[h]);
-#pragma unroll
-        for (int h = 0; h < kGvFp4Ahead; ++h) compute(k0 + h * kStepRows, q[h]);
-    }
-    for (; k0 < k_end; k0 += kStepRows) {
-        uint2 q1[4];
-        load(k0, q1);
-        compute(k0, q1);
-    }
-
-    // ---- partial sums of the four k groups -> shared memory -> per-column epilogue ----------------
-    if (t < 2) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int col = c_first + (kStored ? 64 * (j >> 2) : 8 * (j >> 2)) + 2 * (j & 3);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {  // tokens 2t, 2t + 1
-                float* dst = red + (size_t)(kg * kGvRows + 2 * t + e) * kGvSlabN + col;
-                *reinterpret_cast<float2*>(dst) = make_float2(acc[j][e], acc[j][2 + e]);
-            }
-        }
-    }
-    gv_draw(a, next);
-    __syncthreads();
-    float v[kGvRows];
-#pragma unroll
-    for (int m = 0; m < kGvRows; ++m) {
-        v[m] = 0.f;
-        if (m < un.rows) {
-#pragma unroll
-            for (int w = 0; w < kGvMmaParts; ++w) v[m] += red[(w * kGvRows + m) * kGvSlabN + threadIdx.x];
-        }
-    }
-    gv_finish<B200MOE_CT_FP4>(a, un, nullptr, xexp, v);
 }
 
 // fp4 prepass, one CTA per x row: the row as f16, times 2^-e with e chosen so that its largest element lies in
@@ -889,19 +501,17 @@ __global__ void __launch_bounds__(256) gv_begin_kernel(int* __restrict__ status,
 // to gain and stays whole.  One token on 8 of 256 experts, 7168 x 4096 fp8 (128 slabs, two parts): 117 -> 72 us = 3.3
 // TB/s; 3 tokens x 4 over 160 experts, 4224 x 3328 int8: 54.6 -> 53.3 us.
 constexpr int kGvPartCost = 2;
-__device__ __forceinline__ int gv_choose_parts(int slabs, int ctas, int K) {
+__device__ __forceinline__ int gv_choose_parts(int slabs, int ctas, int K, int max_parts) {
     const int blocks = (K + kGvPartRows - 1) / kGvPartRows;
     const int s = (threadIdx.x & 31) + 1, per = (blocks + s - 1) / s;
     unsigned cost = 0xFFFFFFFFu;
-    if (s == 1 || ((long long)slabs * s <= kGvMaxParts && per > 1 && (blocks + per - 1) / per == s))
+    if (s == 1 || ((long long)slabs * s <= max_parts && per > 1 && (blocks + per - 1) / per == s))
         cost = min((unsigned)((slabs * (long long)s + ctas - 1) / ctas) * (unsigned)(per + kGvPartCost), 0x03FFFFFFu) * 32u + (unsigned)(s - 1);
     return (int)(__reduce_min_sync(0xffffffffu, cost) & 31u) + 1;
 }
 
-// fp4 is launched as two kernels over the same work items: PATH 1 takes the passes whose x rows are all exact as
-// scaled f16 (tensor-core path), PATH 2 the others (fp32 multiply-adds; normally none: the kernel leaves at once when the
-// prepass found no such row); PATH 0: every other mode, and fp4 without the prepass.  Separate kernels keep the
-// registers of one path from weighing on the other.
+// fp4 is launched as two kernels over the same rows: gemv_ring_kernel, and behind it this one as PATH 1 for the passes of which an x
+// row is not exact as scaled f16 (normally none: it leaves at once when the prepass found no such row).
 template <int MODE, int PATH = 0>
 __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -911,11 +521,8 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
     uintptr_t p = (reinterpret_cast<uintptr_t>(order + (a.by_rows ? a.G : 0)) + 15) & ~uintptr_t(15);
     float* red = reinterpret_cast<float*>(p);                                     // [8][4][256]
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(red + kGvWarps * kGvRows * kGvSlabN);  // [4][K]
-    float* xsum = reinterpret_cast<float*>(xs + a.K);  // [4], in the pad behind the first row
-    int* xexp = reinterpret_cast<int*>(xsum + kGvRows);  // [4], the other half of it
-    static_assert(kGvXPad * sizeof(__nv_bfloat16) == 2 * kGvRows * sizeof(float), "pad of a staged row");
 
-    if (PATH == 2) {
+    if (PATH == 1) {
         grid_dep_wait();
         if (*reinterpret_cast<volatile int*>(a.status + 3) == 0) return;
     }
@@ -954,7 +561,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             at += passes_of(i);
         }
         if (threadIdx.x == 0) pass_start[a.G] = total;
-        const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K);
+        const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K, a.max_parts);
         if (threadIdx.x == 0) {
             // (kept in shared memory: a unit's loop needs every register)
             s_parts = parts;
@@ -971,7 +578,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
     for (;;) {
         if (threadIdx.x == 0) s_ticket = next;
         __syncthreads();
-        const unsigned unit = (unsigned)(s_ticket - (PATH == 2 ? 1 : 0));
+        const unsigned unit = (unsigned)(s_ticket - (PATH == 1 ? 1 : 0));
         if (unit >= s_units) break;
         // every thread looks at its experts, the one that finds the unit describes it to the others: a binary search
         // with its divisions by one thread was a tenth of a short unit (2048 rows of fp4)
@@ -1000,57 +607,33 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
         {
             // (copies: the stores of the staging loop could alias the descriptor)
             const int r = un.r0, rows = un.rows, v0 = un.k0 / 8, v1 = un.k1 / 8;
-            // fp4: the tensor-core path when every row of the pass is exact as scaled f16 (prepared by the prepass)
-            bool fp4_mma = false;
-            if constexpr (PATH != 0) {
-                fp4_mma = true;
-                for (int m = 0; m < rows; ++m) fp4_mma = fp4_mma && a.xexp[r + m] != kGvNotF16;
-                if (fp4_mma != (PATH == 1)) {  // the other kernel's pass
+            if constexpr (PATH == 1) {
+                bool exact = true;
+                for (int m = 0; m < rows; ++m) exact = exact && a.xexp[r + m] != kGvNotF16;
+                if (exact) {  // the other kernel's pass
                     gv_draw(a, next);
                     __syncthreads();
                     continue;
                 }
-                if (fp4_mma && threadIdx.x < rows) xexp[threadIdx.x] = a.xexp[r + threadIdx.x];
             }
-            // ---- stage the x rows (and their sums, for the offset term) ----
-            if (threadIdx.x < 4) xsum[threadIdx.x] = 0.f;
-            __syncthreads();
+            // ---- stage the x rows ----
             for (int m = 0; m < rows; ++m) {
-                const uint4* src = fp4_mma ? reinterpret_cast<const uint4*>(a.x16 + (size_t)(r + m) * a.K)
-                                           : reinterpret_cast<const uint4*>(a.x + (size_t)(r + m) * a.K);
+                const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)(r + m) * a.K);
                 uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)m * (a.K + kGvXPad));
-                float s = 0.f;
 #pragma unroll 4
                 for (int i = v0 + threadIdx.x; i < v1; i += kGvThreads) {
                     const uint4 v = PATH == 1 ? __ldca(src + i) : __ldg(src + i);
                     dst[i] = v;
-                    if (MODE == B200MOE_CT_INT8 && a.offset != nullptr) {
-                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) s += __uint_as_float(w4[j] << 16) + __uint_as_float(w4[j] & 0xFFFF0000u);
-                    }
-                }
-                if (MODE == B200MOE_CT_INT8 && a.offset != nullptr) {
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if ((threadIdx.x & 31) == 0) atomicAdd(&xsum[m], s);
                 }
             }
             __syncthreads();
-            // fp8: the tensor-core path also wins with one row (its decode is two-wide); int8 with one
-            // row is faster on the scalar path; fp4 takes the tensor-core path whenever x is exact in f16
-            if constexpr (PATH == 1) {
-                if (a.fp4_stored) gv_compute_fp4_mma<true>(a, un, reinterpret_cast<const __half*>(xs), xexp, red, next);
-                else gv_compute_fp4_mma<false>(a, un, reinterpret_cast<const __half*>(xs), xexp, red, next);
-            } else if (MODE == B200MOE_CT_FP4 && a.fp4_stored) {
+            if (MODE == B200MOE_CT_FP4 && a.fp4_stored) {
                 if (rows == 1) gv_compute_fp4_stored<1>(a, un, xs, red, next);
                 else if (rows == 2) gv_compute_fp4_stored<2>(a, un, xs, red, next);
                 else gv_compute_fp4_stored<4>(a, un, xs, red, next);
-            } else if constexpr (MODE == B200MOE_CT_FP8) gv_compute_mma<MODE>(a, un, xs, xsum, red, next);
-            else if (rows == 1) gv_compute<MODE, 1>(a, un, xs, xsum, red, next);
-            else if constexpr (MODE == B200MOE_CT_INT8) gv_compute_mma<MODE>(a, un, xs, xsum, red, next);
-            else if (rows == 2) gv_compute<MODE, 2>(a, un, xs, xsum, red, next);
-            else gv_compute<MODE, 4>(a, un, xs, xsum, red, next);
+            } else if (rows == 1) gv_compute<MODE, 1>(a, un, xs, red, next);
+            else if (rows == 2) gv_compute<MODE, 2>(a, un, xs, red, next);
+            else gv_compute<MODE, 4>(a, un, xs, red, next);
         }
     }
 }
@@ -1065,7 +648,7 @@ static size_t gv_smem_bytes(int G, int K, bool by_rows) {
 template <int MODE, int PATH = 0>
 static int gv_launch(const GemvArgs& a0, cudaStream_t stream) {
     GemvArgs a = a0;
-    a.ticket = a.status + (PATH == 2 ? 3 : 2);
+    a.ticket = a.status + (PATH == 1 ? 3 : 2);
     size_t smem = gv_smem_bytes(a.G, a.K, true);
     // (the order must not cost the second CTA of a multiprocessor, nor a shape that fits without it)
     a.by_rows = smem <= 110 * 1024 || (smem <= 226 * 1024 && gv_smem_bytes(a.G, a.K, false) > 110 * 1024);
@@ -1078,17 +661,14 @@ static int gv_launch(const GemvArgs& a0, cudaStream_t stream) {
     if (per_sm == 1) smem = std::max<size_t>(smem, 116 * 1024);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemv_kernel<MODE, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    // (behind gv_begin_kernel or the fp4 prepass; the fp32 kernel of fp4 stays behind the tensor-core one)
-    if (PATH != 2) {
-        B200MOE_CUDA_TRY(launch_dependent(grouped_gemv_kernel<MODE, PATH>, (unsigned)(per_sm * sm_count()), kGvThreads, smem, stream, a));
-    } else {
-        grouped_gemv_kernel<MODE, PATH><<<per_sm * sm_count(), kGvThreads, smem, stream>>>(a);
-        B200MOE_CUDA_TRY(cudaGetLastError());
-    }
+    // (behind gv_begin_kernel, or as PATH 1 behind the tensor-core kernel)
+    B200MOE_CUDA_TRY(launch_dependent(grouped_gemv_kernel<MODE, PATH>, (unsigned)(per_sm * sm_count()), kGvThreads, smem, stream, a));
     return B200MOE_OK;
 }
 
 }  // namespace b200moe
+
+#include "gemv_ring.cuh"
 
 using namespace b200moe;
 
@@ -1153,6 +733,7 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
     a.part_count = nullptr;
     a.part_sums = nullptr;
+    a.max_parts = kGvMaxParts;
     if (workspace_bytes >= gv_parts_offset(need) + kGvPartBytes) {
         uint8_t* parts = static_cast<uint8_t*>(workspace) + gv_parts_offset(need);
         a.part_count = reinterpret_cast<unsigned*>(parts);
@@ -1176,13 +757,19 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
                                           const_cast<int*>(a.xexp), a.K, a.status));
     }
     switch (compute_type) {
-        case B200MOE_CT_INT8: return gv_launch<B200MOE_CT_INT8>(a, s);
-        case B200MOE_CT_FP8: return gv_launch<B200MOE_CT_FP8>(a, s);
+        case B200MOE_CT_INT8: return gv_ring_launch<B200MOE_CT_INT8>(a, s);
+        case B200MOE_CT_FP8: return gv_ring_launch<B200MOE_CT_FP8>(a, s);
         case B200MOE_CT_INT4: return gv_launch<B200MOE_CT_INT4>(a, s);
         default: {
             if (a.x16 == nullptr) return gv_launch<B200MOE_CT_FP4>(a, s);
-            const int rc = gv_launch<B200MOE_CT_FP4, 1>(a, s);
-            return rc != B200MOE_OK ? rc : gv_launch<B200MOE_CT_FP4, 2>(a, s);
+            a.max_parts = kGvMaxParts / 2;  // half of the room for each of the two kernels
+            const int rc = a.fp4_stored ? gv_ring_launch<B200MOE_CT_FP4, true>(a, s) : gv_ring_launch<B200MOE_CT_FP4, false>(a, s);
+            if (rc != B200MOE_OK) return rc;
+            if (a.part_count != nullptr) {
+                a.part_count += kGvMaxParts / 2;
+                a.part_sums += (size_t)(kGvMaxParts / 2) * kGvSlotFloats;
+            }
+            return gv_launch<B200MOE_CT_FP4, 1>(a, s);
         }
     }
 }

@@ -1,0 +1,41 @@
+"""The GEMV kernel that streams its operands through shared memory: row counts around its eight rows a unit, k ranges that end in
+the middle of a stage, a last slab of 128 columns, more stages than the ring holds."""
+import pytest
+import torch
+
+from oracle import oracle as O
+from tests.test_gpu_gemv import SENTINEL, _fp4_case, _int8_case, run_gemv
+from tests.util import assert_close_to_golden
+
+pytestmark = pytest.mark.gpu
+COUNTS = [8, 0, 9, 16, 17, 1, 7]
+
+
+@pytest.mark.parametrize("ct,K,N", [
+    ("int8", 64, 256), ("int8", 192, 512), ("int8", 1408, 768),
+    ("fp8", 128, 128), ("fp8", 1408, 384),
+    ("fp4", 64, 256), ("fp4", 320, 512), ("fp4", 2176, 256),
+])
+def test_matches_oracle(ct, K, N):
+    import ascend_kernel_b200 as ak
+
+    gen = torch.Generator().manual_seed(K + N)
+    G, cnt, offset = len(COUNTS), torch.tensor(COUNTS, dtype=torch.int64), None
+    if ct == "int8":
+        x, w, scale, offset, cnt = _int8_case(COUNTS, K, N, K + N, True)
+    elif ct == "fp8":
+        x = torch.randn(sum(COUNTS), K, generator=gen).to(torch.bfloat16)
+        w = torch.randint(0, 256, (G, K, N), generator=gen, dtype=torch.uint8)
+        scale = torch.randn(G, K // 128, N // 128, generator=gen)
+    else:
+        x, w, scale, cnt = _fp4_case(COUNTS, K, N, K + N)
+        x[3, 5] = 2.0 ** -100   # a row for the fp32 kernel, in a unit whose second four rows are not done again
+        x[8:17, 1] = 2.0 ** -90  # and units that it does as a whole
+    x = torch.cat([x, torch.full((2, K), float("nan"), dtype=torch.bfloat16)])  # rows of no expert, beside the last unit's
+    gold = O.golden_f32(x, w, scale, offset, cnt, ct, O.GROUP_LIST_COUNTS, weight_layout="canonical", gemv=True)
+    for lay in ("canonical", "ascend") if ct == "fp4" else ("canonical",):
+        wd = ak.fp4_layout(w.cuda(), to_ascend=True).cpu() if lay == "ascend" else w
+        out, st = run_gemv(x, wd, scale, cnt, ct, offset, gl_type=1, layout=lay)
+        assert st == (0, 0)
+        assert (out[sum(COUNTS):].float() == SENTINEL).all()
+        assert_close_to_golden(out, gold, ulps=1.0 if ct == "int8" else 2.0)
