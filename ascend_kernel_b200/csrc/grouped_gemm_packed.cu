@@ -610,10 +610,203 @@ __device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUt
     }
 }
 
+// ---- few rows an expert: the legacy tensor instruction on weights streamed through shared memory -----------------------
+// With at most 16 rows on every expert the pass is bound by the weights' way from HBM, and handing every 64-k stage through
+// registers, tensor memory and three roles took a third longer than that (~1000 cycles a stage against 700).  Here the packed stages (128 k of a
+// 256-column tile, 32 KB in one piece) land in a ring in shared memory and 16 warps take 16 columns each, all of k: no
+// hand-over but the ring's, no sums across warps.  mma.sync m16n8k16, weights as the 16 x 16 operand: lane (g, t) holds columns g and g + 8
+// and, of each 16-k chunk, word t of the column's 16 bytes, whose (k, k + 1) pairs the conversion gives as they are; x
+// enters with the same k order.
+struct Gemv {
+    static constexpr int kMaxR = 16, kStages = 4, kWarps = 16, kWarp0 = 4;
+    static constexpr int kWBytes = 2 * kStageWBytes, kXBytes = 2 * kSmallBox * kBK * 2, kSlotBytes = kWBytes + kXBytes;
+    static constexpr int kOutBytes = kMaxR * kTileN * 4;
+    static constexpr int kBytes = kStages * kSlotBytes + kOutBytes + kBarrierBytes;
+    static_assert(kStages <= Decode::kStages && kBytes <= Prefill::kBytes, "barriers, shared memory");
+};
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <bool GATE_UP>
+__device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xs, const uint8_t* __restrict__ weight, const GemmArgs& a, uint8_t* base,
+                                          const int* row_start, int* tile_prefix, __nv_bfloat16* const* s_dst_base) {
+    uint8_t* ring = base;
+    float* out = reinterpret_cast<float*>(ring + Gemv::kStages * Gemv::kSlotBytes);  // [16 rows][256 columns]
+    Barriers* sb = reinterpret_cast<Barriers*>(reinterpret_cast<uint8_t*>(out) + Gemv::kOutBytes);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_nt = a.N / kTileN, n_kt = a.K / kBK;
+    if (warp == 0) {
+        int lo, hi, mine = 0, total;
+        lane_experts(a.G, lo, hi);
+        for (int g = lo; g < hi; ++g) mine += (row_start[g + 1] - row_start[g] + Gemv::kMaxR - 1) / Gemv::kMaxR;
+        int at = warp_exclusive_sum(mine, total);
+        for (int g = lo; g < hi; ++g) {
+            tile_prefix[g] = at * n_nt;
+            at += (row_start[g + 1] - row_start[g] + Gemv::kMaxR - 1) / Gemv::kMaxR;
+        }
+        if (lane == 0) {
+            tile_prefix[a.G] = total * n_nt;
+            sb->n_tiles = total * n_nt;
+        }
+    }
+    if (threadIdx.x == 32) {
+        sb->abort = 0;
+        for (int i = 0; i < kTileRing; ++i) sb->tile_ring[i] = tile_entry(0u, 0u, 0u, 0u, 0u);
+        for (int i = 0; i < Gemv::kStages; ++i) {
+            ptx::mbar_init(ptx::smem_u32(&sb->full[i]), 1);
+            ptx::mbar_init(ptx::smem_u32(&sb->empty[i]), Gemv::kWarps);
+        }
+        ptx::mbar_init(ptx::smem_u32(&sb->t_full), Gemv::kWarps);  // the consumers among themselves
+        ptx::fence_mbar_init();
+        ptx::prefetch_tensormap(&tmap_xs);
+    }
+    __syncthreads();
+    if (warp == kWarpProd) {
+        if (lane != 0) return;
+        const int n_tiles = sb->n_tiles;
+        int* ticket = a.status + 2;
+        int held = atomicAdd(ticket, 1);
+        uint32_t it = 0, published = 0;
+        for (bool ok = true; ok;) {
+            const bool live = held < n_tiles;
+            TileInfo ti;
+            TileEntry entry = tile_entry(published + 1, 0u, 0u, 0u, 0u);  // rows 0: the schedule has ended
+            if (live) {
+                ti = locate_tile<Gemv::kMaxR>(held, tile_prefix, row_start, a.G, n_nt);
+                entry = tile_entry(published + 1, (uint32_t)ti.row0, (uint32_t)ti.rows, (uint32_t)ti.g, (uint32_t)ti.j);
+                held = atomicAdd(ticket, 1);
+            }
+            // (the consumers are at most the ring's four stages, so five tiles, behind: a slot has been read before it is written again)
+            ring_store(&sb->tile_ring[published % kTileRing], entry);
+            ++published;
+            if (!live) break;
+            const uint8_t* wp = weight + ((size_t)ti.g * n_nt + ti.j) * n_kt * (size_t)kStageWBytes;
+            for (int kt = 0; kt < n_kt; kt += 2, ++it) {
+                const uint32_t s = it % Gemv::kStages, ph = (it / Gemv::kStages) & 1;
+                if (it >= Gemv::kStages && !pk_wait(&sb->empty[s], ph ^ 1, sb, a.status, 10 + (int)s)) { ok = false; break; }
+                const uint32_t bar = ptx::smem_u32(&sb->full[s]), at = ptx::smem_u32(ring + s * Gemv::kSlotBytes);
+                const int n = min(2, n_kt - kt);  // 64-k halves
+                ptx::mbar_arrive_expect_tx(bar, (uint32_t)(n * (Gemv::kSlotBytes / 2)));
+                ptx::bulk_load(at, wp + (size_t)kt * kStageWBytes, (uint32_t)(n * kStageWBytes), bar);
+                for (int h = 0; h < n; ++h)
+                    ptx::tma_load_2d(at + Gemv::kWBytes + h * (Gemv::kXBytes / 2), &tmap_xs, bar, (kt + h) * kBK, ti.row0);
+            }
+        }
+        if (*reinterpret_cast<volatile int*>(&sb->abort))  // copies in flight land before the shared memory goes
+            for (uint32_t j = (it > Gemv::kStages ? it - Gemv::kStages : 0); j < it; ++j)
+                (void)ptx::mbar_wait(ptx::smem_u32(&sb->full[j % Gemv::kStages]), (j / Gemv::kStages) & 1);
+        return;
+    }
+    if (warp < Gemv::kWarp0 || warp >= Gemv::kWarp0 + Gemv::kWarps) return;
+
+    const int w = warp - Gemv::kWarp0, tid = threadIdx.x - Gemv::kWarp0 * 32, g = lane >> 2, t = lane & 3;
+    const uint32_t ring_u32 = ptx::smem_u32(ring);
+    const uint32_t w_at = (uint32_t)((w >> 1) * 2048 + ((w & 1) * 16 + g) * 16 + t * 4);
+    const uint32_t x_at = (uint32_t)(Gemv::kWBytes + g * 128 + (t & 1) * 8);
+    const bool has_offset = a.offset != nullptr;
+    const int ld_out = GATE_UP ? (a.N >> 1) : a.N;
+    constexpr int kCols = GATE_UP ? 128 : kTileN, kStep = Gemv::kWarps * 32 / kCols;  // output columns of a tile; rows stored at a time
+    const int col = tid & (kCols - 1), row_first = tid / kCols;
+    uint32_t s = 0, ph = 0, sync_ph = 0, seq = 0;
+    bool scattered = false;
+    auto sync = [&]() {
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->t_full));
+        const bool ok = __all_sync(0xffffffffu, pk_wait(&sb->t_full, sync_ph, sb, a.status, 60));
+        sync_ph ^= 1u;
+        return ok;
+    };
+    for (;;) {
+        TileInfo ti;
+        if (!__all_sync(0xffffffffu, next_tile(sb, seq, ti, a.status))) break;
+        // the scales of the thread's output column, while the weights are on their way
+        const __nv_bfloat16* sp = static_cast<const __nv_bfloat16*>(a.scale) + (size_t)ti.g * a.N;
+        const __nv_bfloat16* op = has_offset ? a.offset + (size_t)ti.g * a.N : nullptr;
+        const int c0 = ti.j * kCols + col;
+        const float s0 = __bfloat162float(sp[c0]), so0 = has_offset ? s0 * __bfloat162float(op[c0]) : 0.f;
+        float s1 = 0.f, so1 = 0.f;
+        if constexpr (GATE_UP) {
+            s1 = __bfloat162float(sp[(a.N >> 1) + c0]);
+            if (has_offset) so1 = s1 * __bfloat162float(op[(a.N >> 1) + c0]);
+        }
+        float acc[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+        const bool two = ti.rows > 8;
+        bool ok = true;
+        for (int kt = 0; kt < n_kt; kt += 2) {
+            ok = __all_sync(0xffffffffu, pk_wait(&sb->full[s], ph, sb, a.status, 40 + (int)s));
+            if (!ok) break;
+            const uint32_t at = ring_u32 + s * Gemv::kSlotBytes;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h == 1 && kt + 1 >= n_kt) break;
+#pragma unroll
+                for (int kc = 0; kc < 4; ++kc) {
+                    uint32_t w0, w1;
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(at + w_at + h * kStageWBytes + kc * 512));
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w1) : "r"(at + w_at + h * kStageWBytes + kc * 512 + 128));
+                    const uint32_t xa = at + x_at + h * (Gemv::kXBytes / 2) + (((2 * kc + (t >> 1)) ^ g) << 4);
+                    uint32_t b0, b1, a0, a1, a2, a3;
+                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(xa));
+                    s8x4_to_bf16_even_odd(w0, a0, a2);
+                    s8x4_to_bf16_even_odd(w1, a1, a3);
+                    mma_16816(acc[0], a0, a1, a2, a3, b0, b1);
+                    if (two) {
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(xa + 1024));
+                        mma_16816(acc[1], a0, a1, a2, a3, b0, b1);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->empty[s]));
+            if (++s == Gemv::kStages) { s = 0; ph ^= 1u; }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (i == 1 && !two) break;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                out[(8 * i + 2 * t + (e & 1)) * kTileN + 16 * w + g + 8 * (e >> 1)] = acc[i][e];
+        }
+        if (!sync()) break;
+        for (int r = row_first; r < ti.rows; r += kStep) {
+            const float rs = has_offset ? __ldg(a.rowsum + ti.row0 + r) : 0.f;
+            float o = fmaf(so0, rs, s0 * (kS8Unit * out[r * kTileN + col]));
+            if constexpr (GATE_UP) {
+                const float gate = __bfloat162float(__float2bfloat16_rn(o));
+                const float up = __bfloat162float(__float2bfloat16_rn(fmaf(so1, rs, s1 * (kS8Unit * out[r * kTileN + 128 + col]))));
+                o = __fdividef(gate, 1.f + __expf(-gate)) * up;
+            }
+            __nv_bfloat16* dst;
+            if (GATE_UP || a.row_code == nullptr) {
+                dst = a.y + (size_t)(ti.row0 + r) * ld_out;
+            } else {
+                // scatter mode: the row's own destination (a code naming none is skipped)
+                const long long code = __ldg(a.row_code + ti.row0 + r);
+                const unsigned int bi = (unsigned int)(code >> 32), ri = (unsigned int)code;
+                if ((int)bi >= a.n_base || (long long)ri >= a.dst_rows) continue;
+                dst = s_dst_base[bi] + (size_t)ri * ld_out;
+                scattered = true;
+            }
+            dst[c0] = __float2bfloat16_rn(o);
+        }
+        if (!sync()) break;
+    }
+    // rows stored into other GPUs' memory must be visible there before a later kernel signals them
+    if (scattered) __threadfence_system();
+}
+
 // What a kernel holds: one shape, or both and the choice between them.
 enum class Which { kDecode, kPrefill, kEither };
 template <Which WHICH>
-constexpr int kRingBytes = WHICH == Which::kDecode ? Decode::kBytes : Prefill::kBytes;
+constexpr int kRingBytes = WHICH == Which::kDecode ? (Decode::kBytes > Gemv::kBytes ? Decode::kBytes : Gemv::kBytes) : Prefill::kBytes;
 static_assert(Decode::kBytes <= Prefill::kBytes, "kEither has room for both");
 
 // kEither: the decode step's shape where 32-row tiles make (nearly) no more waves of the grid than 160-row ones, and so
@@ -634,27 +827,29 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     int* tile_prefix = row_start + (a.G + 1);
 
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
-    if constexpr (WHICH == Which::kEither) {
-        __shared__ int s_decode;
+    if constexpr (WHICH != Which::kPrefill) {
+        __shared__ int s_how;  // 0: gemv_body, 1: 32-row tiles, 2: 160-row tiles
         if (threadIdx.x < 32) {
-            int lo, hi, t32 = 0, t160 = 0;
+            int lo, hi, t32 = 0, t160 = 0, most = 0;
             lane_experts(a.G, lo, hi);
             for (int g = lo; g < hi; ++g) {
                 const int rows = row_start[g + 1] - row_start[g];
                 t32 += (rows + Decode::kMaxR - 1) / Decode::kMaxR;
                 t160 += (rows + Prefill::kMaxR - 1) / Prefill::kMaxR;
+                most = max(most, rows);
             }
             const int n_nt = a.N / kTileN, ctas = (int)gridDim.x;
             const int w32 = (__reduce_add_sync(0xffffffffu, t32) * n_nt + ctas - 1) / ctas;
             const int w160 = (__reduce_add_sync(0xffffffffu, t160) * n_nt + ctas - 1) / ctas;
-            if (threadIdx.x == 0) s_decode = 16LL * w32 <= 17LL * w160;
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (threadIdx.x == 0) s_how = most <= Gemv::kMaxR ? 0 : (WHICH == Which::kDecode || 16LL * w32 <= 17LL * w160 ? 1 : 2);
         }
         __syncthreads();
-        if (s_decode) packed_body<GATE_UP, Decode>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+        if (s_how == 0) gemv_body<GATE_UP>(tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+        else if (WHICH == Which::kDecode || s_how == 1) packed_body<GATE_UP, Decode>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
         else packed_body<GATE_UP, Prefill>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
     } else {
-        using Only = std::conditional_t<WHICH == Which::kDecode, Decode, Prefill>;
-        packed_body<GATE_UP, Only>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
+        packed_body<GATE_UP, Prefill>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
     }
 }
 
