@@ -20,7 +20,8 @@ FP4_SCALE_NONE, FP4_SCALE_E8M0_PER32 = 0, 1
 STATUS_BYTES = 256
 
 EXPORTS = [
-    "b200moe_grouped_gemm", "b200moe_grouped_gemm_workspace_bytes", "b200moe_grouped_gemv",
+    "b200moe_grouped_gemm", "b200moe_grouped_gemm_workspace_bytes", "b200moe_grouped_gemm_scratch", "b200moe_grouped_gemm_scratch_bytes",
+    "b200moe_grouped_gemv",
     "b200moe_grouped_gemv_workspace_bytes", "b200moe_grouped_gemv_split_workspace_bytes", "b200moe_fp4_dequant", "b200moe_fp4_layout", "b200moe_silu_mul",
     "b200moe_ep_finish", "b200moe_gather_rows", "b200moe_gather_rows_sum", "b200moe_grouped_gemm_int8_packed_rowsum", "b200moe_grouped_gemm_int8_packed_bounded", "b200moe_combine", "b200moe_read_status", "b200moe_read_sticky_status", "b200moe_strerror", "b200moe_version",
     "b200moe_moe_route", "b200moe_moe_regroup_index", "b200moe_grouped_gemm_int8_noalloc", "b200moe_grouped_gemm_int8_noalloc_max_rows", "b200moe_noalloc_read_status",
@@ -62,10 +63,12 @@ def _load() -> ctypes.CDLL:
     gemm_args = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, i32, i32, vp, sz, vp]
     lib.b200moe_grouped_gemm.argtypes = gemm_args
     lib.b200moe_grouped_gemm.restype = i32
+    lib.b200moe_grouped_gemm_scratch.argtypes = gemm_args[:-1] + [vp, sz, vp]
+    lib.b200moe_grouped_gemm_scratch.restype = i32
     lib.b200moe_grouped_gemv.argtypes = gemm_args
     lib.b200moe_grouped_gemv.restype = i32
     for f in (lib.b200moe_grouped_gemm_workspace_bytes, lib.b200moe_grouped_gemv_workspace_bytes,
-              lib.b200moe_grouped_gemv_split_workspace_bytes):
+              lib.b200moe_grouped_gemv_split_workspace_bytes, lib.b200moe_grouped_gemm_scratch_bytes):
         f.argtypes = [i64, i64, i64, i64, i32, i32]
         f.restype = sz
     lib.b200moe_grouped_gemm_int8_silu.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i32, vp, sz, vp]

@@ -173,9 +173,19 @@ void GroupedGemm(at::Tensor x, at::Tensor weight, at::Tensor antiquantScaleOptio
     auto stream = c10::cuda::getCurrentCUDAStream();
     const size_t ws_bytes = b200moe_grouped_gemm_workspace_bytes(d.M, d.K, d.N, d.G, ct, layout);
     at::Tensor ws = workspace_for(x, ws_bytes, stream.stream());
-    raise_on(b200moe_grouped_gemm(x.data_ptr(), weight.data_ptr(), scale_ptr, offset,
-                                  groupListOptional.data_ptr<int64_t>(), output.data_ptr(), d.M, d.K, d.N, d.G, ct,
-                                  (int)group_list_type, layout, ws.data_ptr(), ws_bytes, stream.stream()),
+    // int4: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
+    const size_t scratch_bytes = b200moe_grouped_gemm_scratch_bytes(d.M, d.K, d.N, d.G, ct, offset != nullptr);
+    at::Tensor scratch;
+    if (scratch_bytes > 0) {
+        try {
+            scratch = at::empty({(int64_t)scratch_bytes}, x.options().dtype(at::kByte));
+        } catch (const c10::OutOfMemoryError&) {
+        }
+    }
+    raise_on(b200moe_grouped_gemm_scratch(x.data_ptr(), weight.data_ptr(), scale_ptr, offset,
+                                          groupListOptional.data_ptr<int64_t>(), output.data_ptr(), d.M, d.K, d.N, d.G, ct,
+                                          (int)group_list_type, layout, ws.data_ptr(), ws_bytes,
+                                          scratch.defined() ? scratch.data_ptr() : nullptr, scratch_bytes, stream.stream()),
              "grouped_gemm");
 }
 

@@ -19,6 +19,11 @@ struct GemmArgs {
     __nv_bfloat16* dst_base[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     int n_base = 0;
     long long dst_rows = 0;
+    // int4 in one pass (grouped_gemm.cu), scratch of the call: the rows' exponents, the tiles that the two-pass kernel does again, and
+    // [0] their number, [1] that kernel's ticket, [2] rows of x that are not exact in f16
+    const int* row_exp = nullptr;
+    int4* redo = nullptr;
+    int* redo_ctl = nullptr;
 };
 
 // out[m] = sum_k x[m, k] in fp32 for the rows the group list uses, and status words 0 .. 3 zeroed (grouped_gemm.cu).

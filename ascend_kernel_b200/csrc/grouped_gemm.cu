@@ -26,6 +26,8 @@
 // Weights never make a round trip through global memory.  Every wait is bounded; on expiry the
 // kernel records an error status, all roles wind down, copies in flight are given time to land
 // and TMEM is released.
+#include <cuda_fp16.h>
+
 #include <mutex>
 
 #include "common.cuh"
@@ -78,10 +80,17 @@ constexpr int kCtFp4Ascend = 16;
 // layer of 256 experts, 4096 tokens x 8, 7168 x 2048 takes 5.08 instead of 8.80 ms, and one of few tokens an eighth.
 constexpr int kCtFp4E8m0 = 17;
 
+// Internal kernel mode: int4 weights as f16, in one pass (see "int4 in one pass" below).
+constexpr int kCtInt4F16 = 18;
+constexpr int kOffsetSlots = 4;         // k rows that a scale group's offsets take
+constexpr int kInt4ScaleShift = 6;      // the scales enter times 2^6
+constexpr int kInt4BadRows = 512;       // one row in as many that is not exact in f16: all tiles go to the two-pass kernel
+constexpr int kRowNotF16 = -(1 << 30);  // in the place of a row's exponent
+
 template <int MODE>
 struct GmTraits {
     static constexpr bool kNibbles = (MODE == B200MOE_CT_FP4 || MODE == B200MOE_CT_INT4 || MODE == kCtFp4Ascend ||
-                                      MODE == kCtFp4E8m0);
+                                      MODE == kCtFp4E8m0 || MODE == kCtInt4F16);
     // int4 with per-128-k scale/offset: (w + o) * s does not fit bf16, so every k block is fed to
     // the tensor core twice -- a stage carries two weight tiles, hi = bf16(v) and lo = bf16(v - hi),
     // multiplied with the same x block; the fp32 accumulator then holds x @ v to about 2^-16 relative.
@@ -97,7 +106,7 @@ struct GmTraits {
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 14 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
-    static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4);
+    static constexpr bool kEightRows = (MODE == kCtFp4Ascend || MODE == B200MOE_CT_INT4 || MODE == kCtInt4F16);
     // Who turns a published tile number into rows and columns: the publisher, once, or each role for itself.  Resolved
     // entries cost the roles less at a tile switch but leave the dequant loop of the modes with 4 rows x 16 columns a thread
     // fewer registers.  Each role | publisher, us, libraries called in turn: 8192 tokens x 8 by popularity over 256 experts,
@@ -344,7 +353,8 @@ template <int MODE>
 struct PackedRegs {
     uint4 q[kDqRows];  // fp4 / int4 use only .x/.y of each
     uint4 s[2];        // fp4 only: the bf16 scales of the thread's 16 columns (one 16-row group)
-    uint32_t e[kDqRows];  // fp4 with e8m0 scales: the scale byte of each of the thread's rows; int4: e[0] locates its scales
+    uint32_t e[kDqRows];  // fp4 with e8m0 scales: the scale byte of each of the thread's rows; int4: e[0] locates its scales,
+                          // in one pass e[1] is 1 + the scale groups the thread has in an offset stage, 0 in the others
     float sf;          // fp8 only: the fp32 scale of the thread's 128 x 128 block
 };
 
@@ -407,7 +417,16 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
         return;
     }
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
-    if constexpr (MODE == B200MOE_CT_INT4) {
+    if constexpr (MODE == kCtInt4F16) {
+        if (it.kt * kBK >= a.K) {  // an offset stage: the thread's eight rows are four each of two scale groups
+            const int n_g = a.K >> 7, g0 = (it.kt * kBK - a.K + d.k0) / kOffsetSlots;
+            r.e[0] = (uint32_t)((((size_t)it.g * n_g + g0) * a.N + it.n0) >> 3) + d.chunk;
+            r.e[1] = 1u + (uint32_t)min(max(n_g - g0, 0), 2);
+            return;
+        }
+        r.e[1] = 0u;
+    }
+    if constexpr (MODE == B200MOE_CT_INT4 || MODE == kCtInt4F16) {
         uint32_t v[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = ldg_stream4(it.wp + (size_t)i * row_bytes);
@@ -647,6 +666,92 @@ __device__ __forceinline__ void convert_block_int4(const PackedRegs<B200MOE_CT_I
     }
 }
 
+// ---- int4 in one pass --------------------------------------------------------------------------------------
+// (w + o) * s has up to 16 significant bits, so one bf16 tile cannot hold it; w * s has at most 11, which f16 does, and f16
+// times f16 runs at the rate of bf16.  So x is written as f16 first (gm_int4_prepare_x_kernel: each row times the power of two that puts
+// its largest element into [2^14, 2^15)), the weights enter as w * s * 2^6, exact for scales of 2^-23 up to 2^7, and
+// what the offsets add, the sum over the scale groups of (o * s) * (sum of the group's x), is a matrix product as well: K / 128
+// groups are further k rows of the same accumulation, in bf16, four slots a group, (hi, lo, hi, lo) of o * s * 2^6, whose 16
+// bits they hold, against (hi, hi, mid, mid) of the fp32 sum, 17 bits of it.  The epilogue multiplies by the row's power
+// of two.  Against the hi + lo pair of tiles: half the MMAs plus 1 / 32, 13 instead of 34 instructions per eight codes.
+// Rows of x that f16 cannot hold (an element more than about 2^-32 below the row's largest, infinities, NaN) and tiles with a scale
+// or offset out of range are done again by the two-pass kernel: the epilogue lists such tiles.  Where more than
+// one row in kInt4BadRows is of that kind, the two-pass kernel does all tiles and this one none.
+// Stages that the offsets add to a tile.
+static int offset_stages(int64_t K) { return (int)((K / 128 * kOffsetSlots + kBK - 1) / kBK); }
+// 16-bit elements of a prepared row.
+static int64_t int4_pitch(int64_t K, bool offsets) { return K + (offsets ? (int64_t)offset_stages(K) * kBK : 0); }
+
+// Whether f16 holds w * s * 2^6 for every code (two bf16 scales a word), and the hi / lo pair of o * s * 2^6 is in bf16's range.
+__device__ __forceinline__ bool int4_scale_fits(uint32_t w) {
+    const uint32_t a = w & 0x7FFFu, b = (w >> 16) & 0x7FFFu;  // 0x3400: 2^-23, 0x4300: 2^7
+    return (a == 0u || a - 0x3400u < 0x0F00u) && (b == 0u || b - 0x3400u < 0x0F00u);
+}
+__device__ __forceinline__ bool int4_offset_fits(uint32_t w) {
+    const uint32_t a = w & 0x7FFFu, b = (w >> 16) & 0x7FFFu;  // 0x1780: 2^-80, 0x5D80: 2^60
+    return (a == 0u || a - 0x1780u < 0x4600u) && (b == 0u || b - 0x1780u < 0x4600u);
+}
+
+// Eight rows of eight columns, in the column order of the fp4 modes; `sa` as in convert_stage_fp4_ascend.
+__device__ __forceinline__ void convert_int4_f16(const PackedRegs<kCtInt4F16>& r, const uint4& s8, uint32_t sa) {
+    const uint4 sp = pair_scales(s8);
+    const uint32_t sb[4] = {sp.x, sp.y, sp.z, sp.w};
+    __half2 sc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const f32x2 up = mul_f32x2(pack_u32x2(sb[i] << 16, sb[i] & 0xFFFF0000u), pack_f32x2(1 << kInt4ScaleShift, 1 << kInt4ScaleShift));
+        sc[i] = __floats2half2_rn(f32x2_lo(up), f32x2_hi(up));
+    }
+    // code ^ 8 under the f16 1024 (or, four bits up, sixteen times it): one add or multiply-add gives the code's value
+    const __half2 k1032 = __float2half2_rn(-1032.f), k16th = __float2half2_rn(0.0625f), k72 = __float2half2_rn(-72.f);
+    const uint32_t w8[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        uint32_t o[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t w = h ? w8[j] >> 8 : w8[j];
+            uint32_t lo, hi;
+            asm("lop3.b32 %0, %1, 0x000F000F, 0x64086408, 0x6A;" : "=r"(lo) : "r"(w));  // (w & m) ^ c
+            asm("lop3.b32 %0, %1, 0x00F000F0, 0x64806480, 0x6A;" : "=r"(hi) : "r"(w));
+            const __half2 v0 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&lo), k1032), sc[2 * h]);
+            const __half2 v1 = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&hi), k16th, k72), sc[2 * h + 1]);
+            o[2 * h] = *reinterpret_cast<const uint32_t*>(&v0);
+            o[2 * h + 1] = *reinterpret_cast<const uint32_t*>(&v1);
+        }
+        sts128((sa ^ (uint32_t)(j << 4)) + (uint32_t)(j * 128), o[0], o[1], o[2], o[3]);
+    }
+}
+
+// The thread's eight rows of an offset stage: two scale groups, four slots each.
+__device__ __forceinline__ void convert_int4_offsets(const GemmArgs& a, uint32_t unit, int groups, uint32_t sa) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        uint32_t hi[4] = {0u, 0u, 0u, 0u}, lo[4] = {0u, 0u, 0u, 0u};
+        if (i < groups) {
+            const uint4 s = __ldg(static_cast<const uint4*>(a.scale) + unit + (size_t)i * (a.N >> 3));
+            const uint4 o = __ldg(reinterpret_cast<const uint4*>(a.offset) + unit + (size_t)i * (a.N >> 3));
+            const uint4 sp = pair_scales(s), op = pair_scales(o);
+            const uint32_t sw[4] = {sp.x, sp.y, sp.z, sp.w}, ow[4] = {op.x, op.y, op.z, op.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const f32x2 up = mul_f32x2(pack_u32x2(sw[c] << 16, sw[c] & 0xFFFF0000u), pack_f32x2(1 << kInt4ScaleShift, 1 << kInt4ScaleShift));
+                const f32x2 v = mul_f32x2(pack_u32x2(ow[c] << 16, ow[c] & 0xFFFF0000u), up);
+                hi[c] = pack_bf16x2(f32x2_lo(v), f32x2_hi(v));
+                const f32x2 rest = sub_f32x2(v, pack_u32x2(hi[c] << 16, hi[c] & 0xFFFF0000u));
+                lo[c] = pack_bf16x2(f32x2_lo(rest), f32x2_hi(rest));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kOffsetSlots; ++k) {
+            const int j = i * kOffsetSlots + k;
+            const uint32_t at = (sa ^ (uint32_t)(j << 4)) + (uint32_t)(j * 128);
+            if (k & 1) sts128(at, lo[0], lo[1], lo[2], lo[3]);
+            else sts128(at, hi[0], hi[1], hi[2], hi[3]);
+        }
+    }
+}
+
 // Position of the x producer's L2 prefetch in the (tile, k-stage) sequence of its CTA.
 struct StageIter {
     int kt;
@@ -659,8 +764,30 @@ struct StageIter {
 template <int MODE>
 __device__ __forceinline__ constexpr int acc_pos(int i) {
     return MODE == B200MOE_CT_INT8 || MODE == B200MOE_CT_FP8 ? ((i & ~3) | ((i & 1) << 1) | ((i >> 1) & 1))
-           : (MODE == kCtFp4Ascend || MODE == kCtFp4E8m0)   ? ((i & ~7) | ((i & 3) << 1) | ((i >> 2) & 1))
+           : (MODE == kCtFp4Ascend || MODE == kCtFp4E8m0 || MODE == kCtInt4F16) ? ((i & ~7) | ((i & 3) << 1) | ((i >> 2) & 1))
                                                             : i;
+}
+
+// One-pass int4: 2^(e - 6) of a row, and the check of a tile by one warp; what does not fit is listed for the two-pass kernel.
+__device__ __forceinline__ float int4_row_unit(int e) {
+    return e == kRowNotF16 ? 0.f : __uint_as_float((uint32_t)(e - kInt4ScaleShift + 127) << 23);
+}
+__device__ __noinline__ void int4_check_tile(const int* __restrict__ row_exp, const uint4* __restrict__ scale, const uint4* __restrict__ offset,
+                                             int n_g, int stride, int g, int row0, int rows, int n0, int4* redo, int* redo_count) {
+    const int lane = threadIdx.x & 31;
+    bool ok = true;
+    for (int i = lane; i < rows; i += 32) ok = ok && __ldca(row_exp + row0 + i) != kRowNotF16;
+    const size_t first = (size_t)g * n_g * stride + (n0 >> 3) + lane;
+#pragma unroll 4
+    for (int i = 0; i < n_g; ++i) {
+        const uint4 s = __ldg(scale + first + (size_t)i * stride);
+        ok = ok && int4_scale_fits(s.x) && int4_scale_fits(s.y) && int4_scale_fits(s.z) && int4_scale_fits(s.w);
+        if (offset != nullptr) {
+            const uint4 o = __ldg(offset + first + (size_t)i * stride);
+            ok = ok && int4_offset_fits(o.x) && int4_offset_fits(o.y) && int4_offset_fits(o.z) && int4_offset_fits(o.w);
+        }
+    }
+    if (!__all_sync(0xffffffffu, ok) && lane == 0) redo[atomicAdd(redo_count, 1)] = make_int4(g, row0, rows, n0);
 }
 
 // SILU (int8, fp4 with e8m0 scales): int8 weight columns come as blocks of 128 gate columns followed by the 128
@@ -685,8 +812,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_nt = (a.N + kBN - 1) / kBN;  // (fp8 only: the last tile may hold 128 columns)
-    const int n_kt = a.K / kBK;  // stages per tile
+    // stages per tile: the weights' and, in one-pass int4, the offsets'
+    const int n_wkt = a.K / kBK;
+    const int n_kt = n_wkt + (MODE == kCtInt4F16 && a.offset != nullptr ? (n_wkt / 2 * kOffsetSlots + kBK - 1) / kBK : 0);
 
+    if constexpr (MODE == B200MOE_CT_INT4) {
+        if (a.redo_ctl != nullptr) {
+            grid_dep_wait();
+            if (__ldcg(a.redo_ctl) == 0 && __ldcg(a.redo_ctl + 2) == 0) return;  // no tile to do again
+        }
+    }
     gm_schedule(a.group_list, a.G, a.M, a.gl_type, n_nt, row_start, tile_prefix, &sb->n_tiles, a.status);
     if (threadIdx.x == 32) {
         sb->abort = 0;
@@ -716,7 +851,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // (launched behind the row sums' kernel, everything up to here ran beside it: it zeroes the tile ticket)
     grid_dep_wait();
 
-    const int n_tiles = sb->n_tiles;
+    int n_tiles = sb->n_tiles;
+    bool listed = false;  // the tiles come from the list of those to do again
+    if constexpr (MODE == kCtInt4F16 || MODE == B200MOE_CT_INT4) {
+        if (a.redo_ctl != nullptr) {
+            const bool all_again = (long long)__ldcg(a.redo_ctl + 2) * kInt4BadRows > row_start[a.G];
+            if (MODE == kCtInt4F16 && all_again) n_tiles = 0;
+            if (MODE == B200MOE_CT_INT4 && !all_again) {
+                listed = true;
+                n_tiles = __ldcg(a.redo_ctl);
+            }
+        }
+    }
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sb->tmem_base);
 
     if (warp == kWarpA) {
@@ -729,7 +875,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             bool ok = true;
             // This thread runs furthest ahead (its L2 prefetch leads everything else), so it draws the
             // tiles.  One ticket is always held in hand, so the atomic's latency is off the path.
-            int* ticket = a.status + 2;  // zero at the start: by a memset before the launch, or by the row sums' kernel
+            // zero at the start: by a memset before the launch, or by the row sums' or x preparing kernel
+            int* ticket = MODE == B200MOE_CT_INT4 && a.redo_ctl != nullptr ? a.redo_ctl + 1 : a.status + 2;
             int held = atomicAdd(ticket, 1);
             StageIter far;  // the tile published last
             far.kt = 0;
@@ -737,7 +884,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 far.valid = held < n_tiles;
                 TileEntry entry = tile_entry(published + 1, RESOLVED ? 0u : ~0u, 0u, 0u, 0u);
                 if (far.valid) {
-                    far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
+                    if (MODE == B200MOE_CT_INT4 && listed) {
+                        const int4 e = __ldcg(a.redo + held);
+                        far.ti.g = e.x;
+                        far.ti.row0 = e.y;
+                        far.ti.rows = e.z;
+                        far.ti.n0 = e.w;
+                    } else {
+                        far.ti = locate_tile(held, tile_prefix, row_start, a.G, n_nt);
+                    }
                     entry = tile_entry(published + 1, (uint32_t)(RESOLVED ? far.ti.row0 : held), (uint32_t)far.ti.rows,
                                        (uint32_t)far.ti.g, (uint32_t)far.ti.n0 / kBN);
                 }
@@ -750,7 +905,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if constexpr (SPLIT) {
                     ptx::tma_prefetch_l2_2d(&tmap_w, far.ti.n0 / 4, far.ti.g * a.K + far.kt * kBK);
                     ptx::tma_prefetch_l2_2d(&tmap_w, (a.N + far.ti.n0) / 4, far.ti.g * a.K + far.kt * kBK);
-                } else if constexpr (!T::kDirect)
+                } else if (!T::kDirect && (MODE != kCtInt4F16 || far.kt < n_wkt))
                     ptx::tma_prefetch_l2_2d(&tmap_w, T::kNibbles ? far.ti.n0 / 2 : far.ti.n0, far.ti.g * a.K + far.kt * kBK);
                 if (++far.kt < n_kt) return;
                 far.kt = 0;
@@ -805,7 +960,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         // small stage / k offset.  The next stage's barrier is polled (non-blocking) right after a stage's MMAs are
         // issued, so that the poll's latency runs beside the commit's.
         const bool leader = ptx::elect_one();
-        const uint32_t idesc = ptx::umma_idesc_bf16(kBM, kBN, true);
+        const uint32_t idesc_bf16 = ptx::umma_idesc_bf16(kBM, kBN, true), idesc_f16 = ptx::umma_idesc_f16(kBM, kBN, true);
         // A: K-major, 8-row groups 1024 B apart, 32 B per 16 k inside the swizzle atom
         const uint64_t da0 = ptx::umma_desc_sw128(ptx::smem_u32(a_ring), 0, 1024);
         // B: MN-major, 64-column blocks kBK*128 B apart (LBO), 8-k groups 1024 B apart (SBO)
@@ -832,6 +987,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if (!ok) break;
                 ptx::tc_fence_after();
                 const uint32_t sn = sa + 1 == NS ? 0u : sa + 1, phn = sa + 1 == NS ? pha ^ 1u : pha;
+                const uint32_t idesc = MODE == kCtInt4F16 && kt < n_wkt ? idesc_f16 : idesc_bf16;
                 if (leader) {
                     const uint64_t da = da0 + (uint64_t)(sa * (kATileBytes >> 4));
 #pragma unroll
@@ -903,12 +1059,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 }
                 __syncwarp();
             }
+            if constexpr (MODE == kCtInt4F16) {
+                if (quarter == 0 && half == 0)  // one warp a tile, while it is being accumulated
+                    int4_check_tile(a.row_exp, static_cast<const uint4*>(a.scale), reinterpret_cast<const uint4*>(a.offset), a.K >> 7,
+                                    a.N >> 3, ti.g, ti.row0, ti.rows, ti.n0, a.redo, a.redo_ctl);
+            }
             if (!__all_sync(0xffffffffu, gm_wait(&sb->t_full[grp], use & 1, sb, a.status, 60 + grp))) break;
             ++use;
             ptx::tc_fence_after();
             {
                 const int row = ti.row0 + half * kBM + quarter * 32 + lane;
                 const bool row_ok = row < ti.row0 + ti.rows;
+                float unit = 1.f;  // (a row that is not exact in f16 comes out as zeros here)
+                if constexpr (MODE == kCtInt4F16) unit = row_ok ? int4_row_unit(__ldca(a.row_exp + row)) : 0.f;
                 const float rs = (has_offset && row_ok) ? __ldca(a.rowsum + row) : 0.f;
                 if constexpr (SILU) {
                     __nv_bfloat16* arow = a.y + (size_t)row * (a.N >> 1) + (ti.n0 >> 1);
@@ -984,6 +1147,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                             v2 = fmaf(o4.z, rs, s4.z * (kS8Unit * v2));
                             v3 = fmaf(o4.w, rs, s4.w * (kS8Unit * v3));
                         }
+                        if constexpr (MODE == kCtInt4F16) { v0 *= unit; v1 *= unit; v2 *= unit; v3 *= unit; }
                         o[2 * q] = pack_bf16x2(v0, v1);
                         o[2 * q + 1] = pack_bf16x2(v2, v3);
                     }
@@ -1040,13 +1204,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 const uint32_t slot = ib % NS;
                 Int4Scales sc4;
                 if constexpr (MODE == B200MOE_CT_INT4) sc4 = load_int4_scales(a, regs[u].e[0]);  // (late: registers)
+                uint4 s8;
+                if constexpr (MODE == kCtInt4F16)
+                    if (regs[u].e[1] == 0u) s8 = __ldg(static_cast<const uint4*>(a.scale) + regs[u].e[0]);
                 bool got = true;
                 if (ib >= NS) got = gm_wait(&sb->empty[slot], ((ib / NS) & 1) ^ 1, sb, a.status, 80 + (int)slot);
                 if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 const uint32_t sa = sa0 + slot * (uint32_t)(P * kBTileBytes);
                 if constexpr (MODE == B200MOE_CT_INT4)
                     convert_block_int4(regs[u], sc4, sa, sa + kBTileBytes);
-                else if constexpr (MODE == kCtFp4Ascend)
+                else if constexpr (MODE == kCtInt4F16) {
+                    if (regs[u].e[1] == 0u) convert_int4_f16(regs[u], s8, sa);
+                    else convert_int4_offsets(a, regs[u].e[0], (int)regs[u].e[1] - 1, sa);
+                } else if constexpr (MODE == kCtFp4Ascend)
                     convert_stage_fp4_ascend(regs[u], sa);
                 else
                     convert_stage<MODE>(regs[u], sa);
@@ -1071,16 +1241,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
 }
 
-// Row sums of x in fp32 (the offset term of the int8 epilogue): one warp per row.  Rows past the
-// last group are skipped (a caller may pass a buffer sized for the worst case as x).  Being the first kernel of its
-// call, it also zeroes status words 0 .. 3, which saves the call a memset of its own, and lets the GEMM start its
-// prologue beside it (4 experts, 128 rows, 256 x 512: 18.1 -> 12.3 us).
-__global__ void rowsum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int M, int K,
-                              const long long* __restrict__ group_list, int G, int gl_type, int* __restrict__ status) {
-    grid_dep_launch();
-    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
-    // rows in use = end of the last group (clamped to M): a warp-level reduction, then one shared
-    // atomic per warp
+// Rows in use = end of the last group (clamped to M), by a whole CTA: a warp-level reduction, then one shared
+// atomic per warp.
+__device__ __forceinline__ int used_rows(const long long* __restrict__ group_list, int G, int gl_type, int M) {
     __shared__ int s_used;
     if (threadIdx.x == 0) s_used = 0;
     __syncthreads();
@@ -1100,7 +1263,18 @@ __global__ void rowsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
         if (gl_type == B200MOE_GROUP_LIST_COUNTS) atomicAdd(&s_used, (int)v); else atomicMax(&s_used, (int)v);
     }
     __syncthreads();
-    const int used = (s_used < 0 || s_used > M) ? M : s_used;  // (a sum of eight clamped parts could wrap)
+    return (s_used < 0 || s_used > M) ? M : s_used;  // (a sum of eight clamped parts could wrap)
+}
+
+// Row sums of x in fp32 (the offset term of the int8 epilogue): one warp per row.  Rows past the
+// last group are skipped (a caller may pass a buffer sized for the worst case as x).  Being the first kernel of its
+// call, it also zeroes status words 0 .. 3, which saves the call a memset of its own, and lets the GEMM start its
+// prologue beside it (4 experts, 128 rows, 256 x 512: 18.1 -> 12.3 us).
+__global__ void rowsum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int M, int K,
+                              const long long* __restrict__ group_list, int G, int gl_type, int* __restrict__ status) {
+    grid_dep_launch();
+    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
+    const int used = used_rows(group_list, G, gl_type, M);
     const int wpb = blockDim.x >> 5;
     for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < used; row += gridDim.x * wpb) {
         const uint4* p = reinterpret_cast<const uint4*>(x + (size_t)row * K);
@@ -1130,11 +1304,84 @@ void launch_rowsum(const void* x, float* out, int64_t M, int64_t K, const int64_
                                                         reinterpret_cast<const long long*>(group_list), (int)G, gl_type, status);
 }
 
+// One-pass int4: a row of x as f16 times 2^-e, e into row_exp (kRowNotF16: not exact), behind it the offset stages' A operand.
+// One warp a row; the row's second reading comes from L1 or L2, so the bound is its bytes in and out.
+__global__ void __launch_bounds__(256)
+gm_int4_prepare_x_kernel(const __nv_bfloat16* __restrict__ x, uint16_t* __restrict__ x16, int* __restrict__ row_exp, int M, int K,
+                         int pitch, const long long* __restrict__ group_list, int G, int gl_type, int* __restrict__ status,
+                         int* __restrict__ ctl) {
+    grid_dep_launch();
+    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
+    const int used = used_rows(group_list, G, gl_type, M);
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, n_vec = K / 8, n_rest = (pitch - K) / 4;  // 8-byte pieces
+    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < used; row += gridDim.x * wpb) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * K);
+        uint4* dst = reinterpret_cast<uint4*>(x16 + (size_t)row * pitch);
+        uint2* rest = reinterpret_cast<uint2*>(x16 + (size_t)row * pitch + K);
+        uint32_t mx = 0u;  // bf16 magnitudes order like integers
+#pragma unroll 8
+        for (int i = lane; i < n_vec; i += 32) {
+            const uint4 q = __ldg(src + i);
+            mx = __vmaxu2(__vmaxu2(mx, __vmaxu2(q.x & 0x7FFF7FFFu, q.y & 0x7FFF7FFFu)), __vmaxu2(q.z & 0x7FFF7FFFu, q.w & 0x7FFF7FFFu));
+        }
+        mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
+        const int e_max = (int)(mx >> 7);  // biased exponent of the largest magnitude
+        const int e = mx == 0u ? 0 : e_max - 127 - 14;
+        // (2^-e and the epilogue's 2^(e - 6) are normal numbers)
+        bool ok = mx == 0u || (e_max >= 32 && e_max < 255);
+        const float down = ok ? __uint_as_float((uint32_t)(127 - e) << 23) : 0.f;
+        // (every lane runs all iterations: the sums' shuffles)
+#pragma unroll 4
+        for (int i0 = 0; i0 < n_vec; i0 += 32) {
+            const int i = i0 + lane;
+            float sum = 0.f;
+            if (i < n_vec) {
+                const uint4 q = __ldg(src + i);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+                uint32_t h[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float f0 = __uint_as_float(w[j] << 16) * down, f1 = __uint_as_float(w[j] & 0xFFFF0000u) * down;
+                    const __half2 hh = __floats2half2_rn(f0, f1);
+                    h[j] = *reinterpret_cast<const uint32_t*>(&hh);
+                    // exact: the same value back, and no zero that was none (f0, f1 themselves may underflow)
+                    const float2 back = __half22float2(hh);
+                    ok = ok && back.x == f0 && back.y == f1 && ((h[j] & 0x7FFFu) != 0u) == ((w[j] & 0x7FFFu) != 0u) &&
+                         ((h[j] & 0x7FFF0000u) != 0u) == ((w[j] & 0x7FFF0000u) != 0u);
+                    sum += f0 + f1;
+                }
+                dst[i] = make_uint4(h[0], h[1], h[2], h[3]);
+            }
+            if (n_rest > 0) {  // a scale group is 16 lanes
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if ((lane & 15) == 0 && i < n_vec) {
+                    const uint32_t hi = pack_bf16x2(sum, sum);
+                    const float r = sum - __uint_as_float(hi << 16);
+                    rest[i >> 4] = make_uint2(hi, pack_bf16x2(r, r));
+                }
+            }
+        }
+        for (int i = n_vec / 16 + lane; i < n_rest; i += 32) rest[i] = make_uint2(0u, 0u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) {
+            row_exp[row] = ok ? e : kRowNotF16;
+            if (!ok) atomicAdd(ctl + 2, 1);
+        }
+    }
+}
+
 // int8 tiles of fewer than 32 stages are resolved by the publisher.  Each role | publisher, us: 4 experts of 32 rows, 256 x 512: 13.2 |
 // 12.3; 32 of 300, 64 x 2048: 45.0 | 41.0; 128 experts, 32768 rows by popularity, 1024 x 4096: 489 | 474, its SiLU form 526 | 513; 64 of
 // 210, 1536 x 2048: 139.2 | 137.4, SiLU 154.7 | 155.9, 2048 x 2048: 172.6 | 170.8, SiLU 189.9 | 191.2; 128 of 32, 4096 x 2048: 363 |
 // 378, SiLU 376 | 398.
 constexpr int kInt8RolesK = 2048;
+
+// Whether a call of int4 goes through f16 in one pass.
+static bool int4_one_pass(int64_t M, int64_t K, int64_t N, int64_t G) {
+    (void)G;
+    return 2.0 * M * K * N >= 1e10;
+}
 
 static size_t gm_smem_bytes(int G) {
     return 1024 + (size_t)kNS * (kATileBytes + kBTileBytes) + kBarrierBytes + sizeof(float) * kEpiWarps * kEpiScaleFloats +
@@ -1146,9 +1393,11 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
     using T = GmTraits<MODE>;
     if (MODE == B200MOE_CT_INT8 && !RESOLVED && a.K < kInt8RolesK) return gm_launch<MODE, SILU, true>(x, w, a, stream);
     CUtensorMap tx, txs, tw;
-    int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)a.M, a.K, kBM, kBK, true);
+    // (one-pass int4: x is the prepared one)
+    const uint64_t x_cols = MODE == kCtInt4F16 ? (uint64_t)int4_pitch(a.K, a.offset != nullptr) : (uint64_t)a.K;
+    int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)a.M, x_cols, kBM, kBK, true);
     if (rc != B200MOE_OK) return rc;
-    rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)a.M, a.K, kSmallRows, kBK, true);
+    rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)a.M, x_cols, kSmallRows, kBK, true);
     if (rc != B200MOE_OK) return rc;
     if (T::kDirect)
         rc = make_tensor_map_2d(&tw, w, 2, (uint64_t)a.G * a.K, a.N, kBK, 64, true);
@@ -1160,7 +1409,7 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
     const size_t smem = gm_smem_bytes(a.G);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, SILU, RESOLVED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    if (a.rowsum != nullptr) {  // launch_rowsum came directly before
+    if (a.rowsum != nullptr || a.redo_ctl != nullptr) {  // the kernel before is launch_rowsum's, or one of one-pass int4
         B200MOE_CUDA_TRY(launch_dependent(grouped_gemm_kernel<MODE, SILU, RESOLVED>, (unsigned)sm_count(), kGemmThreads, smem, stream, tx, txs, tw,
                                           static_cast<const uint8_t*>(w), a));
     } else {
@@ -1171,6 +1420,20 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
 }
 
 static size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
+
+// Scratch of a one-pass int4 call: control words, row exponents, the list of tiles to do again, x as f16.
+struct Int4Scratch {
+    size_t exp, redo, x16, bytes;
+};
+static Int4Scratch int4_scratch(int64_t M, int64_t K, int64_t N, int64_t G, bool offsets) {
+    const size_t tiles = (size_t)(N / kBN) * (size_t)(M / kTileM + (M < G ? M : G));  // at most
+    Int4Scratch s;
+    s.exp = 256;
+    s.redo = s.exp + align256((size_t)M * sizeof(int));
+    s.x16 = s.redo + align256(tiles * sizeof(int4));
+    s.bytes = s.x16 + (size_t)M * (size_t)int4_pitch(K, offsets) * 2;
+    return s;
+}
 
 }  // namespace b200moe
 
@@ -1184,10 +1447,24 @@ extern "C" size_t b200moe_grouped_gemm_workspace_bytes(int64_t M, int64_t K, int
     return b;
 }
 
+extern "C" size_t b200moe_grouped_gemm_scratch_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type, int has_offset) {
+    if (compute_type != B200MOE_CT_INT4 || M <= 0 || K <= 0 || N <= 0 || G <= 0 || (K % 128) != 0 || (N % kBN) != 0) return 0;
+    if (!int4_one_pass(M, K, N, G)) return 0;
+    return int4_scratch(M, K, N, G, has_offset != 0).bytes;
+}
+
 extern "C" int b200moe_grouped_gemm(const void* x, const void* weight, const void* scale, const void* offset,
                                     const int64_t* group_list, void* y, int64_t M, int64_t K, int64_t N, int64_t G,
                                     int compute_type, int group_list_type, int weight_layout, void* workspace,
                                     size_t workspace_bytes, void* stream) {
+    return b200moe_grouped_gemm_scratch(x, weight, scale, offset, group_list, y, M, K, N, G, compute_type, group_list_type,
+                                        weight_layout, workspace, workspace_bytes, nullptr, 0, stream);
+}
+
+extern "C" int b200moe_grouped_gemm_scratch(const void* x, const void* weight, const void* scale, const void* offset,
+                                            const int64_t* group_list, void* y, int64_t M, int64_t K, int64_t N, int64_t G,
+                                            int compute_type, int group_list_type, int weight_layout, void* workspace,
+                                            size_t workspace_bytes, void* scratch, size_t scratch_bytes, void* stream) {
     if (compute_type < B200MOE_CT_FP8 || compute_type > B200MOE_CT_BF16) return B200MOE_ERR_COMPUTE_TYPE;
     if (group_list_type != B200MOE_GROUP_LIST_CUMSUM && group_list_type != B200MOE_GROUP_LIST_COUNTS)
         return B200MOE_ERR_ARGUMENT;
@@ -1210,8 +1487,11 @@ extern "C" int b200moe_grouped_gemm(const void* x, const void* weight, const voi
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200MOE_ERR_WORKSPACE;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // (the row sums' kernel zeroes the status words itself)
-    if (compute_type != B200MOE_CT_INT8 || offset == nullptr) B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
+    const size_t scratch_need = b200moe_grouped_gemm_scratch_bytes(M, K, N, G, compute_type, offset != nullptr);
+    const bool one_pass = scratch_need != 0 && scratch != nullptr && scratch_bytes >= scratch_need && aligned16(scratch);
+    // (the row sums' kernel zeroes the status words itself, and so does the one that prepares x for one-pass int4)
+    if (one_pass) B200MOE_CUDA_TRY(cudaMemsetAsync(scratch, 0, 16, s));
+    else if (compute_type != B200MOE_CT_INT8 || offset == nullptr) B200MOE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
     uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
     GemmArgs a;
     a.scale = scale;
@@ -1236,7 +1516,20 @@ extern "C" int b200moe_grouped_gemm(const void* x, const void* weight, const voi
     }
     if (compute_type == B200MOE_CT_INT4) {
         a.offset = static_cast<const __nv_bfloat16*>(offset);  // folded into the weights by the dequant warps
-        return gm_launch<B200MOE_CT_INT4>(x, weight, a, s);
+        if (!one_pass) return gm_launch<B200MOE_CT_INT4>(x, weight, a, s);
+        const Int4Scratch at = int4_scratch(M, K, N, G, offset != nullptr);
+        uint8_t* sc = static_cast<uint8_t*>(scratch);
+        int* exps = reinterpret_cast<int*>(sc + at.exp);
+        void* x16 = sc + at.x16;
+        a.row_exp = exps;
+        a.redo = reinterpret_cast<int4*>(sc + at.redo);
+        a.redo_ctl = reinterpret_cast<int*>(sc);
+        gm_int4_prepare_x_kernel<<<rowsum_blocks(M), 256, 0, s>>>(
+            static_cast<const __nv_bfloat16*>(x), static_cast<uint16_t*>(x16), exps, (int)M, (int)K, (int)int4_pitch(K, offset != nullptr),
+            reinterpret_cast<const long long*>(group_list), (int)G, group_list_type, a.status, a.redo_ctl);
+        B200MOE_CUDA_TRY(cudaGetLastError());
+        const int rc = gm_launch<kCtInt4F16>(x16, weight, a, s);
+        return rc != B200MOE_OK ? rc : gm_launch<B200MOE_CT_INT4>(x, weight, a, s);
     }
     if (compute_type == B200MOE_CT_FP8) return gm_launch<B200MOE_CT_FP8>(x, weight, a, s);
     if (compute_type == B200MOE_CT_BF16) return gm_launch<B200MOE_CT_BF16>(x, weight, a, s);

@@ -218,6 +218,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t
 // as given.
 // (Both operands must carry the same 16-bit format: a bf16 A with an fp16 B is rejected by the
 // hardware as an illegal instruction.)
+// umma_idesc_f16: both f16 (format 0).
+__device__ __forceinline__ uint32_t umma_idesc_f16(int m, int n, bool b_mn_major) {
+    return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n, bool b_mn_major) {
     uint32_t d = 0;
     d |= 1u << 4;                      // D format: f32

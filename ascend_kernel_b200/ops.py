@@ -164,11 +164,22 @@ def grouped_gemm(x, weight, antiquantScaleOptional, antiquantOffsetOptional, gro
     offset = antiquantOffsetOptional if ct in (CT["int8"], CT["int4"]) else None  # ignored for fp8/fp4
     if offset is not None:
         _check_scale(offset, ct, G, K, N, "antiquantOffsetOptional")
-    ws = _run(_lib.b200moe_grouped_gemm, _lib.b200moe_grouped_gemm_workspace_bytes, "grouped_gemm", x, weight,
+    # int4: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
+    scratch, scratch_bytes = None, _lib.b200moe_grouped_gemm_scratch_bytes(M, K, N, G, ct, int(offset is not None))
+    if scratch_bytes > 0:
+        try:
+            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=x.device)
+        except torch.cuda.OutOfMemoryError:
+            pass
+
+    def fn(*args):
+        return _lib.b200moe_grouped_gemm_scratch(*args[:-1], _ptr(scratch), scratch_bytes, args[-1])
+
+    ws = _run(fn, _lib.b200moe_grouped_gemm_workspace_bytes, "grouped_gemm", x, weight,
               antiquantScaleOptional, offset, groupListOptional, output, ct, group_list_type,
               LAYOUT[weight_layout], M, K, N, G)
-    if M > 0:  # GEMM + row sums for the int8 offset term (pre-shuffled fp4 weights are read in place)
-        _count(1 + (offset is not None and ct == CT["int8"]))
+    if M > 0:  # GEMM + row sums for the int8 offset term (pre-shuffled fp4 weights are read in place), or one-pass int4's three
+        _count(3 if scratch is not None else 1 + (offset is not None and ct == CT["int8"]))
     return ws if return_workspace else None
 
 
