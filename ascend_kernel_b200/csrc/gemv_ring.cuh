@@ -1,25 +1,31 @@
 // Grouped GEMV on the tensor core with its operands streamed through a shared-memory ring (part of grouped_gemv.cu).
 //
-// One CTA a multiprocessor: a producer warp and 16 consumer warps.  The producer's lane draws the units (up to 8 rows of an
-// expert, slab of 256 columns, part of the k range), and copies their stages by TMA: 128 k rows of the slab's
+// Two CTAs a multiprocessor, each a producer warp and 8 consumer warps.  The producer's lane draws the units (up to 8 rows of an
+// expert, slab of 256 columns, part of the k range), and copies their stages by TMA: 64 k rows of the slab's
 // packed weights, of the group scales (fp4) and of the unit's x rows.  It runs ahead of the consumers by the ring, over the
 // end of a unit, so the next unit's first weights arrive while the sums of this one are being put together; with loads
 // into registers a unit started cold: ticket, look-up, staging of x, first loads, each waited for in turn.
 // Every consumer warp takes 16 k rows x 128 columns of each stage: eight mma.sync m16n8k16 with the weights as the 16 x 16
 // operand and up to eight x rows as the other (a legacy instruction on purpose: the tile is 16 x 8 and HBM is the bound).
+// us, register kernel | one CTA of 16 consumer warps and stages of 128 k | this, called in turn with the register kernel: int8, 32 tokens x 8
+// over 256 experts, 7168 x 4096: 886 | 830, 875 | 784 (6.1 TB/s); stored fp4, 37 tokens x 8, 2048 x 7168: 427 | 376, 419 | 354 (4.6
+// TB/s); fp8, one token on 8 experts, 7168 x 4096: 70.3 | 74.4, 70.3 | 67.1.  One CTA leaves its multiprocessor without work
+// while its sums are put together (1200 .. 1700 cycles a unit); what is left at two is issue slots (about 3 per fp8 weight, 2 per fp4
+// and int8 one).
 #pragma once
 
 #include "ptx.cuh"
 
 namespace b200moe {
 
-constexpr int kRgWarps = 16;                      // consumers
+constexpr int kRgK = 64;                          // k rows of a stage
+constexpr int kRgKGroups = kRgK / 16;             // warps along k; two along the columns
+constexpr int kRgWarps = 2 * kRgKGroups;          // consumers
 constexpr int kRgThreads = (kRgWarps + 1) * 32;
 constexpr int kRgRows = 8;                        // x rows per unit: the instruction's n
-constexpr int kRgK = 128;                         // k rows of a stage
-constexpr int kRgKGroups = kRgK / 16;             // warps along k; two along the columns
 constexpr int kRgRedRows = 4;                     // rows whose sums are put together at a time
-constexpr int kRgXBytes = kRgRows * kRgK * 2;     // two swizzled boxes of 8 rows x 64 k
+constexpr int kRgXBytes = kRgRows * kRgK * 2;     // a swizzled box of 8 rows x 64 k
+static_assert(kRgWarps * 32 == kGvSlabN, "one thread a column");
 constexpr int kRgSlotFloats = 2 * kGvSlotFloats;  // (a slot holds eight rows)
 static_assert(kRgSlotFloats >= kRgRows * kGvSlabN + kRgRows, "slot");
 
@@ -29,8 +35,8 @@ struct RgTraits {
     static constexpr int kWBytes = kRgK * (kFp4 ? kGvSlabN / 2 : kGvSlabN);
     static constexpr int kSBytes = kFp4 ? kRgK / 16 * kGvSlabN * 2 : 0;
     static constexpr int kStageBytes = kWBytes + kSBytes + kRgXBytes;
-    static constexpr int kStages = kFp4 ? 8 : 5;
-    static_assert(kWBytes % 1024 == 0 && kSBytes % 1024 == 0 && kRgXBytes % 2048 == 0, "swizzled boxes");
+    static constexpr int kStages = kFp4 ? 7 : 5;
+    static_assert(kWBytes % 1024 == 0 && kSBytes % 1024 == 0 && kRgXBytes % 1024 == 0, "swizzled boxes");
 };
 
 struct RgUnit {
@@ -167,7 +173,7 @@ __device__ __forceinline__ void rg_step_fp4(const uint2 (&q)[4], const uint4& s0
 }
 
 template <int MODE, bool STORED>
-__global__ void __launch_bounds__(kRgThreads, 1)
+__global__ void __launch_bounds__(kRgThreads, 2)
 gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                  const __grid_constant__ CUtensorMap tmap_x, const GemvArgs a) {
     using T = RgTraits<MODE>;
@@ -275,7 +281,6 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     const uint32_t s = it % T::kStages, ph = (it / T::kStages) & 1;
                     if (it >= T::kStages && !rg_wait(&sb->empty[s], ph ^ 1, sb, a.status, 10 + (int)s)) { ok = false; break; }
                     const uint32_t bar = ptx::smem_u32(&sb->full[s]), at = ptx::smem_u32(ring + s * T::kStageBytes);
-                    // (a half last stage reads 64 rows too many: the next expert's, or zeros past the end, which no warp takes)
                     ptx::mbar_arrive_expect_tx(bar, (uint32_t)(upper ? T::kStageBytes : T::kStageBytes - T::kWBytes / 2));
                     if constexpr (T::kFp4) {
                         ptx::tma_load_2d(at, &tmap_w, bar, u.n0 / 2, u.g * a.K + k);
@@ -285,7 +290,6 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                         if (upper) ptx::tma_load_2d(at + T::kWBytes / 2, &tmap_w, bar, u.n0 + 128, u.g * a.K + k);
                     }
                     ptx::tma_load_2d(at + T::kWBytes + T::kSBytes, &tmap_x, bar, k, u.r0);
-                    ptx::tma_load_2d(at + T::kWBytes + T::kSBytes + kRgXBytes / 2, &tmap_x, bar, k + 64, u.r0);
                 }
                 if (!ok) break;
             }
@@ -304,7 +308,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint32_t w_at[2];
     if constexpr (T::kFp4 && STORED) {
         // stored order: row (b * 4 + aa) * 8 + p of a 64-row block, bytes 32 q ..: four rows' codes of eight columns
-        w_at[0] = (uint32_t)((kl >> 6) * 8192 + (((kl >> 4) & 3) * 8 + 4 * hc + (g >> 2)) * 128 + (g & 3) * 32 + 8 * t);
+        w_at[0] = (uint32_t)((kg * 8 + 4 * hc + (g >> 2)) * 128 + (g & 3) * 32 + 8 * t);
         w_at[1] = w_at[0] + 4 * 8 * 128;  // b = 1: rows 8 .. 15 of the scale group
     } else if constexpr (T::kFp4) {
         // 64 bytes = 128 columns of a row; the 16-byte pieces are swizzled with the row
@@ -314,8 +318,8 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         w_at[0] = (uint32_t)(hc * (T::kWBytes / 2) + (kl + 2 * t) * 128 + ((g ^ (2 * t)) << 4));
         w_at[1] = (uint32_t)(hc * (T::kWBytes / 2) + (kl + 2 * t + 1) * 128 + ((g ^ (2 * t + 1)) << 4));
     }
-    const uint32_t x_at = (uint32_t)(T::kWBytes + T::kSBytes + (kg >> 2) * (kRgXBytes / 2) + g * 128 + 4 * t);
-    const uint32_t x0 = x_at + (((2 * (kg & 3)) ^ g) << 4), x1 = x_at + (((2 * (kg & 3) + 1) ^ g) << 4);
+    const uint32_t x_at = (uint32_t)(T::kWBytes + T::kSBytes + g * 128 + 4 * t);
+    const uint32_t x0 = x_at + (((2 * kg) ^ g) << 4), x1 = x_at + (((2 * kg + 1) ^ g) << 4);
     const uint32_t s_at = (uint32_t)(T::kWBytes + kg * (kGvSlabN * 2) + c_first * 2);
     const uint32_t ring_u32 = ptx::smem_u32(ring);
     const bool sums = MODE == B200MOE_CT_INT8 && a.offset != nullptr;
@@ -342,7 +346,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             ok = __all_sync(0xffffffffu, rg_wait(&sb->full[s], ph, sb, a.status, 40 + (int)s));
             if (!ok) break;
             const uint32_t at = ring_u32 + s * T::kStageBytes;
-            if (k + kl < u.k1 && cols_on) {
+            if (cols_on) {
                 uint32_t b0 = 0u, b1 = 0u;
                 if (x_on) {
                     b0 = lds32(at + x0);
@@ -377,35 +381,36 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         if (!ok) break;
 
-        // ---- the eight k groups' sums -> shared memory -> one thread per column and two rows of four ----
+        // ---- the k groups' sums -> shared memory -> one thread per column ----
         if (sums && hc == 0) {
             xs += __shfl_xor_sync(0xffffffffu, xs, 1);
             xs += __shfl_xor_sync(0xffffffffu, xs, 2);
             if (t == 0) sb->xsum[kg][g] = xs;  // (read between the two barriers below)
         }
-        const int col = threadIdx.x & (kGvSlabN - 1), pair = threadIdx.x >> 8;
-        float v[kRgRows / kRgRedRows][2], xv[kRgRows / kRgRedRows][2];
+        const int col = threadIdx.x;
+        float v[kRgRows], xv[kRgRows];
 #pragma unroll
-        for (int r = 0; r < kRgRows / kRgRedRows; ++r) {
-            v[r][0] = v[r][1] = xv[r][0] = xv[r][1] = 0.f;
-            if (r * kRgRedRows < u.rows) {
-                if ((t >> 1) == r) {
+        for (int m = 0; m < kRgRows; ++m) v[m] = xv[m] = 0.f;
+#pragma unroll
+        for (int r = 0; r < kRgRows; r += kRgRedRows) {
+            if (r < u.rows) {
+                if (2 * t >= r && 2 * t < r + kRgRedRows) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const int cc = T::kFp4 && STORED ? c_first + 64 * (j >> 2) + 2 * (j & 3) : c_first + 2 * j;
 #pragma unroll
                         for (int e = 0; e < 2; ++e)  // rows 2t, 2t + 1
-                            *reinterpret_cast<float2*>(red + (kg * kRgRedRows + 2 * (t & 1) + e) * kGvSlabN + cc) = make_float2(c[j][e], c[j][2 + e]);
+                            *reinterpret_cast<float2*>(red + (kg * kRgRedRows + 2 * t - r + e) * kGvSlabN + cc) = make_float2(c[j][e], c[j][2 + e]);
                     }
                 }
                 if (!rg_sync(sb, sync_ph, a.status)) return;
 #pragma unroll
-                for (int w = 0; w < kRgKGroups; ++w) {
-                    v[r][0] += red[(w * kRgRedRows + 2 * pair) * kGvSlabN + col];
-                    v[r][1] += red[(w * kRgRedRows + 2 * pair + 1) * kGvSlabN + col];
-                    if (sums) {
-                        xv[r][0] += sb->xsum[w][r * kRgRedRows + 2 * pair];
-                        xv[r][1] += sb->xsum[w][r * kRgRedRows + 2 * pair + 1];
+                for (int m = 0; m < kRgRedRows; ++m) {
+                    if (r + m >= u.rows) break;
+#pragma unroll
+                    for (int w = 0; w < kRgKGroups; ++w) {
+                        v[r + m] += red[(w * kRgRedRows + m) * kGvSlabN + col];
+                        if (sums) xv[r + m] += sb->xsum[w][r + m];
                     }
                 }
                 if (!rg_sync(sb, sync_ph, a.status)) return;
@@ -416,13 +421,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if (u.n_split > 1) {
             float* slot = a.part_sums + (size_t)(u.slot + u.split) * kRgSlotFloats;
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int m = r * kRgRedRows + 2 * pair + e;
-                    if (m >= u.rows) continue;
-                    __stcg(slot + m * kGvSlabN + col, v[r][e]);
-                    if (sums && col == 0) __stcg(slot + kRgRows * kGvSlabN + m, xv[r][e]);
+            for (int m = 0; m < kRgRows; ++m)
+                if (m < u.rows) {
+                    __stcg(slot + m * kGvSlabN + col, v[m]);
+                    if (sums && col == 0) __stcg(slot + kRgRows * kGvSlabN + m, xv[m]);
                 }
             __threadfence();
             if (!rg_sync(sb, sync_ph, a.status)) return;
@@ -432,15 +434,12 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             __threadfence();
             const float* first = a.part_sums + (size_t)u.slot * kRgSlotFloats;
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int m = r * kRgRedRows + 2 * pair + e;
-                    if (m >= u.rows) continue;
-                    v[r][e] = xv[r][e] = 0.f;
+            for (int m = 0; m < kRgRows; ++m)
+                if (m < u.rows) {
+                    v[m] = xv[m] = 0.f;
                     for (int p = 0; p < u.n_split; ++p) {
-                        v[r][e] += __ldcg(first + (size_t)p * kRgSlotFloats + m * kGvSlabN + col);
-                        if (sums) xv[r][e] += __ldcg(first + (size_t)p * kRgSlotFloats + kRgRows * kGvSlabN + m);
+                        v[m] += __ldcg(first + (size_t)p * kRgSlotFloats + m * kGvSlabN + col);
+                        if (sums) xv[m] += __ldcg(first + (size_t)p * kRgSlotFloats + kRgRows * kGvSlabN + m);
                     }
                 }
         }
@@ -452,13 +451,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (sums) so_n = s_n * __bfloat162float(a.offset[(size_t)u.g * a.N + col_y]);
         }
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int m = r * kRgRedRows + 2 * pair + e;
-                if (m >= u.rows) continue;
-                float o = v[r][e];
-                if constexpr (MODE == B200MOE_CT_INT8) o = fmaf(so_n, xv[r][e], s_n * (kS8Unit * o));
+        for (int m = 0; m < kRgRows; ++m)
+            if (m < u.rows) {
+                float o = v[m];
+                if constexpr (MODE == B200MOE_CT_INT8) o = fmaf(so_n, xv[m], s_n * (kS8Unit * o));
                 if constexpr (T::kFp4) {
                     const int ex = __ldca(a.xexp + u.r0 + m);
                     o = scalbnf(o, ex == kGvNotF16 ? 0 : ex);
@@ -486,7 +482,7 @@ static int gv_ring_launch(const GemvArgs& a0, cudaStream_t stream) {
     const size_t smem = 1024 + (size_t)T::kStages * T::kStageBytes + sizeof(float) * kRgKGroups * kRgRedRows * kGvSlabN +
                         sizeof(RgBarriers) + sizeof(int) * 2 * (size_t)(a.G + 1);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(gemv_ring_kernel<MODE, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    B200MOE_CUDA_TRY(launch_dependent(gemv_ring_kernel<MODE, STORED>, (unsigned)sm_count(), kRgThreads, smem, stream, tw, ts, tx, a));
+    B200MOE_CUDA_TRY(launch_dependent(gemv_ring_kernel<MODE, STORED>, 2u * (unsigned)sm_count(), kRgThreads, smem, stream, tw, ts, tx, a));
     return B200MOE_OK;
 }
 
