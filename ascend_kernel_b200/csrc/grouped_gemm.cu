@@ -63,6 +63,11 @@ constexpr int kAHalfBytes = kBM * kBK * 2;   // one 128-row box
 constexpr int kATileBytes = 2 * kAHalfBytes;  // an x stage holds both row halves
 constexpr int kSmallRows = 32;                 // rows of the small x box (a nearly empty last row half)
 constexpr int kSmallBytes = kSmallRows * kBK * 2;
+// A last row half of at most this many rows is multiplied with M = 64, and its x comes in boxes of 32 rows: no less time on the tensor
+// core, but half of its shared-memory reads of x, and fewer x bytes from L2.  us with M = 128 | this: int8 / fp8 / int4 / fp4, 65536 rows by
+// popularity over 256 experts (two thirds of them with at most 64), 7168 x 4096: 5174 | 5018, 5908 | 5550, 5586 | 5390, fp4 with 32 rows on
+// every expert, 2048 x 7168: 1215 | 1100, fp4-stored layer of 4096 tokens x 8: 4810 | 4620 (scaled to one GPU by the start's times).
+constexpr int kHalfM = 64;
 constexpr int kBTileBytes = kBK * kBN * 2;
 constexpr uint32_t kTmemCols = 512;
 
@@ -916,14 +921,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 TileInfo ti;
                 if (!next_tile<RESOLVED>(sb, seq, ti, tile_prefix, row_start, a.G, n_nt, a.status) || !ok) break;
                 // The last row half of a tile often holds only a few rows of the expert (a second half
-                // of a dozen rows when an expert has a little over 128): a box of kSmallRows rows then
-                // replaces the 128-row box.  The MMA still reads 128 rows; what the rows beyond the box
+                // of a dozen rows when an expert has a little over 128): up to kHalfM rows come in one or two boxes of kSmallRows
+                // rows.  The MMA reads kHalfM rows then; what those beyond the boxes
                 // hold is left over from earlier stages and lands in accumulator rows that are never
                 // stored.
                 const int last_rows = ti.rows - (ti.halves - 1) * kBM;
-                const bool small_last = last_rows <= kSmallRows;
-                const uint32_t stage_bytes = (uint32_t)((ti.halves - 1) * kAHalfBytes + (small_last ? kSmallBytes : kAHalfBytes));
-                const CUtensorMap* last_map = small_last ? &tmap_xs : &tmap_x;
+                const int n_small = last_rows <= kHalfM ? (last_rows + kSmallRows - 1) / kSmallRows : 0;
+                const uint32_t stage_bytes = (uint32_t)((ti.halves - 1) * kAHalfBytes + (n_small ? n_small * kSmallBytes : kAHalfBytes));
                 for (int kt = 0; kt < n_kt; ++kt, ++ia) {
                     const uint32_t s = ia % NS, ph = (ia / NS) & 1;
                     if (ia >= NS && !gm_wait(&sb->empty[s], ph ^ 1, sb, a.status, 10 + (int)s)) { ok = false; break; }
@@ -936,13 +940,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                             ptx::tma_load_2d(ptx::smem_u32(b_ring + s * kBTileBytes + blk * (kBK * 128)), &tmap_w, bar,
                                              ti.n0 + blk * 64, ti.g * a.K + kx);
                     }
+                    uint32_t dst = ptx::smem_u32(a_ring + s * kATileBytes);
+                    int row = ti.row0;
                     if (ti.halves == 2) {
-                        ptx::tma_load_2d(ptx::smem_u32(a_ring + s * kATileBytes), &tmap_x, bar, kx, ti.row0);
-                        ptx::tma_load_2d(ptx::smem_u32(a_ring + s * kATileBytes + kAHalfBytes), last_map, bar, kx,
-                                         ti.row0 + kBM);
-                    } else {
-                        ptx::tma_load_2d(ptx::smem_u32(a_ring + s * kATileBytes), last_map, bar, kx, ti.row0);
+                        ptx::tma_load_2d(dst, &tmap_x, bar, kx, row);
+                        dst += kAHalfBytes;
+                        row += kBM;
                     }
+                    if (n_small == 0) ptx::tma_load_2d(dst, &tmap_x, bar, kx, row);
+                    for (int b = 0; b < n_small; ++b) ptx::tma_load_2d(dst + b * kSmallBytes, &tmap_xs, bar, kx, row + b * kSmallRows);
                     if (far.valid) far_step();
                 }
             }
@@ -980,6 +986,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             if (ok && use1 && uses1 >= 1) ok = gm_wait(&sb->t_empty[1], (uses1 - 1) & 1, sb, a.status, 31);
             if (!__all_sync(0xffffffffu, ok)) break;
             const uint32_t acc0 = tmem_base + (use0 ? 0u : (uint32_t)kBN);
+            // M = 64 instead of 128 in the last row half: what is taken off the instruction descriptors
+            const uint32_t less = ti.rows - (ti.halves - 1) * kBM <= kHalfM ? (uint32_t)((kBM - kHalfM) >> 4) << 24 : 0u;
             ptx::tc_fence_after();
             uint32_t accumulate = 0;
             for (int kt = 0; kt < n_kt; ++kt) {
@@ -995,13 +1003,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                         const uint64_t db = db0 + (uint64_t)((sa * P + p) * (kBTileBytes >> 4));
 #pragma unroll
                         for (int k16 = 0; k16 < kBK / 16; ++k16)
-                            ptx::umma_bf16(acc0, da + (uint64_t)(k16 * 2), db + (uint64_t)(k16 * 128), idesc,
+                            ptx::umma_bf16(acc0, da + (uint64_t)(k16 * 2), db + (uint64_t)(k16 * 128), ti.halves == 2 ? idesc : idesc - less,
                                            accumulate | (uint32_t)(k16 + p));
                         if (ti.halves == 2) {
 #pragma unroll
                             for (int k16 = 0; k16 < kBK / 16; ++k16)
                                 ptx::umma_bf16(acc0 + kBN, da + (uint64_t)((kAHalfBytes >> 4) + k16 * 2),
-                                               db + (uint64_t)(k16 * 128), idesc, accumulate | (uint32_t)(k16 + p));
+                                               db + (uint64_t)(k16 * 128), idesc - less, accumulate | (uint32_t)(k16 + p));
                         }
                     }
                 }
@@ -1068,8 +1076,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             ++use;
             ptx::tc_fence_after();
             {
-                const int row = ti.row0 + half * kBM + quarter * 32 + lane;
-                const bool row_ok = row < ti.row0 + ti.rows;
+                // (M = 64 leaves row i in TMEM lane 32 * (i / 16) + i % 16)
+                const bool half_m = ti.rows - half * kBM <= kHalfM;
+                const int row = ti.row0 + half * kBM + (half_m ? quarter * 16 + (lane & 15) : quarter * 32 + lane);
+                const bool row_ok = row < ti.row0 + ti.rows && !(half_m && lane >= 16);
                 float unit = 1.f;  // (a row that is not exact in f16 comes out as zeros here)
                 if constexpr (MODE == kCtInt4F16) unit = row_ok ? int4_row_unit(__ldca(a.row_exp + row)) : 0.f;
                 const float rs = (has_offset && row_ok) ? __ldca(a.rowsum + row) : 0.f;
