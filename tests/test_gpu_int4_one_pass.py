@@ -27,10 +27,10 @@ def _one_pass(x, K, N, G, offsets):
 
 
 @pytest.mark.parametrize("counts,K,N,offsets", [
-    ([1, 0, 127, 128, 129, 300, 1200], 2176, 1024, True),   # 17 scale groups: a second offset stage, nearly empty
-    ([700, 1, 33, 1000], 2048, 1024, False),                # no offset stages
-    ([4096 + 17, 256, 32, 8192], 128, 3584, True),          # one scale group: two weight stages and one of offsets
-    ([2] * 200 + [900], 896, 5120, True),
+    ([1, 0, 127, 128, 129, 300, 1200], 2176, 4096, True),   # 17 scale groups: a second offset stage, nearly empty
+    ([700, 1, 33, 1000], 2048, 4096, False),                # no offset stages
+    ([1] * 596 + [300, 129, 256, 64], 128, 1536, True),     # one scale group: two weight stages and one of offsets
+    ([2] * 200 + [900], 896, 1024, True),
 ])
 def test_matches_oracle(counts, K, N, offsets):
     x, w, s, o, cnt = _case(counts, K, N, offsets, 5)
@@ -53,7 +53,7 @@ def test_what_f16_does_not_hold_goes_through_the_two_pass_kernel(kind):
     import ascend_kernel_b200 as ak
     from ascend_kernel_b200 import _abi
 
-    K, N, counts = 1024, 2048, [1300, 0, 257, 1100]
+    K, N, counts = 2048, 4096, [1300, 0, 257, 1100]
     x, w, s, o, cnt = _case(counts, K, N, True, 6)
     assert _one_pass(x, K, N, len(counts), True)
     redone = torch.zeros(x.shape[0], N, dtype=torch.bool)
@@ -96,7 +96,7 @@ def test_captured_graph_replays_on_new_inputs():
     """Scratch of a captured call comes from the graph's pool; the list of tiles to do again is made anew by each replay."""
     import ascend_kernel_b200 as ak
 
-    K, N, counts = 1024, 1024, [1500, 0, 3100, 400]
+    K, N, counts = 2048, 2048, [1500, 0, 3100, 400]
     x, w, s, o, cnt = (t.cuda() for t in _case(counts, K, N, True, 8))
     assert _one_pass(x, K, N, 4, True)
     out = torch.zeros(x.shape[0], N, dtype=torch.bfloat16, device="cuda")
