@@ -616,7 +616,7 @@ __device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUt
 // 256-column tile, 32 KB in one piece) land in a ring in shared memory and 16 warps take 16 columns each, all of k: no
 // hand-over but the ring's, no sums across warps.  mma.sync m16n8k16, weights as the 16 x 16 operand: lane (g, t) holds columns g and g + 8
 // and, of each 16-k chunk, word t of the column's 16 bytes, whose (k, k + 1) pairs the conversion gives as they are; x
-// enters with the same k order.
+// enters with the same k order.  Layer of 256 experts, 32 tokens x 8, 7168 x 2048, called in turn with the 32-row shape alone: 1553 -> 1355 us.
 struct Gemv {
     static constexpr int kMaxR = 16, kStages = 5, kWarps = 16, kWarp0 = 4;
     static constexpr int kWBytes = 2 * kStageWBytes, kXBytes = 2 * kMaxR * kBK * 2, kSlotBytes = kWBytes + kXBytes;
@@ -803,13 +803,13 @@ __device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xg, const uint
     if (scattered) __threadfence_system();
 }
 
-// What a kernel holds: one shape, or both and the choice between them.
+// What a kernel holds: the 160-row shape, or gemv_body with the 32-row shape or with both, and the choice between them by the group list.
 enum class Which { kDecode, kPrefill, kEither };
 template <Which WHICH>
 constexpr int kRingBytes = WHICH == Which::kDecode ? (Decode::kBytes > Gemv::kBytes ? Decode::kBytes : Gemv::kBytes) : Prefill::kBytes;
 static_assert(Decode::kBytes <= Prefill::kBytes, "kEither has room for both");
 
-// kEither: the decode step's shape where 32-row tiles make (nearly) no more waves of the grid than 160-row ones, and so
+// No expert with more than 16 rows: gemv_body.  Otherwise, kEither: the 32-row shape where 32-row tiles make (nearly) no more waves of the grid than 160-row ones, and so
 // (nearly) no more dequantisation.  Time of the 160-row shape over that of the 32-row one, 256 experts, 7168 x 4096 / 2048 x 7168: one to
 // eight rows an expert, evenly or 8 of 256 experts a token: 1.03 .. 1.25 / 1.08 .. 1.22, with the same tiles; by popularity
 // (Zipf 1.2), 1, 2, 4 rows on average: 1.03, 1.11, 1.15 / 1.15, 1.14, 1.04 with 1.04 .. 1.11 times the waves; 6 and 8 rows: 0.99,
@@ -864,10 +864,11 @@ static int launch_one(const CUtensorMap& tx, const CUtensorMap& txs, const CUten
 }
 
 // More than eight rows an expert on average: prefill.  No expert with more than 32 rows (the caller says so, or there are no more),
-// or 32-row tiles in one wave however the rows are spread: decode.  Otherwise only the group list tells, and the kernel that holds
+// or 32-row tiles in one wave however the rows are spread: kDecode.  Otherwise only the group list tells, and the kernel that holds
 // both shapes decides; it needs the larger one's shared memory, whose place L1 then lacks.  256 experts, 7168 x 4096 with SiLU /
 // 2048 x 7168, us on the 160-row shape, the 32-row shape, through the choice: 32 tokens x 8: 1124, 999, 1029 / 590, 525, 545; 256 tokens
-// x 8: 1706, 1532, 1570 / 902, 797, 830; 1024 rows by popularity: 1245, 1234, 1281; 2048 rows on one expert: 123, 337, 122.  Two
+// x 8: 1706, 1532, 1570 / 902, 797, 830; 1024 rows by popularity: 1245, 1234, 1281; 2048 rows on one expert: 123, 337, 122 (before gemv_body,
+// which takes the first of these lists in either kernel).  Two
 // launches of which one leaves at once came to the same for long calls and cost short ones 4 us.
 template <bool GATE_UP>
 static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const CUtensorMap& txg, const void* packed, const GemmArgs& a, int64_t max_rows, cudaStream_t s) {
