@@ -617,9 +617,10 @@ __device__ __forceinline__ void packed_body(const CUtensorMap& tmap_x, const CUt
 // hand-over but the ring's, no sums across warps.  mma.sync m16n8k16, weights as the 16 x 16 operand: lane (g, t) holds columns g and g + 8
 // and, of each 16-k chunk, word t of the column's 16 bytes, whose (k, k + 1) pairs the conversion gives as they are; x
 // enters with the same k order.  Layer of 256 experts, 32 tokens x 8, 7168 x 2048, called in turn with the 32-row shape alone: 1553 -> 1355 us.
+// (x boxes of 16 rows and a fifth stage: 1337 -> 1329, within the runs' spread.)
 struct Gemv {
-    static constexpr int kMaxR = 16, kStages = 5, kWarps = 16, kWarp0 = 4;
-    static constexpr int kWBytes = 2 * kStageWBytes, kXBytes = 2 * kMaxR * kBK * 2, kSlotBytes = kWBytes + kXBytes;
+    static constexpr int kMaxR = 16, kStages = 4, kWarps = 16, kWarp0 = 4;
+    static constexpr int kWBytes = 2 * kStageWBytes, kXBytes = 2 * kSmallBox * kBK * 2, kSlotBytes = kWBytes + kXBytes;
     static constexpr int kOutBytes = kMaxR * kTileN * 4;
     static constexpr int kBytes = kStages * kSlotBytes + kOutBytes + kBarrierBytes;
     static_assert(kStages <= Decode::kStages && kBytes <= Prefill::kBytes, "barriers, shared memory");
@@ -633,7 +634,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 }
 
 template <bool GATE_UP>
-__device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xg, const uint8_t* __restrict__ weight, const GemmArgs& a, uint8_t* base,
+__device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xs, const uint8_t* __restrict__ weight, const GemmArgs& a, uint8_t* base,
                                           const int* row_start, int* tile_prefix, __nv_bfloat16* const* s_dst_base) {
     uint8_t* ring = base;
     float* out = reinterpret_cast<float*>(ring + Gemv::kStages * Gemv::kSlotBytes);  // [16 rows][256 columns]
@@ -663,7 +664,7 @@ __device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xg, const uint
         }
         ptx::mbar_init(ptx::smem_u32(&sb->t_full), Gemv::kWarps);  // the consumers among themselves
         ptx::fence_mbar_init();
-        ptx::prefetch_tensormap(&tmap_xg);
+        ptx::prefetch_tensormap(&tmap_xs);
     }
     __syncthreads();
     if (warp == kWarpProd) {
@@ -681,7 +682,7 @@ __device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xg, const uint
                 entry = tile_entry(published + 1, (uint32_t)ti.row0, (uint32_t)ti.rows, (uint32_t)ti.g, (uint32_t)ti.j);
                 held = atomicAdd(ticket, 1);
             }
-            // (the consumers are at most the ring's five stages, so six tiles, behind: a slot has been read before it is written again)
+            // (the consumers are at most the ring's four stages, so five tiles, behind: a slot has been read before it is written again)
             ring_store(&sb->tile_ring[published % kTileRing], entry);
             ++published;
             if (!live) break;
@@ -694,7 +695,7 @@ __device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xg, const uint
                 ptx::mbar_arrive_expect_tx(bar, (uint32_t)(n * (Gemv::kSlotBytes / 2)));
                 ptx::bulk_load(at, wp + (size_t)kt * kStageWBytes, (uint32_t)(n * kStageWBytes), bar);
                 for (int h = 0; h < n; ++h)
-                    ptx::tma_load_2d(at + Gemv::kWBytes + h * (Gemv::kXBytes / 2), &tmap_xg, bar, (kt + h) * kBK, ti.row0);
+                    ptx::tma_load_2d(at + Gemv::kWBytes + h * (Gemv::kXBytes / 2), &tmap_xs, bar, (kt + h) * kBK, ti.row0);
             }
         }
         if (*reinterpret_cast<volatile int*>(&sb->abort))  // copies in flight land before the shared memory goes
@@ -818,7 +819,7 @@ static_assert(Decode::kBytes <= Prefill::kBytes, "kEither has room for both");
 template <bool GATE_UP, Which WHICH>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xs,
-                           const __grid_constant__ CUtensorMap tmap_xg, const uint8_t* __restrict__ weight, const GemmArgs a) {
+                           const uint8_t* __restrict__ weight, const GemmArgs a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __nv_bfloat16* s_dst_base[8];  // scatter mode: the destination tensors (indexed per row)
@@ -845,7 +846,7 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
             if (threadIdx.x == 0) s_how = most <= Gemv::kMaxR ? 0 : (WHICH == Which::kDecode || 16LL * w32 <= 17LL * w160 ? 1 : 2);
         }
         __syncthreads();
-        if (s_how == 0) gemv_body<GATE_UP>(tmap_xg, weight, a, base, row_start, tile_prefix, s_dst_base);
+        if (s_how == 0) gemv_body<GATE_UP>(tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
         else if (WHICH == Which::kDecode || s_how == 1) packed_body<GATE_UP, Decode>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
         else packed_body<GATE_UP, Prefill>(tmap_x, tmap_xs, weight, a, base, row_start, tile_prefix, s_dst_base);
     } else {
@@ -854,11 +855,11 @@ grouped_gemm_packed_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
 }
 
 template <bool GATE_UP, Which WHICH>
-static int launch_one(const CUtensorMap& tx, const CUtensorMap& txs, const CUtensorMap& txg, const void* packed, const GemmArgs& a, cudaStream_t s) {
+static int launch_one(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, cudaStream_t s) {
     const size_t smem = 1024 + (size_t)kRingBytes<WHICH> + sizeof(int) * 2 * (size_t)(a.G + 1);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_packed_kernel<GATE_UP, WHICH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    grouped_gemm_packed_kernel<GATE_UP, WHICH><<<grid_ctas(), kThreads, smem, s>>>(tx, txs, txg, static_cast<const uint8_t*>(packed), a);
+    grouped_gemm_packed_kernel<GATE_UP, WHICH><<<grid_ctas(), kThreads, smem, s>>>(tx, txs, static_cast<const uint8_t*>(packed), a);
     B200MOE_CUDA_TRY(cudaGetLastError());
     return B200MOE_OK;
 }
@@ -871,13 +872,13 @@ static int launch_one(const CUtensorMap& tx, const CUtensorMap& txs, const CUten
 // which takes the first of these lists in either kernel).  Two
 // launches of which one leaves at once came to the same for long calls and cost short ones 4 us.
 template <bool GATE_UP>
-static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const CUtensorMap& txg, const void* packed, const GemmArgs& a, int64_t max_rows, cudaStream_t s) {
-    if (a.M > 8LL * a.G) return launch_one<GATE_UP, Which::kPrefill>(tx, txs, txg, packed, a, s);
+static int launch(const CUtensorMap& tx, const CUtensorMap& txs, const void* packed, const GemmArgs& a, int64_t max_rows, cudaStream_t s) {
+    if (a.M > 8LL * a.G) return launch_one<GATE_UP, Which::kPrefill>(tx, txs, packed, a, s);
     const long long experts = std::min(a.G, a.M);
     const long long tiles = (experts + (a.M - experts) / Decode::kMaxR) * (a.N / kTileN);  // at most
     if (std::min<int64_t>(max_rows, a.M) <= Decode::kMaxR || tiles <= grid_ctas())
-        return launch_one<GATE_UP, Which::kDecode>(tx, txs, txg, packed, a, s);
-    return launch_one<GATE_UP, Which::kEither>(tx, txs, txg, packed, a, s);
+        return launch_one<GATE_UP, Which::kDecode>(tx, txs, packed, a, s);
+    return launch_one<GATE_UP, Which::kEither>(tx, txs, packed, a, s);
 }
 
 // [G, K, N] int8 -> the packed order.  One thread writes one lane's 16 bytes of a k-chunk.
@@ -980,14 +981,12 @@ static int packed_launch(const void* x, const void* packed, const void* scale, c
             a.rowsum = rowsum;
         }
     }
-    CUtensorMap tx, txs, txg;
+    CUtensorMap tx, txs;
     int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)M, (uint64_t)K, pk::kBigBox, pk::kBK, true);
     if (rc != B200MOE_OK) return rc;
     rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)M, (uint64_t)K, pk::kSmallBox, pk::kBK, true);
     if (rc != B200MOE_OK) return rc;
-    rc = make_tensor_map_2d(&txg, x, 2, (uint64_t)M, (uint64_t)K, pk::Gemv::kMaxR, pk::kBK, true);
-    if (rc != B200MOE_OK) return rc;
-    return gate_up_silu ? pk::launch<true>(tx, txs, txg, packed, a, max_rows, s) : pk::launch<false>(tx, txs, txg, packed, a, max_rows, s);
+    return gate_up_silu ? pk::launch<true>(tx, txs, packed, a, max_rows, s) : pk::launch<false>(tx, txs, packed, a, max_rows, s);
 }
 
 extern "C" int b200moe_grouped_gemm_int8_packed(const void* x, const void* packed, const void* scale, const void* offset,
