@@ -108,6 +108,9 @@ struct GmTraits {
     // into the B ring (a 64 k x 128-byte box with the 128-byte swizzle is exactly one block of the
     // MN-major operand layout) and the dequant warps have nothing to do
     static constexpr bool kDirect = (MODE == B200MOE_CT_BF16);
+    // last row halves of at most this many rows are multiplied with M = 64 (not bf16, whose B tiles never pass the warps: 128 experts of
+    // 30 rows, 256 x 256, 12.3 us without, 12.75 with)
+    static constexpr int kShortRows = kDirect ? 0 : kHalfM;
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
     // columns instead of 16 (222 -> 14 bytes of spills; 8192 tokens x 8 over 256 experts, 7168 x 4096: 11.3 -> 9.2 ms)
@@ -926,7 +929,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 // hold is left over from earlier stages and lands in accumulator rows that are never
                 // stored.
                 const int last_rows = ti.rows - (ti.halves - 1) * kBM;
-                const int n_small = last_rows <= kHalfM ? (last_rows + kSmallRows - 1) / kSmallRows : 0;
+                const int n_small = last_rows <= max(T::kShortRows, kSmallRows) ? (last_rows + kSmallRows - 1) / kSmallRows : 0;
                 const uint32_t stage_bytes = (uint32_t)((ti.halves - 1) * kAHalfBytes + (n_small ? n_small * kSmallBytes : kAHalfBytes));
                 for (int kt = 0; kt < n_kt; ++kt, ++ia) {
                     const uint32_t s = ia % NS, ph = (ia / NS) & 1;
@@ -987,7 +990,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             if (!__all_sync(0xffffffffu, ok)) break;
             const uint32_t acc0 = tmem_base + (use0 ? 0u : (uint32_t)kBN);
             // M = 64 instead of 128 in the last row half: what is taken off the instruction descriptors
-            const uint32_t less = ti.rows - (ti.halves - 1) * kBM <= kHalfM ? (uint32_t)((kBM - kHalfM) >> 4) << 24 : 0u;
+            const uint32_t less = ti.rows - (ti.halves - 1) * kBM <= T::kShortRows ? (uint32_t)((kBM - kHalfM) >> 4) << 24 : 0u;
             ptx::tc_fence_after();
             uint32_t accumulate = 0;
             for (int kt = 0; kt < n_kt; ++kt) {
@@ -1077,7 +1080,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             ptx::tc_fence_after();
             {
                 // (M = 64 leaves row i in TMEM lane 32 * (i / 16) + i % 16)
-                const bool half_m = ti.rows - half * kBM <= kHalfM;
+                const bool half_m = ti.rows - half * kBM <= T::kShortRows;
                 const int row = ti.row0 + half * kBM + (half_m ? quarter * 16 + (lane & 15) : quarter * 32 + lane);
                 const bool row_ok = row < ti.row0 + ti.rows && !(half_m && lane >= 16);
                 float unit = 1.f;  // (a row that is not exact in f16 comes out as zeros here)
