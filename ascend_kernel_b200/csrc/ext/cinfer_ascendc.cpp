@@ -173,7 +173,7 @@ void GroupedGemm(at::Tensor x, at::Tensor weight, at::Tensor antiquantScaleOptio
     auto stream = c10::cuda::getCurrentCUDAStream();
     const size_t ws_bytes = b200moe_grouped_gemm_workspace_bytes(d.M, d.K, d.N, d.G, ct, layout);
     at::Tensor ws = workspace_for(x, ws_bytes, stream.stream());
-    // int4: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
+    // int4 without offsets: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
     const size_t scratch_bytes = b200moe_grouped_gemm_scratch_bytes(d.M, d.K, d.N, d.G, ct, offset != nullptr);
     at::Tensor scratch;
     if (scratch_bytes > 0) {

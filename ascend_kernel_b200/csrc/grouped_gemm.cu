@@ -87,7 +87,6 @@ constexpr int kCtFp4E8m0 = 17;
 
 // Internal kernel mode: int4 weights as f16, in one pass (see "int4 in one pass" below).
 constexpr int kCtInt4F16 = 18;
-constexpr int kOffsetSlots = 4;         // k rows that a scale group's offsets take
 constexpr int kInt4ScaleShift = 6;      // the scales enter times 2^6
 constexpr int kInt4BadRows = 512;       // one row in as many that is not exact in f16: all tiles go to the two-pass kernel
 constexpr int kRowNotF16 = -(1 << 30);  // in the place of a row's exponent
@@ -361,8 +360,7 @@ template <int MODE>
 struct PackedRegs {
     uint4 q[kDqRows];  // fp4 / int4 use only .x/.y of each
     uint4 s[2];        // fp4 only: the bf16 scales of the thread's 16 columns (one 16-row group)
-    uint32_t e[kDqRows];  // fp4 with e8m0 scales: the scale byte of each of the thread's rows; int4: e[0] locates its scales,
-                          // in one pass e[1] is 1 + the scale groups the thread has in an offset stage, 0 in the others
+    uint32_t e[kDqRows];  // fp4 with e8m0 scales: the scale byte of each of the thread's rows; int4: e[0] locates its scales
     float sf;          // fp8 only: the fp32 scale of the thread's 128 x 128 block
 };
 
@@ -425,15 +423,6 @@ __device__ __forceinline__ void load_packed(PackedRegs<MODE>& r, const DqIter& i
         return;
     }
     const size_t row_bytes = T::kNibbles ? (size_t)a.N / 2 : (size_t)a.N;
-    if constexpr (MODE == kCtInt4F16) {
-        if (it.kt * kBK >= a.K) {  // an offset stage: the thread's eight rows are four each of two scale groups
-            const int n_g = a.K >> 7, g0 = (it.kt * kBK - a.K + d.k0) / kOffsetSlots;
-            r.e[0] = (uint32_t)((((size_t)it.g * n_g + g0) * a.N + it.n0) >> 3) + d.chunk;
-            r.e[1] = 1u + (uint32_t)min(max(n_g - g0, 0), 2);
-            return;
-        }
-        r.e[1] = 0u;
-    }
     if constexpr (MODE == B200MOE_CT_INT4 || MODE == kCtInt4F16) {
         uint32_t v[8];
 #pragma unroll
@@ -675,29 +664,24 @@ __device__ __forceinline__ void convert_block_int4(const PackedRegs<B200MOE_CT_I
 }
 
 // ---- int4 in one pass --------------------------------------------------------------------------------------
-// (w + o) * s has up to 16 significant bits, so one bf16 tile cannot hold it; w * s has at most 11, which f16 does, and f16
+// For calls without offsets.  w * s has at most 11 significant bits, which one f16 tile holds where bf16 takes a pair of tiles, and f16
 // times f16 runs at the rate of bf16.  So x is written as f16 first (gm_int4_prepare_x_kernel: each row times the power of two that puts
-// its largest element into [2^14, 2^15)), the weights enter as w * s * 2^6, exact for scales of 2^-23 up to 2^7, and
-// what the offsets add, the sum over the scale groups of (o * s) * (sum of the group's x), is a matrix product as well: K / 128
-// groups are further k rows of the same accumulation, in bf16, four slots a group, (hi, lo, hi, lo) of o * s * 2^6, whose 16
-// bits they hold, against (hi, hi, mid, mid) of the fp32 sum, 17 bits of it.  The epilogue multiplies by the row's power
-// of two.  Against the hi + lo pair of tiles: half the MMAs plus 1 / 32, 13 instead of 34 instructions per eight codes.
+// its largest element into [2^14, 2^15)) and the weights enter as w * s * 2^6, exact for scales of 2^-23 up to 2^7; the epilogue
+// multiplies by the row's power of two.  Against the hi + lo pair of tiles: half the MMAs, 13 instead of 34 instructions per eight codes.
+// Every product is exact and the accumulator takes half as many, so the fp32 sums are the closer ones (16 experts of 40 rows, 7168 x 2048,
+// error against 64 bits: 0.7e-5 .. 0.8e-5, the pair of tiles 1.3e-5 .. 1.6e-5).
+// With an offset (w + o) * s has up to 16 bits, which f16 does not hold, and w * s and o * s as separate products cancel where the offset does
+// what a zero point is for: sums of both signs, each many times the result, in an accumulator that drops what lies 24 bits
+// below it (codes with zero points, positive x: 1.0e-4 .. 3.2e-4 against 1.1e-5; codes 5 .. 7 under offsets about -6, positive x: 1.4e-2
+// against 1.5e-5).  Such calls take the pair.
 // Rows of x that f16 cannot hold (an element more than about 2^-32 below the row's largest, infinities, NaN) and tiles with a scale
-// or offset out of range are done again by the two-pass kernel: the epilogue lists such tiles.  Where more than
+// out of range are done again by the two-pass kernel: the epilogue lists such tiles.  Where more than
 // one row in kInt4BadRows is of that kind, the two-pass kernel does all tiles and this one none.
-// Stages that the offsets add to a tile.
-static int offset_stages(int64_t K) { return (int)((K / 128 * kOffsetSlots + kBK - 1) / kBK); }
-// 16-bit elements of a prepared row.
-static int64_t int4_pitch(int64_t K, bool offsets) { return K + (offsets ? (int64_t)offset_stages(K) * kBK : 0); }
 
-// Whether f16 holds w * s * 2^6 for every code (two bf16 scales a word), and the hi / lo pair of o * s * 2^6 is in bf16's range.
+// Whether f16 holds w * s * 2^6 for every code (two bf16 scales a word).
 __device__ __forceinline__ bool int4_scale_fits(uint32_t w) {
     const uint32_t a = w & 0x7FFFu, b = (w >> 16) & 0x7FFFu;  // 0x3400: 2^-23, 0x4300: 2^7
     return (a == 0u || a - 0x3400u < 0x0F00u) && (b == 0u || b - 0x3400u < 0x0F00u);
-}
-__device__ __forceinline__ bool int4_offset_fits(uint32_t w) {
-    const uint32_t a = w & 0x7FFFu, b = (w >> 16) & 0x7FFFu;  // 0x1780: 2^-80, 0x5D80: 2^60
-    return (a == 0u || a - 0x1780u < 0x4600u) && (b == 0u || b - 0x1780u < 0x4600u);
 }
 
 // Eight rows of eight columns, in the column order of the fp4 modes; `sa` as in convert_stage_fp4_ascend.
@@ -731,35 +715,6 @@ __device__ __forceinline__ void convert_int4_f16(const PackedRegs<kCtInt4F16>& r
     }
 }
 
-// The thread's eight rows of an offset stage: two scale groups, four slots each.
-__device__ __forceinline__ void convert_int4_offsets(const GemmArgs& a, uint32_t unit, int groups, uint32_t sa) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        uint32_t hi[4] = {0u, 0u, 0u, 0u}, lo[4] = {0u, 0u, 0u, 0u};
-        if (i < groups) {
-            const uint4 s = __ldg(static_cast<const uint4*>(a.scale) + unit + (size_t)i * (a.N >> 3));
-            const uint4 o = __ldg(reinterpret_cast<const uint4*>(a.offset) + unit + (size_t)i * (a.N >> 3));
-            const uint4 sp = pair_scales(s), op = pair_scales(o);
-            const uint32_t sw[4] = {sp.x, sp.y, sp.z, sp.w}, ow[4] = {op.x, op.y, op.z, op.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const f32x2 up = mul_f32x2(pack_u32x2(sw[c] << 16, sw[c] & 0xFFFF0000u), pack_f32x2(1 << kInt4ScaleShift, 1 << kInt4ScaleShift));
-                const f32x2 v = mul_f32x2(pack_u32x2(ow[c] << 16, ow[c] & 0xFFFF0000u), up);
-                hi[c] = pack_bf16x2(f32x2_lo(v), f32x2_hi(v));
-                const f32x2 rest = sub_f32x2(v, pack_u32x2(hi[c] << 16, hi[c] & 0xFFFF0000u));
-                lo[c] = pack_bf16x2(f32x2_lo(rest), f32x2_hi(rest));
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kOffsetSlots; ++k) {
-            const int j = i * kOffsetSlots + k;
-            const uint32_t at = (sa ^ (uint32_t)(j << 4)) + (uint32_t)(j * 128);
-            if (k & 1) sts128(at, lo[0], lo[1], lo[2], lo[3]);
-            else sts128(at, hi[0], hi[1], hi[2], hi[3]);
-        }
-    }
-}
-
 // Position of the x producer's L2 prefetch in the (tile, k-stage) sequence of its CTA.
 struct StageIter {
     int kt;
@@ -780,8 +735,7 @@ __device__ __forceinline__ constexpr int acc_pos(int i) {
 __device__ __forceinline__ float int4_row_unit(int e) {
     return e == kRowNotF16 ? 0.f : __uint_as_float((uint32_t)(e - kInt4ScaleShift + 127) << 23);
 }
-__device__ __noinline__ void int4_check_tile(const int* __restrict__ row_exp, const uint4* __restrict__ scale, const uint4* __restrict__ offset,
-                                             int n_g, int stride, int g, int row0, int rows, int n0, int4* redo, int* redo_count) {
+__device__ __noinline__ void int4_check_tile(const int* __restrict__ row_exp, const uint4* __restrict__ scale, int n_g, int stride, int g, int row0, int rows, int n0, int4* redo, int* redo_count) {
     const int lane = threadIdx.x & 31;
     bool ok = true;
     for (int i = lane; i < rows; i += 32) ok = ok && __ldca(row_exp + row0 + i) != kRowNotF16;
@@ -790,10 +744,6 @@ __device__ __noinline__ void int4_check_tile(const int* __restrict__ row_exp, co
     for (int i = 0; i < n_g; ++i) {
         const uint4 s = __ldg(scale + first + (size_t)i * stride);
         ok = ok && int4_scale_fits(s.x) && int4_scale_fits(s.y) && int4_scale_fits(s.z) && int4_scale_fits(s.w);
-        if (offset != nullptr) {
-            const uint4 o = __ldg(offset + first + (size_t)i * stride);
-            ok = ok && int4_offset_fits(o.x) && int4_offset_fits(o.y) && int4_offset_fits(o.z) && int4_offset_fits(o.w);
-        }
     }
     if (!__all_sync(0xffffffffu, ok) && lane == 0) redo[atomicAdd(redo_count, 1)] = make_int4(g, row0, rows, n0);
 }
@@ -820,9 +770,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_nt = (a.N + kBN - 1) / kBN;  // (fp8 only: the last tile may hold 128 columns)
-    // stages per tile: the weights' and, in one-pass int4, the offsets'
-    const int n_wkt = a.K / kBK;
-    const int n_kt = n_wkt + (MODE == kCtInt4F16 && a.offset != nullptr ? (n_wkt / 2 * kOffsetSlots + kBK - 1) / kBK : 0);
+    const int n_kt = a.K / kBK;  // stages per tile
 
     if constexpr (MODE == B200MOE_CT_INT4) {
         if (a.redo_ctl != nullptr) {
@@ -913,7 +861,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if constexpr (SPLIT) {
                     ptx::tma_prefetch_l2_2d(&tmap_w, far.ti.n0 / 4, far.ti.g * a.K + far.kt * kBK);
                     ptx::tma_prefetch_l2_2d(&tmap_w, (a.N + far.ti.n0) / 4, far.ti.g * a.K + far.kt * kBK);
-                } else if (!T::kDirect && (MODE != kCtInt4F16 || far.kt < n_wkt))
+                } else if constexpr (!T::kDirect)
                     ptx::tma_prefetch_l2_2d(&tmap_w, T::kNibbles ? far.ti.n0 / 2 : far.ti.n0, far.ti.g * a.K + far.kt * kBK);
                 if (++far.kt < n_kt) return;
                 far.kt = 0;
@@ -969,7 +917,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         // small stage / k offset.  The next stage's barrier is polled (non-blocking) right after a stage's MMAs are
         // issued, so that the poll's latency runs beside the commit's.
         const bool leader = ptx::elect_one();
-        const uint32_t idesc_bf16 = ptx::umma_idesc_bf16(kBM, kBN, true), idesc_f16 = ptx::umma_idesc_f16(kBM, kBN, true);
+        const uint32_t idesc = MODE == kCtInt4F16 ? ptx::umma_idesc_f16(kBM, kBN, true) : ptx::umma_idesc_bf16(kBM, kBN, true);
         // A: K-major, 8-row groups 1024 B apart, 32 B per 16 k inside the swizzle atom
         const uint64_t da0 = ptx::umma_desc_sw128(ptx::smem_u32(a_ring), 0, 1024);
         // B: MN-major, 64-column blocks kBK*128 B apart (LBO), 8-k groups 1024 B apart (SBO)
@@ -998,7 +946,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 if (!ok) break;
                 ptx::tc_fence_after();
                 const uint32_t sn = sa + 1 == NS ? 0u : sa + 1, phn = sa + 1 == NS ? pha ^ 1u : pha;
-                const uint32_t idesc = MODE == kCtInt4F16 && kt < n_wkt ? idesc_f16 : idesc_bf16;
                 if (leader) {
                     const uint64_t da = da0 + (uint64_t)(sa * (kATileBytes >> 4));
 #pragma unroll
@@ -1072,8 +1019,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             }
             if constexpr (MODE == kCtInt4F16) {
                 if (quarter == 0 && half == 0)  // one warp a tile, while it is being accumulated
-                    int4_check_tile(a.row_exp, static_cast<const uint4*>(a.scale), reinterpret_cast<const uint4*>(a.offset), a.K >> 7,
-                                    a.N >> 3, ti.g, ti.row0, ti.rows, ti.n0, a.redo, a.redo_ctl);
+                    int4_check_tile(a.row_exp, static_cast<const uint4*>(a.scale), a.K >> 7, a.N >> 3, ti.g, ti.row0, ti.rows, ti.n0, a.redo, a.redo_ctl);
             }
             if (!__all_sync(0xffffffffu, gm_wait(&sb->t_full[grp], use & 1, sb, a.status, 60 + grp))) break;
             ++use;
@@ -1218,18 +1164,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 Int4Scales sc4;
                 if constexpr (MODE == B200MOE_CT_INT4) sc4 = load_int4_scales(a, regs[u].e[0]);  // (late: registers)
                 uint4 s8;
-                if constexpr (MODE == kCtInt4F16)
-                    if (regs[u].e[1] == 0u) s8 = __ldg(static_cast<const uint4*>(a.scale) + regs[u].e[0]);
+                if constexpr (MODE == kCtInt4F16) s8 = __ldg(static_cast<const uint4*>(a.scale) + regs[u].e[0]);
                 bool got = true;
                 if (ib >= NS) got = gm_wait(&sb->empty[slot], ((ib / NS) & 1) ^ 1, sb, a.status, 80 + (int)slot);
                 if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 const uint32_t sa = sa0 + slot * (uint32_t)(P * kBTileBytes);
                 if constexpr (MODE == B200MOE_CT_INT4)
                     convert_block_int4(regs[u], sc4, sa, sa + kBTileBytes);
-                else if constexpr (MODE == kCtInt4F16) {
-                    if (regs[u].e[1] == 0u) convert_int4_f16(regs[u], s8, sa);
-                    else convert_int4_offsets(a, regs[u].e[0], (int)regs[u].e[1] - 1, sa);
-                } else if constexpr (MODE == kCtFp4Ascend)
+                else if constexpr (MODE == kCtInt4F16)
+                    convert_int4_f16(regs[u], s8, sa);
+                else if constexpr (MODE == kCtFp4Ascend)
                     convert_stage_fp4_ascend(regs[u], sa);
                 else
                     convert_stage<MODE>(regs[u], sa);
@@ -1317,20 +1261,19 @@ void launch_rowsum(const void* x, float* out, int64_t M, int64_t K, const int64_
                                                         reinterpret_cast<const long long*>(group_list), (int)G, gl_type, status);
 }
 
-// One-pass int4: a row of x as f16 times 2^-e, e into row_exp (kRowNotF16: not exact), behind it the offset stages' A operand.
+// One-pass int4: a row of x as f16 times 2^-e, e into row_exp (kRowNotF16: not exact).
 // One warp a row; the row's second reading comes from L1 or L2, so the bound is its bytes in and out.
 __global__ void __launch_bounds__(256)
 gm_int4_prepare_x_kernel(const __nv_bfloat16* __restrict__ x, uint16_t* __restrict__ x16, int* __restrict__ row_exp, int M, int K,
-                         int pitch, const long long* __restrict__ group_list, int G, int gl_type, int* __restrict__ status,
+                         const long long* __restrict__ group_list, int G, int gl_type, int* __restrict__ status,
                          int* __restrict__ ctl) {
     grid_dep_launch();
     if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
     const int used = used_rows(group_list, G, gl_type, M);
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, n_vec = K / 8, n_rest = (pitch - K) / 4;  // 8-byte pieces
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, n_vec = K / 8;
     for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < used; row += gridDim.x * wpb) {
         const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * K);
-        uint4* dst = reinterpret_cast<uint4*>(x16 + (size_t)row * pitch);
-        uint2* rest = reinterpret_cast<uint2*>(x16 + (size_t)row * pitch + K);
+        uint4* dst = reinterpret_cast<uint4*>(x16 + (size_t)row * K);
         uint32_t mx = 0u;  // bf16 magnitudes order like integers
 #pragma unroll 8
         for (int i = lane; i < n_vec; i += 32) {
@@ -1343,39 +1286,23 @@ gm_int4_prepare_x_kernel(const __nv_bfloat16* __restrict__ x, uint16_t* __restri
         // (2^-e and the epilogue's 2^(e - 6) are normal numbers)
         bool ok = mx == 0u || (e_max >= 32 && e_max < 255);
         const float down = ok ? __uint_as_float((uint32_t)(127 - e) << 23) : 0.f;
-        // (every lane runs all iterations: the sums' shuffles)
 #pragma unroll 4
-        for (int i0 = 0; i0 < n_vec; i0 += 32) {
-            const int i = i0 + lane;
-            float sum = 0.f;
-            if (i < n_vec) {
-                const uint4 q = __ldg(src + i);
-                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-                uint32_t h[4];
+        for (int i = lane; i < n_vec; i += 32) {
+            const uint4 q = __ldg(src + i);
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+            uint32_t h[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float f0 = __uint_as_float(w[j] << 16) * down, f1 = __uint_as_float(w[j] & 0xFFFF0000u) * down;
-                    const __half2 hh = __floats2half2_rn(f0, f1);
-                    h[j] = *reinterpret_cast<const uint32_t*>(&hh);
-                    // exact: the same value back, and no zero that was none (f0, f1 themselves may underflow)
-                    const float2 back = __half22float2(hh);
-                    ok = ok && back.x == f0 && back.y == f1 && ((h[j] & 0x7FFFu) != 0u) == ((w[j] & 0x7FFFu) != 0u) &&
-                         ((h[j] & 0x7FFF0000u) != 0u) == ((w[j] & 0x7FFF0000u) != 0u);
-                    sum += f0 + f1;
-                }
-                dst[i] = make_uint4(h[0], h[1], h[2], h[3]);
+            for (int j = 0; j < 4; ++j) {
+                const float f0 = __uint_as_float(w[j] << 16) * down, f1 = __uint_as_float(w[j] & 0xFFFF0000u) * down;
+                const __half2 hh = __floats2half2_rn(f0, f1);
+                h[j] = *reinterpret_cast<const uint32_t*>(&hh);
+                // exact: the same value back, and no zero that was none (f0, f1 themselves may underflow)
+                const float2 back = __half22float2(hh);
+                ok = ok && back.x == f0 && back.y == f1 && ((h[j] & 0x7FFFu) != 0u) == ((w[j] & 0x7FFFu) != 0u) &&
+                     ((h[j] & 0x7FFF0000u) != 0u) == ((w[j] & 0x7FFF0000u) != 0u);
             }
-            if (n_rest > 0) {  // a scale group is 16 lanes
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if ((lane & 15) == 0 && i < n_vec) {
-                    const uint32_t hi = pack_bf16x2(sum, sum);
-                    const float r = sum - __uint_as_float(hi << 16);
-                    rest[i >> 4] = make_uint2(hi, pack_bf16x2(r, r));
-                }
-            }
+            dst[i] = make_uint4(h[0], h[1], h[2], h[3]);
         }
-        for (int i = n_vec / 16 + lane; i < n_rest; i += 32) rest[i] = make_uint2(0u, 0u);
         ok = __all_sync(0xffffffffu, ok);
         if (lane == 0) {
             row_exp[row] = ok ? e : kRowNotF16;
@@ -1390,7 +1317,7 @@ gm_int4_prepare_x_kernel(const __nv_bfloat16* __restrict__ x, uint16_t* __restri
 // 378, SiLU 376 | 398.
 constexpr int kInt8RolesK = 2048;
 
-// Whether a call of int4 goes through f16 in one pass: where the tiles of a multiprocessor come to at least 48 stages of 64 k, the
+// Whether a call of int4 without offsets goes through f16 in one pass: where the tiles of a multiprocessor come to at least 48 stages of 64 k, the
 // preparation of x and the two launches more (6 .. 10 us, and the bytes of x twice) are won back; where whole experts are long and N is a
 // single column tile, they are not.  us, hi and lo | one pass, back to back, experts : rows : K x N (even lists unless said): 8 : 1024 : 2048 x 2048
 // (32 stages) 49.5 | 59.7; 32 : 1024 : 2048 x 1024 (32) 47.5 | 56.5; 16 : 4096 : 256 x 4096 (16) 45.4 | 44.4; 16 : 1024 : 256 x 1024 (4) 16.6 | 23.1;
@@ -1411,11 +1338,9 @@ static int gm_launch(const void* x, const void* w, const GemmArgs& a, cudaStream
     using T = GmTraits<MODE>;
     if (MODE == B200MOE_CT_INT8 && !RESOLVED && a.K < kInt8RolesK) return gm_launch<MODE, SILU, true>(x, w, a, stream);
     CUtensorMap tx, txs, tw;
-    // (one-pass int4: x is the prepared one)
-    const uint64_t x_cols = MODE == kCtInt4F16 ? (uint64_t)int4_pitch(a.K, a.offset != nullptr) : (uint64_t)a.K;
-    int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)a.M, x_cols, kBM, kBK, true);
+    int rc = make_tensor_map_2d(&tx, x, 2, (uint64_t)a.M, a.K, kBM, kBK, true);
     if (rc != B200MOE_OK) return rc;
-    rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)a.M, x_cols, kSmallRows, kBK, true);
+    rc = make_tensor_map_2d(&txs, x, 2, (uint64_t)a.M, a.K, kSmallRows, kBK, true);
     if (rc != B200MOE_OK) return rc;
     if (T::kDirect)
         rc = make_tensor_map_2d(&tw, w, 2, (uint64_t)a.G * a.K, a.N, kBK, 64, true);
@@ -1443,13 +1368,13 @@ static size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 struct Int4Scratch {
     size_t exp, redo, x16, bytes;
 };
-static Int4Scratch int4_scratch(int64_t M, int64_t K, int64_t N, int64_t G, bool offsets) {
+static Int4Scratch int4_scratch(int64_t M, int64_t K, int64_t N, int64_t G) {
     const size_t tiles = (size_t)(N / kBN) * (size_t)(M / kTileM + (M < G ? M : G));  // at most
     Int4Scratch s;
     s.exp = 256;
     s.redo = s.exp + align256((size_t)M * sizeof(int));
     s.x16 = s.redo + align256(tiles * sizeof(int4));
-    s.bytes = s.x16 + (size_t)M * (size_t)int4_pitch(K, offsets) * 2;
+    s.bytes = s.x16 + (size_t)M * (size_t)K * 2;
     return s;
 }
 
@@ -1467,8 +1392,8 @@ extern "C" size_t b200moe_grouped_gemm_workspace_bytes(int64_t M, int64_t K, int
 
 extern "C" size_t b200moe_grouped_gemm_scratch_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type, int has_offset) {
     if (compute_type != B200MOE_CT_INT4 || M <= 0 || K <= 0 || N <= 0 || G <= 0 || (K % 128) != 0 || (N % kBN) != 0) return 0;
-    if (!int4_one_pass(M, K, N, G)) return 0;
-    return int4_scratch(M, K, N, G, has_offset != 0).bytes;
+    if (has_offset != 0 || !int4_one_pass(M, K, N, G)) return 0;
+    return int4_scratch(M, K, N, G).bytes;
 }
 
 extern "C" int b200moe_grouped_gemm(const void* x, const void* weight, const void* scale, const void* offset,
@@ -1535,7 +1460,7 @@ extern "C" int b200moe_grouped_gemm_scratch(const void* x, const void* weight, c
     if (compute_type == B200MOE_CT_INT4) {
         a.offset = static_cast<const __nv_bfloat16*>(offset);  // folded into the weights by the dequant warps
         if (!one_pass) return gm_launch<B200MOE_CT_INT4>(x, weight, a, s);
-        const Int4Scratch at = int4_scratch(M, K, N, G, offset != nullptr);
+        const Int4Scratch at = int4_scratch(M, K, N, G);
         uint8_t* sc = static_cast<uint8_t*>(scratch);
         int* exps = reinterpret_cast<int*>(sc + at.exp);
         void* x16 = sc + at.x16;
@@ -1543,7 +1468,7 @@ extern "C" int b200moe_grouped_gemm_scratch(const void* x, const void* weight, c
         a.redo = reinterpret_cast<int4*>(sc + at.redo);
         a.redo_ctl = reinterpret_cast<int*>(sc);
         gm_int4_prepare_x_kernel<<<rowsum_blocks(M), 256, 0, s>>>(
-            static_cast<const __nv_bfloat16*>(x), static_cast<uint16_t*>(x16), exps, (int)M, (int)K, (int)int4_pitch(K, offset != nullptr),
+            static_cast<const __nv_bfloat16*>(x), static_cast<uint16_t*>(x16), exps, (int)M, (int)K,
             reinterpret_cast<const long long*>(group_list), (int)G, group_list_type, a.status, a.redo_ctl);
         B200MOE_CUDA_TRY(cudaGetLastError());
         const int rc = gm_launch<kCtInt4F16>(x16, weight, a, s);

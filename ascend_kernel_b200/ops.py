@@ -164,7 +164,7 @@ def grouped_gemm(x, weight, antiquantScaleOptional, antiquantOffsetOptional, gro
     offset = antiquantOffsetOptional if ct in (CT["int8"], CT["int4"]) else None  # ignored for fp8/fp4
     if offset is not None:
         _check_scale(offset, ct, G, K, N, "antiquantOffsetOptional")
-    # int4: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
+    # int4 without offsets: scratch for the one-pass kernel, from the caching allocator and back to it; without it the two-pass kernel runs
     scratch, scratch_bytes = None, _lib.b200moe_grouped_gemm_scratch_bytes(M, K, N, G, ct, int(offset is not None))
     if scratch_bytes > 0:
         try:

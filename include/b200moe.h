@@ -95,11 +95,11 @@ int b200moe_grouped_gemm(const void* x, const void* weight, const void* scale, c
 size_t b200moe_grouped_gemm_workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type,
                                             int weight_layout);
 
-/* The same with scratch memory for the call: int4 calls of many rows then keep x as scaled f16 there and multiply every
- * weight once instead of as a pair of bf16 numbers.  scratch_bytes says how much
+/* The same with scratch memory for the call: int4 calls of many rows and without offsets then keep x as scaled f16 there and multiply
+ * every weight once instead of as a pair of bf16 numbers.  scratch_bytes says how much
  * that takes (about 2 * M * K bytes); 0: the call has no use for any.  Without it, or with less, the call runs as
  * b200moe_grouped_gemm does.  The scratch belongs to the call until it has completed on the stream; its contents mean nothing after that.
- * has_offset: whether the call will pass an offset. */
+ * has_offset: whether the call will pass an offset (no use for scratch then). */
 size_t b200moe_grouped_gemm_scratch_bytes(int64_t M, int64_t K, int64_t N, int64_t G, int compute_type, int has_offset);
 int b200moe_grouped_gemm_scratch(const void* x, const void* weight, const void* scale, const void* offset,
                                  const int64_t* group_list, void* y, int64_t M, int64_t K, int64_t N, int64_t G,

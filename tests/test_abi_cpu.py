@@ -133,11 +133,12 @@ def test_gemv_split_workspace_comes_on_top_of_the_plain_one():
 
 
 def test_one_pass_int4_scratch_where_the_rule_says():
-    """Scratch of the int4 GEMM: none for other formats, for few stages a multiprocessor, for one column tile under long experts."""
+    """Scratch of the int4 GEMM: none for other formats, with offsets, for few stages a multiprocessor, for one column tile under long
+    experts."""
     f = _lib().lib.b200moe_grouped_gemm_scratch_bytes
     big = (65536, 7168, 4096, 256)
-    assert f(*big, 3, 1) > 2 * 65536 * 7168 and f(*big, 3, 1) - f(*big, 3, 0) == 65536 * 256 * 2  # 56 groups x 4: four stages of 64
-    assert all(f(*big, ct, 1) == 0 for ct in (0, 1, 2, 4))
-    assert f(1024, 2048, 2048, 8, 3, 1) == 0 and f(4096, 1024, 1024, 64, 3, 1) > 0
-    assert f(65536, 7168, 256, 256, 3, 1) == 0 and f(4096, 7168, 256, 256, 3, 1) > 0
-    assert f(0, 7168, 4096, 256, 3, 1) == 0 and f(64, 7104, 4096, 256, 3, 1) == 0 and f(64, 7168, 4000, 256, 3, 1) == 0
+    assert f(*big, 3, 0) > 2 * 65536 * 7168 and f(*big, 3, 1) == 0
+    assert all(f(*big, ct, 0) == 0 for ct in (0, 1, 2, 4))
+    assert f(1024, 2048, 2048, 8, 3, 0) == 0 and f(4096, 1024, 1024, 64, 3, 0) > 0
+    assert f(65536, 7168, 256, 256, 3, 0) == 0 and f(4096, 7168, 256, 256, 3, 0) > 0
+    assert f(0, 7168, 4096, 256, 3, 0) == 0 and f(64, 7104, 4096, 256, 3, 0) == 0 and f(64, 7168, 4000, 256, 3, 0) == 0

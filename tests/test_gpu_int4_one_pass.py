@@ -1,5 +1,5 @@
-"""int4 GEMM in one pass (x and the weights as scaled f16) against the oracle and the two-pass kernel: ragged row counts, offsets,
-rows and scales that f16 does not hold."""
+"""int4 GEMM in one pass (calls without offsets: x and the weights as scaled f16) against the oracle and the two-pass kernel: ragged
+row counts, rows and scales that f16 does not hold; and calls with offsets, which take the two-pass kernel."""
 import pytest
 import torch
 
@@ -27,14 +27,16 @@ def _one_pass(x, K, N, G, offsets):
 
 
 @pytest.mark.parametrize("counts,K,N,offsets", [
-    ([1, 0, 127, 128, 129, 300, 1200], 2176, 4096, True),   # 17 scale groups: a second offset stage, nearly empty
-    ([700, 1, 33, 1000], 2048, 4096, False),                # no offset stages
-    ([1] * 596 + [300, 129, 256, 64], 128, 1536, True),     # one scale group: two weight stages and one of offsets
+    ([1, 0, 127, 128, 129, 300, 1200], 2176, 4096, False),
+    ([1, 0, 127, 128, 129, 300, 1200], 2176, 4096, True),
+    ([700, 1, 33, 1000], 2048, 4096, False),
+    ([1] * 950 + [300, 129, 256, 64], 128, 1536, False),    # one scale group: two stages a tile
+    ([2] * 200 + [900], 896, 1024, False),
     ([2] * 200 + [900], 896, 1024, True),
 ])
 def test_matches_oracle(counts, K, N, offsets):
     x, w, s, o, cnt = _case(counts, K, N, offsets, 5)
-    assert _one_pass(x, K, N, len(counts), offsets)
+    assert _one_pass(x, K, N, len(counts), offsets) == (not offsets)
     x[3] *= 2.0 ** 60      # rows of any magnitude keep their accuracy
     x[5] *= 2.0 ** -70
     x[7] = 0
@@ -54,31 +56,30 @@ def test_what_f16_does_not_hold_goes_through_the_two_pass_kernel(kind):
     from ascend_kernel_b200 import _abi
 
     K, N, counts = 2048, 4096, [1300, 0, 257, 1100]
-    x, w, s, o, cnt = _case(counts, K, N, True, 6)
-    assert _one_pass(x, K, N, len(counts), True)
+    x, w, s, o, cnt = _case(counts, K, N, False, 6)
+    assert _one_pass(x, K, N, len(counts), False)
     redone = torch.zeros(x.shape[0], N, dtype=torch.bool)
     if kind == "few_rows":
         x[300, 5] = 2.0 ** -60           # rows 256 .. 511 of expert 0
         x[1299] = 0
         x[1299, 1:3] = torch.tensor([2.0 ** -50, 1.0])
         w[0, 2] = 0                      # with the weights of the large element zero
-        o[0, 0] = 0
         redone[256:512] = redone[1280:1300] = True
     elif kind == "most_rows":
         x[::2, 7] = 2.0 ** -80
         redone[:sum(counts)] = True
     else:
         s[2, 3, 300] = 2.0 ** -30        # expert 2, columns 256 .. 511
-        o[3, 1, 0] = 2.0 ** 70           # expert 3, columns 0 .. 255
+        s[3, 1, 0] = 2.0 ** 10           # expert 3, columns 0 .. 255
         redone[1300:1557, 256:512] = redone[1557:2657, 0:256] = True
     gold = O.golden_f32(x, w, s, o, cnt, "int4", O.GROUP_LIST_COUNTS)
     out, st = run_gemm(x, w, s, o, cnt, "int4", gl_type=1)
     assert st == (0, 0)
-    d = [t.cuda() for t in (x, w, s, o, cnt)]
+    d = [t.cuda() for t in (x, w, s, cnt)]
     two = torch.full((x.shape[0], N), SENTINEL, dtype=torch.bfloat16, device="cuda")
     need = _abi.lib.b200moe_grouped_gemm_workspace_bytes(x.shape[0], K, N, 4, _abi.CT["int4"], 0)
     ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
-    rc = _abi.lib.b200moe_grouped_gemm(*[t.data_ptr() for t in d], two.data_ptr(), x.shape[0], K, N, 4, _abi.CT["int4"], 1, 0,
+    rc = _abi.lib.b200moe_grouped_gemm(*[t.data_ptr() for t in d[:3]], None, d[3].data_ptr(), two.data_ptr(), x.shape[0], K, N, 4, _abi.CT["int4"], 1, 0,
                                        ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert rc == 0 and ak.read_status(ws) == (0, 0)
@@ -97,16 +98,16 @@ def test_captured_graph_replays_on_new_inputs():
     import ascend_kernel_b200 as ak
 
     K, N, counts = 2048, 2048, [1500, 0, 3100, 400]
-    x, w, s, o, cnt = (t.cuda() for t in _case(counts, K, N, True, 8))
-    assert _one_pass(x, K, N, 4, True)
+    x, w, s, cnt = (t.cuda() for t in _case(counts, K, N, False, 8) if t is not None)
+    assert _one_pass(x, K, N, 4, False)
     out = torch.zeros(x.shape[0], N, dtype=torch.bfloat16, device="cuda")
     side = torch.cuda.Stream()
     with torch.cuda.stream(side):
-        ak.grouped_gemm(x, w, s, o, cnt, "int4", out, group_list_type=1)
+        ak.grouped_gemm(x, w, s, None, cnt, "int4", out, group_list_type=1)
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=side):
-        ak.grouped_gemm(x, w, s, o, cnt, "int4", out, group_list_type=1)
+        ak.grouped_gemm(x, w, s, None, cnt, "int4", out, group_list_type=1)
     for step in range(3):
         x.copy_(x.flip(0))
         if step == 1:
@@ -114,7 +115,33 @@ def test_captured_graph_replays_on_new_inputs():
         graph.replay()
         torch.cuda.synchronize()
         want = torch.zeros_like(out)
-        ak.grouped_gemm(x, w, s, o, cnt, "int4", want, group_list_type=1)
+        ak.grouped_gemm(x, w, s, None, cnt, "int4", want, group_list_type=1)
         torch.cuda.synchronize()
         assert torch.equal(out[:5000].view(torch.int16), want[:5000].view(torch.int16))
     assert ak.last_status() == (0, 0)
+
+
+@pytest.mark.parametrize("positive", [False, True])
+def test_offsets_that_cancel_the_codes(positive):
+    """Codes 5 .. 7 under offsets about -6: the result is a small part of the codes' and of the offsets' own sums, so it holds only
+    where (w + o) * s is formed before the sum.  Rounding to bf16 leaves 2^-9 of each value at most, the fp32 sum about 1e-4 of it."""
+    import ascend_kernel_b200 as ak
+
+    gen = torch.Generator().manual_seed(9)
+    G, rows, K, N = 16, 40, 7168, 2048
+    x = torch.randn(G * rows, K, generator=gen)
+    x = (x.abs() if positive else x).to(torch.bfloat16).cuda()
+    w = torch.randint(5, 8, (G, K, N), generator=gen, dtype=torch.int8).cuda()
+    s = (torch.rand(G, K // 128, N, generator=gen) * 0.045 + 0.005).to(torch.bfloat16).cuda()
+    o = (torch.rand(G, K // 128, N, generator=gen) * 0.2 - 6.1).to(torch.bfloat16).cuda()
+    packed = (w[:, :, 0::2] | (w[:, :, 1::2] << 4)).contiguous()
+    counts = torch.full((G,), rows, dtype=torch.int64, device="cuda")
+    y = torch.empty(G * rows, N, dtype=torch.bfloat16, device="cuda")
+    ak.grouped_gemm(x, packed, s, o, counts, "int4", y, group_list_type=1)
+    err = ref = 0.0
+    for g in range(G):
+        v = (w[g].double() + o[g].double().repeat_interleave(128, 0)) * s[g].double().repeat_interleave(128, 0)
+        want = x[g * rows:(g + 1) * rows].double() @ v
+        err += float((y[g * rows:(g + 1) * rows].double() - want).square().sum())
+        ref += float(want.square().sum())
+    assert (err / ref) ** 0.5 < 2.0 ** -9 + 1e-4
