@@ -19,7 +19,7 @@ SCRIPTS = [
 ]
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference checkout not present")
+@pytest.mark.skipif(not all(os.path.isfile(os.path.join(REF, s)) for s in SCRIPTS), reason="reference checkout not present")
 @pytest.mark.parametrize("script", SCRIPTS)
 def test_reference_script_passes_against_oracle(script):
     r = subprocess.run([sys.executable, os.path.join(HERE, "ref_shim_runner.py"), os.path.join(REF, script)],
