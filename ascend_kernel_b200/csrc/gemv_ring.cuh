@@ -5,11 +5,12 @@
 // packed weights, of the group scales (fp4) and of the unit's x rows.  It runs ahead of the consumers by the ring, over the
 // end of a unit, so the next unit's first weights arrive while the sums of this one are being put together; with loads
 // into registers a unit started cold: ticket, look-up, staging of x, first loads, each waited for in turn.
-// Every consumer warp takes 16 k rows x 128 columns of each stage: eight mma.sync m16n8k16 with the weights as the 16 x 16
+// Every consumer warp takes 16 k rows x 128 columns of each stage, or 32 x 64: eight mma.sync m16n8k16 with the weights as the 16 x 16
 // operand and up to eight x rows as the other (a legacy instruction on purpose: the tile is 16 x 8 and HBM is the bound).
 // us, register kernel | one CTA of 16 consumer warps and stages of 128 k | this, called in turn with the register kernel: int8, 32 tokens x 8
 // over 256 experts, 7168 x 4096: 886 | 830, 875 | 784 (6.1 TB/s); stored fp4, 37 tokens x 8, 2048 x 7168: 427 | 376, 419 | 354 (4.6
-// TB/s); fp8, one token on 8 experts, 7168 x 4096: 70.3 | 74.4, 70.3 | 67.1.  One CTA leaves its multiprocessor without work
+// TB/s); fp8, one token on 8 experts, 7168 x 4096: 70.3 | 74.4, 70.2 | 63.5, 32 tokens x 8: 906 | 890 (5.4 TB/s; 968 with 16 x 128 a
+// warp and the block's scale read in front of each stage).  One CTA leaves its multiprocessor without work
 // while its sums are put together (1200 .. 1700 cycles a unit); what is left at two is issue slots (about 3 per fp8 weight, 2 per fp4
 // and int8 one).
 #pragma once
@@ -19,11 +20,9 @@
 namespace b200moe {
 
 constexpr int kRgK = 64;                          // k rows of a stage
-constexpr int kRgKGroups = kRgK / 16;             // warps along k; two along the columns
-constexpr int kRgWarps = 2 * kRgKGroups;          // consumers
+constexpr int kRgWarps = 8;                       // consumers
 constexpr int kRgThreads = (kRgWarps + 1) * 32;
 constexpr int kRgRows = 8;                        // x rows per unit: the instruction's n
-constexpr int kRgRedRows = 4;                     // rows whose sums are put together at a time
 constexpr int kRgXBytes = kRgRows * kRgK * 2;     // a swizzled box of 8 rows x 64 k
 static_assert(kRgWarps * 32 == kGvSlabN, "one thread a column");
 constexpr int kRgSlotFloats = 2 * kGvSlotFloats;  // (a slot holds eight rows)
@@ -36,6 +35,13 @@ struct RgTraits {
     static constexpr int kSBytes = kFp4 ? kRgK / 16 * kGvSlabN * 2 : 0;
     static constexpr int kStageBytes = kWBytes + kSBytes + kRgXBytes;
     static constexpr int kStages = kFp4 ? 7 : 5;
+    // A warp's share of a stage: 16 k rows (one scale group) x 128 columns of fp4, 32 x 64 of the byte formats: the same
+    // weights a lane, but the fp32 scaling of fp8 comes once for two chained instructions instead of for each, and the sums of two k groups
+    // meet instead of four.
+    static constexpr int kKGroups = kFp4 ? 4 : 2, kKRows = kRgK / kKGroups;  // warps along k, rows of each
+    static constexpr int kCols = kGvSlabN * kKGroups / kRgWarps;             // columns of a warp
+    static constexpr int kAcc = kCols / 16;                                  // 16 x 8 accumulators of a warp
+    static constexpr int kRedRows = 16 / kKGroups;                           // rows whose sums are put together at a time
     static_assert(kWBytes % 1024 == 0 && kSBytes % 1024 == 0 && kRgXBytes % 1024 == 0, "swizzled boxes");
 };
 
@@ -53,7 +59,7 @@ struct RgBarriers {
     RgUnit unit[2];
     int abort, last;
     int per_pass, units, parts, part_rows;
-    float xsum[kRgKGroups][kRgRows];
+    float xsum[4][kRgRows];
 };
 
 __device__ __noinline__ bool rg_wait_slow(uint32_t bar, uint32_t parity, RgBarriers* sb, int* status, int id) {
@@ -102,37 +108,43 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
     return v;
 }
 
-// A warp's 16 k rows x 128 columns of a stage into its sums.  Lane (g, t) = (lane / 4, lane % 4) holds the k rows
-// {2t, 2t + 1, 2t + 8, 2t + 9} (the instruction's own k indices) of 16 columns, and of x row g.
-// `w0`, `w1`: shared addresses of the lane's columns in rows 2t, 2t + 1; c[j]: columns 2j, 2j + 1 of the 16 x two x rows.
+// Lane (g, t) = (lane / 4, lane % 4) holds, of every 16 k rows, {2t, 2t + 1, 2t + 8, 2t + 9} (the instruction's own k indices)
+// of its columns, and of x row g; c[j]: columns 2j, 2j + 1 of the lane's x two x rows.
+// Byte formats: a warp's 32 k rows x 64 columns of a stage; `w0`, `w1`: shared addresses of the lane's eight columns in rows 2t, 2t + 1
+// (rows 8 apart are 1024 bytes apart and share their swizzle), b[h]: x of rows 16h ...  int8 goes on in c, fp8 starts from zero.
 template <int MODE>
-__device__ __forceinline__ void rg_step_bytes(uint32_t w0, uint32_t w1, uint32_t b0, uint32_t b1, float sf, float (&c)[8][4]) {
-    // rows 2t and 2t + 8 are 1024 bytes apart and share their swizzle, and so do 2t + 1 and 2t + 9
-    const uint4 q0 = lds128(w0), q1 = lds128(w1), q2 = lds128(w0 + 1024), q3 = lds128(w1 + 1024);
-    const uint32_t r0w[4] = {q0.x, q0.y, q0.z, q0.w}, r1w[4] = {q1.x, q1.y, q1.z, q1.w};
-    const uint32_t r2w[4] = {q2.x, q2.y, q2.z, q2.w}, r3w[4] = {q3.x, q3.y, q3.z, q3.w};
+__device__ __forceinline__ void rg_step_bytes(uint32_t w0, uint32_t w1, const uint32_t (&b)[2][2], float sf, float (&c)[4][4]) {
+    float d[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int h = 0; h < 2; ++h) {
+        const uint2 q0 = lds64(w0 + h * 2048), q1 = lds64(w1 + h * 2048), q2 = lds64(w0 + h * 2048 + 1024), q3 = lds64(w1 + h * 2048 + 1024);
+        const uint32_t r0w[2] = {q0.x, q0.y}, r1w[2] = {q1.x, q1.y}, r2w[2] = {q2.x, q2.y}, r3w[2] = {q3.x, q3.y};
 #pragma unroll
-        for (int o = 0; o < 2; ++o) {  // byte pairs (0,1) and (2,3) of word i: instruction j = 2i + o
-            uint32_t a0, a1, a2, a3;
-            if constexpr (MODE == B200MOE_CT_INT8) {
-                const uint32_t sel = o == 0 ? 0x5410u : 0x7632u;
-                s8x4_to_bf16_even_odd(prmt(r0w[i], r1w[i], sel), a0, a1);  // rows (2t, 2t+1) at the two columns
-                s8x4_to_bf16_even_odd(prmt(r2w[i], r3w[i], sel), a2, a3);  // rows (2t+8, 2t+9)
-                mma_16816(c[2 * i + o], a0, a1, a2, a3, b0, b1);
-            } else {
-                // byte b of both rows into the high bytes of the two lanes (the low bytes are masked off)
-                const uint32_t s0 = o == 0 ? 0x4000u : 0x6020u, s1 = o == 0 ? 0x5010u : 0x7030u;
-                a0 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s0));
-                a1 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s1));
-                a2 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s0));
-                a3 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s1));
-                // the 128 x 128 block's fp32 scale multiplies the step's sums
-                float d[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_16816(d, a0, a1, a2, a3, b0, b1);
+        for (int i = 0; i < 2; ++i) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) c[2 * i + o][e] = fmaf(sf, d[e], c[2 * i + o][e]);
+            for (int o = 0; o < 2; ++o) {  // byte pairs (0,1) and (2,3) of word i: accumulator j = 2i + o
+                uint32_t a0, a1, a2, a3;
+                if constexpr (MODE == B200MOE_CT_INT8) {
+                    const uint32_t sel = o == 0 ? 0x5410u : 0x7632u;
+                    s8x4_to_bf16_even_odd(prmt(r0w[i], r1w[i], sel), a0, a1);  // rows (2t, 2t+1) at the two columns
+                    s8x4_to_bf16_even_odd(prmt(r2w[i], r3w[i], sel), a2, a3);  // rows (2t+8, 2t+9)
+                    mma_16816(c[2 * i + o], a0, a1, a2, a3, b[h][0], b[h][1]);
+                } else {
+                    // byte b of both rows into the high bytes of the two lanes (the low bytes are masked off)
+                    const uint32_t s0 = o == 0 ? 0x4000u : 0x6020u, s1 = o == 0 ? 0x5010u : 0x7030u;
+                    a0 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s0));
+                    a1 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s1));
+                    a2 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s0));
+                    a3 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s1));
+                    float (&dd)[4] = d[2 * i + o];
+                    if (h == 0) dd[0] = dd[1] = dd[2] = dd[3] = 0.f;
+                    mma_16816(dd, a0, a1, a2, a3, b[h][0], b[h][1]);
+                    // the 128 x 128 block's fp32 scale multiplies the step's sums
+                    if (h == 1) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c[2 * i + o][e] = fmaf(sf, dd[e], c[2 * i + o][e]);
+                    }
+                }
             }
         }
     }
@@ -179,8 +191,8 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     using T = RgTraits<MODE>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* red = reinterpret_cast<float*>(ring + T::kStages * T::kStageBytes);  // [8 k groups][4 rows][256]
-    RgBarriers* sb = reinterpret_cast<RgBarriers*>(red + kRgKGroups * kRgRedRows * kGvSlabN);
+    float* red = reinterpret_cast<float*>(ring + T::kStages * T::kStageBytes);  // [kKGroups][kRedRows][256]
+    RgBarriers* sb = reinterpret_cast<RgBarriers*>(red + T::kKGroups * T::kRedRows * kGvSlabN);
     int* row_start = reinterpret_cast<int*>(sb + 1);
     int* pass_start = row_start + (a.G + 1);  // [G + 1] passes (of up to 8 rows) before the i-th expert
 
@@ -301,25 +313,26 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
 
     // ------------------------------ consumers ------------------------------
-    const int g = lane >> 2, t = lane & 3, hc = warp & 1, kg = warp >> 1;
-    const int kl = kg * 16;  // the warp's first k row in a stage
-    // the lane's places in a stage
-    const int c_first = T::kFp4 && STORED ? 128 * hc + 32 * (g >> 2) + 8 * (g & 3) : 128 * hc + 16 * g;  // first of its 16 columns
+    const int g = lane >> 2, t = lane & 3, hc = warp % (kRgWarps / T::kKGroups), kg = warp / (kRgWarps / T::kKGroups);
+    const int c_warp = hc * T::kCols, kl = kg * T::kKRows;  // the warp's first column in a slab, first k row in a stage
+    // the lane's places in a stage; its first column
+    const int c_first = c_warp + (!T::kFp4 ? 8 * g : STORED ? 32 * (g >> 2) + 8 * (g & 3) : 16 * g);
     uint32_t w_at[2];
     if constexpr (T::kFp4 && STORED) {
         // stored order: row (b * 4 + aa) * 8 + p of a 64-row block, bytes 32 q ..: four rows' codes of eight columns
         w_at[0] = (uint32_t)((kg * 8 + 4 * hc + (g >> 2)) * 128 + (g & 3) * 32 + 8 * t);
         w_at[1] = w_at[0] + 4 * 8 * 128;  // b = 1: rows 8 .. 15 of the scale group
-    } else if constexpr (T::kFp4) {
-        // 64 bytes = 128 columns of a row; the 16-byte pieces are swizzled with the row
-        w_at[0] = (uint32_t)((kl + 2 * t) * 128 + (((4 * hc + (g >> 1)) ^ (2 * t)) << 4) + (g & 1) * 8);
-        w_at[1] = (uint32_t)((kl + 2 * t + 1) * 128 + (((4 * hc + (g >> 1)) ^ (2 * t + 1)) << 4) + (g & 1) * 8);
     } else {
-        w_at[0] = (uint32_t)(hc * (T::kWBytes / 2) + (kl + 2 * t) * 128 + ((g ^ (2 * t)) << 4));
-        w_at[1] = (uint32_t)(hc * (T::kWBytes / 2) + (kl + 2 * t + 1) * 128 + ((g ^ (2 * t + 1)) << 4));
+        // 16-byte pieces of a 128-byte row (fp4: of its 256 columns; else of 128), swizzled with the row
+        const int row = kl + 2 * t, piece = T::kFp4 ? 4 * hc + (g >> 1) : 4 * (hc & 1) + (g >> 1);
+        const int box = T::kFp4 ? 0 : (hc >> 1) * (T::kWBytes / 2);
+        w_at[0] = (uint32_t)(box + row * 128 + ((piece ^ (2 * t)) << 4) + (g & 1) * 8);
+        w_at[1] = (uint32_t)(box + (row + 1) * 128 + ((piece ^ (2 * t + 1)) << 4) + (g & 1) * 8);
     }
-    const uint32_t x_at = (uint32_t)(T::kWBytes + T::kSBytes + g * 128 + 4 * t);
-    const uint32_t x0 = x_at + (((2 * kg) ^ g) << 4), x1 = x_at + (((2 * kg + 1) ^ g) << 4);
+    const uint32_t x_row = (uint32_t)(T::kWBytes + T::kSBytes + g * 128 + 4 * t);
+    uint32_t x_at[T::kKRows / 8];  // the lane's words of x row g, 8 k apart
+#pragma unroll
+    for (int i = 0; i < T::kKRows / 8; ++i) x_at[i] = x_row + (uint32_t)(((kl / 8 + i) ^ g) << 4);
     const uint32_t s_at = (uint32_t)(T::kWBytes + kg * (kGvSlabN * 2) + c_first * 2);
     const uint32_t ring_u32 = ptx::smem_u32(ring);
     const bool sums = MODE == B200MOE_CT_INT8 && a.offset != nullptr;
@@ -331,26 +344,35 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->unit_empty[n & 1]));
         if (u.rows == 0) break;
-        float c[8][4];
+        float c[T::kAcc][4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+        for (int j = 0; j < T::kAcc; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
         float xs = 0.f;
-        const bool x_on = g < u.rows, cols_on = u.n0 + 128 * hc < a.N;
+        const bool x_on = g < u.rows, cols_on = u.n0 + c_warp < a.N;
         bool ok = true;
+        // fp8: the scale of the block (128 k rows: two stages; a part starts with one) is read a block ahead
+        const float* sf_at = nullptr;
+        float sf = 1.f, sf_next = 1.f;
+        if constexpr (MODE == B200MOE_CT_FP8)
+            if (cols_on) {
+                sf_at = static_cast<const float*>(a.scale) + ((size_t)u.g * (a.K >> 7) + (u.k0 >> 7)) * (a.N >> 7) + ((u.n0 + c_warp) >> 7);
+                sf_next = __ldg(sf_at);
+            }
         for (int k = u.k0; k < u.k1; k += kRgK) {
-            float sf = 1.f;
             if constexpr (MODE == B200MOE_CT_FP8)
-                if (cols_on)
-                    sf = __ldg(static_cast<const float*>(a.scale) + ((size_t)u.g * (a.K >> 7) + (k >> 7)) * (a.N >> 7) +
-                               ((u.n0 + 128 * hc) >> 7));
+                if (cols_on && (k & kRgK) == 0) {
+                    sf = sf_next;
+                    sf_at += a.N >> 7;
+                    if (k + 2 * kRgK < u.k1) sf_next = __ldg(sf_at);
+                }
             ok = __all_sync(0xffffffffu, rg_wait(&sb->full[s], ph, sb, a.status, 40 + (int)s));
             if (!ok) break;
             const uint32_t at = ring_u32 + s * T::kStageBytes;
             if (cols_on) {
-                uint32_t b0 = 0u, b1 = 0u;
+                uint32_t b[T::kKRows / 16][2] = {};
                 if (x_on) {
-                    b0 = lds32(at + x0);
-                    b1 = lds32(at + x1);
+#pragma unroll
+                    for (int i = 0; i < T::kKRows / 8; ++i) b[i / 2][i % 2] = lds32(at + x_at[i]);
                 }
                 if constexpr (T::kFp4) {
                     uint2 q[4];
@@ -367,12 +389,15 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                         q[2] = make_uint2(r0w.y, r1w.y);
                         q[3] = make_uint2(r8w.y, r9w.y);
                     }
-                    rg_step_fp4(q, lds128(at + s_at), lds128(at + s_at + (STORED ? 128 : 16)), b0, b1, c);
+                    rg_step_fp4(q, lds128(at + s_at), lds128(at + s_at + (STORED ? 128 : 16)), b[0][0], b[0][1], c);
                 } else {
-                    rg_step_bytes<MODE>(at + w_at[0], at + w_at[1], b0, b1, sf, c);
-                    if (sums && hc == 0)
-                        xs += (__uint_as_float(b0 << 16) + __uint_as_float(b0 & 0xFFFF0000u)) +
-                              (__uint_as_float(b1 << 16) + __uint_as_float(b1 & 0xFFFF0000u));
+                    rg_step_bytes<MODE>(at + w_at[0], at + w_at[1], b, sf, c);
+                    if (sums && hc == 0) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            xs += (__uint_as_float(b[h][0] << 16) + __uint_as_float(b[h][0] & 0xFFFF0000u)) +
+                                  (__uint_as_float(b[h][1] << 16) + __uint_as_float(b[h][1] & 0xFFFF0000u));
+                    }
                 }
             }
             __syncwarp();
@@ -392,24 +417,24 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
         for (int m = 0; m < kRgRows; ++m) v[m] = xv[m] = 0.f;
 #pragma unroll
-        for (int r = 0; r < kRgRows; r += kRgRedRows) {
+        for (int r = 0; r < kRgRows; r += T::kRedRows) {
             if (r < u.rows) {
-                if (2 * t >= r && 2 * t < r + kRgRedRows) {
+                if (2 * t >= r && 2 * t < r + T::kRedRows) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < T::kAcc; ++j) {
                         const int cc = T::kFp4 && STORED ? c_first + 64 * (j >> 2) + 2 * (j & 3) : c_first + 2 * j;
 #pragma unroll
                         for (int e = 0; e < 2; ++e)  // rows 2t, 2t + 1
-                            *reinterpret_cast<float2*>(red + (kg * kRgRedRows + 2 * t - r + e) * kGvSlabN + cc) = make_float2(c[j][e], c[j][2 + e]);
+                            *reinterpret_cast<float2*>(red + (kg * T::kRedRows + 2 * t - r + e) * kGvSlabN + cc) = make_float2(c[j][e], c[j][2 + e]);
                     }
                 }
                 if (!rg_sync(sb, sync_ph, a.status)) return;
 #pragma unroll
-                for (int m = 0; m < kRgRedRows; ++m) {
+                for (int m = 0; m < T::kRedRows; ++m) {
                     if (r + m >= u.rows) break;
 #pragma unroll
-                    for (int w = 0; w < kRgKGroups; ++w) {
-                        v[r + m] += red[(w * kRgRedRows + m) * kGvSlabN + col];
+                    for (int w = 0; w < T::kKGroups; ++w) {
+                        v[r + m] += red[(w * T::kRedRows + m) * kGvSlabN + col];
                         if (sums) xv[r + m] += sb->xsum[w][r + m];
                     }
                 }
@@ -479,7 +504,7 @@ static int gv_ring_launch(const GemvArgs& a0, cudaStream_t stream) {
     if (rc != B200MOE_OK) return rc;
     rc = make_tensor_map_2d(&tx, T::kFp4 ? static_cast<const void*>(a.x16) : a.x, 2, (uint64_t)a.M, a.K, kRgRows, 64, true);
     if (rc != B200MOE_OK) return rc;
-    const size_t smem = 1024 + (size_t)T::kStages * T::kStageBytes + sizeof(float) * kRgKGroups * kRgRedRows * kGvSlabN +
+    const size_t smem = 1024 + (size_t)T::kStages * T::kStageBytes + sizeof(float) * T::kKGroups * T::kRedRows * kGvSlabN +
                         sizeof(RgBarriers) + sizeof(int) * 2 * (size_t)(a.G + 1);
     B200MOE_CUDA_TRY(cudaFuncSetAttribute(gemv_ring_kernel<MODE, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     B200MOE_CUDA_TRY(launch_dependent(gemv_ring_kernel<MODE, STORED>, 2u * (unsigned)sm_count(), kRgThreads, smem, stream, tw, ts, tx, a));

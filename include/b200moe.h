@@ -216,7 +216,7 @@ int64_t b200moe_grouped_gemm_int8_noalloc_max_rows(void);
 int b200moe_noalloc_read_status(int32_t out[2], void* stream);
 
 /* Grouped GEMV for decode-sized expert batches (any number of rows per expert is accepted;
- * it is bandwidth-optimal up to 8 rows per expert, int4 up to 4).  Dequantised weights stay fp32, x is
+ * up to 8 rows of an expert, int4 up to 4, take one pass over its weights).  Dequantised weights stay fp32, x is
  * widened to fp32, one final round to bf16.  `offset` only for int8/int4 (may be NULL).
  * fp4: a short first kernel writes x as f16 into the workspace, each row scaled by a power of two, and the
  * multiply-adds then run on the tensor core -- for the rows where that copy is exact (every element within about
