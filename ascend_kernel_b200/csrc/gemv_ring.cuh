@@ -494,8 +494,6 @@ static int gv_ring_launch(const GemvArgs& a0, cudaStream_t stream) {
     using T = RgTraits<MODE>;
     GemvArgs a = a0;
     a.ticket = a.status + 2;
-    // (K up to what the register kernel's staged x rows allow)
-    if (gv_smem_bytes(a.G, a.K, false) > 227 * 1024) return B200MOE_ERR_SHAPE;
     CUtensorMap tw, ts, tx;
     int rc = make_tensor_map_2d(&tw, a.weight, 1, (uint64_t)a.G * a.K, T::kFp4 ? a.N / 2 : a.N, kRgK, 128, !(T::kFp4 && STORED));
     if (rc != B200MOE_OK) return rc;

@@ -638,6 +638,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
     }
 }
 
+constexpr size_t kGvSmemLimit = 227 * 1024;
 static size_t gv_smem_bytes(int G, int K, bool by_rows) {
     size_t b = (sizeof(int) * (size_t)((by_rows ? 3 : 2) * G + 2) + 15) & ~size_t(15);
     b += sizeof(float) * kGvWarps * kGvRows * kGvSlabN;
@@ -653,7 +654,6 @@ static int gv_launch(const GemvArgs& a0, cudaStream_t stream) {
     // (the order must not cost the second CTA of a multiprocessor, nor a shape that fits without it)
     a.by_rows = smem <= 110 * 1024 || (smem <= 226 * 1024 && gv_smem_bytes(a.G, a.K, false) > 110 * 1024);
     if (!a.by_rows) smem = gv_smem_bytes(a.G, a.K, false);
-    if (smem > 227 * 1024) return B200MOE_ERR_SHAPE;
     // One CTA a multiprocessor: room for exactly one.  A kernel that starts beside the one before it has its CTAs put wherever
     // there is room, and where two fitted, some SMs got two and others none (stored fp4, 16 tokens x 8 over 64 experts,
     // 10240 x 1024, 115 KB: 236 us; 188 with one on each).
@@ -718,6 +718,8 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
         return B200MOE_ERR_ALIGNMENT;
     const size_t need = b200moe_grouped_gemv_workspace_bytes(M, K, N, G, compute_type, weight_layout);
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200MOE_ERR_WORKSPACE;
+    // (K up to what the fp32 kernels' staged x rows allow: one limit for every format, refused before anything is launched)
+    if (gv_smem_bytes((int)G, (int)K, false) > kGvSmemLimit) return B200MOE_ERR_SHAPE;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     GemvArgs a;

@@ -142,3 +142,13 @@ def test_one_pass_int4_scratch_where_the_rule_says():
     assert f(1024, 2048, 2048, 8, 3, 0) == 0 and f(4096, 1024, 1024, 64, 3, 0) > 0
     assert f(65536, 7168, 256, 256, 3, 0) == 0 and f(4096, 7168, 256, 256, 3, 0) > 0
     assert f(0, 7168, 4096, 256, 3, 0) == 0 and f(64, 7104, 4096, 256, 3, 0) == 0 and f(64, 7168, 4000, 256, 3, 0) == 0
+
+
+def test_gemv_refuses_a_k_range_that_does_not_fit_before_it_launches_anything():
+    """K beyond what the fp32 kernel can hold of four x rows is an invalid shape for every format; here, without a GPU, a launch
+    would give a CUDA error instead."""
+    lib = _lib().lib
+    K, N, G, M = 32768, 256, 1, 1
+    for ct in (0, 1, 2, 3):
+        need = lib.b200moe_grouped_gemv_workspace_bytes(M, K, N, G, ct, 0)
+        assert lib.b200moe_grouped_gemv(4096, 4096, 4096, None, 4096, 4096, M, K, N, G, ct, 1, 0, 4096, need, None) == 3
