@@ -25,8 +25,10 @@ constexpr int kRgThreads = (kRgWarps + 1) * 32;
 constexpr int kRgRows = 8;                        // x rows per unit: the instruction's n
 constexpr int kRgXBytes = kRgRows * kRgK * 2;     // a swizzled box of 8 rows x 64 k
 static_assert(kRgWarps * 32 == kGvSlabN, "one thread a column");
-constexpr int kRgSlotFloats = 2 * kGvSlotFloats;  // (a slot holds eight rows)
-static_assert(kRgSlotFloats >= kRgRows * kGvSlabN + kRgRows, "slot");
+// A part's slot holds four rows' sums, or eight where an expert has more than four rows: then there is room for half as many parts, and
+// there are half as many units as with passes of four rows.
+constexpr int kRgSlotFloats = 2 * kGvSlotFloats;
+static_assert(kRgSlotFloats >= kRgRows * (kGvSlabN + 1) && kGvSlotFloats >= kGvRows * (kGvSlabN + 1), "slot: sums of the columns, sums of x");
 
 template <int MODE>
 struct RgTraits {
@@ -58,7 +60,7 @@ struct RgBarriers {
     uint64_t sync;
     RgUnit unit[2];
     int abort, last;
-    int per_pass, units, parts, part_rows;
+    int per_pass, units, parts, part_rows, slot_rows;
     float xsum[4][kRgRows];
 };
 
@@ -200,9 +202,13 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const int n_slabs = (a.N + kGvSlabN - 1) / kGvSlabN;
     load_row_starts(a.group_list, a.G, a.M, a.gl_type, row_start, a.status);
     if (threadIdx.x < 32) {
-        int lo, hi, mine = 0, total;
+        int lo, hi, mine = 0, total, most = 0;
         lane_experts(a.G, lo, hi);
-        for (int i = lo; i < hi; ++i) mine += (row_start[i + 1] - row_start[i] + kRgRows - 1) / kRgRows;
+        for (int i = lo; i < hi; ++i) {
+            mine += (row_start[i + 1] - row_start[i] + kRgRows - 1) / kRgRows;
+            most = max(most, row_start[i + 1] - row_start[i]);
+        }
+        const int slot_rows = __reduce_max_sync(0xffffffffu, most) > kGvRows ? kRgRows : kGvRows;
         int at = warp_exclusive_sum(mine, total);
         for (int i = lo; i < hi; ++i) {
             pass_start[i] = at;
@@ -210,10 +216,11 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         const int parts = a.part_count == nullptr
                               ? 1
-                              : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K, a.max_parts / 2);
+                              : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K, kGvMaxParts * kGvRows / slot_rows);
         if (threadIdx.x == 0) {
             pass_start[a.G] = total;
             sb->parts = parts;
+            sb->slot_rows = slot_rows;
             sb->per_pass = n_slabs * parts;                               // units of one pass
             sb->units = (int)((unsigned)total * (unsigned)sb->per_pass);  // (as many would need 2 TB of y to not fit)
             sb->part_rows = ((a.K + kGvPartRows - 1) / kGvPartRows + parts - 1) / parts * kGvPartRows;
@@ -444,12 +451,13 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
         // ---- a slab in parts: the CTA that arrives last adds them in their order ----
         if (u.n_split > 1) {
-            float* slot = a.part_sums + (size_t)(u.slot + u.split) * kRgSlotFloats;
+            const int slot_rows = sb->slot_rows, slot_floats = slot_rows == kGvRows ? kGvSlotFloats : kRgSlotFloats;
+            float* slot = a.part_sums + (size_t)(u.slot + u.split) * slot_floats;
 #pragma unroll
             for (int m = 0; m < kRgRows; ++m)
                 if (m < u.rows) {
                     __stcg(slot + m * kGvSlabN + col, v[m]);
-                    if (sums && col == 0) __stcg(slot + kRgRows * kGvSlabN + m, xv[m]);
+                    if (sums && col == 0) __stcg(slot + slot_rows * kGvSlabN + m, xv[m]);
                 }
             __threadfence();
             if (!rg_sync(sb, sync_ph, a.status)) return;
@@ -457,14 +465,15 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (!rg_sync(sb, sync_ph, a.status)) return;
             if (!*reinterpret_cast<volatile int*>(&sb->last)) continue;
             __threadfence();
-            const float* first = a.part_sums + (size_t)u.slot * kRgSlotFloats;
+            if (threadIdx.x == 0) a.part_count[u.slot] = 0u;  // (fp4: the fp32 kernel behind this one counts there too)
+            const float* first = a.part_sums + (size_t)u.slot * slot_floats;
 #pragma unroll
             for (int m = 0; m < kRgRows; ++m)
                 if (m < u.rows) {
                     v[m] = xv[m] = 0.f;
                     for (int p = 0; p < u.n_split; ++p) {
-                        v[m] += __ldcg(first + (size_t)p * kRgSlotFloats + m * kGvSlabN + col);
-                        if (sums) xv[m] += __ldcg(first + (size_t)p * kRgSlotFloats + kRgRows * kGvSlabN + m);
+                        v[m] += __ldcg(first + (size_t)p * slot_floats + m * kGvSlabN + col);
+                        if (sums) xv[m] += __ldcg(first + (size_t)p * slot_floats + slot_rows * kGvSlabN + m);
                     }
                 }
         }

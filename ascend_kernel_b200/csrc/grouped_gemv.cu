@@ -43,13 +43,13 @@ struct GemvArgs {
     const int* xexp;
     unsigned* part_count;  // [kGvMaxParts] finished parts of a slab, zero at the launch; null: k is not split
     float* part_sums;      // [kGvMaxParts][kGvSlotFloats]
-    int max_parts;         // parts there is room for
     int* ticket;           // status word 2 (the fp32 kernel of fp4: 3, from 1 on)
     int by_rows;           // experts in the order of their row counts: shared memory has room for the order
 };
 
 // Split of the k range: parts are multiples of kGvPartRows rows, at most kGvMaxParts of them per launch (four waves of
-// two CTAs on 148 SMs; 4.9 MB of partial sums), each with the sums of 4 rows x 256 columns and of the x rows.
+// two CTAs on 148 SMs; 4.9 MB of partial sums), each with the sums of 4 rows x 256 columns and of the x rows; the tensor-core kernel
+// takes two such slots a part where its units have more than four rows.
 constexpr int kGvPartRows = 128;
 constexpr int kGvMaxParts = 1184;
 constexpr int kGvSlotFloats = kGvRows * kGvSlabN + 16;
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) grouped_gemv_kernel(const GemvA
             at += passes_of(i);
         }
         if (threadIdx.x == 0) pass_start[a.G] = total;
-        const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K, a.max_parts);
+        const int parts = a.part_count == nullptr ? 1 : gv_choose_parts((int)min((long long)total * n_slabs, 1LL << 30), gridDim.x, a.K, kGvMaxParts);
         if (threadIdx.x == 0) {
             // (kept in shared memory: a unit's loop needs every register)
             s_parts = parts;
@@ -735,7 +735,6 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
     uint8_t* ws = static_cast<uint8_t*>(workspace) + B200MOE_STATUS_BYTES;
     a.part_count = nullptr;
     a.part_sums = nullptr;
-    a.max_parts = kGvMaxParts;
     if (workspace_bytes >= gv_parts_offset(need) + kGvPartBytes) {
         uint8_t* parts = static_cast<uint8_t*>(workspace) + gv_parts_offset(need);
         a.part_count = reinterpret_cast<unsigned*>(parts);
@@ -764,13 +763,8 @@ extern "C" int b200moe_grouped_gemv(const void* x, const void* weight, const voi
         case B200MOE_CT_INT4: return gv_launch<B200MOE_CT_INT4>(a, s);
         default: {
             if (a.x16 == nullptr) return gv_launch<B200MOE_CT_FP4>(a, s);
-            a.max_parts = kGvMaxParts / 2;  // half of the room for each of the two kernels
             const int rc = a.fp4_stored ? gv_ring_launch<B200MOE_CT_FP4, true>(a, s) : gv_ring_launch<B200MOE_CT_FP4, false>(a, s);
             if (rc != B200MOE_OK) return rc;
-            if (a.part_count != nullptr) {
-                a.part_count += kGvMaxParts / 2;
-                a.part_sums += (size_t)(kGvMaxParts / 2) * kGvSlotFloats;
-            }
             return gv_launch<B200MOE_CT_FP4, 1>(a, s);
         }
     }

@@ -39,3 +39,51 @@ def test_matches_oracle(ct, K, N):
         assert st == (0, 0)
         assert (out[sum(COUNTS):].float() == SENTINEL).all()
         assert_close_to_golden(out, gold, ulps=1.0 if ct == "int8" else 2.0)
+
+
+def _call(x, w, scale, cnt, ct, y, layout=0):
+    """The C entry on a workspace of the test's own, which comes back: status words, operands, counters and sums of the parts."""
+    from ascend_kernel_b200 import _abi
+
+    (M, K), N, G = x.shape, y.shape[1], cnt.numel()
+    need = _abi.lib.b200moe_grouped_gemv_split_workspace_bytes(M, K, N, G, _abi.CT[ct], layout)
+    ws = torch.full((need,), 0xFF, dtype=torch.uint8, device="cuda")
+    ws[:256] = 0
+    rc = _abi.lib.b200moe_grouped_gemv(x.data_ptr(), w.data_ptr(), scale.data_ptr(), None, cnt.data_ptr(), y.data_ptr(), M, K, N, G,
+                                       _abi.CT[ct], 1, layout, ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0
+    return ws
+
+
+@pytest.mark.parametrize("ct,G,N,rows", [
+    ("int8", 20, 4096, 1),   # 320 units in two parts of 1024 k: 640 slots of four rows
+    ("fp8", 20, 4096, 4),
+    ("fp4", 20, 2048, 1),    # 160 units in three parts
+    ("int8", 20, 2048, 8),   # slots of eight rows
+    ("fp4", 20, 1024, 7),
+])
+def test_parts_of_the_k_range(ct, G, N, rows):
+    """Calls of one or two waves are cut along k as far as there is room for the parts' sums: the sums were written, and what comes
+    out is what the oracle gives.  fp4 has rows in every third place that the fp32 kernel does, in parts too."""
+    import ascend_kernel_b200 as ak
+
+    K, counts = 2048, [rows] * G
+    if ct == "int8":
+        x, w, scale, _, cnt = _int8_case(counts, K, N, 3, False)
+    elif ct == "fp8":
+        gen = torch.Generator().manual_seed(4)
+        x, cnt = torch.randn(rows * G, K, generator=gen).to(torch.bfloat16), torch.tensor(counts)
+        w = torch.randint(0, 256, (G, K, N), generator=gen, dtype=torch.uint8)
+        scale = torch.randn(G, K // 128, N // 128, generator=gen)
+    else:
+        x, w, scale, cnt = _fp4_case(counts, K, N, 5)
+        x[::3, 5] = 2.0 ** -100
+    gold = O.golden_f32(x, w, scale, None, cnt, ct, O.GROUP_LIST_COUNTS, weight_layout="canonical", gemv=True)
+    x, w, scale, cnt = (t.cuda() for t in (x, w, scale, cnt))
+    y = torch.full((rows * G, N), SENTINEL, dtype=torch.bfloat16, device="cuda")
+    ws = _call(x, w, scale, cnt, ct, y)
+    assert ak.read_status(ws) == (0, 0)
+    assert_close_to_golden(y, gold, ulps=1.0 if ct == "int8" else 2.0)
+    slots = ws[ws.numel() - 1184 * 1040 * 4:]  # behind the counters
+    assert (slots != 0xFF).any(), "the k range was not cut"
