@@ -64,9 +64,9 @@ constexpr int kATileBytes = 2 * kAHalfBytes;  // an x stage holds both row halve
 constexpr int kSmallRows = 32;                 // rows of the small x box (a nearly empty last row half)
 constexpr int kSmallBytes = kSmallRows * kBK * 2;
 // A last row half of at most this many rows is multiplied with M = 64, and its x comes in boxes of 32 rows: no less time on the tensor
-// core, but half of its shared-memory reads of x, and fewer x bytes from L2.  us with M = 128 | this: int8 / fp8 / int4 / fp4, 65536 rows by
-// popularity over 256 experts (two thirds of them with at most 64), 7168 x 4096: 5174 | 5018, 5908 | 5550, 5586 | 5390, fp4 with 32 rows on
-// every expert, 2048 x 7168: 1215 | 1100, fp4-stored layer of 4096 tokens x 8: 4810 | 4620 (scaled to one GPU by the start's times).
+// core, but half of its shared-memory reads of x, fewer x bytes from L2, and less power.  us in a steady loop, M = 128 | M = 64: 65536 rows by
+// popularity over 256 experts (two thirds of them with at most 64), 7168 x 4096: int8 4773 | 4604, fp8 5428 | 5222; stored fp4, 1021 tokens x 8
+// over 256 experts, 2048 x 7168: 1143 | 1069; fp4-stored layer of 4096 tokens x 8: 4575 | 4378.
 constexpr int kHalfM = 64;
 constexpr int kBTileBytes = kBK * kBN * 2;
 constexpr uint32_t kTmemCols = 512;
@@ -107,8 +107,8 @@ struct GmTraits {
     // into the B ring (a 64 k x 128-byte box with the 128-byte swizzle is exactly one block of the
     // MN-major operand layout) and the dequant warps have nothing to do
     static constexpr bool kDirect = (MODE == B200MOE_CT_BF16);
-    // last row halves of at most this many rows are multiplied with M = 64 (not bf16, whose B tiles never pass the warps: 128 experts of
-    // 30 rows, 256 x 256, 12.3 us without, 12.75 with)
+    // last row halves of at most this many rows are multiplied with M = 64 (not bf16, whose B tiles never pass the warps; it is free of
+    // what the M = 64 forms cost: with it, 40 bytes of spills and 5 % at every size)
     static constexpr int kShortRows = kDirect ? 0 : kHalfM;
     // a dequant thread converts 8 rows x 8 columns of a stage (one 16-byte chunk of each of its rows) instead of
     // 4 rows x 16 columns: stored-order fp4 comes that way, int4 then holds and unpacks the scales and offsets of 8
@@ -879,6 +879,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                 const int last_rows = ti.rows - (ti.halves - 1) * kBM;
                 const int n_small = last_rows <= max(T::kShortRows, kSmallRows) ? (last_rows + kSmallRows - 1) / kSmallRows : 0;
                 const uint32_t stage_bytes = (uint32_t)((ti.halves - 1) * kAHalfBytes + (n_small ? n_small * kSmallBytes : kAHalfBytes));
+                const CUtensorMap* last_map = n_small ? &tmap_xs : &tmap_x;
                 for (int kt = 0; kt < n_kt; ++kt, ++ia) {
                     const uint32_t s = ia % NS, ph = (ia / NS) & 1;
                     if (ia >= NS && !gm_wait(&sb->empty[s], ph ^ 1, sb, a.status, 10 + (int)s)) { ok = false; break; }
@@ -898,8 +899,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                         dst += kAHalfBytes;
                         row += kBM;
                     }
-                    if (n_small == 0) ptx::tma_load_2d(dst, &tmap_x, bar, kx, row);
-                    for (int b = 0; b < n_small; ++b) ptx::tma_load_2d(dst + b * kSmallBytes, &tmap_xs, bar, kx, row + b * kSmallRows);
+                    // (no loop over the boxes: 32 experts, 264 tokens x 4, 4096 x 1024: int8 91.3 -> 80.2 us, stored fp4 51.7 -> 47.1)
+                    ptx::tma_load_2d(dst, last_map, bar, kx, row);
+                    if (T::kShortRows > kSmallRows && n_small == 2) ptx::tma_load_2d(dst + kSmallBytes, &tmap_xs, bar, kx, row + kSmallRows);
                     if (far.valid) far_step();
                 }
             }
@@ -938,7 +940,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             if (!__all_sync(0xffffffffu, ok)) break;
             const uint32_t acc0 = tmem_base + (use0 ? 0u : (uint32_t)kBN);
             // M = 64 instead of 128 in the last row half: what is taken off the instruction descriptors
-            const uint32_t less = ti.rows - (ti.halves - 1) * kBM <= T::kShortRows ? (uint32_t)((kBM - kHalfM) >> 4) << 24 : 0u;
+            const uint32_t less = T::kShortRows > 0 && ti.rows - (ti.halves - 1) * kBM <= T::kShortRows ? (uint32_t)((kBM - kHalfM) >> 4) << 24 : 0u;
             ptx::tc_fence_after();
             uint32_t accumulate = 0;
             for (int kt = 0; kt < n_kt; ++kt) {
@@ -1026,9 +1028,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             ptx::tc_fence_after();
             {
                 // (M = 64 leaves row i in TMEM lane 32 * (i / 16) + i % 16)
-                const bool half_m = ti.rows - half * kBM <= T::kShortRows;
-                const int row = ti.row0 + half * kBM + (half_m ? quarter * 16 + (lane & 15) : quarter * 32 + lane);
-                const bool row_ok = row < ti.row0 + ti.rows && !(half_m && lane >= 16);
+                const bool half_m = T::kShortRows > 0 && ti.rows - half * kBM <= T::kShortRows;
+                int row;
+                bool row_ok;
+                if constexpr (T::kNibbles) {
+                    // one number for both (0 .. 18 bytes of spills; with two, as below, 44 .. 80, and stored fp4 lost 5 to 10 % on short calls)
+                    int at = half * kBM + quarter * 32 + lane;
+                    if (half_m) at = half * kBM + ((lane & 16) << 4) + quarter * 16 + (lane & 15);  // (lanes from 16 on: past any tile's rows)
+                    row = ti.row0 + at;
+                    row_ok = at < ti.rows;
+                } else {
+                    row = ti.row0 + half * kBM + (half_m ? quarter * 16 + (lane & 15) : quarter * 32 + lane);
+                    row_ok = row < ti.row0 + ti.rows && !(half_m && lane >= 16);
+                }
                 float unit = 1.f;  // (a row that is not exact in f16 comes out as zeros here)
                 if constexpr (MODE == kCtInt4F16) unit = row_ok ? int4_row_unit(__ldca(a.row_exp + row)) : 0.f;
                 const float rs = (has_offset && row_ok) ? __ldca(a.rowsum + row) : 0.f;
