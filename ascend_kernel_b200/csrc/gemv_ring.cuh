@@ -278,7 +278,6 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     u.slot = parts > 1 ? ((pass_start[lo] + (int)pass) * n_slabs + slab) * parts : 0;
                     u.k0 = split * sb->part_rows;
                     u.k1 = min(u.k0 + sb->part_rows, a.K);
-                    held = (unsigned)atomicAdd(a.ticket, 1);
                     if constexpr (T::kFp4) {
                         // the fp32 kernel does every four rows (from the expert's first on) of which one is not exact in f16
                         bool all_again = true;
@@ -287,7 +286,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                             for (int m = q; m < min(q + kGvRows, u.rows); ++m) bad = bad || __ldca(a.xexp + u.r0 + m) == kGvNotF16;
                             all_again = bad;
                         }
-                        if (all_again) continue;
+                        if (all_again) {
+                            held = (unsigned)atomicAdd(a.ticket, 1);
+                            continue;
+                        }
                     }
                 }
                 if (n >= 2 && !rg_wait(&sb->unit_empty[n & 1], ((n >> 1) & 1) ^ 1, sb, a.status, 70)) break;
@@ -297,6 +299,12 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 if (!live) break;
                 const bool upper = T::kFp4 || u.n0 + 128 < a.N;  // (fp8: the last slab may hold 128 columns)
                 for (int k = u.k0; k < u.k1; k += kRgK, ++it) {
+                    // The next ticket is drawn when the ring has been filled twice (or with the last stage).  Drawn with the first stage, a CTA
+                    // that starts a few us late -- behind the one CTA a row that prepares fp4's x -- found the units of a single wave taken by
+                    // others as their second; drawn with the last, two even waves became three on some CTAs.  First stage | twice the ring | last
+                    // stage, us: stored fp4, 16 experts of 2 rows, 7168 x 2048, 256 units: 85.9 | 54.9 | 55.0; fp8, 5 tokens x 8, 7168 x 4096, 592 units:
+                    // 226 | 226 | 267.
+                    if (k == min(u.k0 + 2 * T::kStages * kRgK, (u.k1 - 1) / kRgK * kRgK)) held = (unsigned)atomicAdd(a.ticket, 1);
                     const uint32_t s = it % T::kStages, ph = (it / T::kStages) & 1;
                     if (it >= T::kStages && !rg_wait(&sb->empty[s], ph ^ 1, sb, a.status, 10 + (int)s)) { ok = false; break; }
                     const uint32_t bar = ptx::smem_u32(&sb->full[s]), at = ptx::smem_u32(ring + s * T::kStageBytes);
