@@ -23,6 +23,7 @@ constexpr int kRgK = 64;                          // k rows of a stage
 constexpr int kRgWarps = 8;                       // consumers
 constexpr int kRgThreads = (kRgWarps + 1) * 32;
 constexpr int kRgRows = 8;                        // x rows per unit: the instruction's n
+constexpr int kRgRun = 8;                         // int8: stages in one partial sum
 constexpr int kRgXBytes = kRgRows * kRgK * 2;     // a swizzled box of 8 rows x 64 k
 static_assert(kRgWarps * 32 == kGvSlabN, "one thread a column");
 // A part's slot holds four rows' sums, or eight where an expert has more than four rows: then there is room for half as many parts, and
@@ -113,7 +114,7 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
 // Lane (g, t) = (lane / 4, lane % 4) holds, of every 16 k rows, {2t, 2t + 1, 2t + 8, 2t + 9} (the instruction's own k indices)
 // of its columns, and of x row g; c[j]: columns 2j, 2j + 1 of the lane's x two x rows.
 // Byte formats: a warp's 32 k rows x 64 columns of a stage; `w0`, `w1`: shared addresses of the lane's eight columns in rows 2t, 2t + 1
-// (rows 8 apart are 1024 bytes apart and share their swizzle), b[h]: x of rows 16h ...  int8 goes on in c, fp8 starts from zero.
+// (rows 8 apart are 1024 bytes apart and share their swizzle), b[h]: x of rows 16h ...
 template <int MODE>
 __device__ __forceinline__ void rg_step_bytes(uint32_t w0, uint32_t w1, const uint32_t (&b)[2][2], float sf, float (&c)[4][4]) {
     float d[4][4];
@@ -130,7 +131,6 @@ __device__ __forceinline__ void rg_step_bytes(uint32_t w0, uint32_t w1, const ui
                     const uint32_t sel = o == 0 ? 0x5410u : 0x7632u;
                     s8x4_to_bf16_even_odd(prmt(r0w[i], r1w[i], sel), a0, a1);  // rows (2t, 2t+1) at the two columns
                     s8x4_to_bf16_even_odd(prmt(r2w[i], r3w[i], sel), a2, a3);  // rows (2t+8, 2t+9)
-                    mma_16816(c[2 * i + o], a0, a1, a2, a3, b[h][0], b[h][1]);
                 } else {
                     // byte b of both rows into the high bytes of the two lanes (the low bytes are masked off)
                     const uint32_t s0 = o == 0 ? 0x4000u : 0x6020u, s1 = o == 0 ? 0x5010u : 0x7030u;
@@ -138,14 +138,14 @@ __device__ __forceinline__ void rg_step_bytes(uint32_t w0, uint32_t w1, const ui
                     a1 = e4m3x2_hi_to_bf16(prmt(r0w[i], r1w[i], s1));
                     a2 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s0));
                     a3 = e4m3x2_hi_to_bf16(prmt(r2w[i], r3w[i], s1));
-                    float (&dd)[4] = d[2 * i + o];
-                    if (h == 0) dd[0] = dd[1] = dd[2] = dd[3] = 0.f;
-                    mma_16816(dd, a0, a1, a2, a3, b[h][0], b[h][1]);
-                    // the 128 x 128 block's fp32 scale multiplies the step's sums
-                    if (h == 1) {
+                }
+                float (&dd)[4] = d[2 * i + o];
+                if (h == 0) dd[0] = dd[1] = dd[2] = dd[3] = 0.f;
+                mma_16816(dd, a0, a1, a2, a3, b[h][0], b[h][1]);
+                if (h == 1) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) c[2 * i + o][e] = fmaf(sf, dd[e], c[2 * i + o][e]);
-                    }
+                    for (int e = 0; e < 4; ++e)  // fp8: the 128 x 128 block's fp32 scale multiplies the step's sums
+                        c[2 * i + o][e] = MODE == B200MOE_CT_INT8 ? c[2 * i + o][e] + dd[e] : fmaf(sf, dd[e], c[2 * i + o][e]);
                 }
             }
         }
@@ -362,6 +362,15 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         float c[T::kAcc][4];
 #pragma unroll
         for (int j = 0; j < T::kAcc; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+        // int8: a step's sums are added in fp32 to `run`, and kRgRun steps' to `c`.  The instruction's own additions drop bits: chained over the whole
+        // of k they showed two to five times the error of the fp32 multiply-adds that one-row units had before the ring (sums that
+        // cancel, 32 experts, 7168 x 4096: 1.1e-7 then, 5.6e-7 chained, 1.1e-7 so; with several rows 2.3e-7 before, 1.0e-7 now), and one
+        // level of additions twice.  (32 tokens x 8 over 256 experts, 7168 x 4096: 710 -> 732 us.)
+        float run[MODE == B200MOE_CT_INT8 ? T::kAcc : 1][4];
+        if constexpr (MODE == B200MOE_CT_INT8) {
+#pragma unroll
+            for (int j = 0; j < T::kAcc; ++j) run[j][0] = run[j][1] = run[j][2] = run[j][3] = 0.f;
+        }
         float xs = 0.f;
         const bool x_on = g < u.rows, cols_on = u.n0 + c_warp < a.N;
         bool ok = true;
@@ -373,51 +382,68 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 sf_at = static_cast<const float*>(a.scale) + ((size_t)u.g * (a.K >> 7) + (u.k0 >> 7)) * (a.N >> 7) + ((u.n0 + c_warp) >> 7);
                 sf_next = __ldg(sf_at);
             }
-        for (int k = u.k0; k < u.k1; k += kRgK) {
-            if constexpr (MODE == B200MOE_CT_FP8)
-                if (cols_on && (k & kRgK) == 0) {
-                    sf = sf_next;
-                    sf_at += a.N >> 7;
-                    if (k + 2 * kRgK < u.k1) sf_next = __ldg(sf_at);
-                }
-            ok = __all_sync(0xffffffffu, rg_wait(&sb->full[s], ph, sb, a.status, 40 + (int)s));
-            if (!ok) break;
-            const uint32_t at = ring_u32 + s * T::kStageBytes;
-            if (cols_on) {
-                uint32_t b[T::kKRows / 16][2] = {};
-                if (x_on) {
+        for (int k = u.k0; k < u.k1;) {
+            const int k_end = MODE == B200MOE_CT_INT8 ? min(k + kRgRun * kRgK, u.k1) : u.k1;
+            for (; k < k_end; k += kRgK) {
+                if constexpr (MODE == B200MOE_CT_FP8)
+                    if (cols_on && (k & kRgK) == 0) {
+                        sf = sf_next;
+                        sf_at += a.N >> 7;
+                        if (k + 2 * kRgK < u.k1) sf_next = __ldg(sf_at);
+                    }
+                ok = __all_sync(0xffffffffu, rg_wait(&sb->full[s], ph, sb, a.status, 40 + (int)s));
+                if (!ok) break;
+                const uint32_t at = ring_u32 + s * T::kStageBytes;
+                if (cols_on) {
+                    uint32_t b[T::kKRows / 16][2] = {};
+                    if (x_on) {
 #pragma unroll
-                    for (int i = 0; i < T::kKRows / 8; ++i) b[i / 2][i % 2] = lds32(at + x_at[i]);
-                }
-                if constexpr (T::kFp4) {
-                    uint2 q[4];
-                    if constexpr (STORED) {
+                        for (int i = 0; i < T::kKRows / 8; ++i) b[i / 2][i % 2] = lds32(at + x_at[i]);
+                    }
+                    if constexpr (T::kFp4) {
+                        uint2 q[4];
+                        if constexpr (STORED) {
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
+                            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                            for (int b = 0; b < 2; ++b) q[2 * i + b] = lds64(at + w_at[b] + i * 256);
+                                for (int b = 0; b < 2; ++b) q[2 * i + b] = lds64(at + w_at[b] + i * 256);
+                        } else {
+                            const uint2 r0w = lds64(at + w_at[0]), r1w = lds64(at + w_at[1]);
+                            const uint2 r8w = lds64(at + w_at[0] + 1024), r9w = lds64(at + w_at[1] + 1024);
+                            q[0] = make_uint2(r0w.x, r1w.x);
+                            q[1] = make_uint2(r8w.x, r9w.x);
+                            q[2] = make_uint2(r0w.y, r1w.y);
+                            q[3] = make_uint2(r8w.y, r9w.y);
+                        }
+                        rg_step_fp4(q, lds128(at + s_at), lds128(at + s_at + (STORED ? 128 : 16)), b[0][0], b[0][1], c);
                     } else {
-                        const uint2 r0w = lds64(at + w_at[0]), r1w = lds64(at + w_at[1]);
-                        const uint2 r8w = lds64(at + w_at[0] + 1024), r9w = lds64(at + w_at[1] + 1024);
-                        q[0] = make_uint2(r0w.x, r1w.x);
-                        q[1] = make_uint2(r8w.x, r9w.x);
-                        q[2] = make_uint2(r0w.y, r1w.y);
-                        q[3] = make_uint2(r8w.y, r9w.y);
-                    }
-                    rg_step_fp4(q, lds128(at + s_at), lds128(at + s_at + (STORED ? 128 : 16)), b[0][0], b[0][1], c);
-                } else {
-                    rg_step_bytes<MODE>(at + w_at[0], at + w_at[1], b, sf, c);
-                    if (sums && hc == 0) {
+                        if constexpr (MODE == B200MOE_CT_INT8) {
+                            rg_step_bytes<MODE>(at + w_at[0], at + w_at[1], b, sf, run);
+                        } else {
+                            rg_step_bytes<MODE>(at + w_at[0], at + w_at[1], b, sf, c);
+                        }
+                        if (sums && hc == 0) {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            xs += (__uint_as_float(b[h][0] << 16) + __uint_as_float(b[h][0] & 0xFFFF0000u)) +
-                                  (__uint_as_float(b[h][1] << 16) + __uint_as_float(b[h][1] & 0xFFFF0000u));
+                            for (int h = 0; h < 2; ++h)
+                                xs += (__uint_as_float(b[h][0] << 16) + __uint_as_float(b[h][0] & 0xFFFF0000u)) +
+                                      (__uint_as_float(b[h][1] << 16) + __uint_as_float(b[h][1] & 0xFFFF0000u));
+                        }
                     }
                 }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->empty[s]));
+                if (++s == T::kStages) { s = 0; ph ^= 1u; }
             }
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sb->empty[s]));
-            if (++s == T::kStages) { s = 0; ph ^= 1u; }
+            if (!ok) break;
+            if constexpr (MODE == B200MOE_CT_INT8) {
+#pragma unroll
+                for (int j = 0; j < T::kAcc; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        c[j][e] += run[j][e];
+                        run[j][e] = 0.f;
+                    }
+            }
         }
         if (!ok) break;
 

@@ -87,3 +87,19 @@ def test_parts_of_the_k_range(ct, G, N, rows):
     assert_close_to_golden(y, gold, ulps=1.0 if ct == "int8" else 2.0)
     slots = ws[ws.numel() - 1184 * 1040 * 4:]  # behind the counters
     assert (slots != 0xFF).any(), "the k range was not cut"
+
+
+def test_one_row_int8_is_as_close_as_fp32_multiply_adds():
+    """Every product has its negative at another place of k, so the exact sum is zero and what comes out is the rounding of the
+    partial sums alone: fp32 additions in a row and in two levels leave about 1e-7 of half the sum, chained tensor instructions twice that."""
+    gen = torch.Generator().manual_seed(6)
+    G, K, N = 8, 7168, 4096
+    half = torch.randn(G, K // 2, generator=gen).to(torch.bfloat16)
+    w = torch.randint(-128, 128, (G, K // 2, N), generator=gen, dtype=torch.int8)
+    at = torch.randperm(K // 2, generator=gen)
+    x = torch.cat([half, -half[:, at]], 1).cuda()
+    scale = torch.ones(G, N, dtype=torch.bfloat16).cuda()
+    y = torch.empty(G, N, dtype=torch.bfloat16, device="cuda")
+    _call(x, torch.cat([w, w[:, at]], 1).cuda(), scale, torch.ones(G, dtype=torch.int64).cuda(), "int8", y)
+    part = torch.einsum("gk,gkn->gn", half.cuda().double(), w.cuda().double())
+    assert float(y.double().square().mean().sqrt() / part.square().mean().sqrt()) < 1.35e-7
