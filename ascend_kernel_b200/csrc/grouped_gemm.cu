@@ -1331,13 +1331,16 @@ constexpr int kInt8RolesK = 2048;
 
 // Whether a call of int4 without offsets goes through f16 in one pass: where the tiles of a multiprocessor come to at least 48 stages of 64 k, the
 // preparation of x and the two launches more (6 .. 10 us, and the bytes of x twice) are won back; where whole experts are long and N is a
-// single column tile, they are not.  us, hi and lo | one pass, back to back, experts : rows : K x N (even lists unless said): 8 : 1024 : 2048 x 2048
+// single column tile, they are not, nor where short ones make a single wave, which waits for its stages'
+// round trips and not for MMAs.  us, hi and lo | one pass, back to back, experts : rows : K x N (even lists unless said): 128 : 8192 : 2048 x 256 50.9 |
+// 69.8; 32 : 1056 : 4096 x 1024 87.0 | 102.3; 16 : 528 : 7168 x 2048 142.1 | 167.6; 20 : 800 : 4096 x 2048 158.8 | 92.0; 8 : 1024 : 2048 x 2048
 // (32 stages) 49.5 | 59.7; 32 : 1024 : 2048 x 1024 (32) 47.5 | 56.5; 16 : 4096 : 256 x 4096 (16) 45.4 | 44.4; 16 : 1024 : 256 x 1024 (4) 16.6 | 23.1;
 // 64 : 4096 by popularity : 1024 x 1024 (48) 64.3 | 52.8; 32 : 256 : 7168 x 2048 (224) 264 | 184; 256 : 1024 : 2048 x 2048 (448) 554 | 345; 64 : 8192 by
 // popularity : 7168 x 1024 409.6 | 330.9; 256 : 8192 : 2048 x 7168 1992 | 1226; 256 : 65536 by popularity : 7168 x 4096 8840 | 5586.
 static bool int4_one_pass(int64_t M, int64_t K, int64_t N, int64_t G) {
     const int64_t tiles = N / kBN * (M / kTileM + (M < G ? M : G)), sms = sm_count();  // (all experts have rows)
-    return (tiles + sms - 1) / sms * (K / kBK) >= 48 && (N >= 2 * kBN || M <= 64 * G);
+    const bool long_experts = M > 64 * G;
+    return (tiles + sms - 1) / sms * (K / kBK) >= 48 && (long_experts ? N >= 2 * kBN : N / kBN * (M < G ? M : G) > sms);
 }
 
 static size_t gm_smem_bytes(int G) {

@@ -134,13 +134,14 @@ def test_gemv_split_workspace_comes_on_top_of_the_plain_one():
 
 def test_one_pass_int4_scratch_where_the_rule_says():
     """Scratch of the int4 GEMM: none for other formats, with offsets, for few stages a multiprocessor, for one column tile under long
-    experts."""
+    experts, for a single wave of short ones."""
     f = _lib().lib.b200moe_grouped_gemm_scratch_bytes
     big = (65536, 7168, 4096, 256)
     assert f(*big, 3, 0) > 2 * 65536 * 7168 and f(*big, 3, 1) == 0
     assert all(f(*big, ct, 0) == 0 for ct in (0, 1, 2, 4))
     assert f(1024, 2048, 2048, 8, 3, 0) == 0 and f(4096, 1024, 1024, 64, 3, 0) > 0
     assert f(65536, 7168, 256, 256, 3, 0) == 0 and f(4096, 7168, 256, 256, 3, 0) > 0
+    assert f(1056, 4096, 1024, 32, 3, 0) == 0 and f(8192, 2048, 256, 128, 3, 0) == 0  # a single wave of short tiles
     assert f(0, 7168, 4096, 256, 3, 0) == 0 and f(64, 7104, 4096, 256, 3, 0) == 0 and f(64, 7168, 4000, 256, 3, 0) == 0
 
 
