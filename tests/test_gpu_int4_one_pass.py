@@ -145,3 +145,47 @@ def test_offsets_that_cancel_the_codes(positive):
         err += float((y[g * rows:(g + 1) * rows].double() - want).square().sum())
         ref += float(want.square().sum())
     assert (err / ref) ** 0.5 < 2.0 ** -9 + 1e-4
+
+
+def _control_words(x, w, s, cnt, y):
+    """One call on scratch of the test's own: tiles listed for the two-pass kernel, and rows of x that f16 does not hold."""
+    from ascend_kernel_b200 import _abi
+
+    (M, K), N, G, ct = x.shape, y.shape[1], cnt.numel(), _abi.CT["int4"]
+    need = _abi.lib.b200moe_grouped_gemm_workspace_bytes(M, K, N, G, ct, 0)
+    scratch = torch.zeros(_abi.lib.b200moe_grouped_gemm_scratch_bytes(M, K, N, G, ct, 0), dtype=torch.uint8, device="cuda")
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    rc = _abi.lib.b200moe_grouped_gemm_scratch(x.data_ptr(), w.data_ptr(), s.data_ptr(), None, cnt.data_ptr(), y.data_ptr(), M, K, N, G, ct, 1, 0,
+                                               ws.data_ptr(), need, scratch.data_ptr(), scratch.numel(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0
+    words = scratch[:12].view(torch.int32).tolist()
+    return words[0], words[2]
+
+
+def test_the_one_pass_kernel_runs_and_lists_what_it_leaves():
+    """No tile is listed for clean input, and exactly the tiles of an inexact row or an outsized scale otherwise; both bindings give the
+    one-pass result, which is not the two-pass one bit for bit."""
+    import ascend_kernel_b200 as ak
+    from ascend_kernel_b200 import _abi, cinfer_ascendc
+
+    K, N, counts = 2048, 4096, [1300, 0, 257, 1100]
+    x, w, s, cnt = (t.cuda() for t in _case(counts, K, N, False, 6) if t is not None)
+    y = torch.zeros(x.shape[0], N, dtype=torch.bfloat16, device="cuda")
+    assert _control_words(x, w, s, cnt, y) == (0, 0)
+    rows = sum(counts)
+    two, need = torch.zeros_like(y), _abi.lib.b200moe_grouped_gemm_workspace_bytes(x.shape[0], K, N, 4, _abi.CT["int4"], 0)
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    assert _abi.lib.b200moe_grouped_gemm(x.data_ptr(), w.data_ptr(), s.data_ptr(), None, cnt.data_ptr(), two.data_ptr(), x.shape[0], K, N, 4,
+                                         _abi.CT["int4"], 1, 0, ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert not torch.equal(y[:rows].view(torch.int16), two[:rows].view(torch.int16))
+    for call in (lambda o: ak.grouped_gemm(x, w, s, None, cnt, "int4", o, group_list_type=1),
+                 lambda o: cinfer_ascendc.grouped_gemm(x, w, s, torch.empty(0, dtype=torch.bfloat16, device="cuda"), cnt, "int4", o, group_list_type=1)):
+        out = torch.zeros_like(y)
+        call(out)
+        torch.cuda.synchronize()
+        assert torch.equal(out[:rows].view(torch.int16), y[:rows].view(torch.int16))
+    x[300, 5] = 2.0 ** -60  # rows 256 .. 511 of expert 0: 16 tiles
+    s[2, 3, 300] = 2.0 ** -30  # expert 2, columns 256 .. 511: two tiles of rows
+    assert _control_words(x, w, s, cnt, y) == (18, 1)
