@@ -484,7 +484,7 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, ui
 __device__ __forceinline__ uint32_t dq_row_addr(uint32_t sa, int j) { return (sa ^ (uint32_t)(j << 5)) + (uint32_t)(j * 256); }
 
 // Stored-order fp4 and fp4 with e8m0 scales enter the tile in the column order (0,4,1,5,2,6,3,7) of every eight, the order
-// in which the decode produces them (e2m1x8_to_bf16_pairs); the epilogue undoes it when it picks accumulator
+// in which the decode produces them (e2m1x8_to_bf16_tiny); the epilogue undoes it when it picks accumulator
 // registers.  Restoring the order here cost four permutes per eight codes (with resolved tiles, fp4-stored layer of 256
 // experts, 4096 tokens x 8, 7168 x 2048: 4.79 -> 4.61 ms).  The scales of eight columns are
 // brought into the same order, once for all rows of the scale group (the canonical order's 16 columns a thread

@@ -626,13 +626,6 @@ struct Gemv {
     static_assert(kStages <= Decode::kStages && kBytes <= Prefill::kBytes, "barriers, shared memory");
 };
 
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 template <bool GATE_UP>
 __device__ __forceinline__ void gemv_body(const CUtensorMap& tmap_xs, const uint8_t* __restrict__ weight, const GemmArgs& a, uint8_t* base,
                                           const int* row_start, int* tile_prefix, __nv_bfloat16* const* s_dst_base) {

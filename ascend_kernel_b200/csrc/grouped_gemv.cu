@@ -293,14 +293,6 @@ __device__ __forceinline__ uint32_t e4m3x2_hi_to_bf16(uint32_t t) {
     return mul_bf16x2(((t >> 4) & 0x07F007F0u) | (t & 0x80008000u), 0x7B807B80u);
 }
 
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                          uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // ---- fp4 weights in the reference's stored (pre-shuffled) order, read in place -----------------
 // Canonical row 16a + 8b + c8 of 64-row block R, byte column 128j + 16p + 4q + s lives at
 //   ((((((2R + b) * 4 + a) * 8 + p) * J + j) * 4 + q) * 8 + c8) * 4 + s,        J = N / 256,
