@@ -489,9 +489,10 @@ __global__ void __launch_bounds__(256) gv_begin_kernel(int* __restrict__ status,
 
 // Parts a slab's k range is cut into, for `slabs` (rows x slab) units on `ctas` CTAs; called by a whole warp, lane i
 // weighs i + 1 parts: waves of CTAs times the blocks of kGvPartRows rows of a part plus kGvPartCost, what a unit costs
-// beyond its weights (x staging, first loads, the sums' way through L2) in blocks.  A launch of many waves has nothing
-// to gain and stays whole.  One token on 8 of 256 experts, 7168 x 4096 fp8 (128 slabs, two parts): 117 -> 72 us = 3.3
-// TB/s; 3 tokens x 4 over 160 experts, 4224 x 3328 int8: 54.6 -> 53.3 us.
+// beyond its weights (first loads, the sums' way through L2; in grouped_gemv_kernel the staging of x too) in blocks.  A launch of many
+// waves has nothing to gain and stays whole.  Whole | in parts, us, register kernel: one token on 8 of 256 experts, 7168 x 4096 fp8 (128
+// slabs, two parts): 117 | 72; 3 tokens x 4 over 160 experts, 4224 x 3328 int8: 54.6 | 53.3.  In the ring kernel costs of 1, 2 and 4 give the
+// same times (32, 128, 160, 336 and 368 slabs, three formats: within 1 %, fp4 at 32 slabs 5 %): the count of waves decides.
 constexpr int kGvPartCost = 2;
 __device__ __forceinline__ int gv_choose_parts(int slabs, int ctas, int K, int max_parts) {
     const int blocks = (K + kGvPartRows - 1) / kGvPartRows;
